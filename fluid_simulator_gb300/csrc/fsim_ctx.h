@@ -39,7 +39,8 @@ struct MGLevelBufs {
     int nx = 0, ny = 0, nz = 0, pz = 0;
     long long ncell = 0;          // nx * ny * pz
     uint8_t* kind = nullptr;      // 0 fluid, 1 air, 2 solid (levels >= 1)
-    uint16_t* code = nullptr;     // same encoding as SolverBufs::code
+    uint16_t* code = nullptr;     // level 0: SolverBufs::code
+    uint32_t* ccode = nullptr;    // levels >= 1: face quarters, Dirichlet eighths, interpolation scale
     float* x = nullptr;           // correction (levels >= 1)
     float* f = nullptr;           // right-hand side (levels >= 1)
     float* r = nullptr;           // residual

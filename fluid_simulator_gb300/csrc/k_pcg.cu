@@ -74,9 +74,6 @@ constexpr float SAFE = 0.25f;
 
 // code bits
 constexpr uint16_t CODE_FLUID = 0x8000;
-// shared-memory copies of the codes (coarsest multigrid levels) also carry the
-// cell's colour, (x + y + z) & 1, so that a half sweep needs no coordinates
-constexpr uint16_t SCODE_ODD = 0x4000;
 __device__ __forceinline__ int code_ns(uint16_t c) { return (c >> 8) & 7; }
 __device__ __forceinline__ int code_nf(uint16_t c) { return __popc(c & 0x3F); }
 
@@ -520,55 +517,50 @@ __global__ void __launch_bounds__(PCG_THREADS) k_update(const PcgArgs a, Vecs<T>
 //
 // z = M^-1 r by one V-cycle.  Level l + 1 halves every dimension (ceil); a
 // coarse cell is fluid if any child is fluid, else air if any child is air,
-// else solid.  Each level's operator is the same integer 7-point stencil
-// rebuilt from its own cells (rediscretisation); in the fine level's units the
-// level-l operator is L_l / 4^l, so the coarse right-hand side is
-// 4 R (f - L x) with R the full-weighting restriction (R = P^T / 8, P the
-// cell-centred trilinear prolongation, weights 3/4 and 1/4 per axis).  The
-// smoother is red-black Gauss-Seidel, NU sweeps red->black before the coarse
-// correction and black->red after it; the coarsest level (at most 4 cells per
-// axis) is smoothed BOTTOM times each way inside one CTA.  Starting every level
-// from zero, the V-cycle is a fixed symmetric linear operator, as CG requires.
-// Sweeps per level group, first measured on the 256^3 fill workload (PCG to 1e-6,
-// steps/s of the whole step; the defaults below were re-measured after the
-// coarse levels got cheaper): (2, 2, 2) took 30 iterations; (3, 6, 6) 16.3
-// iterations, 34.0 steps/s; (2, 6, 6) 17 iterations, 35.4; (1, 6, 6) 18.8, 35.8;
-// (2, 4, 6) 17.8, 35.3.  A fine-level sweep costs ~107 us in place, a level-1
-// sweep ~22 us: the coarse correction near the free surface is the weak part of
-// the cycle, so coarse smoothing pays for itself and fine smoothing does not.
+// else solid.  Level 0 is the integer stencil; a coarse level's operator is a
+// 7-point stencil built from the finer level's faces (k_mg_code).  In the fine
+// level's units the level-l operator is L_l / 4^l, so the coarse right-hand
+// side is 4 R (f - L x) with R = P^T / 8 and P the cell-centred trilinear
+// prolongation (weights 3/4 and 1/4 per axis) divided by the weight of the
+// coarse neighbours that are not solid (k_mg_pscale).  The smoother is
+// red-black Gauss-Seidel, NU sweeps red->black before the coarse correction and
+// black->red after it; the coarsest level (at most 4 cells per axis) is smoothed
+// BOTTOM times each way inside one CTA.  Starting every level from zero, the
+// V-cycle is a fixed symmetric linear operator, as CG requires.
+//
+// Both rules are what makes V(1,1) converge like the textbook cycle here:
+// without the division interpolation loses a quarter of a constant at every
+// wall, and with coarse cells rediscretised from their own kinds a cell cut by
+// the free surface is tied to p = 0 as weakly as a full one.  Iterations to
+// 1e-6 with one sweep on every level (128^3 dam break / porous random mask):
+// 26 / 55 with neither, 16 / 11 with the face operator alone, 9 / 9 with both,
+// the same from 32^3 to 256^3.  With the rediscretised operator the best sweep
+// counts were 1-2 / 4 / 6 / 8, plus three band sweeps at the surface:
+// 17 iterations and 12.1 ms at 256^3, against 8 iterations and 5.7 ms now
+// (one GB300, half-filled box).
+//
 // MIXED precision: the FP32 recursion is folded into the FP64 solution (true
 // FP64 residual, CG restart) each time the residual norm fell this many decades.
 // The FP32 correction restarts from zero at every fold, so the drift between the
 // recursive and the true residual stays near FP32 rounding of the fold's
 // residual, far below a 10^-3 drop.  One decade per fold (the first setting)
-// cost 5 refinements per 1e-6 solve at 256^3.
+// cost 5 refinements per 1e-6 solve at 256^3; four or five decades also need
+// two, at the same time.
 constexpr int MIXED_REFINE_DIGITS = 3;
-// Per-level defaults re-measured on the 256^3 fill workload (steps/s, level 1 /
-// deeper separate levels / cluster levels): 4/6/8 45.2, 4/8/6 45.0, 6/4/6 45.0,
-// 5/5/8 44.9, 4/4/8 44.7 (18 iterations), 6/6/6 44.4, 4/8/10 44.0, 6/6/4 43.6.
-// Level 0 with the free-surface band sweeps (steps/s on the same box; full
-// sweeps / band sweeps): 2/0 46.8 (17.2 iterations), 1/0 47.8 (19.4), 1/2
-// 48.7 (17.8), 1/3 49.3 (17.1), 1/4 49.0 (17.0), 1/5 48.6, 2/4 46.9 (16.0),
-// 2/6 45.8: one full sweep plus three band sweeps recover the iterations a
-// second full sweep saved, for about a third of its cost.  On smaller grids the
-// band's launches cost more than the full sweep they replace (128^3 dam break:
-// 173 -> 158 steps/s, 32^3: 480 -> 399), so the band is the default only from
-// MG_BAND_MIN_CELLS cells on.
-constexpr long long MG_BAND_MIN_CELLS = 1ll << 23;
-constexpr int MG_NU_DEFAULT_BIG = 1;       // level 0, grids of MG_BAND_MIN_CELLS cells or more
-constexpr int MG_NB_DEFAULT_BIG = 3;       // level 0 free-surface band, same grids
-constexpr int MG_NU_DEFAULT = 2;           // level 0, smaller grids (no band)
-constexpr int MG_NU_L1_DEFAULT = 4;        // level 1 (128^3 at 256^3)
-constexpr int MG_NU_COARSE_DEFAULT = 6;    // deeper separately launched levels
-constexpr int MG_NU_CLUSTER_DEFAULT = 8;   // cluster levels in global or distributed shared memory
-constexpr int MG_NU_SMALL_DEFAULT = 6;     // levels rank 0 runs alone (<= 4096 cells): 8/6 45.5, 8/8 45.2,
-                                           // 10/6 45.3, 12/4 45.3, 8/4 45.0 (17.75 iterations)
-constexpr int MG_BOTTOM_SWEEPS = 4;  // on the <= 4^3 bottom level; 12 gave the same iterations, 12 us/it slower
+// Sweeps per level: level 0 / separately launched coarse levels / cluster levels,
+// ms of a solve to 1e-6 (32^3 and 128^3 dam break, 256^3 half filled, random
+// mask 72x100x85): 1/1/1 1.04, 1.86, 5.81, 1.99; 1/2/2 1.01, 1.77, 5.75, 1.87;
+// 2/2/2 0.99, 1.69, 6.00, 1.80; 2/1/1 1.03, 1.99, 6.68, 1.95.  Band sweeps no
+// longer pay: 1/1/1 with two, 1.26, 2.10, 6.12, 2.33.
+constexpr int MG_NU_DEFAULT = 1;         // level 0
+constexpr int MG_NU_COARSE_DEFAULT = 2;  // all coarser levels
+constexpr int MG_BOTTOM_SWEEPS = 4;  // on the <= 4^3 bottom level
 constexpr int MG_BOTTOM_MAX = 4096;
 
 struct MGLev {
     int nx, ny, nz, pz;
-    const uint16_t* code;
+    const uint16_t* code;   // level 0
+    const uint32_t* ccode;  // levels >= 1 (coarse_* helpers)
     float* x;
     const float* f;
     const float* f1;  // level 0: the rhs is the current PCG residual buffer (r[0] or r[1])
@@ -579,10 +571,41 @@ __device__ __forceinline__ const float* mg_rhs(const PcgArgs& A, const MGLev& L)
     return (L.f1 && (A.st->bufsel & 1)) ? L.f1 : L.f;
 }
 
-__device__ __forceinline__ long long mg_off(const MGLev& L, int k) {
-    const long long st = (k >> 1) == 0 ? (long long)L.pz * L.ny : ((k >> 1) == 1 ? (long long)L.pz : 1ll);
-    return (k & 1) ? -st : st;
+// Coarse cell code (levels >= 1): bits 3k..3k+2 the open quarters (0..4) of the
+// face towards neighbour k (+x, -x, +y, -y, +z, -z), bits 18-22 the Dirichlet
+// weight in eighths, bits 23-28 the interpolation scale (below); 0 = no unknown.
+constexpr uint32_t CC_OP = 0x7FFFFF;      // faces and Dirichlet weight
+constexpr uint32_t CC_INTERIOR = 0x24924; // six open faces, no Dirichlet weight
+constexpr int CC_DIRICHLET = 18, CC_SCALE = 23;
+constexpr int DIRICHLET_MAX = 24;         // eighths
+// colour and slab bits of the copies in shared memory
+constexpr uint32_t CS_ODD = 1u << 29, CS_XLO = 1u << 30, CS_XHI = 1u << 31;
+
+// eight times the diagonal: two per open quarter face plus the Dirichlet eighths
+__device__ __forceinline__ int coarse_diag8(uint32_t cc) {
+    const uint32_t a = (cc & 0x71C7u) + ((cc >> 3) & 0x71C7u);
+    return 2 * (int)((a + (a >> 6) + (a >> 12)) & 0x3Fu) + (int)((cc >> CC_DIRICHLET) & 31u);
 }
+// small unsigned integer to float without the quarter-rate conversion unit
+__device__ __forceinline__ float small_float(uint32_t v) { return __uint_as_float(0x4B000000u | v) - 8388608.f; }
+__device__ __forceinline__ float coarse_face(uint32_t cc, int k) { return small_float((cc >> (3 * k)) & 7u); }
+// f + neighbours over the diagonal; sum4 = sum of (quarters * neighbour value)
+__device__ __forceinline__ float coarse_solve(uint32_t cc, float f, float sum4) {
+    return __fdividef(8.f * f + 2.f * sum4, small_float((uint32_t)coarse_diag8(cc)));
+}
+__device__ __forceinline__ float coarse_resid(uint32_t cc, float f, float x, float sum4) {
+    return f - (0.125f * small_float((uint32_t)coarse_diag8(cc)) * x - 0.25f * sum4);
+}
+
+// Interpolation scale.  The trilinear weights (27, 9, 9, 9, 3, 3, 3, 1)/64 of a
+// cell's eight coarse neighbours are divided by the sum over those that are
+// not solid (k / 64), so that interpolation reproduces constants next to walls
+// (zero normal derivative) and still falls to zero towards air (p = 0).  Codes
+// store 64 - k (0 in the interior; the cell's own parent is fluid, so k >= 27):
+// level 0 in the code's six spare bits, coarse levels in bits 23-28.
+__constant__ float c_pscale[64];  // 64 / (64 - i)
+__device__ __forceinline__ float code_pscale(uint16_t c) { return c_pscale[((c >> 6) & 3) | ((c >> 9) & 0x3C)]; }
+__device__ __forceinline__ float coarse_pscale(uint32_t c) { return c_pscale[(c >> CC_SCALE) & 63u]; }
 
 // ---- quad kernels -----------------------------------------------------------
 // Every multigrid kernel (and the MG-path PCG kernels) gives each thread a quad:
@@ -609,6 +632,15 @@ __device__ __forceinline__ void codes4(const uint16_t* code, long long c0, uint1
 __device__ __forceinline__ bool any_fluid(const uint16_t (&cc)[4]) {
     return ((cc[0] | cc[1] | cc[2] | cc[3]) & CODE_FLUID) != 0;
 }
+__device__ __forceinline__ void codes4(const uint32_t* code, long long c0, uint32_t (&cc)[4]) {
+    const uint4 w = *reinterpret_cast<const uint4*>(code + c0);
+    cc[0] = w.x; cc[1] = w.y; cc[2] = w.z; cc[3] = w.w;
+}
+__device__ __forceinline__ bool any_fluid(const uint32_t (&cc)[4]) {
+    return ((cc[0] | cc[1] | cc[2] | cc[3]) & CC_OP) != 0;
+}
+__device__ __forceinline__ bool is_fluid(uint16_t c) { return (c & CODE_FLUID) != 0; }
+__device__ __forceinline__ bool is_fluid(uint32_t c) { return (c & CC_OP) != 0; }
 
 // a field around a quad: centre and the four face-neighbour quads, plus z ends
 struct Q7 {
@@ -642,6 +674,42 @@ __device__ __forceinline__ float nbsum(const Q7& q, int i, uint16_t cc) {
     if (cc & 32) s += (i > 0) ? q.c[i - 1] : q.zm;
     return s;
 }
+
+// the same on a coarse level: sum of (open quarters * neighbour value)
+__device__ __forceinline__ float nbsum4(const Q7& q, int i, uint32_t cc) {
+    const float zp = (i < 3) ? q.c[i + 1] : q.zp, zm = (i > 0) ? q.c[i - 1] : q.zm;
+    if ((cc & CC_OP) == CC_INTERIOR) return 4.f * (q.xp[i] + q.xm[i] + q.yp[i] + q.ym[i] + zp + zm);
+    // closed faces are skipped, not multiplied by zero: a cell without an unknown
+    // may hold an earlier solve's non-finite value
+    float s = 0.f;
+    if (cc & 7u) s += coarse_face(cc, 0) * q.xp[i];
+    if (cc & (7u << 3)) s += coarse_face(cc, 1) * q.xm[i];
+    if (cc & (7u << 6)) s += coarse_face(cc, 2) * q.yp[i];
+    if (cc & (7u << 9)) s += coarse_face(cc, 3) * q.ym[i];
+    if (cc & (7u << 12)) s += coarse_face(cc, 4) * zp;
+    if (cc & (7u << 15)) s += coarse_face(cc, 5) * zm;
+    return s;
+}
+
+// Gauss-Seidel value and residual of lane i, on either kind of level
+__device__ __forceinline__ float gs_value(const Q7& q, int i, uint16_t cc, float f, bool first) {
+    return (first ? f : f + nbsum(q, i, cc)) * c_rcp[code_ns(cc)];
+}
+__device__ __forceinline__ float gs_value(const Q7& q, int i, uint32_t cc, float f, bool first) {
+    return coarse_solve(cc, f, first ? 0.f : nbsum4(q, i, cc));
+}
+__device__ __forceinline__ float resid_value(const Q7& q, int i, uint16_t cc, float f) {
+    return f - ((float)code_ns(cc) * q.c[i] - nbsum(q, i, cc));
+}
+__device__ __forceinline__ float resid_value(const Q7& q, int i, uint32_t cc, float f) {
+    return coarse_resid(cc, f, q.c[i], nbsum4(q, i, cc));
+}
+__device__ __forceinline__ float pscale_of(uint16_t c) { return code_pscale(c); }
+__device__ __forceinline__ float pscale_of(uint32_t c) { return coarse_pscale(c); }
+template <bool FINE>
+struct LevCode { using T = uint16_t; static __device__ __forceinline__ const T* of(const MGLev& L) { return L.code; } };
+template <>
+struct LevCode<false> { using T = uint32_t; static __device__ __forceinline__ const T* of(const MGLev& L) { return L.ccode; } };
 
 // all quads of a coarse level, thread i0 + k * step
 // (x, y, z0) of quad i of a level, in 32-bit arithmetic (levels stay below 2^31 cells)
@@ -683,12 +751,13 @@ __device__ __forceinline__ void mg_for_quads(const PcgArgs& A, const MGLev& L, F
 __device__ __forceinline__ long long lev_sx(const MGLev& L) { return (long long)L.pz * L.ny; }
 
 // one red-black Gauss-Seidel half sweep of a quad; first: the other colour is still zero
+template <bool FINE>
 __device__ __forceinline__ void smooth_quad(const MGLev& L, const float* rhs, int color, int first, int x, int y,
                                             int z0, long long c0) {
     // every load is issued before the fluid test (one round trip, not two; the
     // levels sit in L2, so the loads of quads without fluid are cheap)
-    uint16_t cc[4];
-    codes4(L.code, c0, cc);
+    typename LevCode<FINE>::T cc[4];
+    codes4(LevCode<FINE>::of(L), c0, cc);
     float f[4];
     unpack4(ld4(rhs + c0), f);
     Q7 q;
@@ -699,10 +768,8 @@ __device__ __forceinline__ void smooth_quad(const MGLev& L, const float* rhs, in
     float out[4] = {q.c[0], q.c[1], q.c[2], q.c[3]};
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        if (((par ^ i) & 1) != color || !(cc[i] & CODE_FLUID)) continue;
-        float sum = f[i];
-        if (!first) sum += nbsum(q, i, cc[i]);
-        out[i] = sum * c_rcp[code_ns(cc[i])];
+        if (((par ^ i) & 1) != color || !is_fluid(cc[i])) continue;
+        out[i] = gs_value(q, i, cc[i], f[i], first != 0);
     }
     st4(L.x + c0, out);
 }
@@ -712,7 +779,7 @@ __global__ void __launch_bounds__(PCG_THREADS) k_mg_smooth(const PcgArgs A, MGLe
     pdl_enter();
     if (A.st->done) return;
     const float* rhs = mg_rhs(A, L);
-    mg_for_quads<FINE>(A, L, [&](int x, int y, int z0, long long c0) { smooth_quad(L, rhs, color, first, x, y, z0, c0); });
+    mg_for_quads<FINE>(A, L, [&](int x, int y, int z0, long long c0) { smooth_quad<FINE>(L, rhs, color, first, x, y, z0, c0); });
 }
 
 // the last post-smoothing half sweep (red, level 0) fused with z.r (modes 0/1 as k_red)
@@ -762,9 +829,12 @@ __global__ void __launch_bounds__(PCG_THREADS) k_mg_smooth_dot(const PcgArgs A, 
     }
 }
 
+// r = (f - A x) times the interpolation scale (restriction is the transpose of
+// the scaled interpolation)
+template <bool FINE>
 __device__ __forceinline__ void residual_quad(const MGLev& L, const float* rhs, int x, int y, int z0, long long c0) {
-    uint16_t cc[4];
-    codes4(L.code, c0, cc);
+    typename LevCode<FINE>::T cc[4];
+    codes4(LevCode<FINE>::of(L), c0, cc);
     float f[4];
     unpack4(ld4(rhs + c0), f);
     Q7 q;
@@ -772,8 +842,7 @@ __device__ __forceinline__ void residual_quad(const MGLev& L, const float* rhs, 
     if (!any_fluid(cc)) return;
     float out[4];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-        out[i] = (cc[i] & CODE_FLUID) ? f[i] - ((float)code_ns(cc[i]) * q.c[i] - nbsum(q, i, cc[i])) : 0.f;
+    for (int i = 0; i < 4; i++) out[i] = is_fluid(cc[i]) ? resid_value(q, i, cc[i], f[i]) * pscale_of(cc[i]) : 0.f;
     st4(L.r + c0, out);
 }
 
@@ -782,15 +851,16 @@ __global__ void __launch_bounds__(PCG_THREADS) k_mg_residual(const PcgArgs A, MG
     pdl_enter();
     if (A.st->done) return;
     const float* rhs = mg_rhs(A, L);
-    mg_for_quads<FINE>(A, L, [&](int x, int y, int z0, long long c0) { residual_quad(L, rhs, x, y, z0, c0); });
+    mg_for_quads<FINE>(A, L, [&](int x, int y, int z0, long long c0) { residual_quad<FINE>(L, rhs, x, y, z0, c0); });
 }
 
 // coarse f = 0.5 * sum_fine P[f,C] r_f  (= 4 R r), per coarse quad:
 // fine z 2 z0 - 1 .. 2 z0 + 8 come from the four fine quads at 2 z0 - 4 .. 2 z0 + 8
+template <bool FINE>
 __device__ __forceinline__ void restrict_quad(const MGLev& F, const MGLev& Cl, int cx, int cy, int cz0, long long ci) {
     {
-        uint16_t ccc[4];
-        codes4(Cl.code, ci, ccc);
+        uint32_t ccc[4];
+        codes4(Cl.ccode, ci, ccc);
         if (!any_fluid(ccc)) return;
         float sum[4] = {0.f, 0.f, 0.f, 0.f};
         const int fz0 = 2 * cz0 - 4;  // first fine z loaded (a multiple of 4)
@@ -812,12 +882,12 @@ __device__ __forceinline__ void restrict_quad(const MGLev& F, const MGLev& Cl, i
                     if (z >= 0 && z < F.pz) {
                         // codes and residual loaded together; r is stale on quads
                         // without fluid (never written), so the codes mask it
-                        uint16_t fc[4];
-                        codes4(F.code, row + z, fc);
+                        typename LevCode<FINE>::T fc[4];
+                        codes4(LevCode<FINE>::of(F), row + z, fc);
                         unpack4(ld4(F.r + row + z), v);
 #pragma unroll
                         for (int e = 0; e < 4; e++)
-                            if (!(fc[e] & CODE_FLUID)) v[e] = 0.f;
+                            if (!is_fluid(fc[e])) v[e] = 0.f;
                     }
 #pragma unroll
                     for (int e = 0; e < 4; e++) fr[4 * k + e] = v[e];
@@ -833,23 +903,25 @@ __device__ __forceinline__ void restrict_quad(const MGLev& F, const MGLev& Cl, i
         unpack4(ld4(Cl.f + ci), out);
 #pragma unroll
         for (int j = 0; j < 4; j++)
-            if (ccc[j] & CODE_FLUID) out[j] = 0.5f * sum[j];
+            if (is_fluid(ccc[j])) out[j] = 0.5f * sum[j];
         st4(const_cast<float*>(Cl.f) + ci, out);
     }
 }
 
+template <bool FINE>
 __global__ void __launch_bounds__(PCG_THREADS) k_mg_restrict(const PcgState* st, MGLev F, MGLev Cl) {
     pdl_enter();
     if (st->done) return;
     mg_for_range(Cl, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x,
-                 [&](int x, int y, int z0, long long c0) { restrict_quad(F, Cl, x, y, z0, c0); });
+                 [&](int x, int y, int z0, long long c0) { restrict_quad<FINE>(F, Cl, x, y, z0, c0); });
 }
 
 // fine x += P x_coarse on fluid fine cells, per fine quad: the quad's coarse z
 // neighbours are z0/2 - 1 .. z0/2 + 2
+template <bool FINE>
 __device__ __forceinline__ void prolong_quad(const MGLev& F, const MGLev& Cl, int x, int y, int z0, long long c0) {
-    uint16_t cc[4];
-    codes4(F.code, c0, cc);
+    typename LevCode<FINE>::T cc[4];
+    codes4(LevCode<FINE>::of(F), c0, cc);
     if (!any_fluid(cc)) return;
     const int px = (x & 1) ? x >> 1 : (x >> 1) - 1;  // lower coarse neighbour per axis
     const int py = (y & 1) ? y >> 1 : (y >> 1) - 1;
@@ -869,19 +941,19 @@ __device__ __forceinline__ void prolong_quad(const MGLev& F, const MGLev& Cl, in
         const float wxy = (ox ? 1.f - wlx : wlx) * (oy ? 1.f - wly : wly);
         const long long row = ((long long)cx * Cl.ny + cy) * Cl.pz;
         float qv[4];
-        uint16_t qc[4];
+        uint32_t qc[4];
         unpack4(ld4(Cl.x + row + hq), qv);
-        codes4(Cl.code, row + hq, qc);
+        codes4(Cl.ccode, row + hq, qc);
         const bool ein = ze >= 0 && ze < Cl.pz;
         const float ev = ein ? Cl.x[row + ze] : 0.f;
-        const uint16_t ec = ein ? Cl.code[row + ze] : (uint16_t)0;
+        const uint32_t ec = ein ? Cl.ccode[row + ze] : 0u;
         float cv[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             // lowq: zc = hq - 1 (the extra value), then hq .. hq + 2; else hq + 1 .. hq + 3, then hq + 4
             const float v = lowq ? (k == 0 ? ev : qv[k - 1]) : (k == 3 ? ev : qv[k + 1]);
-            const uint16_t c = lowq ? (k == 0 ? ec : qc[k - 1]) : (k == 3 ? ec : qc[k + 1]);
-            cv[k] = (c & CODE_FLUID) ? v : 0.f;
+            const uint32_t c = lowq ? (k == 0 ? ec : qc[k - 1]) : (k == 3 ? ec : qc[k + 1]);
+            cv[k] = is_fluid(c) ? v : 0.f;
         }
         // lanes: z0 (lower zc, w 1/4), z0+1 (zc+1, 3/4), z0+2 (zc+1, 1/4), z0+3 (zc+2, 3/4)
         sum[0] += wxy * (0.25f * cv[0] + 0.75f * cv[1]);
@@ -893,7 +965,7 @@ __device__ __forceinline__ void prolong_quad(const MGLev& F, const MGLev& Cl, in
     unpack4(ld4(F.x + c0), xv);
 #pragma unroll
     for (int i = 0; i < 4; i++)
-        if (cc[i] & CODE_FLUID) xv[i] += sum[i];
+        if (is_fluid(cc[i])) xv[i] += sum[i] * pscale_of(cc[i]);
     st4(F.x + c0, xv);
 }
 
@@ -901,7 +973,7 @@ template <bool FINE>
 __global__ void __launch_bounds__(PCG_THREADS) k_mg_prolong(const PcgArgs A, MGLev F, MGLev Cl) {
     pdl_enter();
     if (A.st->done) return;
-    mg_for_quads<FINE>(A, F, [&](int x, int y, int z0, long long c0) { prolong_quad(F, Cl, x, y, z0, c0); });
+    mg_for_quads<FINE>(A, F, [&](int x, int y, int z0, long long c0) { prolong_quad<FINE>(F, Cl, x, y, z0, c0); });
 }
 
 // ---- free-surface band of the finest level ------------------------------------
@@ -949,7 +1021,7 @@ __global__ void __launch_bounds__(PCG_THREADS) k_mg_smooth_bnd(const PcgArgs A, 
     const int n = *count;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int4 q = list[i];
-        smooth_quad(L, rhs, color, 0, q.x, q.y, q.z, ((long long)q.x * L.ny + q.y) * L.pz + q.z);
+        smooth_quad<true>(L, rhs, color, 0, q.x, q.y, q.z, ((long long)q.x * L.ny + q.y) * L.pz + q.z);
     }
 }
 
@@ -1098,8 +1170,25 @@ __global__ void __launch_bounds__(PCG_THREADS) k_update_q(const PcgArgs a, Vecs<
     }
 }
 
+// dense copies of a coarse level in shared memory: colour test and neighbour sum
+// (a closed face is not read: its neighbour may lie outside the array)
+__device__ __forceinline__ bool smem_color(uint32_t cc, int color) {
+    return (cc & CC_OP) && ((cc & CS_ODD) != 0) == (color != 0);
+}
+__device__ __forceinline__ float smem_nbsum4(const float* x, int i, uint32_t cc, int sx, int sy) {
+    if ((cc & CC_OP) == CC_INTERIOR) return 4.f * (x[i + sx] + x[i - sx] + x[i + sy] + x[i - sy] + x[i + 1] + x[i - 1]);
+    float s = 0.f;
+    if (cc & 7u) s += coarse_face(cc, 0) * x[i + sx];
+    if (cc & (7u << 3)) s += coarse_face(cc, 1) * x[i - sx];
+    if (cc & (7u << 6)) s += coarse_face(cc, 2) * x[i + sy];
+    if (cc & (7u << 9)) s += coarse_face(cc, 3) * x[i - sy];
+    if (cc & (7u << 12)) s += coarse_face(cc, 4) * x[i + 1];
+    if (cc & (7u << 15)) s += coarse_face(cc, 5) * x[i - 1];
+    return s;
+}
+
 // coarsest level: symmetric red-black Gauss-Seidel in shared memory, one CTA
-__device__ void mg_bottom_block(const MGLev& L, float* sx, float* sf, uint16_t* sc) {
+__device__ void mg_bottom_block(const MGLev& L, float* sx, float* sf, uint32_t* sc) {
     const int n = L.nx * L.ny * L.nz;  // dense in shared memory, padded in global
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const int z = i % L.nz, t = i / L.nz;
@@ -1107,7 +1196,7 @@ __device__ void mg_bottom_block(const MGLev& L, float* sx, float* sf, uint16_t* 
         const int odd = (t / L.ny + t % L.ny + z) & 1;
         sx[i] = 0.f;
         sf[i] = L.f[gi];
-        sc[i] = L.code[gi] | (odd ? SCODE_ODD : 0);
+        sc[i] = L.ccode[gi] | (odd ? CS_ODD : 0);
     }
     __syncthreads();
     const int sxs = L.ny * L.nz, sys = L.nz;
@@ -1115,18 +1204,10 @@ __device__ void mg_bottom_block(const MGLev& L, float* sx, float* sf, uint16_t* 
         // forward half: red then black; backward half: black then red
         for (int h = 0; h < 2; h++) {
             const int color = (pass < MG_BOTTOM_SWEEPS) ? h : 1 - h;
-            const uint16_t want = CODE_FLUID | (color ? SCODE_ODD : 0);
             for (int i = threadIdx.x; i < n; i += blockDim.x) {
-                const uint16_t cc = sc[i];
-                if ((cc & (CODE_FLUID | SCODE_ODD)) != want) continue;
-                float sum = sf[i];
-                if (cc & 1) sum += sx[i + sxs];
-                if (cc & 2) sum += sx[i - sxs];
-                if (cc & 4) sum += sx[i + sys];
-                if (cc & 8) sum += sx[i - sys];
-                if (cc & 16) sum += sx[i + 1];
-                if (cc & 32) sum += sx[i - 1];
-                sx[i] = sum * c_rcp[code_ns(cc)];
+                const uint32_t cc = sc[i];
+                if (!smem_color(cc, color)) continue;
+                sx[i] = coarse_solve(cc, sf[i], smem_nbsum4(sx, i, cc, sxs, sys));
             }
             __syncthreads();
         }
@@ -1139,7 +1220,7 @@ __global__ void __launch_bounds__(1024) k_mg_bottom(const PcgState* st, MGLev L)
     if (st->done) return;
     __shared__ float sx[MG_BOTTOM_MAX];
     __shared__ float sf[MG_BOTTOM_MAX];
-    __shared__ uint16_t sc[MG_BOTTOM_MAX];
+    __shared__ uint32_t sc[MG_BOTTOM_MAX];
     mg_bottom_block(L, sx, sf, sc);
 }
 
@@ -1160,7 +1241,6 @@ constexpr int MG_CLUSTER_SMEM = 200 * 1024;  // dynamic shared memory limit of t
 struct MGChain {
     MGLev lev[MG_MAX_LEVELS];
     int lc, last, nu;
-    int nu_small;  // sweeps on the shared-memory levels ls .. last-1
     int ls;  // first level small enough to run in one CTA's shared memory (<= last)
     // levels lc .. ls-1 as x slabs in distributed shared memory (slab != 0):
     // planes per CTA and float offset of each level in the pool, then the offset
@@ -1182,7 +1262,7 @@ constexpr int MG_SMEM_CELLS = 4096;
 struct SLev {
     int nx, ny, nz, n;
     float *x, *f, *r;
-    uint16_t* code;
+    uint32_t* code;
 };
 
 __device__ __forceinline__ int sidx(const SLev& L, int x, int y, int z) { return (x * L.ny + y) * L.nz + z; }
@@ -1193,20 +1273,8 @@ __device__ __forceinline__ int sidx(const SLev& L, int x, int y, int z) { return
 constexpr int SCELLS_PER_THREAD = 4;
 static_assert(SCELLS_PER_THREAD * MG_CLUSTER_THREADS >= MG_SMEM_CELLS, "shared-memory level cells per thread");
 
-__device__ __forceinline__ float s_nbsum(const SLev& L, int i, uint16_t cc, int sx, int sy) {
-    float s = 0.f;
-    if (cc & 1) s += L.x[i + sx];
-    if (cc & 2) s += L.x[i - sx];
-    if (cc & 4) s += L.x[i + sy];
-    if (cc & 8) s += L.x[i - sy];
-    if (cc & 16) s += L.x[i + 1];
-    if (cc & 32) s += L.x[i - 1];
-    return s;
-}
-
 __device__ void s_smooth(const SLev L, int color) {
     const int sx = L.ny * L.nz, sy = L.nz;
-    const uint16_t want = CODE_FLUID | (color ? SCODE_ODD : 0);
     float nv[SCELLS_PER_THREAD];
     bool act[SCELLS_PER_THREAD];
 #pragma unroll
@@ -1215,10 +1283,10 @@ __device__ void s_smooth(const SLev L, int color) {
         act[k] = false;
         nv[k] = 0.f;
         if (i >= L.n) continue;
-        const uint16_t cc = L.code[i];
-        if ((cc & (CODE_FLUID | SCODE_ODD)) != want) continue;
+        const uint32_t cc = L.code[i];
+        if (!smem_color(cc, color)) continue;
         act[k] = true;
-        nv[k] = (L.f[i] + s_nbsum(L, i, cc, sx, sy)) * c_rcp[code_ns(cc)];
+        nv[k] = coarse_solve(cc, L.f[i], smem_nbsum4(L.x, i, cc, sx, sy));
     }
 #pragma unroll
     for (int k = 0; k < SCELLS_PER_THREAD; k++)
@@ -1234,8 +1302,9 @@ __device__ void s_residual(const SLev L) {
         const int i = threadIdx.x + k * MG_CLUSTER_THREADS;
         rv[k] = 0.f;
         if (i >= L.n) continue;
-        const uint16_t cc = L.code[i];
-        if (cc & CODE_FLUID) rv[k] = L.f[i] - ((float)code_ns(cc) * L.x[i] - s_nbsum(L, i, cc, sx, sy));
+        const uint32_t cc = L.code[i];
+        if (is_fluid(cc))
+            rv[k] = coarse_resid(cc, L.f[i], L.x[i], smem_nbsum4(L.x, i, cc, sx, sy)) * coarse_pscale(cc);
     }
 #pragma unroll
     for (int k = 0; k < SCELLS_PER_THREAD; k++) {
@@ -1252,7 +1321,7 @@ __device__ void s_restrict(const SLev F, const SLev C) {
     for (int i = threadIdx.x; i < C.n; i += blockDim.x) {
         const int cz = i % C.nz, cy = (i / C.nz) % C.ny, cx = i / (C.nz * C.ny);
         C.x[i] = 0.f;
-        if (!(C.code[i] & CODE_FLUID)) {
+        if (!is_fluid(C.code[i])) {
             C.f[i] = 0.f;
             continue;
         }
@@ -1284,7 +1353,7 @@ __device__ void s_restrict(const SLev F, const SLev C) {
 // fine x += P x_coarse on fluid fine cells (coarse fluid values only)
 __device__ void s_prolong(const SLev F, const SLev C) {
     for (int i = threadIdx.x; i < F.n; i += blockDim.x) {
-        if (!(F.code[i] & CODE_FLUID)) continue;
+        if (!is_fluid(F.code[i])) continue;
         const int z = i % F.nz, y = (i / F.nz) % F.ny, x = i / (F.nz * F.ny);
         const int p[3] = {(x & 1) ? x >> 1 : (x >> 1) - 1, (y & 1) ? y >> 1 : (y >> 1) - 1,
                           (z & 1) ? z >> 1 : (z >> 1) - 1};
@@ -1295,17 +1364,16 @@ __device__ void s_prolong(const SLev F, const SLev C) {
             const int cx = p[0] + ox, cy = p[1] + oy, cz = p[2] + oz;
             if (cx < 0 || cy < 0 || cz < 0 || cx >= C.nx || cy >= C.ny || cz >= C.nz) continue;
             const int ci = sidx(C, cx, cy, cz);
-            if (!(C.code[ci] & CODE_FLUID)) continue;
+            if (!is_fluid(C.code[ci])) continue;
             sum += (ox ? 1.f - wl[0] : wl[0]) * (oy ? 1.f - wl[1] : wl[1]) * (oz ? 1.f - wl[2] : wl[2]) * C.x[ci];
         }
-        F.x[i] += sum;
+        F.x[i] += sum * coarse_pscale(F.code[i]);
     }
     __syncthreads();
 }
 
 // Levels ls..last in one CTA's shared memory, dense (z fastest), laid out from
-// `smem` level by level: x, f, r (n floats each), then the codes (n uint16,
-// padded to whole floats).  load_f: level ls's rhs comes from global memory
+// `smem` level by level: x, f, r (n floats each), then the codes (n words).  load_f: level ls's rhs comes from global memory
 // (otherwise the caller's restriction writes it into this layout).
 __device__ void smem_levels_init(const MGChain& C, float* smem, SLev* S, bool load_f) {
     if (threadIdx.x == 0) {
@@ -1318,8 +1386,8 @@ __device__ void smem_levels_init(const MGChain& C, float* smem, SLev* S, bool lo
             L.x = p; p += L.n;
             L.f = p; p += L.n;
             L.r = p; p += L.n;
-            L.code = reinterpret_cast<uint16_t*>(p);
-            p += (L.n + 1) / 2;
+            L.code = reinterpret_cast<uint32_t*>(p);
+            p += L.n;
         }
     }
     __syncthreads();
@@ -1330,7 +1398,7 @@ __device__ void smem_levels_init(const MGChain& C, float* smem, SLev* S, bool lo
             const int z = i % L.nz, t = i / L.nz;
             const long long gi = (long long)t * G.pz + z;
             const int odd = (t / L.ny + t % L.ny + z) & 1;
-            L.code[i] = G.code[gi] | (odd ? SCODE_ODD : 0);
+            L.code[i] = G.ccode[gi] | (odd ? CS_ODD : 0);
             L.x[i] = 0.f;
             if (l == C.ls && load_f) L.f[i] = G.f[gi];
         }
@@ -1342,7 +1410,7 @@ __device__ void smem_levels_init(const MGChain& C, float* smem, SLev* S, bool lo
 // global memory (otherwise the caller's prolongation reads it in place)
 __device__ void smem_levels_run(const MGChain& C, const SLev* S, bool store_x) {
     for (int l = C.ls; l < C.last; l++) {
-        for (int k = 0; k < C.nu_small; k++) {
+        for (int k = 0; k < C.nu; k++) {
             s_smooth(S[l], 0);
             s_smooth(S[l], 1);
         }
@@ -1359,7 +1427,7 @@ __device__ void smem_levels_run(const MGChain& C, const SLev* S, bool store_x) {
     }
     for (int l = C.last - 1; l >= C.ls; l--) {
         s_prolong(S[l], S[l + 1]);
-        for (int k = 0; k < C.nu_small; k++) {
+        for (int k = 0; k < C.nu; k++) {
             s_smooth(S[l], 1);
             s_smooth(S[l], 0);
         }
@@ -1394,12 +1462,11 @@ __device__ __forceinline__ unsigned cluster_size() {
 // The restriction into level ls writes straight into rank 0's shared-memory
 // levels, and the prolongation from ls reads them there, so only level lc's
 // rhs comes from global memory and only its correction goes back.
-constexpr uint16_t SCODE_XLO = 0x2000;  // slab copies: x - 1 lies in the previous CTA
-constexpr uint16_t SCODE_XHI = 0x1000;  // slab copies: x + 1 lies in the next CTA
+// (CS_XLO / CS_XHI in the slab copies' codes: x - 1 / x + 1 lies in the previous / next CTA)
 
 struct DLev {
     float *x, *f, *r;
-    uint16_t* code;
+    uint32_t* code;
     int nx, ny, nz, P, np, x0, plane;
 };
 
@@ -1416,7 +1483,7 @@ __device__ __forceinline__ DLev dlev(const MGChain& C, int l, float* pool, unsig
     D.x = p;
     D.f = p + m;
     D.r = p + 2 * m;
-    D.code = reinterpret_cast<uint16_t*>(p + 3 * m);
+    D.code = reinterpret_cast<uint32_t*>(p + 3 * m);
     return D;
 }
 
@@ -1428,36 +1495,35 @@ __device__ __forceinline__ T* dsm(T* p, unsigned rank) {
     return reinterpret_cast<T*>(out);
 }
 
-__device__ __forceinline__ float slab_nbsum(const DLev& D, int i, uint16_t cc, const float* xp, const float* xn) {
+__device__ __forceinline__ float slab_nbsum4(const DLev& D, int i, uint32_t cc, const float* xp, const float* xn) {
+    if ((cc & (CC_OP | CS_XLO | CS_XHI)) == CC_INTERIOR)
+        return 4.f * (D.x[i + D.plane] + D.x[i - D.plane] + D.x[i + D.nz] + D.x[i - D.nz] + D.x[i + 1] + D.x[i - 1]);
     float s = 0.f;
-    if (cc & 1) s += (cc & SCODE_XHI) ? xn[i - (D.np - 1) * D.plane] : D.x[i + D.plane];
-    if (cc & 2) s += (cc & SCODE_XLO) ? xp[i + (D.P - 1) * D.plane] : D.x[i - D.plane];
-    if (cc & 4) s += D.x[i + D.nz];
-    if (cc & 8) s += D.x[i - D.nz];
-    if (cc & 16) s += D.x[i + 1];
-    if (cc & 32) s += D.x[i - 1];
+    if (cc & 7u) s += coarse_face(cc, 0) * ((cc & CS_XHI) ? xn[i - (D.np - 1) * D.plane] : D.x[i + D.plane]);
+    if (cc & (7u << 3)) s += coarse_face(cc, 1) * ((cc & CS_XLO) ? xp[i + (D.P - 1) * D.plane] : D.x[i - D.plane]);
+    if (cc & (7u << 6)) s += coarse_face(cc, 2) * D.x[i + D.nz];
+    if (cc & (7u << 9)) s += coarse_face(cc, 3) * D.x[i - D.nz];
+    if (cc & (7u << 12)) s += coarse_face(cc, 4) * D.x[i + 1];
+    if (cc & (7u << 15)) s += coarse_face(cc, 5) * D.x[i - 1];
     return s;
 }
 
 // red-black half sweep; first: the other colour is still zero
 __device__ void slab_smooth(const DLev& D, int color, bool first, const float* xp, const float* xn) {
-    const uint16_t want = CODE_FLUID | (color ? SCODE_ODD : 0);
     const int n = D.np * D.plane;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const uint16_t cc = D.code[i];
-        if ((cc & (CODE_FLUID | SCODE_ODD)) != want) continue;
-        float sum = D.f[i];
-        if (!first) sum += slab_nbsum(D, i, cc, xp, xn);
-        D.x[i] = sum * c_rcp[code_ns(cc)];
+        const uint32_t cc = D.code[i];
+        if (!smem_color(cc, color)) continue;
+        D.x[i] = coarse_solve(cc, D.f[i], first ? 0.f : slab_nbsum4(D, i, cc, xp, xn));
     }
 }
 
 __device__ void slab_residual(const DLev& D, const float* xp, const float* xn) {
     const int n = D.np * D.plane;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const uint16_t cc = D.code[i];
+        const uint32_t cc = D.code[i];
         float rv = 0.f;
-        if (cc & CODE_FLUID) rv = D.f[i] - ((float)code_ns(cc) * D.x[i] - slab_nbsum(D, i, cc, xp, xn));
+        if (is_fluid(cc)) rv = coarse_resid(cc, D.f[i], D.x[i], slab_nbsum4(D, i, cc, xp, xn)) * coarse_pscale(cc);
         D.r[i] = rv;
     }
 }
@@ -1475,7 +1541,7 @@ __device__ void slab_restrict(const MGChain& C, int l, float* pool, unsigned ran
     const int i0 = to_slab ? (int)threadIdx.x : (int)(rank * blockDim.x + threadIdx.x);
     const int step = to_slab ? (int)blockDim.x : (int)(cs * blockDim.x);
     float* fout = to_slab ? D.f : dsm(spool + nsm, 0);
-    const uint16_t* cin = to_slab ? D.code : reinterpret_cast<const uint16_t*>(dsm(spool + 3 * nsm, 0));
+    const uint32_t* cin = to_slab ? D.code : reinterpret_cast<const uint32_t*>(dsm(spool + 3 * nsm, 0));
     for (int i = i0; i < n; i += step) {
         int cx, cy, cz;
         if (to_slab) {
@@ -1489,7 +1555,7 @@ __device__ void slab_restrict(const MGChain& C, int l, float* pool, unsigned ran
             cy = t % Gc.ny;
             cx = t / Gc.ny;
         }
-        if (!(cin[i] & CODE_FLUID)) {
+        if (!is_fluid(cin[i])) {
             fout[i] = 0.f;
             continue;
         }
@@ -1526,10 +1592,10 @@ __device__ void slab_prolong(const MGChain& C, int l, float* pool, unsigned rank
     const DLev D = dlev(C, l + 1, pool, rank);  // used only when from_slab
     const int nsm = Gc.nx * Gc.ny * Gc.nz;
     const float* sx0 = from_slab ? nullptr : dsm(spool, 0);
-    const uint16_t* sc0 = from_slab ? nullptr : reinterpret_cast<const uint16_t*>(dsm(spool + 3 * nsm, 0));
+    const uint32_t* sc0 = from_slab ? nullptr : reinterpret_cast<const uint32_t*>(dsm(spool + 3 * nsm, 0));
     const int n = F.np * F.plane;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        if (!(F.code[i] & CODE_FLUID)) continue;
+        if (!is_fluid(F.code[i])) continue;
         const int xl = i / F.plane, t = i - xl * F.plane;
         const int x = F.x0 + xl, y = t / F.nz, z = t - y * F.nz;
         const int p[3] = {(x & 1) ? x >> 1 : (x >> 1) - 1, (y & 1) ? y >> 1 : (y >> 1) - 1,
@@ -1542,7 +1608,7 @@ __device__ void slab_prolong(const MGChain& C, int l, float* pool, unsigned rank
             const int cx = p[0] + ox, cy = p[1] + oy, cz = p[2] + oz;
             if (cx < 0 || cy < 0 || cz < 0 || cx >= Gc.nx || cy >= Gc.ny || cz >= Gc.nz) continue;
             float v;
-            uint16_t c;
+            uint32_t c;
             if (from_slab) {
                 const unsigned ro = (unsigned)(cx / D.P);
                 const int li = ((cx - (int)ro * D.P) * Gc.ny + cy) * Gc.nz + cz;
@@ -1553,10 +1619,10 @@ __device__ void slab_prolong(const MGChain& C, int l, float* pool, unsigned rank
                 v = sx0[ci];
                 c = sc0[ci];
             }
-            if (!(c & CODE_FLUID)) continue;
+            if (!is_fluid(c)) continue;
             sum += (ox ? 1.f - wl[0] : wl[0]) * (oy ? 1.f - wl[1] : wl[1]) * (oz ? 1.f - wl[2] : wl[2]) * v;
         }
-        F.x[i] += sum;
+        F.x[i] += sum * coarse_pscale(F.code[i]);
     }
 }
 
@@ -1574,10 +1640,10 @@ __global__ void __launch_bounds__(MG_CLUSTER_THREADS) k_mg_coarse(const PcgArgs 
             for (int i = threadIdx.x; i < D.np * D.plane; i += blockDim.x) {
                 const int xl = i / D.plane, t = i - xl * D.plane, y = t / D.nz, z = t - y * D.nz;
                 const long long gi = ((long long)(D.x0 + xl) * G.ny + y) * G.pz + z;
-                uint16_t cc = G.code[gi];
-                if ((D.x0 + xl + y + z) & 1) cc |= SCODE_ODD;
-                if (xl == 0) cc |= SCODE_XLO;
-                if (xl == D.np - 1) cc |= SCODE_XHI;
+                uint32_t cc = G.ccode[gi];
+                if ((D.x0 + xl + y + z) & 1) cc |= CS_ODD;
+                if (xl == 0) cc |= CS_XLO;
+                if (xl == D.np - 1) cc |= CS_XHI;
                 D.code[i] = cc;
                 D.x[i] = 0.f;
                 if (l == C.lc) D.f[i] = G.f[gi];
@@ -1630,15 +1696,15 @@ __global__ void __launch_bounds__(MG_CLUSTER_THREADS) k_mg_coarse(const PcgArgs 
     for (int l = C.lc; l < C.ls; l++) {
         const MGLev& L = C.lev[l];
         for (int k = 0; k < C.nu; k++) {
-            mg_for_range(L, i0, step, [&](int x, int y, int z0, long long c0) { smooth_quad(L, L.f, 0, k == 0, x, y, z0, c0); });
+            mg_for_range(L, i0, step, [&](int x, int y, int z0, long long c0) { smooth_quad<false>(L, L.f, 0, k == 0, x, y, z0, c0); });
             cluster_barrier();
-            mg_for_range(L, i0, step, [&](int x, int y, int z0, long long c0) { smooth_quad(L, L.f, 1, 0, x, y, z0, c0); });
+            mg_for_range(L, i0, step, [&](int x, int y, int z0, long long c0) { smooth_quad<false>(L, L.f, 1, 0, x, y, z0, c0); });
             cluster_barrier();
         }
-        mg_for_range(L, i0, step, [&](int x, int y, int z0, long long c0) { residual_quad(L, L.f, x, y, z0, c0); });
+        mg_for_range(L, i0, step, [&](int x, int y, int z0, long long c0) { residual_quad<false>(L, L.f, x, y, z0, c0); });
         cluster_barrier();
         const MGLev& Cl = C.lev[l + 1];
-        mg_for_range(Cl, i0, step, [&](int x, int y, int z0, long long c0) { restrict_quad(L, Cl, x, y, z0, c0); });
+        mg_for_range(Cl, i0, step, [&](int x, int y, int z0, long long c0) { restrict_quad<false>(L, Cl, x, y, z0, c0); });
         cluster_barrier();
     }
     if (rank == 0) {
@@ -1649,12 +1715,12 @@ __global__ void __launch_bounds__(MG_CLUSTER_THREADS) k_mg_coarse(const PcgArgs 
     for (int l = C.ls - 1; l >= C.lc; l--) {
         const MGLev& L = C.lev[l];
         const MGLev& Cl = C.lev[l + 1];
-        mg_for_range(L, i0, step, [&](int x, int y, int z0, long long c0) { prolong_quad(L, Cl, x, y, z0, c0); });
+        mg_for_range(L, i0, step, [&](int x, int y, int z0, long long c0) { prolong_quad<false>(L, Cl, x, y, z0, c0); });
         cluster_barrier();
         for (int k = 0; k < C.nu; k++) {
-            mg_for_range(L, i0, step, [&](int x, int y, int z0, long long c0) { smooth_quad(L, L.f, 1, 0, x, y, z0, c0); });
+            mg_for_range(L, i0, step, [&](int x, int y, int z0, long long c0) { smooth_quad<false>(L, L.f, 1, 0, x, y, z0, c0); });
             cluster_barrier();
-            mg_for_range(L, i0, step, [&](int x, int y, int z0, long long c0) { smooth_quad(L, L.f, 0, 0, x, y, z0, c0); });
+            mg_for_range(L, i0, step, [&](int x, int y, int z0, long long c0) { smooth_quad<false>(L, L.f, 0, 0, x, y, z0, c0); });
             cluster_barrier();
         }
     }
@@ -1681,31 +1747,83 @@ __global__ void k_mg_coarsen(MGLev F, const uint8_t* fkind, const uint8_t* fflag
     ckind[ci] = (uint8_t)best;
 }
 
-// per-cell code of a coarse level from its kinds (outside the level = solid)
-__global__ void k_mg_code(MGLev L, const uint8_t* kind, uint16_t* code) {
+// Coarse operator: the Galerkin operator of piecewise-constant interpolation,
+// halved (its energy counts a linear profile twice), kept as a 7-point stencil.
+// A coarse face carries the mean of its four fine faces, so that faces partly
+// closed by solids conduct less; the fine cells' Dirichlet weights (fluid-air
+// faces at level 0) add up, halved and bounded, so that a coarse cell that is
+// cut by the free surface stays tied to p = 0 as the fine cells are.  Weights
+// are rounded to quarters and eighths: both cells of a face round the same
+// sum, so the operator stays symmetric.
+// FINE: the finer level is level 0 (16-bit codes).
+template <bool FINE>
+__global__ void k_mg_code(MGLev F, MGLev L, uint32_t* code) {
     const long long n = (long long)L.nx * L.ny * L.nz;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const unsigned iu = (unsigned)i, t = iu / (unsigned)L.nz, u = t / (unsigned)L.ny;
     const int z = (int)(iu - t * (unsigned)L.nz), y = (int)(t - u * (unsigned)L.ny), x = (int)u;
     const long long ci = ((long long)x * L.ny + y) * L.pz + z;
-    if (kind[ci] != 0) {
-        code[ci] = 0;
-        return;
+    int face[6] = {0, 0, 0, 0, 0, 0}, dir = 0;
+#pragma unroll
+    for (int o = 0; o < 8; o++) {
+        const int ox = o >> 2, oy = (o >> 1) & 1, oz = o & 1;
+        const int fx = 2 * x + ox, fy = 2 * y + oy, fz = 2 * z + oz;
+        if (fx >= F.nx || fy >= F.ny || fz >= F.nz) continue;
+        const long long fi = ((long long)fx * F.ny + fy) * F.pz + fz;
+        const int kx = ox ? 0 : 1, ky = oy ? 2 : 3, kz = oz ? 4 : 5;  // the faces this child shares with the coarse cell
+        if (FINE) {
+            const uint16_t c = F.code[fi];
+            if (!(c & CODE_FLUID)) continue;
+            face[kx] += 4 * ((c >> kx) & 1);
+            face[ky] += 4 * ((c >> ky) & 1);
+            face[kz] += 4 * ((c >> kz) & 1);
+            dir += 8 * (code_ns(c) - code_nf(c));
+        } else {
+            const uint32_t c = F.ccode[fi];
+            face[kx] += (int)((c >> (3 * kx)) & 7u);
+            face[ky] += (int)((c >> (3 * ky)) & 7u);
+            face[kz] += (int)((c >> (3 * kz)) & 7u);
+            dir += (int)((c >> CC_DIRICHLET) & 31u);
+        }
     }
-    uint16_t cd = CODE_FLUID;
-    int ns = 0;
-    const int pos[3] = {x, y, z}, lim[3] = {L.nx, L.ny, L.nz};
+    uint32_t cc = 0;
 #pragma unroll
     for (int k = 0; k < 6; k++) {
-        const int a = k >> 1, dir = (k & 1) ? -1 : 1;
-        const int q = pos[a] + dir;
-        if (q < 0 || q >= lim[a]) continue;
-        const uint8_t kn = kind[ci + mg_off(L, k)];
-        if (kn == 0) cd |= (uint16_t)(1u << k);
-        if (kn != 2) ns++;
+        int w = (face[k] + 2) >> 2;  // mean of four faces in quarters
+        if (face[k] > 0 && w == 0) w = 1;
+        cc |= (uint32_t)w << (3 * k);
     }
-    code[ci] = cd | (uint16_t)(ns << 8);
+    cc |= (uint32_t)min((dir + 1) >> 1, DIRICHLET_MAX) << CC_DIRICHLET;
+    code[ci] = cc;
+}
+
+// interpolation scale of a level's fluid cells from the next level's kinds
+// (outside the level = solid)
+template <bool FINE>
+__global__ void k_mg_pscale(MGLev F, MGLev Cl, const uint8_t* ckind, uint16_t* code, uint32_t* ccode) {
+    const long long n = (long long)F.nx * F.ny * F.nz;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const unsigned iu = (unsigned)i, t = iu / (unsigned)F.nz, u = t / (unsigned)F.ny;
+    const int z = (int)(iu - t * (unsigned)F.nz), y = (int)(t - u * (unsigned)F.ny), x = (int)u;
+    const long long fi = ((long long)x * F.ny + y) * F.pz + z;
+    if (FINE ? !is_fluid(code[fi]) : !is_fluid(ccode[fi])) return;
+    const int px = (x >> 1) - 1 + (x & 1), py = (y >> 1) - 1 + (y & 1), pz = (z >> 1) - 1 + (z & 1);
+    int k = 0;
+#pragma unroll
+    for (int o = 0; o < 8; o++) {
+        const int ox = o >> 2, oy = (o >> 1) & 1, oz = o & 1;
+        const int cx = px + ox, cy = py + oy, cz = pz + oz;
+        if (cx < 0 || cy < 0 || cz < 0 || cx >= Cl.nx || cy >= Cl.ny || cz >= Cl.nz) continue;
+        if (ckind[((long long)cx * Cl.ny + cy) * Cl.pz + cz] == 2) continue;
+        // the lower neighbour weighs 3 (of 4) for odd cells, 1 for even ones
+        k += ((x & 1) != ox ? 3 : 1) * ((y & 1) != oy ? 3 : 1) * ((z & 1) != oz ? 3 : 1);
+    }
+    const unsigned s = (unsigned)(64 - k) & 63u;
+    if (!s) return;
+    if (FINE) code[fi] = (uint16_t)(code[fi] | ((s & 3u) << 6) | ((s & 0x3Cu) << 9));
+    else ccode[fi] |= s << CC_SCALE;
 }
 
 // phi += x; x = 0   (fold the FP32 accumulator into the FP64 solution)
@@ -1767,6 +1885,9 @@ int solver_alloc(fsim_ctx* ctx) {
     float rcp[7];
     for (int ns = 0; ns < 7; ns++) rcp[ns] = ns > 0 ? 1.f / ns : 1.f;
     FSIM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_rcp, rcp, sizeof(rcp)));
+    float psc[64];
+    for (int i = 0; i < 64; i++) psc[i] = 64.f / (64 - i);
+    FSIM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_pscale, psc, sizeof(psc)));
     // multigrid hierarchy: halve until every dimension is <= 4
     MGLevelBufs l0;
     l0.nx = g.nx; l0.ny = g.ny; l0.nz = g.nz; l0.pz = g.pz; l0.ncell = g.ncell;
@@ -1780,14 +1901,14 @@ int solver_alloc(fsim_ctx* ctx) {
         c.nx = (f.nx + 1) / 2; c.ny = (f.ny + 1) / 2; c.nz = (f.nz + 1) / 2; c.pz = (c.nz + 3) & ~3;
         c.ncell = (long long)c.nx * c.ny * c.pz;
         FSIM_CUDA_TRY(ctx, cudaMalloc(&c.kind, c.ncell));
-        FSIM_CUDA_TRY(ctx, cudaMalloc(&c.code, c.ncell * sizeof(uint16_t)));
+        FSIM_CUDA_TRY(ctx, cudaMalloc(&c.ccode, c.ncell * sizeof(uint32_t)));
         FSIM_CUDA_TRY(ctx, cudaMalloc(&c.x, c.ncell * sizeof(float)));
         FSIM_CUDA_TRY(ctx, cudaMalloc(&c.f, c.ncell * sizeof(float)));
         FSIM_CUDA_TRY(ctx, cudaMalloc(&c.r, c.ncell * sizeof(float)));
         FSIM_CUDA_TRY(ctx, cudaMemset(c.x, 0, c.ncell * sizeof(float)));
         FSIM_CUDA_TRY(ctx, cudaMemset(c.f, 0, c.ncell * sizeof(float)));
         FSIM_CUDA_TRY(ctx, cudaMemset(c.r, 0, c.ncell * sizeof(float)));
-        FSIM_CUDA_TRY(ctx, cudaMemset(c.code, 0, c.ncell * sizeof(uint16_t)));
+        FSIM_CUDA_TRY(ctx, cudaMemset(c.ccode, 0, c.ncell * sizeof(uint32_t)));
         FSIM_CUDA_TRY(ctx, cudaMemset(c.kind, 2, c.ncell));
         S.mg.push_back(c);
     }
@@ -1830,6 +1951,7 @@ static MGLev mg_lev(const SolverBufs& S, int l, const float* f0, const float* f1
     MGLev L;
     L.nx = b.nx; L.ny = b.ny; L.nz = b.nz; L.pz = b.pz;
     L.code = b.code;
+    L.ccode = b.ccode;
     L.r = b.r;
     if (l == 0) {
         L.x = x0; L.f = f0; L.f1 = f1;
@@ -1849,16 +1971,21 @@ static void mg_setup(fsim_ctx* ctx) {
         const long long n = S.mg[l].ncell;
         k_mg_coarsen<<<ceil_div(n, 256), 256, 0, st>>>(F, l == 1 ? nullptr : S.mg[l - 1].kind, ctx->flags, Cl,
                                                        S.mg[l].kind);
-        k_mg_code<<<ceil_div(n, 256), 256, 0, st>>>(Cl, S.mg[l].kind, S.mg[l].code);
-        ctx->launches += 2;
+        const long long nf = S.mg[l - 1].ncell;
+        if (l == 1) {
+            k_mg_code<true><<<ceil_div(n, 256), 256, 0, st>>>(F, Cl, S.mg[l].ccode);
+            k_mg_pscale<true><<<ceil_div(nf, 256), 256, 0, st>>>(F, Cl, S.mg[l].kind, S.code, nullptr);
+        } else {
+            k_mg_code<false><<<ceil_div(n, 256), 256, 0, st>>>(F, Cl, S.mg[l].ccode);
+            k_mg_pscale<false><<<ceil_div(nf, 256), 256, 0, st>>>(F, Cl, S.mg[l].kind, nullptr, S.mg[l - 1].ccode);
+        }
+        ctx->launches += 3;
     }
 }
 
-// free-surface band sweeps on level l (only the finest level has a band)
-static int mg_band_sweeps(const SolverBufs& S, const fsim_params& P, int l) {
-    if (l != 0 || P.mg_boundary_sweeps < 0) return 0;
-    if (P.mg_boundary_sweeps > 0) return P.mg_boundary_sweeps;
-    return S.mg[0].ncell >= MG_BAND_MIN_CELLS ? MG_NB_DEFAULT_BIG : 0;
+// free-surface band sweeps on level l (only the finest level has a band; none unless asked for)
+static int mg_band_sweeps(const fsim_params& P, int l) {
+    return l == 0 && P.mg_boundary_sweeps > 0 ? P.mg_boundary_sweeps : 0;
 }
 
 // z = V-cycle(r); r is the current PCG residual (r0 or r1 by device state).
@@ -1867,11 +1994,9 @@ static int mg_band_sweeps(const SolverBufs& S, const fsim_params& P, int l) {
 static void mg_vcycle(fsim_ctx* ctx, const PcgArgs& A, int l, const float* r0, const float* r1, float* z,
                       bool first_fused, int dot_mode) {
     const fsim_params& P = ctx->prm;
-    const bool big = ctx->sv.mg[0].ncell >= MG_BAND_MIN_CELLS;
-    const int NU0 = P.mg_sweeps > 0 ? P.mg_sweeps : (big ? MG_NU_DEFAULT_BIG : MG_NU_DEFAULT);
-    const int NU1 = P.mg_coarse_sweeps > 0 ? P.mg_coarse_sweeps : MG_NU_COARSE_DEFAULT;
-    const int NUC = P.mg_cluster_sweeps > 0 ? P.mg_cluster_sweeps : MG_NU_CLUSTER_DEFAULT;
-    const int NU = l == 0 ? NU0 : (P.mg_coarse_sweeps > 0 ? NU1 : (l == 1 ? MG_NU_L1_DEFAULT : NU1));
+    const int NU = l == 0 ? (P.mg_sweeps > 0 ? P.mg_sweeps : MG_NU_DEFAULT)
+                          : (P.mg_coarse_sweeps > 0 ? P.mg_coarse_sweeps : MG_NU_COARSE_DEFAULT);
+    const int NUC = P.mg_cluster_sweeps > 0 ? P.mg_cluster_sweeps : MG_NU_COARSE_DEFAULT;
     SolverBufs& S = ctx->sv;
     cudaStream_t st = ctx->stream;
     const int G = S.grid_blocks;
@@ -1888,7 +2013,6 @@ static void mg_vcycle(fsim_ctx* ctx, const PcgArgs& A, int l, const float* r0, c
         C.lc = 0;
         C.last = last - l;
         C.nu = NUC;
-        C.nu_small = P.mg_cluster_sweeps > 0 ? NUC : MG_NU_SMALL_DEFAULT;
         // the levels from ls on run in shared memory (x, f, r floats + codes per cell)
         C.ls = C.last;
         size_t smem = 0;
@@ -1901,7 +2025,7 @@ static void mg_vcycle(fsim_ctx* ctx, const PcgArgs& A, int l, const float* r0, c
         for (int k = C.ls; k <= C.last; k++) {
             const MGLevelBufs& b = S.mg[l + k];
             const long long n = (long long)b.nx * b.ny * b.nz;
-            smem += (size_t)(3 * n + (n + 1) / 2) * sizeof(float);
+            smem += (size_t)(4 * n) * sizeof(float);
         }
         // levels lc .. ls-1 as x slabs in the cluster's distributed shared memory
         // when they fit beside rank 0's levels (else they run in global memory)
@@ -1912,7 +2036,7 @@ static void mg_vcycle(fsim_ctx* ctx, const PcgArgs& A, int l, const float* r0, c
             const long long m = (long long)P * b.ny * b.nz;
             C.P[k] = P;
             C.off[k] = (int)slab_floats;
-            slab_floats += (size_t)((3 * m + (m + 1) / 2 + 3) & ~3ll);
+            slab_floats += (size_t)((4 * m + 3) & ~3ll);
         }
         C.soff = (int)slab_floats;
         const size_t slab_bytes = slab_floats * sizeof(float) + smem;
@@ -1946,7 +2070,7 @@ static void mg_vcycle(fsim_ctx* ctx, const PcgArgs& A, int l, const float* r0, c
         smooth(1, 0);
         ctx->launches += 2;
     }
-    const int NB = mg_band_sweeps(S, P, l);
+    const int NB = mg_band_sweeps(P, l);
     auto smooth_band = [&](int color) {
         launch_pdl(k_mg_smooth_bnd, G, PCG_THREADS, st, A, L, (const int4*)S.bnd_quads, (const int*)S.d_nbnd, color);
         ctx->launches += 1;
@@ -1959,7 +2083,8 @@ static void mg_vcycle(fsim_ctx* ctx, const PcgArgs& A, int l, const float* r0, c
     else launch_pdl(k_mg_residual<false>, nb, PCG_THREADS, st, A, L);
     MGLev Cl = mg_lev(S, l + 1, nullptr, nullptr, nullptr);
     const int nbc = std::min(G, ceil_div(S.mg[l + 1].ncell, 256));
-    launch_pdl(k_mg_restrict, nbc, PCG_THREADS, st, A.st, L, Cl);
+    if (l == 0) launch_pdl(k_mg_restrict<true>, nbc, PCG_THREADS, st, A.st, L, Cl);
+    else launch_pdl(k_mg_restrict<false>, nbc, PCG_THREADS, st, A.st, L, Cl);
     mg_vcycle(ctx, A, l + 1, nullptr, nullptr, nullptr, false, -1);
     if (l == 0) launch_pdl(k_mg_prolong<true>, nb, PCG_THREADS, st, A, L, Cl);
     else launch_pdl(k_mg_prolong<false>, nb, PCG_THREADS, st, A, L, Cl);
@@ -2002,7 +2127,7 @@ void solver_free(fsim_ctx* ctx) {
     for (size_t l = 0; l < S.mg.size(); l++) {
         cudaFree(S.mg[l].r);
         if (l > 0) {
-            cudaFree(S.mg[l].kind); cudaFree(S.mg[l].code); cudaFree(S.mg[l].x); cudaFree(S.mg[l].f);
+            cudaFree(S.mg[l].kind); cudaFree(S.mg[l].ccode); cudaFree(S.mg[l].x); cudaFree(S.mg[l].f);
         }
     }
     S = SolverBufs{};
@@ -2109,7 +2234,7 @@ static int run_pcg(fsim_ctx* ctx, PcgArgs& A, Vecs<T> v, int precision, int prec
         }
     };
     if (mg) mg_setup(ctx);
-    if (mg && mg_band_sweeps(S, ctx->prm, 0) > 0) {
+    if (mg && mg_band_sweeps(ctx->prm, 0) > 0) {
         if (!S.bnd_quads) {
             FSIM_CUDA_TRY(ctx, cudaMalloc(&S.bnd_quads, (size_t)(ctx->g.ncell / 4 + 1) * sizeof(int4)));
             FSIM_CUDA_TRY(ctx, cudaMalloc(&S.d_nbnd, sizeof(int)));
