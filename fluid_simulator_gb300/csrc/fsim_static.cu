@@ -60,6 +60,9 @@ cudaError_t scratch_address(unsigned char** out) {
         void* p = nullptr;
         e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
         if (e != cudaSuccess) return e;
+        // every P2G tile variant now: a later call with another grid size must
+        // not be the one that loads its kernel
+        if ((e = p2g_load_all()) != cudaSuccess) return e;
         g_scratch_addr[dev] = static_cast<unsigned char*>(p);
     }
     *out = g_scratch_addr[dev];

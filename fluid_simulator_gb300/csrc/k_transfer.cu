@@ -61,7 +61,8 @@ struct P2GShape {
     static constexpr int SMEM = 7 * PCELLS * (int)sizeof(float);
     static constexpr int NTHREADS = THREADS, MIN_BLOCKS = MINB;
 };
-// the default: 8x16x16 tiles (57,344 B), three warp quads per CTA, two CTAs per SM
+// the default on large grids: 8x16x16 tiles (57,344 B), three warp quads per CTA, two
+// CTAs per SM; smaller tiles on smaller grids (p2g_fast)
 using P2GFast = P2GShape<8, 16, 16, 384, 2>;
 // bit-reproducible (fsim_params.deterministic): one warp quad per CTA, so each
 // shared accumulator is added to by a single warp in program order (a warp's
@@ -537,7 +538,52 @@ cudaError_t launch_p2g_shape(P2GArgs a, bool apic, cudaStream_t stream) {
         k_p2g<false, S><<<nb, S::NTHREADS, S::SMEM, stream>>>(a);
     return cudaGetLastError();
 }
+
+template <class S>
+long long p2g_tiles(const GridGeom& g) {
+    return (long long)ceil_div(g.nx, S::PX) * ceil_div(g.ny, S::PY) * ceil_div(g.nz, S::PZ);
+}
+
+// The largest tile that still gives P2G_MIN_TILES CTAs (about three per SM; part of
+// them hold no fluid).  A warp quad walks its tile's cell blocks one after the
+// other, 35 blocks for 8x16x16 tiles, so a grid of few large tiles takes as long
+// as one tile does: 16 CTAs and 167 us at 32^3.  Smaller tiles read more halo
+// cells (1.6 times the cells at 8x16x16, 2.0 at 8x8x8, 3.4 at 4x4x4), which costs
+// more than it gives once every SM is busy.  Sort + P2G in us, by tile 4x4x4 /
+// 4x4x8 / 4x8x8 / 8x8x16 / 8x16x16: 32^3 dam 64 / 69 / 83 / 140 / 210, 48^3 dam
+// 90 / 83 / 98 / 168 / 249, 64^3 dam 145 / 120 / 109 / 169 / 260, 90x61x75 half
+// filled 294 / 244 / 220 / 198 / 288, 96^3 dam 408 / 317 / 263 / 245 / 362, 128^3
+// dam 941 / 707 / 571 / 467 / 445.
+constexpr long long P2G_MIN_TILES = 480;
+using T1 = P2GShape<8, 8, 16, 384, 2>;
+using T2 = P2GShape<4, 8, 8, 384, 2>;
+using T3 = P2GShape<4, 4, 8, 384, 2>;
+using T4 = P2GShape<4, 4, 4, 384, 2>;
+cudaError_t p2g_fast(const P2GArgs& a, bool apic, cudaStream_t stream) {
+    if (p2g_tiles<P2GFast>(a.g) >= P2G_MIN_TILES) return launch_p2g_shape<P2GFast>(a, apic, stream);
+    if (p2g_tiles<T1>(a.g) >= P2G_MIN_TILES) return launch_p2g_shape<T1>(a, apic, stream);
+    if (p2g_tiles<T2>(a.g) >= P2G_MIN_TILES) return launch_p2g_shape<T2>(a, apic, stream);
+    if (p2g_tiles<T3>(a.g) >= P2G_MIN_TILES) return launch_p2g_shape<T3>(a, apic, stream);
+    return launch_p2g_shape<T4>(a, apic, stream);
+}
+
+template <class S>
+cudaError_t p2g_load_shape() {
+    cudaError_t e = set_smem_limit((const void*)k_p2g<true, S>, S::SMEM);
+    return e != cudaSuccess ? e : set_smem_limit((const void*)k_p2g<false, S>, S::SMEM);
+}
 }  // namespace
+
+// loads every tile variant on the current device (set-up calls of callers that
+// may not trigger a lazy module load later)
+cudaError_t p2g_load_all() {
+    cudaError_t e = p2g_load_shape<P2GFast>();
+    if (e == cudaSuccess) e = p2g_load_shape<T1>();
+    if (e == cudaSuccess) e = p2g_load_shape<T2>();
+    if (e == cudaSuccess) e = p2g_load_shape<T3>();
+    if (e == cudaSuccess) e = p2g_load_shape<T4>();
+    return e;
+}
 
 void launch_p2g(fsim_ctx* ctx) {
     P2GArgs a;
@@ -551,7 +597,7 @@ void launch_p2g(fsim_ctx* ctx) {
     ctx->launches += 1;
     const bool apic = ctx->prm.transfer == FSIM_APIC;
     if (ctx->prm.deterministic) launch_p2g_shape<P2GDet>(a, apic, ctx->stream);
-    else launch_p2g_shape<P2GFast>(a, apic, ctx->stream);
+    else p2g_fast(a, apic, ctx->stream);
 }
 
 // P2G on caller-provided buffers (used by the allocation-free entry point in
@@ -566,7 +612,7 @@ cudaError_t launch_p2g_raw(ParticleBuf p, const uint32_t* perm, const int* cstar
     for (int k = 0; k < 3; k++) a.u[k] = u[k];
     a.flags = flags;
     a.avg = avg;
-    return launch_p2g_shape<P2GFast>(a, apic, stream);
+    return p2g_fast(a, apic, stream);
 }
 
 // TMA descriptors of the six face arrays (v2 x/y/z, v x/y/z): 3D tensors

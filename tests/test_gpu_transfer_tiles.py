@@ -1,0 +1,86 @@
+"""P2G and G2P over the grid sizes at which their tile shapes change, against a
+plain FP64 restatement in numpy: ragged boxes (no axis a multiple of a tile),
+grids just below and above each change, sparse particles (empty tiles) and
+crowded cells.  h is a power of two, so pos / h is exact in FP32 and the
+tolerances are those of the parity tests."""
+import numpy as np
+import pytest
+
+from fluid_simulator_gb300 import native as N
+
+from parity_util import REL_GRID, assert_close_field
+
+pytestmark = pytest.mark.gpu
+
+RES = 128
+
+
+def particles(shape, n, seed):
+    """n particles: most spread over the lower 60 % of the box, some crowded into one cell."""
+    rng = np.random.default_rng(seed)
+    lo, hi = np.full(3, 1.3), np.array(shape) - 1.3
+    pos = lo + rng.random((n, 3)) * (hi - lo) * [1.0, 0.6, 1.0]
+    pos[: n // 50] = np.array(shape) // 2 + rng.random((n // 50, 3)) * 0.99
+    pos = (pos / RES).astype(np.float32)
+    vel = (rng.standard_normal((n, 3))).astype(np.float32)
+    c = (rng.standard_normal((n, 9)) * 20).astype(np.float32)
+    return pos, vel, c
+
+
+def p2g_ref(shape, pos, vel, c):
+    """(u[3], weights[3], avgPNum): trilinear scatter in FP64."""
+    h = 1.0 / RES
+    p, g = pos.astype(np.float64), pos.astype(np.float64) * RES
+    out, wts = [], []
+    for a in range(4):
+        off = np.array([0.0 if d == a else 0.5 for d in range(3)])
+        base = np.floor(g - off)
+        f = g - off - base
+        num, den = np.zeros(shape), np.zeros(shape)
+        for o in range(8):
+            b = np.array([(o >> 2) & 1, (o >> 1) & 1, o & 1])
+            w = np.where(b, f, 1.0 - f).prod(1)
+            at = (base + b).astype(np.int64) - np.array([1 if d == a else 0 for d in range(3)])
+            ok = ((at >= 0) & (at < shape)).all(1)
+            idx = tuple(at[ok].T)
+            np.add.at(den, idx, w[ok])
+            if a < 3:
+                val = vel[:, a].astype(np.float64)
+                if c is not None:
+                    val = val + (c[:, 3 * a:3 * a + 3] * ((base + b + off) * h - p)).sum(1)
+                np.add.at(num, idx, (w * val)[ok])
+        if a == 3:
+            return out, wts, den
+        out.append(np.where(den > 1e-6, num / np.maximum(den, 1e-300), 0.0))
+        wts.append(den)
+
+
+# CTAs of 8x16x16 tiles below and above the change: 23x29x30 and 37x21x44 run 4x4x4 tiles,
+# 48^3 4x4x8, 64^3 and 66x70x50 4x8x8, 90x61x75 8x8x16, 128x112x128 (448) 8x8x16,
+# 128x128x120 (512) 8x16x16
+SHAPES = [(7, 9, 5), (23, 29, 30), (37, 21, 44), (48, 48, 48), (66, 70, 50), (90, 61, 75), (128, 112, 128),
+          (128, 128, 120)]
+
+
+@pytest.mark.parametrize("transfer", [N.FLIP, N.APIC])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_p2g_matches_fp64_at_every_tile_shape(gpu, shape, transfer):
+    n = min(120_000, 8 * int(np.prod(np.array(shape) - 2)))
+    pos, vel, c = particles(shape, n, sum(shape))
+    prm = N.default_params(transfer=transfer, resolution=RES)
+    sim = N.Simulation(RES, prm, dims=[(k + 0.01) / RES for k in shape])
+    assert sim.shape == shape
+    sim.set_particles(pos, vel, c)
+    sim.stage(N.STAGE_P2G, 0.01)
+    ref, wts, avg = p2g_ref(shape, pos, vel, c if transfer == N.APIC else None)
+    for a, f in enumerate((N.F_VX, N.F_VY, N.F_VZ)):
+        # a face whose weight sum is within FP32 rounding of the 1e-6 threshold may go either way
+        near = np.abs(wts[a] - 1e-6) < 1e-9
+        assert_close_field(np.where(near, 0, sim.grid(f)), np.where(near, 0, ref[a]), REL_GRID, f"u{a}")
+    assert_close_field(sim.grid(N.F_AVGPNUM), avg, REL_GRID, "avgPNum")
+    cells = np.floor(pos.astype(np.float64) * RES).astype(np.int64)
+    count = np.zeros(shape, np.int64)
+    np.add.at(count, tuple(cells.T), 1)
+    assert np.array_equal(sim.grid(N.F_COUNT), count)
+    assert np.array_equal(sim.grid(N.F_FLAGS) == N.WATER, count > 0)
+    sim.close()
