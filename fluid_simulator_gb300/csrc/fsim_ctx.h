@@ -132,8 +132,9 @@ struct fsim_ctx {
     int* disc_cells_dev = nullptr;
     long long disc_cells_cap = 0;
 
-    // TMA descriptors for the G2P tile loads (v2 x/y/z, v x/y/z)
-    CUtensorMap tmap[6];
+    // TMA descriptors for the G2P tile loads: v2 x/y/z and v x/y/z with the FLIP
+    // tile's box, v2 x/y/z with the PIC / APIC tile's
+    CUtensorMap tmap[9];
     bool tmap_ok = false;
 
     // device error word + pinned mirrors

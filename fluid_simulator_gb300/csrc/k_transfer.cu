@@ -1,7 +1,7 @@
 // k_transfer.cu -- particle <-> grid transfers on cell-sorted particles.
 //
-// Both kernels work on tiles of cells (one CTA per tile): P2G on PX x PY x PZ,
-// G2P on TX x TY x TZ.
+// Both kernels work on tiles of cells (one CTA per tile), whose shape depends on
+// the grid size (p2g_fast, g2p_pick).
 //
 // P2G (Simulator::p2gTransfer, simulator.cpp:314-352, fused with
 // markFluidCellsAndCalculateParticleDensities, simulator.cpp:354-368): the CTA
@@ -28,11 +28,14 @@
 
 namespace {
 
-constexpr int TX = 8, TY = 8, TZ = 32;
-
-// G2P staged box: x in [x0-1, x0+TX], y in [y0-1, y0+TY], z in [z0-4, z0+TZ+4)
-constexpr int BX = TX + 2, BY = TY + 2, BZ = TZ + 8;
-constexpr int BOXN = BX * BY * BZ;
+// G2P tile and its staged box: x in [x0-1, x0+TX], y in [y0-1, y0+TY],
+// z in [z0-4, z0+TZ+4) (16-byte aligned start)
+template <int X, int Y, int Z>
+struct G2PShape {
+    static constexpr int TX = X, TY = Y, TZ = Z, BX = X + 2, BY = Y + 2, BZ = Z + 8;
+    static constexpr int BOXN = BX * BY * BZ;
+    static constexpr int ROWS = X * Y;
+};
 constexpr int G2P_THREADS = 256;
 
 struct P2GArgs {
@@ -292,19 +295,21 @@ struct G2PArgs {
 };
 
 // MODE: 0 PIC, 1 FLIP, 2 APIC
-template <int MODE>
+template <int MODE, class S>
 __global__ void __launch_bounds__(G2P_THREADS) k_g2p(const G2PArgs a, const __grid_constant__ CUtensorMap m0,
                                                      const __grid_constant__ CUtensorMap m1,
                                                      const __grid_constant__ CUtensorMap m2,
                                                      const __grid_constant__ CUtensorMap m3,
                                                      const __grid_constant__ CUtensorMap m4,
                                                      const __grid_constant__ CUtensorMap m5) {
+    constexpr int TX = S::TX, TY = S::TY, TZ = S::TZ, BY = S::BY, BZ = S::BZ, BOXN = S::BOXN, ROWS = S::ROWS;
+    static_assert(ROWS == 16 || ROWS == 32 || ROWS == 64, "a row per lane of one or two warps");
     extern __shared__ __align__(128) unsigned char smraw[];
     float* sv2 = reinterpret_cast<float*>(smraw);  // [3][BOXN]
     float* su = sv2 + 3 * BOXN;                    // [3][BOXN] (FLIP)
     __shared__ __align__(8) uint64_t mbar;
-    __shared__ int seg_beg[TX * TY];
-    __shared__ int seg_pre[TX * TY + 1];
+    __shared__ int seg_beg[64];
+    __shared__ int seg_pre[65];
 
     const int bt = blockIdx.x;
     const int tz = bt % a.ntz, ty = (bt / a.ntz) % a.nty, tx = bt / (a.ntz * a.nty);
@@ -331,7 +336,7 @@ __global__ void __launch_bounds__(G2P_THREADS) k_g2p(const G2PArgs a, const __gr
         const int r = threadIdx.x;
         const int x = x0 + r / TY, y = y0 + r % TY;
         int beg = 0, len = 0;
-        if (x < a.g.nx && y < a.g.ny) {
+        if (r < ROWS && x < a.g.nx && y < a.g.ny) {
             const long long base = gidx(a.g, x, y, 0);
             const int ze = min(z0 + TZ, a.g.pz);
             beg = a.cstart[base + z0];
@@ -351,13 +356,13 @@ __global__ void __launch_bounds__(G2P_THREADS) k_g2p(const G2PArgs a, const __gr
     __syncthreads();
     if (threadIdx.x >= 32 && threadIdx.x < 64) seg_pre[threadIdx.x + 1] += seg_pre[32];
     __syncthreads();
-    const int total = seg_pre[TX * TY];
+    const int total = seg_pre[64];  // rows past ROWS are empty
     // sorted slot of the tile's j-th particle: its row by binary search for a
     // thread's first particle, then by stepping forward from the previous row
     // (a thread's particles come in increasing j, a row is ~TZ*8 particles)
     int row = 0;
     auto slot_of = [&](int j) {
-        int lo = 0, hi = TX * TY - 1;
+        int lo = 0, hi = ROWS - 1;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
             if (seg_pre[mid] <= j) lo = mid; else hi = mid - 1;
@@ -366,17 +371,23 @@ __global__ void __launch_bounds__(G2P_THREADS) k_g2p(const G2PArgs a, const __gr
         return seg_beg[lo] + (j - seg_pre[lo]);
     };
     auto slot_next = [&](int j) {
-        while (row + 1 < TX * TY && seg_pre[row + 1] <= j) row++;
+        while (row + 1 < ROWS && seg_pre[row + 1] <= j) row++;
         return seg_beg[row] + (j - seg_pre[row]);
     };
-    // software pipeline: each thread's next particle (slot, index, position) is
-    // loaded one iteration ahead; the first one while the grid tile is in flight
-    int kn = 0;
-    uint32_t in = 0;
+    // software pipeline: a thread's next position and the index of the particle
+    // after it are loaded one iteration ahead (the index two ahead, so that no
+    // position load waits for its index); the first ones while the tile is in flight
+    const int step = (int)blockDim.x;
+    int kn = 0, kn2 = 0;
+    uint32_t in = 0, in2 = 0;
     float pn[3] = {0.f, 0.f, 0.f};
     if ((int)threadIdx.x < total) {
         kn = slot_of(threadIdx.x);
         in = a.perm[kn];
+        if ((int)threadIdx.x + step < total) {
+            kn2 = slot_next(threadIdx.x + step);
+            in2 = a.perm[kn2];
+        }
         pn[0] = a.src.p[0][in]; pn[1] = a.src.p[1][in]; pn[2] = a.src.p[2][in];
     }
     // wait for the staged grid (bounded: about 2^31 cycles, then report and leave;
@@ -400,15 +411,33 @@ __global__ void __launch_bounds__(G2P_THREADS) k_g2p(const G2PArgs a, const __gr
         }
     }
     const float hinv = a.g.hinv, hzinv = a.g.hzinv;
-    for (int j = threadIdx.x; j < total; j += blockDim.x) {
+    for (int j = threadIdx.x; j < total; j += step) {
         const int k = kn;
         const uint32_t i = in;
         const float px = pn[0], py = pn[1], pz = pn[2];
-        if (j + (int)blockDim.x < total) {
-            kn = slot_next(j + blockDim.x);
-            in = a.perm[kn];
+        if (j + step < total) {
+            kn = kn2;
+            in = in2;
             pn[0] = a.src.p[0][in]; pn[1] = a.src.p[1][in]; pn[2] = a.src.p[2][in];
+            if (j + 2 * step < total) {
+                kn2 = slot_next(j + 2 * step);
+                in2 = a.perm[kn2];
+            }
         }
+        // what this particle only carries along is loaded before any of its stores: the
+        // compiler must assume that a store may change a later load's source
+        float vold[3], cold[9];
+        if (MODE == 1) {
+#pragma unroll
+            for (int ax = 0; ax < 3; ax++) vold[ax] = a.src.v[ax][i];
+        }
+        if (MODE != 2) {
+            if (a.move_c) {
+#pragma unroll
+                for (int q = 0; q < 9; q++) cold[q] = a.src.c[q][i];
+            }
+        }
+        const uint32_t id = a.ids ? a.src.id[i] : 0u;
         const float g[3] = {px * hinv, py * hinv, pz * hzinv};
         float vnew[3];
         float cnew[9];
@@ -489,7 +518,7 @@ __global__ void __launch_bounds__(G2P_THREADS) k_g2p(const G2PArgs a, const __gr
                 c2 = w1[0][0] * Q[0] + w1[0][1] * Q[1];
             }
             if (MODE == 0) vnew[ax] = pic;
-            if (MODE == 1) vnew[ax] = pic * a.pic_w + (flip + a.src.v[ax][i]) * a.fr;
+            if (MODE == 1) vnew[ax] = pic * a.pic_w + (flip + vold[ax]) * a.fr;
             if (MODE == 2) {
                 vnew[ax] = pic;
                 cnew[3 * ax] = c0;
@@ -515,9 +544,9 @@ __global__ void __launch_bounds__(G2P_THREADS) k_g2p(const G2PArgs a, const __gr
             for (int q = 0; q < 9; q++) a.dst.c[q][k] = cnew[q];
         } else if (a.move_c) {
 #pragma unroll
-            for (int q = 0; q < 9; q++) a.dst.c[q][k] = a.src.c[q][i];
+            for (int q = 0; q < 9; q++) a.dst.c[q][k] = cold[q];
         }
-        if (a.ids) a.dst.id[k] = a.src.id[i];
+        if (a.ids) a.dst.id[k] = id;
     }
 }
 
@@ -615,6 +644,48 @@ cudaError_t launch_p2g_raw(ParticleBuf p, const uint32_t* perm, const int* cstar
     return p2g_fast(a, apic, stream);
 }
 
+namespace {
+using G2PBig = G2PShape<8, 8, 32>;
+using G2PMid = G2PShape<4, 8, 16>;
+using G2PSmall = G2PShape<4, 4, 8>;
+template <class S>
+long long g2p_tiles(const GridGeom& g) {
+    return (long long)ceil_div(g.nx, S::TX) * ceil_div(g.ny, S::TY) * ceil_div(g.nz, S::TZ);
+}
+
+// Tile by grid size (0 big, 1 mid, 2 small).  A CTA works through its tile's
+// particles 256 at a time, 64 rounds for a full 8x8x32 tile, so few large tiles
+// leave SMs idle and a small tile re-stages more halo.  FLIP stages six boxes (96
+// KB at 8x8x32, two CTAs per SM) and stays with the mid tile.  G2P call in us
+// (with its host synchronisation), big / mid / small: 32^3 dam FLIP 71 / 42 / 33,
+// 64^3 dam APIC 74 / 43 / 40, 90x61x75 half filled FLIP 119 / 68 / 76, 128^3 dam
+// APIC 102 / 95 / 145, 128^3 half filled FLIP 251 / 199 / 258, 256^3 dam APIC
+// 478 / 582 / 1009, 256^3 dam FLIP 866 / 750 / 1254.
+constexpr long long G2P_MIN_MID = 480, G2P_MIN_BIG = 4096;
+int g2p_pick(const GridGeom& g, bool flip) {
+    if (g2p_tiles<G2PMid>(g) < G2P_MIN_MID) return 2;
+    return flip || g2p_tiles<G2PBig>(g) < G2P_MIN_BIG ? 1 : 0;
+}
+
+template <class S>
+void launch_g2p_shape(G2PArgs a, int mode, const CUtensorMap* m, cudaStream_t stream) {
+    a.ntx = ceil_div(a.g.nx, S::TX);
+    a.nty = ceil_div(a.g.ny, S::TY);
+    a.ntz = ceil_div(a.g.nz, S::TZ);
+    const int nb = a.ntx * a.nty * a.ntz;
+    const int smem = ((mode == FSIM_FLIP) ? 6 : 3) * S::BOXN * (int)sizeof(float);
+    auto go = [&](auto kern) {
+        set_smem_limit((const void*)kern, smem);
+        // PIC and APIC read the first three boxes only
+        const int o = mode == FSIM_FLIP ? 3 : 0;
+        kern<<<nb, G2P_THREADS, smem, stream>>>(a, m[0], m[1], m[2], m[o], m[o + 1], m[o + 2]);
+    };
+    if (mode == FSIM_PIC) go(k_g2p<0, S>);
+    else if (mode == FSIM_FLIP) go(k_g2p<1, S>);
+    else go(k_g2p<2, S>);
+}
+}  // namespace
+
 // TMA descriptors of the six face arrays (v2 x/y/z, v x/y/z): 3D tensors
 // (z innermost, padded pitch pz), box BZ x BY x BX floats, zero fill outside.
 bool make_tensor_maps(fsim_ctx* ctx) {
@@ -629,12 +700,15 @@ bool make_tensor_maps(fsim_ctx* ctx) {
     const GridGeom& g = ctx->g;
     cuuint64_t dims[3] = {(cuuint64_t)g.pz, (cuuint64_t)g.ny, (cuuint64_t)g.nx};
     cuuint64_t strides[2] = {(cuuint64_t)g.pz * 4, (cuuint64_t)g.pz * g.ny * 4};
-    cuuint32_t box[3] = {BZ, BY, BX};
+    const cuuint32_t boxes[3][3] = {{G2PBig::BZ, G2PBig::BY, G2PBig::BX},
+                                    {G2PMid::BZ, G2PMid::BY, G2PMid::BX},
+                                    {G2PSmall::BZ, G2PSmall::BY, G2PSmall::BX}};
     cuuint32_t estr[3] = {1, 1, 1};
     float* arrays[6] = {ctx->v2[0], ctx->v2[1], ctx->v2[2], ctx->u[0], ctx->u[1], ctx->u[2]};
-    for (int k = 0; k < 6; k++) {
-        CUresult r = encode(&ctx->tmap[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, arrays[k], dims, strides,
-                            box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+    for (int k = 0; k < 9; k++) {
+        // 0-5: the FLIP tile's boxes (v2, v), 6-8: the PIC / APIC tile's (v2)
+        CUresult r = encode(&ctx->tmap[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, arrays[k % 6], dims, strides,
+                            boxes[g2p_pick(g, k < 6)], estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) {
             ctx->err = "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")";
@@ -653,27 +727,19 @@ int launch_g2p(fsim_ctx* ctx) {
     a.perm = ctx->perm;
     a.cstart = ctx->cstart;
     a.g = g;
-    a.ntx = ceil_div(g.nx, TX);
-    a.nty = ceil_div(g.ny, TY);
-    a.ntz = ceil_div(g.nz, TZ);
     a.fr = ctx->prm.flip_ratio;
     a.pic_w = 1.0f - ctx->prm.flip_ratio;
     a.ids = ctx->prm.track_ids ? 1 : 0;
     a.move_c = 1;
     a.err = ctx->d_err;
-    const int nb = a.ntx * a.nty * a.ntz;
     const int mode = ctx->prm.transfer;
     ctx->launches += 1;
-    const size_t smem = (size_t)((mode == FSIM_FLIP) ? 6 : 3) * BOXN * sizeof(float);
-    set_smem_limit((const void*)k_g2p<0>, 3 * BOXN * 4);
-    set_smem_limit((const void*)k_g2p<1>, 6 * BOXN * 4);
-    set_smem_limit((const void*)k_g2p<2>, 3 * BOXN * 4);
-    const CUtensorMap* m = ctx->tmap;
-    if (mode == FSIM_PIC)
-        k_g2p<0><<<nb, G2P_THREADS, smem, ctx->stream>>>(a, m[0], m[1], m[2], m[3], m[4], m[5]);
-    else if (mode == FSIM_FLIP)
-        k_g2p<1><<<nb, G2P_THREADS, smem, ctx->stream>>>(a, m[0], m[1], m[2], m[3], m[4], m[5]);
-    else
-        k_g2p<2><<<nb, G2P_THREADS, smem, ctx->stream>>>(a, m[0], m[1], m[2], m[3], m[4], m[5]);
+    const bool flip = mode == FSIM_FLIP;
+    const CUtensorMap* m = flip ? ctx->tmap : ctx->tmap + 6;
+    switch (g2p_pick(g, flip)) {
+        case 0: launch_g2p_shape<G2PBig>(a, mode, m, ctx->stream); break;
+        case 1: launch_g2p_shape<G2PMid>(a, mode, m, ctx->stream); break;
+        default: launch_g2p_shape<G2PSmall>(a, mode, m, ctx->stream); break;
+    }
     return 0;
 }

@@ -84,3 +84,54 @@ def test_p2g_matches_fp64_at_every_tile_shape(gpu, shape, transfer):
     assert np.array_equal(sim.grid(N.F_COUNT), count)
     assert np.array_equal(sim.grid(N.F_FLAGS) == N.WATER, count > 0)
     sim.close()
+
+
+def g2p_ref(shape, transfer, v2, u, pos, vel, fr):
+    """Particle velocities (and APIC matrices) from the grid, FP64, particles in cell order."""
+    g = pos.astype(np.float64) * RES
+    vout, cout = np.empty(pos.shape), np.empty((len(pos), 9))
+    for a in range(3):
+        off = np.array([0.0 if d == a else 0.5 for d in range(3)])
+        base = np.floor(g - off)
+        f = g - off - base
+        val, dif, grad = np.zeros(len(pos)), np.zeros(len(pos)), np.zeros((len(pos), 3))
+        for o in range(8):
+            b = np.array([(o >> 2) & 1, (o >> 1) & 1, o & 1])
+            w = np.where(b, f, 1.0 - f)
+            at = tuple(((base + b).astype(np.int64) - np.array([1 if d == a else 0 for d in range(3)])).T)
+            x = v2[a][at].astype(np.float64)
+            val += w.prod(1) * x
+            dif += w.prod(1) * (x - u[a][at])
+            for d in range(3):
+                sign = np.where(f[:, d] - b[d] > 0, -1.0, 1.0)
+                grad[:, d] += sign * RES * np.delete(w, d, 1).prod(1) * x
+        vout[:, a] = val if transfer != N.FLIP else val * (1.0 - fr) + (dif + vel[:, a]) * fr
+        cout[:, 3 * a:3 * a + 3] = grad
+    return vout, cout
+
+
+@pytest.mark.parametrize("transfer", [N.PIC, N.FLIP, N.APIC])
+@pytest.mark.parametrize("shape", SHAPES + [(130, 200, 175)])
+def test_g2p_matches_fp64_at_every_tile_shape(gpu, shape, transfer):
+    n = min(150_000, 8 * int(np.prod(np.array(shape) - 2)))
+    pos, vel, c = particles(shape, n, sum(shape) + 1)
+    prm = N.default_params(transfer=transfer, resolution=RES)
+    sim = N.Simulation(RES, prm, dims=[(k + 0.01) / RES for k in shape], track_ids=True)
+    sim.set_particles(pos, vel, c)
+    sim.stage(N.STAGE_P2G, 0.01)
+    rng = np.random.default_rng(7)
+    v2 = [rng.standard_normal(shape).astype(np.float32) for _ in range(3)]
+    for a, f in enumerate((N.F_V2X, N.F_V2Y, N.F_V2Z)):
+        sim.set_grid(f, v2[a])
+    u = [sim.grid(f).astype(np.float64) for f in (N.F_VX, N.F_VY, N.F_VZ)]
+    sim.stage(N.STAGE_G2P, 0.01)
+    gp, gv, gc = sim.particles()
+    rv, rc = g2p_ref(shape, transfer, v2, u, pos, vel.astype(np.float64), np.float64(np.float32(0.95)))
+    assert np.array_equal(gp, pos)
+    assert_close_field(gv, rv, 1e-5, "velocity")
+    # APIC takes the gradient of v2; PIC and FLIP carry C along unchanged
+    if transfer == N.APIC:
+        assert_close_field(gc.reshape(-1, 9), rc, 1e-4, "C")
+    else:
+        assert np.array_equal(gc.reshape(-1, 9), c)
+    sim.close()
