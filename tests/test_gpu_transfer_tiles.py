@@ -135,3 +135,41 @@ def test_g2p_matches_fp64_at_every_tile_shape(gpu, shape, transfer):
     else:
         assert np.array_equal(gc.reshape(-1, 9), c)
     sim.close()
+
+
+@pytest.mark.parametrize("shape", [(6, 7, 8), (9, 10, 11), (33, 40, 12)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_device_exchange_at_any_alignment(gpu, shape, shift):
+    """Grid fields and particle records to and from device buffers that start on a
+    16-byte boundary or not, rows padded (nz not a multiple of 4) or not; particle
+    counts around the block size."""
+    import torch
+
+    sim = N.Simulation(RES, N.default_params(resolution=RES), dims=[(k + 0.01) / RES for k in shape])
+    cells = int(np.prod(shape))
+    rng = np.random.default_rng(cells + shift)
+    for f, dt in ((N.F_VX, np.float32), (N.F_FLAGS, np.uint8)):
+        a = (rng.random(cells) * 3).astype(dt)
+        src = torch.zeros(cells + 8, dtype=torch.from_numpy(a).dtype, device="cuda")
+        dst = torch.zeros_like(src)
+        src[shift:shift + cells] = torch.from_numpy(a).cuda()
+        torch.cuda.synchronize()
+        p = src.data_ptr() + shift * src.element_size()
+        sim._check(sim.lib.fsim_set_grid(sim.ctx, f, p, N.DEVICE), "set")
+        assert np.array_equal(sim.grid(f).ravel(), a)
+        sim._check(sim.lib.fsim_get_grid(sim.ctx, f, dst.data_ptr() + shift * src.element_size(), N.DEVICE), "get")
+        assert torch.equal(dst, src)
+    for n in (1, 255, 256, 257, 1000):
+        pos = rng.random((n, 3)).astype(np.float32)
+        vel, c = rng.random((n, 3)).astype(np.float32), rng.random((n, 9)).astype(np.float32)
+        sim.set_particles(pos, vel, c)
+        gp, gv, gc = sim.particles()
+        assert np.array_equal(gp, pos) and np.array_equal(gv, vel) and np.array_equal(gc.reshape(-1, 9), c)
+        out = torch.zeros(n * 9 + 4, device="cuda")
+        torch.cuda.synchronize()
+        import ctypes
+        got = ctypes.c_int64()
+        sim._check(sim.lib.fsim_get_particles(sim.ctx, None, None, out.data_ptr() + 4 * shift, n, ctypes.byref(got),
+                                              N.DEVICE), "particles")
+        assert np.array_equal(out.cpu().numpy()[shift:shift + 9 * n].reshape(n, 9), c)
+    sim.close()
