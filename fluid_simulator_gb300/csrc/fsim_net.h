@@ -31,14 +31,16 @@ struct ConvLaunch {
 
 struct WgradLaunch {
     int taps, n, d, h, w, cin, cout;
-    const __nv_bfloat16* x;    // [vox][cin]
-    const __nv_bfloat16* g;    // [vox][cout]
     float* dw;                 // [taps][cout][cin], accumulated
     unsigned* err;
+    const CUtensorMap* mx;     // input map [vox][cin] (wgrad_x_map)
+    const CUtensorMap* mg;     // gradient map [vox][cout] (wgrad_g_map)
 };
 
 bool conv_act_map(CUtensorMap* m, const void* base, int n, int d, int h, int w, int c, int taps);
 bool conv_wt_map(CUtensorMap* m, const void* base, int taps, int rows, int kdim, int nt);
+bool wgrad_x_map(CUtensorMap* m, const void* base, int n, int d, int h, int w, int c, int taps);
+bool wgrad_g_map(CUtensorMap* m, const void* base, int n, int d, int h, int w, int c, int taps);
 int conv_nt(int taps, int cout);
 int launch_conv_mma(const ConvLaunch& L, cudaStream_t s);
 int launch_conv_wgrad(const WgradLaunch& L, cudaStream_t s);
@@ -86,7 +88,8 @@ struct fsim_net {
     size_t ws_bytes = 0;
     std::vector<NetBuf> act;      // forward tensors
     std::vector<NetBuf> gbuf;     // backward tensors
-    std::vector<CUtensorMap> amap;  // activation maps (forward inputs, gradient inputs)
+    std::vector<CUtensorMap> amap;  // activation maps (forward inputs, gradient inputs, weight
+                                    // gradients' inputs and output gradients)
     float* out = nullptr;         // [vox] FP32 prediction
     float* res = nullptr;         // [vox] residual of the prediction (training)
     float* gout = nullptr;        // [vox] loss gradient w.r.t. the prediction (training)

@@ -27,10 +27,7 @@
 // (so encoder outputs land directly in their concatenation slice).
 //
 // Weight-gradient kernel (k_conv_wgrad): D[(tap, c), n] = sum_v X[v + off(tap), c]
-// * G[v, n] with K = voxels.  Threads stage the shifted input transposed into
-// the K-major layout (16 voxels per step) with plain loads, a proxy fence
-// makes the stores visible to the tensor core, and one thread issues the
-// MMAs; the FP32 result is added to the gradient with atomics.
+// * G[v, n] with K = voxels, operands in the MN-major layout (described there).
 //
 // Every wait is bounded; a timeout sets an error bit, waits (bounded) for the
 // MMAs already issued, frees TMEM and returns.
@@ -561,138 +558,240 @@ __global__ void __launch_bounds__(PERS_THREADS, 1) k_conv_pers(const PersArgs p,
 // ---------------------------------------------------------------------------
 // weight gradient
 // ---------------------------------------------------------------------------
-constexpr int WG_MAX_MT = 8;
+// D[(kd, c), n] of tap (kd, kh, kw) = sum over voxels v of X[v + off, c] * G[v, n]:
+// K = voxels, and both operands sit in memory with their M / N index (channels)
+// contiguous, which is the tensor core's MN-major layout -- TMA boxes are used
+// as they land, nothing is transposed.  A tile is 8 (w) x 16 (h) x WG planes of
+// voxels; X comes as one box per d-plane, laid out [octet][h][w][8 channels] with
+// the halo, so the channel octets of a plane and then of the next planes are
+// one equally spaced sequence: with 4 octets (32 input channels) the 16 groups
+// of M = 128 are (d-shift kd = 0..2, octet), 12 of them used.  A shift in h or w
+// is a start offset, so 9 accumulators (kh, kw) of N columns each cover the 27
+// taps.  One MMA takes 16 voxels (two h rows of 8).  Voxels outside the volume are
+// zero-filled by TMA (planes outside the sample are fetched at a coordinate
+// outside the tensor).  For the pointwise layers the sequence is 16 octets (128
+// input channels) of one plane and there is one accumulator.
+//
+// The tensor core truncates when it adds to its FP32 accumulator, so long chains
+// drift: the accumulators are drained into FP32 registers every few planes (864
+// MMAs deep, the sums over 2M voxels were 4-6 times less exact than with the
+// kernel this one replaced, 215 deep; at 64 they are more exact).  They come in
+// parts (the three kh; pointwise: even and odd planes), each drained by its
+// own four warps while the other parts' MMAs run.  One CTA per SM: warps 0-11 drain
+// and finally add to the gradient, warp 12 streams tiles through two stages, warp
+// 13 issues the MMAs.  Every wait is bounded, as in k_conv_pers.
+// What bounds it: the MMAs' operand reads (A 4 KB, B 32 N bytes per MMA at 128 bytes
+// per cycle: 36 cycles at N = 16, 288 MMAs per tile).  Training pass of 8 x 64^3:
+// 15.8 ms of weight gradients with the kernel this one replaced (threads
+// transposing 27 shifted copies of X into shared memory, two bytes at a time).
+constexpr int WG_THREADS = 448;  // 12 draining warps, TMA, MMA
+template <int TAPS>
+struct Wg {
+    static constexpr int H = TAPS == 27 ? 1 : 0;
+    static constexpr int OCT = TAPS == 27 ? 4 : 16;     // octets of one X chunk
+    static constexpr int PD = TAPS == 27 ? 4 : 2;       // planes of a tile
+    static constexpr int XW = TW + 2 * H, XH = TH + 2 * H, XD = PD + 2 * H;
+    static constexpr int X_OCT = XW * XH * 16;          // bytes of one octet of a plane
+    static constexpr int X_PLANE = OCT * X_OCT;
+    static constexpr int X_BYTES = XD * X_PLANE;
+    static constexpr int G_OCT = TW * TH * 16;
+    static constexpr int ACC = TAPS == 27 ? 9 : 1;      // accumulators (kh, kw)
+    static constexpr int PARTS = TAPS == 27 ? 3 : 2;    // groups of accumulators drained apart: kh; even / odd planes
+    static constexpr int PACC = TAPS == 27 ? 3 : 1;     // accumulators of a part
+};
 
 struct WgArgs {
-    const __nv_bfloat16* x;  // input activation [vox][cin]
-    const __nv_bfloat16* g;  // gradient of the pre-activation output [vox][cout]
-    int taps, cin, cout;
+    int cin, cout;
     int n, d, h, w;
-    int rows;                // taps * cin
-    int mt;                  // 128-row tiles per CTA
-    int groups;
-    long long vox;           // voxels
-    long long steps;         // ceil(voxels / 16); the ragged last step is zero-padded
-    int ksplit;
+    int tiles_w, tiles_h, tiles_d, tiles;
+    int nchunk, nparts, ksplit;
+    int interval;            // planes per drain of an accumulator
+    int stage_bytes, ncols;
     float* dw;               // [taps][cout][cin], accumulated
     unsigned* err;
 };
 
-__global__ void __launch_bounds__(CONV_THREADS) k_conv_wgrad(const WgArgs a) {
+// both operands MN-major (bits 15, 16)
+__host__ __device__ constexpr uint32_t idesc_bf16_mn(int n) { return idesc_bf16(n) | (1u << 15) | (1u << 16); }
+// MN-major, no swizzle: lbo = bytes between 8-voxel groups (K), sbo = between
+// 8-channel groups (M / N); inside a group a voxel's 8 channels are 16 bytes
+__device__ __forceinline__ uint64_t sdesc_mn(uint32_t saddr, uint32_t lbo, uint32_t sbo) { return sdesc(saddr, lbo, sbo); }
+
+// drains part `pt` of the accumulators `uses` times into registers, then adds them to the gradient
+template <int TAPS, int NT>
+__device__ __forceinline__ void wgrad_drain(const WgArgs& a, uint32_t tmem, int pt, int uses, int chunk, int cpart,
+                                            uint64_t* acc_full, uint64_t* acc_empty, volatile int* stop) {
+    using W = Wg<TAPS>;
+    constexpr int COLS = W::PACC * NT;
+    const int lane = threadIdx.x & 31, q = (threadIdx.x >> 5) & 3;
+    const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(pt * COLS);
+    float r[COLS];
+#pragma unroll
+    for (int k = 0; k < COLS; k++) r[k] = 0.f;
+    for (int u = 0; u < uses; u++) {
+        if (!mbar_wait_ab(acc_full, (unsigned)(u & 1), stop, a.err)) return;
+        fence_after();
+#pragma unroll
+        for (int c0 = 0; c0 < COLS; c0 += 32) {
+            uint32_t v0[16], v1[16];
+            tmem_ld16_async(taddr + (uint32_t)c0, v0);
+            if (c0 + 16 < COLS) tmem_ld16_async(taddr + (uint32_t)(c0 + 16), v1);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                r[c0 + j] += __uint_as_float(v0[j]);
+                if (c0 + 16 < COLS) r[c0 + 16 + j] += __uint_as_float(v1[j]);
+            }
+        }
+        fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty);
+    }
+    // row m = (kd, octet, channel); rows past the used groups hold sums over other data
+    const int m = q * 32 + lane;
+    const int kd = (m >> 3) / W::OCT, c = chunk * W::OCT * 8 + ((m >> 3) % W::OCT) * 8 + (m & 7);
+    if (kd >= (TAPS == 27 ? 3 : 1) || c >= a.cin) return;
+#pragma unroll
+    for (int k = 0; k < W::PACC; k++) {
+        const int tap = TAPS == 27 ? kd * 9 + pt * 3 + k : 0;
+        float* o = a.dw + ((long long)tap * a.cout + cpart * NT) * a.cin + c;
+#pragma unroll
+        for (int j = 0; j < NT; j++) atomicAdd(o + (long long)j * a.cin, r[k * NT + j]);
+    }
+}
+
+template <int TAPS, int NT>
+__global__ void __launch_bounds__(WG_THREADS, 1) k_conv_wgrad(const WgArgs a, const __grid_constant__ CUtensorMap tx,
+                                                              const __grid_constant__ CUtensorMap tg) {
+    using W = Wg<TAPS>;
+    constexpr int G_PLANE = (NT >> 3) * W::G_OCT;
     extern __shared__ __align__(128) unsigned char smraw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>(((uintptr_t)smraw + 127) & ~(uintptr_t)127);
-    __shared__ __align__(8) uint64_t bar[2], done;
+    __shared__ __align__(8) uint64_t full[2], empty[2], acc_full[3], acc_empty[3], done;
     __shared__ uint32_t tmem_base;
+    __shared__ int s_stop, s_issued, s_consumed;
 
-    const int grp = blockIdx.x % a.groups;
-    const int ks = blockIdx.x / a.groups;
-    const int R = a.mt * 128;  // rows staged per step
-    const int row0 = grp * R;
-    const int A_KC = R * 16;
-    const int B_KC = a.cout * 16;
-    const int stage_bytes = 2 * A_KC + 2 * B_KC;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int ncols = tmem_cols(a.mt * a.cout);
-    const long long s_begin = a.steps * ks / a.ksplit, s_end = a.steps * (ks + 1) / a.ksplit;
+    const int chunk = (int)blockIdx.x % a.nchunk;
+    const int part = ((int)blockIdx.x / a.nchunk) % a.nparts;
+    const int ks = (int)blockIdx.x / (a.nchunk * a.nparts);
+    const int my_tiles = (a.tiles - 1 - ks) / a.ksplit + 1;  // ks < ksplit <= tiles
+    const int planes = my_tiles * W::PD;
 
     if (threadIdx.x == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
+        for (int q = 0; q < 2; q++) {
+            mbar_init(&full[q], 1);
+            mbar_init(&empty[q], 1);
+        }
+        for (int q = 0; q < W::PARTS; q++) {
+            mbar_init(&acc_full[q], 1);
+            mbar_init(&acc_empty[q], 4);
+        }
         mbar_init(&done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        s_stop = 0;
+        s_issued = 0;
+        s_consumed = 0;
     }
-    if (warp == 0) tmem_alloc(&tmem_base, ncols);
+    if (warp == 0) tmem_alloc(&tmem_base, a.ncols);
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tmem = tmem_base;
-    const uint32_t idesc = idesc_bf16(a.cout);
-    const int k = threadIdx.x & 15;  // this thread's voxel within each step
-    const long long plane = (long long)a.h * a.w;
-    bool ok = true;
+    volatile int* stop = &s_stop;
 
-    for (long long s = s_begin; s < s_end; s++) {
-        const int it = (int)(s - s_begin);
-        const int st = it & 1;
-        // the MMAs that read this stage two steps ago must be done
-        if (it >= 2 && !mbar_wait(&bar[st], (unsigned)(((it - 2) >> 1) & 1))) ok = false;
-        if (__syncthreads_or(!ok)) {
-            ok = false;
-            break;
-        }
-        unsigned char* A = sm + st * stage_bytes;
-        unsigned char* Bm = A + 2 * A_KC;
-        const long long v = s * 16 + k;
-        const bool live = v < a.vox;
-        const int vw = (int)(v % a.w), vh = (int)((v / a.w) % a.h), vd = (int)((v / plane) % a.d);
-        const int kc = k >> 3, kk = k & 7;
-        // A: rows (tap, c) of this group, column k
-        for (int u = threadIdx.x >> 4; u < R / 8; u += CONV_THREADS / 16) {
-            const int r = row0 + u * 8;
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if (live && r < a.rows) {
-                const int tap = r / a.cin, c = r % a.cin;
-                int dd = 0, dh = 0, dw = 0;
-                if (a.taps == 27) {
-                    dd = tap / 9 - 1;
-                    dh = (tap / 3) % 3 - 1;
-                    dw = tap % 3 - 1;
+    if (warp == 12) {
+        if (lane == 0) {
+            int issued = 0;
+            for (int j = 0; j < my_tiles; j++) {
+                const int q = j & 1;
+                if (j >= 2 && !mbar_wait_ab(&empty[q], (unsigned)(((j >> 1) - 1) & 1), stop, a.err)) break;
+                int t = ks + j * a.ksplit;
+                const int w0 = (t % a.tiles_w) * TW;
+                t /= a.tiles_w;
+                const int h0 = (t % a.tiles_h) * TH;
+                t /= a.tiles_h;
+                const int d0 = (t % a.tiles_d) * W::PD, nb = t / a.tiles_d;
+                unsigned char* st = sm + q * a.stage_bytes;
+                mbar_expect_tx(&full[q], (unsigned)(W::X_BYTES + W::PD * G_PLANE));
+                for (int z = 0; z < W::XD; z++) {
+                    const int dd = d0 + z - W::H;
+                    const bool in = dd >= 0 && dd < a.d;
+                    tma_5d(st + z * W::X_PLANE, &tx, 0, w0 - W::H, h0 - W::H, chunk * W::OCT,
+                           in ? nb * a.d + dd : a.n * a.d, &full[q]);
                 }
-                const int sw = vw + dw, sh = vh + dh, sd = vd + dd;
-                if (sw >= 0 && sw < a.w && sh >= 0 && sh < a.h && sd >= 0 && sd < a.d) {
-                    const long long sv = v + ((long long)dd * a.h + dh) * a.w + dw;
-                    val = *reinterpret_cast<const uint4*>(a.x + sv * a.cin + c);
+                for (int z = 0; z < W::PD; z++) {
+                    const int dd = d0 + z;
+                    tma_5d(st + W::X_BYTES + z * G_PLANE, &tg, 0, w0, h0, part * (NT >> 3),
+                           dd < a.d ? nb * a.d + dd : a.n * a.d, &full[q]);
                 }
+                issued = j + 1;
             }
-            const unsigned short* e = reinterpret_cast<const unsigned short*>(&val);
-            unsigned short* base = reinterpret_cast<unsigned short*>(A + kc * A_KC + (u * 8) * 16) + kk;
-#pragma unroll
-            for (int j = 0; j < 8; j++) base[j * 8] = e[j];
+            s_issued = issued;
         }
-        // B: rows n, column k
-        for (int u = threadIdx.x >> 4; u < a.cout / 8; u += CONV_THREADS / 16) {
-            const uint4 val = live ? *reinterpret_cast<const uint4*>(a.g + v * a.cout + u * 8) : make_uint4(0, 0, 0, 0);
-            const unsigned short* e = reinterpret_cast<const unsigned short*>(&val);
-            unsigned short* base = reinterpret_cast<unsigned short*>(Bm + kc * B_KC + (u * 8) * 16) + kk;
+    } else if (warp == 13) {
+        if (lane == 0) {
+            constexpr uint32_t idesc = idesc_bf16_mn(NT);
+            int consumed = 0;
+            bool ok = true;
+            for (int j = 0; ok && j < my_tiles; j++) {
+                const int q = j & 1;
+                if (!mbar_wait_ab(&full[q], (unsigned)((j >> 1) & 1), stop, a.err)) break;
+                consumed = j + 1;
+                fence_after();
+                const uint32_t xb = s32(sm + q * a.stage_bytes), gb = xb + W::X_BYTES;
+                const uint64_t ad0 = sdesc_mn(xb, W::XW * 16, W::X_OCT);
+                const uint64_t bd0 = sdesc_mn(gb, TW * 16, W::G_OCT);
+#pragma unroll 1
+                for (int z = 0; ok && z < W::PD; z++) {
+                    const int p = j * W::PD + z;  // pointwise: plane p >> 1 of part p & 1
+                    // start-address fields are in 16-byte units
+                    const uint64_t adz = ad0 + (uint64_t)(z * W::X_PLANE / 16);
+                    const uint64_t bdz = bd0 + (uint64_t)(z * G_PLANE / 16);
+#pragma unroll 1
+                    for (int pt = 0; pt < W::PARTS; pt++) {
+                        if (TAPS == 1 && (p & 1) != pt) continue;
+                        const int pp = TAPS == 1 ? p >> 1 : p, np = TAPS == 1 ? (planes + 1 - pt) / 2 : planes;
+                        const int use = pp / a.interval, at = pp - use * a.interval;
+                        if (at == 0 && use > 0 &&
+                            !mbar_wait_ab(&acc_empty[pt], (unsigned)((use - 1) & 1), stop, a.err)) {
+                            ok = false;
+                            break;
+                        }
+                        fence_after();
+                        const uint64_t adp = adz + (uint64_t)(TAPS == 27 ? pt * W::XW : 0);  // kh = pt
+                        const uint32_t acc0 = tmem + (uint32_t)(pt * W::PACC * NT);
 #pragma unroll
-            for (int j = 0; j < 8; j++) base[j * 8] = e[j];
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            fence_after();
-            const uint64_t bdesc = sdesc(s32(Bm), (uint32_t)B_KC, 128);
-            for (int mt = 0; mt < a.mt; mt++) {
-                const uint64_t adesc = sdesc(s32(A + mt * 128 * 16), (uint32_t)A_KC, 128);
-                mma_bf16(tmem + (uint32_t)(mt * a.cout), adesc, bdesc, idesc, it > 0 ? 1u : 0u);
+                        for (int hp = 0; hp < TH / 2; hp++)
+#pragma unroll
+                            for (int k = 0; k < W::PACC; k++)  // kw = k
+                                mma_bf16(acc0 + (uint32_t)(k * NT), adp + (uint64_t)(2 * hp * W::XW + k),
+                                         bdz + (uint64_t)(2 * hp * TW), idesc, (hp > 0 || at > 0) ? 1u : 0u);
+                        if (at == a.interval - 1 || pp == np - 1) mma_commit(&acc_full[pt]);
+                    }
+                }
+                mma_commit(&empty[q]);
             }
-            mma_commit(&bar[st]);
+            s_consumed = ok ? consumed : -1;
+            mma_commit(&done);  // arrives once every MMA issued above has completed
         }
+    } else if (warp < 4 * W::PARTS) {
+        const int pt = warp >> 2;
+        const int np = TAPS == 27 ? planes : (planes + 1 - pt) / 2;
+        wgrad_drain<TAPS, NT>(a, tmem, pt, (np + a.interval - 1) / a.interval, chunk, part, &acc_full[pt],
+                              &acc_empty[pt], stop);
     }
-    if (threadIdx.x == 0) mma_commit(&done);
     __syncthreads();
     const bool fin = mbar_wait(&done, 0);
-    if (__syncthreads_or(!fin || !ok)) {
-        if (threadIdx.x == 0) atomicOr(a.err, 4u);
-    } else if (s_end > s_begin) {
-        fence_after();
-        for (int mt = 0; mt < a.mt; mt++) {
-            const int r = row0 + mt * 128 + warp * 32 + lane;
-            const int tap = r / a.cin, c = r % a.cin;
-            for (int n0 = 0; n0 < a.cout; n0 += 16) {
-                uint32_t v[16];
-                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mt * a.cout + n0), v);
-                if (r < a.rows) {
-#pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        atomicAdd(a.dw + ((long long)tap * a.cout + n0 + j) * a.cin + c, __uint_as_float(v[j]));
-                }
-            }
-        }
+    if (__syncthreads_or(!fin || s_stop || s_consumed != my_tiles) && threadIdx.x == 0) {
+        atomicOr(a.err, 4u);
+        // let the copies still in flight land before the CTA's shared memory goes away
+        for (int j = s_issued > 2 ? s_issued - 2 : 0; j < s_issued; j++)
+            mbar_wait(&full[j & 1], (unsigned)((j >> 1) & 1));
     }
     fence_before();
     __syncthreads();
-    if (warp == 0) tmem_free(tmem, ncols);
+    if (warp == 0) tmem_free(tmem, a.ncols);
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encoder() {
@@ -743,6 +842,32 @@ bool conv_wt_map(CUtensorMap* m, const void* base, int taps, int rows, int kdim,
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, str, box, es,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// weight-gradient operands: [n*d][h][w][c] bf16 with the channel octets as a
+// dimension of their own, so that a box holds [octet][h][w][8 channels] of a plane
+static bool wgrad_map(CUtensorMap* m, const void* base, long long planes, int h, int w, int c, int oct, int bw, int bh) {
+    auto enc = encoder();
+    if (!enc || (reinterpret_cast<uintptr_t>(base) & 15) || c % 16) return false;
+    cuuint64_t dims[5] = {8, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)(c / 8), (cuuint64_t)planes};
+    cuuint64_t str[4] = {(cuuint64_t)c * 2, (cuuint64_t)c * 2 * w, 16, (cuuint64_t)c * 2 * w * h};
+    cuuint32_t box[5] = {8, (cuuint32_t)bw, (cuuint32_t)bh, (cuuint32_t)oct, 1};
+    cuuint32_t es[5] = {1, 1, 1, 1, 1};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, str, box, es,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+bool wgrad_x_map(CUtensorMap* m, const void* base, int n, int d, int h, int w, int c, int taps) {
+    return taps == 27 ? wgrad_map(m, base, (long long)n * d, h, w, c, Wg<27>::OCT, Wg<27>::XW, Wg<27>::XH)
+                      : wgrad_map(m, base, (long long)n * d, h, w, c, Wg<1>::OCT, Wg<1>::XW, Wg<1>::XH);
+}
+// output channels per CTA: nine accumulators of nt columns share TMEM with 3x3x3 taps
+static int wgrad_nt(int taps, int cout) {
+    if (taps == 1 || cout <= 32) return cout;
+    return cout % 32 == 0 ? 32 : 16;
+}
+bool wgrad_g_map(CUtensorMap* m, const void* base, int n, int d, int h, int w, int c, int taps) {
+    return wgrad_map(m, base, (long long)n * d, h, w, c, wgrad_nt(taps, c) / 8, TW, TH);
 }
 
 int conv_nt(int taps, int cout) { return pick_nt(cout, taps == 27 ? 64 : 128); }
@@ -816,34 +941,59 @@ int launch_conv_mma(const ConvLaunch& L, cudaStream_t s) {
     return cudaGetLastError() == cudaSuccess ? FSIM_OK : FSIM_E_CUDA;
 }
 
-int launch_conv_wgrad(const WgradLaunch& L, cudaStream_t s) {
-    if ((L.taps != 27 && L.taps != 1) || L.cin % 16 || L.cout % 16 || L.cout > 64) return FSIM_E_INVALID;
-    const long long vox = (long long)L.n * L.d * L.h * L.w;
-    if (vox <= 0) return FSIM_OK;
+template <int TAPS, int NT>
+static int launch_wgrad(const WgradLaunch& L, cudaStream_t s) {
+    using W = Wg<TAPS>;
     WgArgs a{};
-    a.x = L.x; a.g = L.g;
-    a.taps = L.taps; a.cin = L.cin; a.cout = L.cout;
+    a.cin = L.cin; a.cout = L.cout;
     a.n = L.n; a.d = L.d; a.h = L.h; a.w = L.w;
-    a.rows = L.taps * L.cin;
-    const int tiles = ceil_div(a.rows, 128);
-    int mt = 512 / tmem_cols(L.cout);
-    if (mt > WG_MAX_MT) mt = WG_MAX_MT;
-    if (mt > tiles) mt = tiles;
-    while (mt > 1 && tmem_cols(mt * L.cout) > 512) mt--;
-    a.mt = mt;
-    a.groups = ceil_div(tiles, mt);
-    a.vox = vox;
-    a.steps = (vox + 15) / 16;
-    int ks = (int)((4LL * 152 + a.groups - 1) / a.groups);
-    const long long max_ks = a.steps / 8 > 0 ? a.steps / 8 : 1;
-    if (ks > max_ks) ks = (int)max_ks;
-    if (ks < 1) ks = 1;
-    a.ksplit = ks;
+    a.tiles_w = ceil_div(L.w, TW);
+    a.tiles_h = ceil_div(L.h, TH);
+    a.tiles_d = ceil_div(L.d, W::PD);
+    const long long tiles = (long long)a.tiles_w * a.tiles_h * a.tiles_d * L.n;
+    if (tiles >= (1ll << 31) || (long long)L.n * L.d >= (1ll << 31) - 1) return FSIM_E_INVALID;
+    a.tiles = (int)tiles;
+    a.nchunk = ceil_div(L.cin, W::OCT * 8);
+    a.nparts = L.cout / NT;
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return FSIM_E_CUDA;
+    // one wave: a CTA keeps its accumulators over all its tiles and adds them once
+    const int groups = a.nchunk * a.nparts;
+    a.ksplit = sms / groups > 0 ? sms / groups : 1;
+    if (a.ksplit > a.tiles) a.ksplit = a.tiles;
+    // Drain depth (8 MMAs per plane): an eighth of the CTA's planes or less, 1 to 8.
+    // Draining after every plane costs the MMAs a third of their rate (8 x 64^3,
+    // 16 -> 16: 326 us against 230), and this stays below the depth at which the
+    // sums were as exact as before (all of a quarter as many voxels).
+    const int planes = ceil_div(a.tiles, a.ksplit) * W::PD / (TAPS == 1 ? 2 : 1);
+    a.interval = 1;
+    while (a.interval < 8 && 2 * a.interval * 10 <= planes) a.interval *= 2;
+    a.stage_bytes = W::X_BYTES + W::PD * (NT / 8) * W::G_OCT;
+    a.ncols = tmem_cols(TAPS == 27 ? W::ACC * NT : 2 * NT);
     a.dw = L.dw;
     a.err = L.err;
-    const int stage = 2 * (mt * 128 * 16) + 2 * L.cout * 16;
-    const int smem = 2 * stage + 128;
-    if (set_smem_limit((const void*)k_conv_wgrad, SMEM_LIMIT) != cudaSuccess) return FSIM_E_CUDA;
-    k_conv_wgrad<<<(unsigned)(a.groups * a.ksplit), CONV_THREADS, smem, s>>>(a);
+    // the unused M groups of the last planes read past the X box, into the stage's G box
+    if ((W::PD - 1) * W::X_PLANE + 16 * W::X_OCT > a.stage_bytes) return FSIM_E_INVALID;
+    int smem = 2 * a.stage_bytes + 128;
+    if (smem > SMEM_LIMIT) return FSIM_E_INVALID;
+    if (smem < SMEM_LIMIT / 2 + 1024) smem = SMEM_LIMIT / 2 + 1024;  // one CTA per SM (TMEM)
+    if (set_smem_limit((const void*)k_conv_wgrad<TAPS, NT>, SMEM_LIMIT) != cudaSuccess) return FSIM_E_CUDA;
+    k_conv_wgrad<TAPS, NT><<<(unsigned)(groups * a.ksplit), WG_THREADS, smem, s>>>(a, *L.mx, *L.mg);
     return cudaGetLastError() == cudaSuccess ? FSIM_OK : FSIM_E_CUDA;
+}
+
+int launch_conv_wgrad(const WgradLaunch& L, cudaStream_t s) {
+    if ((L.taps != 27 && L.taps != 1) || L.cin % 16 || L.cout % 16 || L.cin <= 0 || L.cout <= 0 || L.cout > 64)
+        return FSIM_E_INVALID;
+    if ((long long)L.n * L.d * L.h * L.w <= 0) return FSIM_OK;
+    const int nt = wgrad_nt(L.taps, L.cout);
+    if (L.taps == 27) return nt == 32 ? launch_wgrad<27, 32>(L, s) : launch_wgrad<27, 16>(L, s);
+    switch (nt) {
+        case 16: return launch_wgrad<1, 16>(L, s);
+        case 32: return launch_wgrad<1, 32>(L, s);
+        case 48: return launch_wgrad<1, 48>(L, s);
+        default: return launch_wgrad<1, 64>(L, s);
+    }
 }

@@ -644,7 +644,7 @@ int ensure_ws(fsim_net* net, int n, int d, int h, int w, bool train) {
     net->gout = train ? (float*)(base + gout_off) : nullptr;
     net->batch_target = train ? (float*)(base + tb_off) : nullptr;
     net->batch_mask = train ? (uint8_t*)(base + mb_off) : nullptr;
-    net->amap.resize(2 * NET_LAYERS);
+    net->amap.resize(4 * NET_LAYERS);
     for (int l = 0; l < NET_LAYERS; l++) {
         const NetBuf& in = net->act[kIn[l]];
         const int lv = in.lev;
@@ -655,6 +655,13 @@ int ensure_ws(fsim_net* net, int n, int d, int h, int w, bool train) {
             if (!conv_act_map(&net->amap[NET_LAYERS + l], gz.p, n, d >> gz.lev, h >> gz.lev, w >> gz.lev, gz.c,
                               net->L[l].taps))
                 return fail(net, "tensor map of a network gradient failed", FSIM_E_CUDA);
+        }
+        if (train) {
+            const NetBuf& gz = net->gbuf[kGz[l]];
+            if (!wgrad_x_map(&net->amap[2 * NET_LAYERS + l], in.p, n, d >> lv, h >> lv, w >> lv, in.c, net->L[l].taps) ||
+                !wgrad_g_map(&net->amap[3 * NET_LAYERS + l], gz.p, n, d >> gz.lev, h >> gz.lev, w >> gz.lev, gz.c,
+                             net->L[l].taps))
+                return fail(net, "tensor map of a weight-gradient operand failed", FSIM_E_CUDA);
         }
     }
     return FSIM_OK;
@@ -739,7 +746,6 @@ namespace {
 int conv_bwd(fsim_net* net, int l) {
     const NetLayer& L = net->L[l];
     const NetBuf& gz = net->gbuf[kGz[l]];
-    const NetBuf& x = net->act[kIn[l]];
     const NetShape& sh = net->shape;
     const int lv = gz.lev;
     // weight gradient
@@ -751,8 +757,8 @@ int conv_bwd(fsim_net* net, int l) {
     wg.w = sh.w >> lv;
     wg.cin = L.cin;
     wg.cout = L.cout;
-    wg.x = x.p;
-    wg.g = gz.p;
+    wg.mx = &net->amap[2 * NET_LAYERS + l];
+    wg.mg = &net->amap[3 * NET_LAYERS + l];
     wg.dw = net->grad + L.w_off;
     wg.err = net->d_err;
     int rc = launch_conv_wgrad(wg, net->stream);
@@ -1225,10 +1231,14 @@ int fsim_net_conv(int taps, int mode, int n, int d, int h, int w, int cin, int c
             L.n = n; L.d = d; L.h = h; L.w = w;
             L.cin = cin;
             L.cout = cout;
-            L.x = bx;
-            L.g = bg;
             L.dw = fo;
             L.err = err;
+            L.mx = &mx;
+            L.mg = &mw;
+            if (!wgrad_x_map(&mx, bx, n, d, h, w, cin, taps) || !wgrad_g_map(&mw, bg, n, d, h, w, cout, taps)) {
+                rc = FSIM_E_CUDA;
+                g_conv_err = "tensor map encoding failed";
+            }
             if (rc == FSIM_OK) rc = launch_conv_wgrad(L, s);
             if (rc) g_conv_err = std::string("weight-gradient launch: ") + cudaGetErrorString(cudaGetLastError());
         }
