@@ -101,24 +101,32 @@ __device__ __forceinline__ double warp_max(double v) {
 }
 
 // Block-wide reduction of K doubles (sum or max per slot, chosen by `is_max`
-// bit k).  Result valid in thread 0.  `scratch` holds 32*K doubles.
+// bit k; at least K warps).  Result valid in thread 0.  `scratch` holds
+// blockDim.x * K doubles: warp k takes value k from there, blockDim.x / 32 per lane
+// and then five shuffles.  FP64 adds issue at 1/64 of the FP32 rate here, and this
+// takes 12 warp instructions per value of a 256-thread block where a shuffle tree
+// in every warp took 45 (with eight such blocks per SM, 2 us a value).
 template <int K>
 __device__ __forceinline__ void block_reduce(double (&v)[K], unsigned is_max, double* scratch) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nw = (blockDim.x + 31) >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = blockDim.x;
 #pragma unroll
-    for (int k = 0; k < K; k++) v[k] = ((is_max >> k) & 1) ? warp_max(v[k]) : warp_sum(v[k]);
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < K; k++) scratch[warp * K + k] = v[k];
+    for (int k = 0; k < K; k++) scratch[k * n + threadIdx.x] = v[k];
     __syncthreads();
-    if (warp == 0) {
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            double t = lane < nw ? scratch[lane * K + k] : (((is_max >> k) & 1) ? -1e300 : 0.0);
-            v[k] = ((is_max >> k) & 1) ? warp_max(t) : warp_sum(t);
+    if (warp < K) {
+        const bool mx = (is_max >> warp) & 1;
+        double t = scratch[warp * n + lane];
+        for (int j = lane + 32; j < n; j += 32) {
+            const double u = scratch[warp * n + j];
+            t = mx ? fmax(t, u) : t + u;
         }
+        t = mx ? warp_max(t) : warp_sum(t);
+        __syncwarp();
+        if (lane == 0) scratch[warp * n] = t;
     }
+    __syncthreads();
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int k = 0; k < K; k++) v[k] = scratch[k * n];
     __syncthreads();
 }
 

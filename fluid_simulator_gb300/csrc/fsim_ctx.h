@@ -18,7 +18,7 @@ struct PcgState {
     double rmax, rr;     // recursive residual max |r|, r.r   (A' units)
     double rr_update;    // r.r right after the last true-residual replacement
     double fold_drop;    // MIXED: fold + restart once r.r < fold_drop * rr_update
-    double bb, bmax;     // rhs norms (A' units)
+    double bb;           // b'.b' (A' units)
     double tol_abs;      // max-norm tolerance in A' units
     double tol_rel2;     // (tol * ||b||)^2 in A' units
     int tol_mode;

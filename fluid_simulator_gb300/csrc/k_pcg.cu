@@ -33,6 +33,7 @@
 // Each reduction finishes in the last CTA to arrive (fixed order, so results
 // are deterministic), which also updates the scalars in device memory; the
 // host only polls a small state block every few iterations.
+#include <algorithm>
 #include <cmath>
 
 #include "fsim_ctx.h"
@@ -205,35 +206,51 @@ __global__ void k_setup(const SetupArgs a) {
     a.brick_flag[((long long)bx * a.B.nby + by) * a.B.nbz + bz] = 1;
 }
 
-// ordered compaction of active bricks (one CTA)
+// ordered compaction of active bricks (one CTA; 16 flags per thread and pass: 65,536
+// bricks at 256^3 take 4 passes, 79 -> 8 us)
 // each entry holds the brick's coordinates and index, int4 {bx, by, bz, b}, so
 // the kernels over active bricks take them with one load, not three divisions
-__global__ void __launch_bounds__(1024) k_compact_bricks(const uint8_t* flag, long long nb, int nby, int nbz,
-                                                         int4* xyz, int* count) {
+constexpr int COMPACT_THREADS = 1024, COMPACT_ITEMS = 16;
+__global__ void __launch_bounds__(COMPACT_THREADS) k_compact_bricks(const uint8_t* flag, long long nb, int nby, int nbz,
+                                                                    int4* xyz, int* count) {
     __shared__ int warp_tot[32];
-    __shared__ int carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (long long base = 0; base < nb; base += blockDim.x) {
-        const long long j = base + threadIdx.x;
-        const int f = (j < nb) ? flag[j] : 0;
-        const unsigned bal = __ballot_sync(0xffffffffu, f);
-        if (lane == 0) warp_tot[warp] = __popc(bal);
-        __syncthreads();
-        int before = 0;
-        for (int w = 0; w < warp; w++) before += warp_tot[w];
-        if (f) {
-            const int pos = carry + before + __popc(bal & ((1u << lane) - 1u));
-            const unsigned ju = (unsigned)j, t = ju / (unsigned)nbz, u = t / (unsigned)nby;
-            xyz[pos] = make_int4((int)u, (int)(t - u * (unsigned)nby), (int)(ju - t * (unsigned)nbz), (int)j);
+    int carry = 0;
+    for (long long base = 0; base < nb; base += COMPACT_THREADS * COMPACT_ITEMS) {
+        const long long j0 = base + (long long)threadIdx.x * COMPACT_ITEMS;
+        // (the flags' allocation is 256-byte aligned; the tail is read byte by byte)
+        alignas(16) uint8_t f[COMPACT_ITEMS];
+        if (j0 + COMPACT_ITEMS <= nb) {
+            *reinterpret_cast<uint4*>(f) = *reinterpret_cast<const uint4*>(flag + j0);
+        } else {
+            for (int k = 0; k < COMPACT_ITEMS; k++) f[k] = j0 + k < nb ? flag[j0 + k] : 0;
         }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int t = 0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += warp_tot[w];
-            carry += t;
+        int mine = 0;
+#pragma unroll
+        for (int k = 0; k < COMPACT_ITEMS; k++) mine += f[k] != 0;
+        int incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
         }
+        if (lane == 31) warp_tot[warp] = incl;
+        __syncthreads();
+        int wt = warp_tot[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, wt, o);
+            if (lane >= o) wt += t;
+        }
+        const int before = __shfl_sync(0xffffffffu, wt, warp > 0 ? warp - 1 : 0);
+        int pos = carry + incl - mine + (warp > 0 ? before : 0);
+        carry += __shfl_sync(0xffffffffu, wt, 31);
+#pragma unroll
+        for (int k = 0; k < COMPACT_ITEMS; k++)
+            if (f[k]) {
+                const unsigned ju = (unsigned)(j0 + k), t = ju / (unsigned)nbz, u = t / (unsigned)nby;
+                xyz[pos++] = make_int4((int)u, (int)(t - u * (unsigned)nby), (int)(ju - t * (unsigned)nbz), (int)ju);
+            }
         __syncthreads();
     }
     if (threadIdx.x == 0) *count = carry;
@@ -264,13 +281,17 @@ struct Vecs {
 };
 
 // r = b' - A' phi (FP64), store into r[rc]; reset x (FP32 accumulator) to 0.
-// first = 1: also reduce |b'| and decide the reference's early-out.
+// first = 1: also reduce |b'| and decide the reference's early-out.  FP64 arithmetic
+// bounds this kernel (1/64 of the FP32 rate): the max norm comes from the stored
+// residual, the rhs norm is needed by the first residual only, and a solve that
+// starts from phi = 0 has r = b, one product per cell.
 template <typename T>
 __global__ void __launch_bounds__(PCG_THREADS) k_residual(const PcgArgs a, Vecs<T> v, int first, int reset_x) {
-    __shared__ double scratch[32 * 4];
+    __shared__ double scratch[PCG_THREADS * 3];
     T* r = (a.st->bufsel & 1) ? v.r[1] : v.r[0];
-    double acc[4] = {0.0, -1e300, 0.0, -1e300};  // rr, rmax, bb, bmax
+    double acc[3] = {0.0, -1e300, 0.0};  // rr, rmax, bb
     T rmaxT = (T)0;
+    const bool from_zero = first && a.phi_zero;
     const int nact = *a.nactive;
     for (int bk = blockIdx.x; bk < nact; bk += gridDim.x) {
         int x, y, z;
@@ -278,30 +299,26 @@ __global__ void __launch_bounds__(PCG_THREADS) k_residual(const PcgArgs a, Vecs<
         if (!brick_cell(a.B, a.bxyz[bk], threadIdx.x, x, y, z, c)) continue;
         const uint16_t cc = a.code[c];
         if (!(cc & CODE_FLUID)) continue;
-        const double* phi = a.phi;
-        double ap = 0.0;
-        if (!(first && a.phi_zero)) {  // from a zero start the first residual is b itself
-            ap = (double)code_ns(cc) * phi[c];
+        const double bc = a.b[c];
+        double rv = bc;
+        if (!from_zero) {
+            const double* phi = a.phi;
+            double ap = (double)code_ns(cc) * phi[c];
 #pragma unroll
             for (int k = 0; k < 6; k++)
                 if ((cc >> k) & 1) ap -= phi[c + nb_off(a.B, k)];
+            rv = bc - ap;
+            acc[0] += rv * rv;
         }
-        const double bc = a.b[c];
-        const double rv = bc - ap;
         const T rt = (T)rv;
         r[c] = rt;
         if (reset_x && sizeof(T) == 4) v.x[c] = (T)0;
-        // FP64 runs at a small fraction of FP32 here: the max norms come from the
-        // stored residual, and the rhs norms are needed by the first residual only
-        acc[0] += rv * rv;
         rmaxT = fmax(rmaxT, fabs(rt));
-        if (first) {
-            acc[2] += bc * bc;
-            acc[3] = fmax(acc[3], fabs(bc));
-        }
+        if (first) acc[2] += bc * bc;
     }
     acc[1] = fmax(acc[1], (double)rmaxT);
-    if (last_block_reduce<4>(acc, 0xA, a.partials, a.counter, scratch)) {
+    if (from_zero) acc[0] = acc[2];
+    if (last_block_reduce<3>(acc, 0x2, a.partials, a.counter, scratch)) {
         if (threadIdx.x == 0) {
             PcgState* s = a.st;
             s->rr = acc[0];
@@ -309,7 +326,6 @@ __global__ void __launch_bounds__(PCG_THREADS) k_residual(const PcgArgs a, Vecs<
             s->rr_update = acc[0];
             if (first) {
                 s->bb = acc[2];
-                s->bmax = acc[3];
                 s->tol_rel2 = a.tol_rel * a.tol_rel * acc[2];
                 s->skip = acc[2] < a.skip_bb ? 1 : 0;
             }
@@ -351,7 +367,7 @@ __global__ void __launch_bounds__(PCG_THREADS) k_black(const PcgArgs a, Vecs<T> 
 // mode 2: beta = z.r / sigma_prev, sigma = z.r                  (after a fold)
 template <typename T>
 __global__ void __launch_bounds__(PCG_THREADS) k_red(const PcgArgs a, Vecs<T> v, int mode) {
-    __shared__ double scratch[32];
+    __shared__ double scratch[PCG_THREADS];
     if (a.st->done) return;
     const int rc = a.st->bufsel & 1;
     const T* r = rc ? v.r[1] : v.r[0];
@@ -405,7 +421,7 @@ __global__ void __launch_bounds__(PCG_THREADS) k_red(const PcgArgs a, Vecs<T> v,
 // s_new = z + beta s_old; q = A' s_new; alpha = sigma / (s.q)
 template <typename T>
 __global__ void __launch_bounds__(PCG_THREADS) k_spmv(const PcgArgs a, Vecs<T> v) {
-    __shared__ double scratch[32];
+    __shared__ double scratch[PCG_THREADS];
     if (a.st->done) return;
     const int sc = (a.st->bufsel >> 1) & 1;
     const double beta = a.st->beta;
@@ -455,7 +471,7 @@ __global__ void __launch_bounds__(PCG_THREADS) k_spmv(const PcgArgs a, Vecs<T> v
 //            zero (red z = r/ns, black z = (r + sum_j r_j/ns_j)/ns)
 template <typename T, int PMODE>
 __global__ void __launch_bounds__(PCG_THREADS) k_update(const PcgArgs a, Vecs<T> v) {
-    __shared__ double scratch[32 * 2];
+    __shared__ double scratch[PCG_THREADS * 2];
     if (a.st->done) return;
     const int rc = a.st->bufsel & 1, sc = (a.st->bufsel >> 1) & 1;
     const T alpha = (T)a.st->alpha;
@@ -536,7 +552,7 @@ __global__ void __launch_bounds__(PCG_THREADS) k_update(const PcgArgs a, Vecs<T>
 // 26 / 55 with neither, 16 / 11 with the face operator alone, 9 / 9 with both,
 // the same from 32^3 to 256^3.  With the rediscretised operator the best sweep
 // counts were 1-2 / 4 / 6 / 8, plus three band sweeps at the surface:
-// 17 iterations and 12.1 ms at 256^3, against 8 iterations and 5.7 ms now
+// 17 iterations and 12.1 ms at 256^3, against 8 iterations and 5.0 ms now
 // (one GB300, half-filled box).
 //
 // MIXED precision: the FP32 recursion is folded into the FP64 solution (true
@@ -549,9 +565,9 @@ __global__ void __launch_bounds__(PCG_THREADS) k_update(const PcgArgs a, Vecs<T>
 constexpr int MIXED_REFINE_DIGITS = 3;
 // Sweeps per level: level 0 / separately launched coarse levels / cluster levels,
 // ms of a solve to 1e-6 (32^3 and 128^3 dam break, 256^3 half filled, random
-// mask 72x100x85): 1/1/1 1.04, 1.86, 5.81, 1.99; 1/2/2 1.01, 1.77, 5.75, 1.87;
-// 2/2/2 0.99, 1.69, 6.00, 1.80; 2/1/1 1.03, 1.99, 6.68, 1.95.  Band sweeps no
-// longer pay: 1/1/1 with two, 1.26, 2.10, 6.12, 2.33.
+// mask 72x100x85): 1/1/1 0.73, 1.52, 5.05, 1.45; 1/2/2 0.68, 1.44, 4.95, 1.38;
+// 2/2/2 0.70, 1.41, 5.28, 1.38; 2/1/1 0.76, 1.66, 5.90, 1.47.  Band sweeps no
+// longer pay: 1/1/1 with two, 0.93, 1.76, 5.35, 1.84.
 constexpr int MG_NU_DEFAULT = 1;         // level 0
 constexpr int MG_NU_COARSE_DEFAULT = 2;  // all coarser levels
 constexpr int MG_BOTTOM_SWEEPS = 4;  // on the <= 4^3 bottom level
@@ -578,8 +594,8 @@ constexpr uint32_t CC_OP = 0x7FFFFF;      // faces and Dirichlet weight
 constexpr uint32_t CC_INTERIOR = 0x24924; // six open faces, no Dirichlet weight
 constexpr int CC_DIRICHLET = 18, CC_SCALE = 23;
 constexpr int DIRICHLET_MAX = 24;         // eighths
-// colour and slab bits of the copies in shared memory
-constexpr uint32_t CS_ODD = 1u << 29, CS_XLO = 1u << 30, CS_XHI = 1u << 31;
+// marks of the copies in shared memory
+constexpr uint32_t CS_ODD = 1u << 29, CS_HIGH = 1u << 30;  // odd x + y + z; upper cell of a z pair
 
 // eight times the diagonal: two per open quarter face plus the Dirichlet eighths
 __device__ __forceinline__ int coarse_diag8(uint32_t cc) {
@@ -784,7 +800,7 @@ __global__ void __launch_bounds__(PCG_THREADS) k_mg_smooth(const PcgArgs A, MGLe
 
 // the last post-smoothing half sweep (red, level 0) fused with z.r (modes 0/1 as k_red)
 __global__ void __launch_bounds__(PCG_THREADS) k_mg_smooth_dot(const PcgArgs A, MGLev L, int mode) {
-    __shared__ double scratch[32];
+    __shared__ double scratch[PCG_THREADS];
     pdl_enter();
     if (A.st->done) return;
     const float* rhs = mg_rhs(A, L);
@@ -839,7 +855,7 @@ __device__ __forceinline__ void residual_quad(const MGLev& L, const float* rhs, 
     unpack4(ld4(rhs + c0), f);
     Q7 q;
     load_q7(q, L.x, c0, L, x, y, z0);
-    if (!any_fluid(cc)) return;
+    if (FINE && !any_fluid(cc)) return;  // (stays zero; a coarse level's quad is written below)
     float out[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) out[i] = is_fluid(cc[i]) ? resid_value(q, i, cc[i], f[i]) * pscale_of(cc[i]) : 0.f;
@@ -854,66 +870,81 @@ __global__ void __launch_bounds__(PCG_THREADS) k_mg_residual(const PcgArgs A, MG
     mg_for_quads<FINE>(A, L, [&](int x, int y, int z0, long long c0) { residual_quad<FINE>(L, rhs, x, y, z0, c0); });
 }
 
-// coarse f = 0.5 * sum_fine P[f,C] r_f  (= 4 R r), per coarse quad:
-// fine z 2 z0 - 1 .. 2 z0 + 8 come from the four fine quads at 2 z0 - 4 .. 2 z0 + 8
-template <bool FINE>
-__device__ __forceinline__ void restrict_quad(const MGLev& F, const MGLev& Cl, int cx, int cy, int cz0, long long ci) {
-    {
-        uint32_t ccc[4];
-        codes4(Cl.ccode, ci, ccc);
-        if (!any_fluid(ccc)) return;
-        float sum[4] = {0.f, 0.f, 0.f, 0.f};
-        const int fz0 = 2 * cz0 - 4;  // first fine z loaded (a multiple of 4)
-        for (int dx = -1; dx <= 2; dx++) {
-            const int fx = 2 * cx + dx;
-            if (fx < 0 || fx >= F.nx) continue;
-            const float wx = (dx == 0 || dx == 1) ? 0.75f : 0.25f;
-            for (int dy = -1; dy <= 2; dy++) {
-                const int fy = 2 * cy + dy;
-                if (fy < 0 || fy >= F.ny) continue;
-                const float wxy = wx * ((dy == 0 || dy == 1) ? 0.75f : 0.25f);
-                const long long row = ((long long)fx * F.ny + fy) * F.pz;
-                // 16 fine values z = fz0 .. fz0 + 15, masked by fine fluid
-                float fr[16];
+// coarse f = 0.5 * sum_fine P[f,C] r_f  (= 4 R r), per coarse quad: the fine
+// plane 2 cx + dx's share (r is zero off the fluid: mg_setup clears level 0's, the
+// coarser residual passes write every quad)
+__device__ __forceinline__ void restrict_plane(const MGLev& F, int cx, int cy, int cz0, int dx, float (&sum)[4]) {
+    const int fx = 2 * cx + dx;
+    if (fx < 0 || fx >= F.nx) return;
+    const float wx = (dx == 0 || dx == 1) ? 0.375f : 0.125f;
+    const int fz = 2 * cz0;  // fine z fz - 1 .. fz + 8
 #pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    const int z = fz0 + 4 * k;
-                    float v[4] = {0.f, 0.f, 0.f, 0.f};
-                    if (z >= 0 && z < F.pz) {
-                        // codes and residual loaded together; r is stale on quads
-                        // without fluid (never written), so the codes mask it
-                        typename LevCode<FINE>::T fc[4];
-                        codes4(LevCode<FINE>::of(F), row + z, fc);
-                        unpack4(ld4(F.r + row + z), v);
+    for (int dy = -1; dy <= 2; dy++) {
+        const int fy = 2 * cy + dy;
+        if (fy < 0 || fy >= F.ny) continue;
+        const float wxy = wx * ((dy == 0 || dy == 1) ? 0.75f : 0.25f);
+        const float* row = F.r + ((long long)fx * F.ny + fy) * F.pz + fz;
+        float fr[10], v[4] = {0.f, 0.f, 0.f, 0.f}, w[4] = {0.f, 0.f, 0.f, 0.f};
+        fr[0] = fz > 0 ? row[-1] : 0.f;
+        if (fz < F.pz) unpack4(ld4(row), v);
+        if (fz + 4 < F.pz) unpack4(ld4(row + 4), w);
 #pragma unroll
-                        for (int e = 0; e < 4; e++)
-                            if (!is_fluid(fc[e])) v[e] = 0.f;
-                    }
-#pragma unroll
-                    for (int e = 0; e < 4; e++) fr[4 * k + e] = v[e];
-                }
-                // coarse lane j takes fine 2(cz0+j) - 1 .. 2(cz0+j) + 2 = fr[3 + 2j .. 6 + 2j]
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    sum[j] += wxy * (0.25f * fr[3 + 2 * j] + 0.75f * fr[4 + 2 * j] + 0.75f * fr[5 + 2 * j] +
-                                     0.25f * fr[6 + 2 * j]);
-            }
+        for (int e = 0; e < 4; e++) {
+            fr[1 + e] = v[e];
+            fr[5 + e] = w[e];
         }
-        float out[4];
-        unpack4(ld4(Cl.f + ci), out);
+        fr[9] = fz + 8 < F.pz ? row[8] : 0.f;
 #pragma unroll
         for (int j = 0; j < 4; j++)
-            if (is_fluid(ccc[j])) out[j] = 0.5f * sum[j];
-        st4(const_cast<float*>(Cl.f) + ci, out);
+            sum[j] += wxy * (0.25f * fr[2 * j] + 0.75f * fr[1 + 2 * j] + 0.75f * fr[2 + 2 * j] + 0.25f * fr[3 + 2 * j]);
     }
 }
+__device__ __forceinline__ void restrict_quad(const MGLev& F, const MGLev& Cl, int cx, int cy, int cz0, long long ci) {
+    uint32_t ccc[4];
+    codes4(Cl.ccode, ci, ccc);
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int dx = -1; dx <= 2; dx++) restrict_plane(F, cx, cy, cz0, dx, sum);
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        if (is_fluid(ccc[j])) const_cast<float*>(Cl.f)[ci + j] = sum[j];
+}
 
-template <bool FINE>
-__global__ void __launch_bounds__(PCG_THREADS) k_mg_restrict(const PcgState* st, MGLev F, MGLev Cl) {
+// Four lanes (l, l + 8, l + 16, l + 24) share a coarse quad, one fine plane each, and
+// a warp's eight quads are neighbours along z (full sectors): with one thread
+// per quad (128 loads one after the other, fine codes among them) a pass took 9-10 us
+// on a small level and 27 us from a half-filled 256^3, now 3-4 and 24.  The coarse
+// level's first half sweep from zero (red: x = f / diagonal) needs nothing else and is
+// done on the way.
+__global__ void __launch_bounds__(PCG_THREADS) k_mg_restrict(const PcgState* st, MGLev F, MGLev Cl, int skip) {
     pdl_enter();
     if (st->done) return;
-    mg_for_range(Cl, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x,
-                 [&](int x, int y, int z0, long long c0) { restrict_quad<FINE>(F, Cl, x, y, z0, c0); });
+    const long long n = (long long)Cl.nx * Cl.ny * (Cl.pz >> 2);
+    const int k = (threadIdx.x & 31) >> 3;
+    const long long step = ((long long)gridDim.x * blockDim.x) >> 2;
+    // whole warps leave together: eight quads per warp, the last ones clamped
+    for (long long i0 = ((long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31)) >> 2; i0 < n; i0 += step) {
+        const long long i = i0 + (threadIdx.x & 7);
+        const bool in = i < n;
+        int cx, cy, cz0;
+        quad_xyz(Cl, in ? i : n - 1, cx, cy, cz0);
+        const long long ci = ((long long)cx * Cl.ny + cy) * Cl.pz + cz0;
+        const uint32_t cc = Cl.ccode[ci + k];
+        float sum[4] = {0.f, 0.f, 0.f, 0.f};
+        // quads without a fluid cell (half of a dam break's) read nothing: 31 to 23 us from
+        // 256^3.  Not on small levels, where the wait for the codes costs 1 us of 4.
+        const unsigned fluid = skip ? __ballot_sync(0xffffffffu, is_fluid(cc)) : 0xffffffffu;
+        if ((fluid >> (threadIdx.x & 7)) & 0x01010101u) restrict_plane(F, cx, cy, cz0, k - 1, sum);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], 8);
+            sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], 16);
+        }
+        if (in && is_fluid(cc)) {
+            const float f = k == 0 ? sum[0] : k == 1 ? sum[1] : k == 2 ? sum[2] : sum[3];
+            const_cast<float*>(Cl.f)[ci + k] = f;
+            if (((cx + cy + cz0 + k) & 1) == 0) Cl.x[ci + k] = coarse_solve(cc, f, 0.f);
+        }
+    }
 }
 
 // fine x += P x_coarse on fluid fine cells, per fine quad: the quad's coarse z
@@ -1028,7 +1059,7 @@ __global__ void __launch_bounds__(PCG_THREADS) k_mg_smooth_bnd(const PcgArgs A, 
 // ---- MG-path PCG kernels on quads (level 0, FP32) ------------------------------
 // s_new = z + beta s_old; q = A' s_new; alpha = sigma / (s.q)
 __global__ void __launch_bounds__(PCG_THREADS) k_spmv_q(const PcgArgs a, Vecs<float> v, MGLev L) {
-    __shared__ double scratch[32];
+    __shared__ double scratch[PCG_THREADS];
     pdl_enter();
     if (a.st->done) return;
     const int sc = (a.st->bufsel >> 1) & 1;
@@ -1086,10 +1117,12 @@ __global__ void __launch_bounds__(PCG_THREADS) k_spmv_q(const PcgArgs a, Vecs<fl
     }
 }
 
-// x += alpha s; r_new = r - alpha q; r.r, max|r|; first red-black sweep of the
-// V-cycle from zero on r_new (red z = r/ns, black z = (r + sum_j r_j/ns_j)/ns)
+// x += alpha s; r_new = r - alpha q; r.r, max|r|; z = r_new / ns, the first red half
+// sweep of the V-cycle from zero (the black one follows as a pass of its own: done
+// here it needed r_new / ns of every neighbour from r, q and the codes, 90 us at
+// 256^3 against 40 + 20)
 __global__ void __launch_bounds__(PCG_THREADS) k_update_q(const PcgArgs a, Vecs<float> v, MGLev L) {
-    __shared__ double scratch[32 * 2];
+    __shared__ double scratch[PCG_THREADS * 2];
     pdl_enter();
     if (a.st->done) return;
     const int rc = a.st->bufsel & 1, sc = (a.st->bufsel >> 1) & 1;
@@ -1097,57 +1130,32 @@ __global__ void __launch_bounds__(PCG_THREADS) k_update_q(const PcgArgs a, Vecs<
     const float* ro = rc ? v.r[1] : v.r[0];
     float* rn = rc ? v.r[0] : v.r[1];
     const float* s = sc ? v.s[1] : v.s[0];
-    const long long sx = lev_sx(L), sy = L.pz;
     Acc<float> rr;
     float rmax = 0.f;
     mg_for_quads<true>(a, L, [&](int x, int y, int z0, long long c0) {
         uint16_t cc[4];
         codes4(a.code, c0, cc);
-        if (!any_fluid(cc)) return;
-        float sv[4], xv[4];
+        float sv[4], xv[4], rv[4], qv[4], zv[4];
         unpack4(ld4(s + c0), sv);
         unpack4(ld4(v.x + c0), xv);
-        Q7 rq, qq;
-        load_q7(rq, ro, c0, L, x, y, z0);
-        load_q7(qq, v.q, c0, L, x, y, z0);
-        // neighbour codes for their 1/ns
-        uint16_t cxp[4], cxm[4], cyp[4], cym[4];
-        codes4_nb(a.code, c0 + sx, x + 1 < L.nx, cxp);
-        codes4_nb(a.code, c0 - sx, x > 0, cxm);
-        codes4_nb(a.code, c0 + sy, y + 1 < L.ny, cyp);
-        codes4_nb(a.code, c0 - sy, y > 0, cym);
-        const uint16_t czm = z0 > 0 ? a.code[c0 - 1] : 0, czp = z0 + 4 < L.pz ? a.code[c0 + 4] : 0;
-        Q7 w;  // r_new / ns around the quad
-        float rnc[4];
+        unpack4(ld4(ro + c0), rv);
+        unpack4(ld4(v.q + c0), qv);
+        if (!any_fluid(cc)) return;
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            rnc[i] = rq.c[i] - alpha * qq.c[i];
-            w.c[i] = rnc[i] * c_rcp[code_ns(cc[i])];
-            w.xp[i] = (rq.xp[i] - alpha * qq.xp[i]) * c_rcp[code_ns(cxp[i])];
-            w.xm[i] = (rq.xm[i] - alpha * qq.xm[i]) * c_rcp[code_ns(cxm[i])];
-            w.yp[i] = (rq.yp[i] - alpha * qq.yp[i]) * c_rcp[code_ns(cyp[i])];
-            w.ym[i] = (rq.ym[i] - alpha * qq.ym[i]) * c_rcp[code_ns(cym[i])];
-        }
-        w.zm = (rq.zm - alpha * qq.zm) * c_rcp[code_ns(czm)];
-        w.zp = (rq.zp - alpha * qq.zp) * c_rcp[code_ns(czp)];
-        const int par = (x + y + z0) & 1;
-        float zv[4], rout[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
+            zv[i] = 0.f;
             if (!(cc[i] & CODE_FLUID)) {
-                zv[i] = 0.f;
-                rout[i] = 0.f;
+                rv[i] = 0.f;
                 continue;
             }
             xv[i] += alpha * sv[i];
-            rout[i] = rnc[i];
-            rr.add(rnc[i] * rnc[i]);
-            rmax = fmaxf(rmax, fabsf(rnc[i]));
-            if (((par ^ i) & 1) == 0) zv[i] = w.c[i];  // red
-            else zv[i] = (rnc[i] + nbsum(w, i, cc[i])) * c_rcp[code_ns(cc[i])];
+            rv[i] -= alpha * qv[i];
+            rr.add(rv[i] * rv[i]);
+            rmax = fmaxf(rmax, fabsf(rv[i]));
+            zv[i] = rv[i] * c_rcp[code_ns(cc[i])];
         }
         st4(v.x + c0, xv);
-        st4(rn + c0, rout);
+        st4(rn + c0, rv);
         st4(v.z + c0, zv);
     });
     double acc[2] = {rr.value(), (double)rmax};
@@ -1230,12 +1238,11 @@ __global__ void __launch_bounds__(1024) k_mg_bottom(const PcgState* st, MGLev L)
 // each pass sees the previous pass's global writes).  Replaces ~11 launches per
 // level of latency-bound small kernels.
 constexpr int MG_MAX_LEVELS = 12;
-constexpr int MG_CLUSTER_THREADS = 1024;
-// Largest level handed to the cluster kernel.  At 256^3 the 64^3 level (262k
-// cells) ran ~8 us per pass on the cluster's 16 SMs and is faster as separate
-// full-GPU launches (35.6 -> 37.5 steps/s); moving the 32^3 level out as well
-// changed nothing.
-constexpr long long MG_CLUSTER_CELLS = 40000;
+constexpr int MG_CLUSTER_THREADS = 512;
+// Largest level handed to the cluster kernel: 32^3 and its like.  A pass over 32^3
+// takes the cluster ~1.3 us and a launch of its own ~3.8; the 64^3 level (262k cells)
+// would not fit the cluster's shared memory, and takes 3.9 us a pass in launches.
+constexpr long long MG_CLUSTER_CELLS = 60000;
 constexpr int MG_CLUSTER_SMEM = 200 * 1024;  // dynamic shared memory limit of the cluster kernel
 
 struct MGChain {
@@ -1251,191 +1258,142 @@ struct MGChain {
     int soff;
 };
 
-// ---- the smallest levels in one CTA's shared memory ----------------------------
-// Levels with at most MG_SMEM_CELLS cells are copied (dense, z fastest) into
-// shared memory and run their part of the V-cycle there: the same red-black
-// Gauss-Seidel, full-weighting restriction (x 0.5) and trilinear prolongation
-// as the global kernels, with __syncthreads between passes instead of cluster
-// barriers and global-memory round trips.
-constexpr int MG_SMEM_CELLS = 4096;
+// ---- levels in shared memory ----------------------------------------------------
+// A level (or a CTA's x slab of one) in shared memory.  Pairs of z-neighbouring
+// cells (2j, 2j + 1) hold one cell of either colour, so x, f, the codes and the
+// reciprocal diagonals are kept as a red and a black array indexed by pair: a half
+// sweep over one colour reads the other colour's array at p, p +- 1, p +- row and
+// p +- plane, free of bank conflicts.  x has a guard plane on either side, rows are
+// padded to whole pairs, so every neighbour's slot exists and is finite.  A slab's
+// guard planes hold its neighbours' boundary planes: whoever writes a boundary
+// cell also writes it there (distributed shared memory), and the cluster barrier
+// separates the passes.  (The passes copy it: a store to the pool could change the
+// shared one.)  The pre-smoothing ends with the black cells and the
+// post-smoothing starts with them, so only red cells have a residual and only red
+// cells need the coarse correction.
+// What bounds it is latency: barriers, shared-memory round trips, and the kernel's own
+// instructions.  It runs once per V-cycle between kernels that stream through the
+// caches, so its code is fetched anew each time: the passes are small functions shared
+// by all levels, not inlined, and only the smoother keeps the operator in registers
+// and is unrolled.  From 16^3 down (32^3 grid) / from 32^3 down on a 128^3 and on a
+// 256^3 grid: 23, 38 and 51 us; with everything inlined and unrolled 19, 39 and 72;
+// with the codes decoded in every pass, both colours in one array and the boundary
+// planes read over the cluster, 29, 49 and 68.
+constexpr int MG_SMEM_CELLS = 4096;  // padded cells of a level rank 0 runs alone
 
 struct SLev {
-    int nx, ny, nz, n;
-    float *x, *f, *r;
-    uint32_t* code;
+    int nx, ny, nz, pr, plane;  // global cells per axis, pairs per row and per plane
+    int x0, P, np, n;           // first plane, planes per CTA, planes and pairs held
+    int xo, xc;                 // pool offset of red x (black: + xc)
+    int fo, fc;                 // red f (black: + fc); then codes, diagonals (red, black) and r
+    float *lo, *hi;             // the neighbours' copies of the first / last red plane, or null
 };
+extern __shared__ float pool[];
+__device__ __forceinline__ int slev_co(const SLev& L) { return L.fo + 2 * L.fc; }
+__device__ __forceinline__ int slev_do(const SLev& L) { return L.fo + 4 * L.fc; }
+__device__ __forceinline__ int slev_ro(const SLev& L) { return L.fo + 6 * L.fc; }
 
-__device__ __forceinline__ int sidx(const SLev& L, int x, int y, int z) { return (x * L.ny + y) * L.nz + z; }
-
-// Each thread holds at most four cells of a shared-memory level (<= 4096 cells,
-// 1024 threads): a pass computes all of them before it stores any, so their
-// loads overlap (a half sweep's cells read only the other colour)
-constexpr int SCELLS_PER_THREAD = 4;
-static_assert(SCELLS_PER_THREAD * MG_CLUSTER_THREADS >= MG_SMEM_CELLS, "shared-memory level cells per thread");
-
-__device__ void s_smooth(const SLev L, int color) {
-    const int sx = L.ny * L.nz, sy = L.nz;
-    float nv[SCELLS_PER_THREAD];
-    bool act[SCELLS_PER_THREAD];
-#pragma unroll
-    for (int k = 0; k < SCELLS_PER_THREAD; k++) {
-        const int i = threadIdx.x + k * MG_CLUSTER_THREADS;
-        act[k] = false;
-        nv[k] = 0.f;
-        if (i >= L.n) continue;
-        const uint32_t cc = L.code[i];
-        if (!smem_color(cc, color)) continue;
-        act[k] = true;
-        nv[k] = coarse_solve(cc, L.f[i], smem_nbsum4(L.x, i, cc, sx, sy));
-    }
-#pragma unroll
-    for (int k = 0; k < SCELLS_PER_THREAD; k++)
-        if (act[k]) L.x[threadIdx.x + k * MG_CLUSTER_THREADS] = nv[k];
-    __syncthreads();
+// floats of a level with `planes` planes
+__host__ __device__ inline long long slev_floats(int planes, int ny, int nz) {
+    const long long plane = (long long)ny * ((nz + 1) / 2);
+    return plane * (9ll * planes + 4);
+}
+__device__ __forceinline__ void slev_make(SLev& L, const MGLev& G, int off, int planes, int x0) {
+    L.nx = G.nx; L.ny = G.ny; L.nz = G.nz;
+    L.pr = (G.nz + 1) >> 1;
+    L.plane = G.ny * L.pr;
+    L.x0 = x0;
+    L.P = planes;
+    L.np = max(0, min(planes, G.nx - x0));
+    L.n = L.np * L.plane;
+    L.xc = (planes + 2) * L.plane;
+    L.fc = planes * L.plane;
+    L.xo = off + L.plane;
+    L.fo = off + 2 * L.xc;
+    L.lo = L.hi = nullptr;
+}
+// pair p: plane, row, place along z; par: its red cell is at z = 2j + par
+__device__ __forceinline__ void slev_pair(const SLev& L, int p, int& xl, int& y, int& j, int& par) {
+    const int row = (int)((unsigned)p / (unsigned)L.pr);
+    j = p - row * L.pr;
+    xl = (int)((unsigned)row / (unsigned)L.ny);
+    y = row - xl * L.ny;
+    par = (L.x0 + xl + y) & 1;
 }
 
-__device__ void s_residual(const SLev L) {
-    const int sx = L.ny * L.nz, sy = L.nz;
-    float rv[SCELLS_PER_THREAD];
+// codes (with the cell's place in its pair) and diagonals from global memory; x, f
+// and r to zero (the guard planes too)
+__device__ __noinline__ void slev_init(const SLev& SL, const MGLev& G) {
+    const SLev L = SL;
+    for (int i = threadIdx.x; i < 2 * L.xc; i += blockDim.x) pool[L.xo - L.plane + i] = 0.f;
+#pragma unroll 1
+    for (int p = threadIdx.x; p < L.n; p += blockDim.x) {
+        int xl, y, j, par;
+        slev_pair(L, p, xl, y, j, par);
+        const uint32_t* row = G.ccode + ((long long)(L.x0 + xl) * G.ny + y) * G.pz + 2 * j;
 #pragma unroll
-    for (int k = 0; k < SCELLS_PER_THREAD; k++) {
-        const int i = threadIdx.x + k * MG_CLUSTER_THREADS;
-        rv[k] = 0.f;
-        if (i >= L.n) continue;
-        const uint32_t cc = L.code[i];
-        if (is_fluid(cc))
-            rv[k] = coarse_resid(cc, L.f[i], L.x[i], smem_nbsum4(L.x, i, cc, sx, sy)) * coarse_pscale(cc);
+        for (int c = 0; c < 2; c++) {
+            const int e = par ^ c;
+            const uint32_t cc = 2 * j + e < L.nz ? row[e] : 0u;
+            pool[slev_co(L) + c * L.fc + p] = __uint_as_float(cc | (e ? CS_HIGH : 0u));
+            pool[slev_do(L) + c * L.fc + p] =
+                is_fluid(cc) ? __fdividef(8.f, small_float((uint32_t)coarse_diag8(cc))) : 0.f;
+            pool[L.fo + c * L.fc + p] = 0.f;
+        }
+        pool[slev_ro(L) + p] = 0.f;
     }
+}
+__device__ __noinline__ void slev_load_f(const SLev& SL, const MGLev& G) {
+    const SLev L = SL;
+#pragma unroll 1
+    for (int p = threadIdx.x; p < L.n; p += blockDim.x) {
+        int xl, y, j, par;
+        slev_pair(L, p, xl, y, j, par);
+        const float* row = G.f + ((long long)(L.x0 + xl) * G.ny + y) * G.pz + 2 * j;
 #pragma unroll
-    for (int k = 0; k < SCELLS_PER_THREAD; k++) {
-        const int i = threadIdx.x + k * MG_CLUSTER_THREADS;
-        if (i < L.n) L.r[i] = rv[k];
+        for (int c = 0; c < 2; c++)
+            if (pool[slev_do(L) + c * L.fc + p] != 0.f) pool[L.fo + c * L.fc + p] = row[par ^ c];
     }
-    __syncthreads();
+}
+__device__ __noinline__ void slev_store_x(const SLev& SL, const MGLev& G) {
+    const SLev L = SL;
+#pragma unroll 1
+    for (int p = threadIdx.x; p < L.n; p += blockDim.x) {
+        int xl, y, j, par;
+        slev_pair(L, p, xl, y, j, par);
+        float* row = G.x + ((long long)(L.x0 + xl) * G.ny + y) * G.pz + 2 * j;
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            const int e = par ^ c;
+            if (2 * j + e < L.nz) row[e] = pool[L.xo + c * L.xc + p];
+        }
+    }
 }
 
-__device__ __forceinline__ float fw_weight(int d) { return (d == 0 || d == 1) ? 0.75f : 0.25f; }
-
-// coarse f = 0.5 * sum_fine P r (fine fluid only), coarse x = 0
-__device__ void s_restrict(const SLev F, const SLev C) {
-    for (int i = threadIdx.x; i < C.n; i += blockDim.x) {
-        const int cz = i % C.nz, cy = (i / C.nz) % C.ny, cx = i / (C.nz * C.ny);
-        C.x[i] = 0.f;
-        if (!is_fluid(C.code[i])) {
-            C.f[i] = 0.f;
-            continue;
-        }
-        // the fine residual is zero off the fine fluid cells (s_residual)
-        float sum = 0.f;
-#pragma unroll
-        for (int dx = -1; dx <= 2; dx++) {
-            const int fx = 2 * cx + dx;
-            if (fx < 0 || fx >= F.nx) continue;
-#pragma unroll
-            for (int dy = -1; dy <= 2; dy++) {
-                const int fy = 2 * cy + dy;
-                if (fy < 0 || fy >= F.ny) continue;
-                const float wxy = fw_weight(dx) * fw_weight(dy);
-                const int row = sidx(F, fx, fy, 0);
-#pragma unroll
-                for (int dz = -1; dz <= 2; dz++) {
-                    const int fz = 2 * cz + dz;
-                    if (fz < 0 || fz >= F.nz) continue;
-                    sum += wxy * fw_weight(dz) * F.r[row + fz];
-                }
-            }
-        }
-        C.f[i] = 0.5f * sum;
-    }
-    __syncthreads();
+// sum of (open quarters * neighbour) around the cell of colour c in pair p, from the
+// other colour's x (all loads are independent of each other and of the code's)
+__device__ __forceinline__ float slev_sum4(const SLev& L, int c, int p, uint32_t cc) {
+    const float* o = pool + L.xo + (1 - c) * L.xc + p;
+    const float a = o[L.plane], b = o[-L.plane], d = o[L.pr], f = o[-L.pr], m = o[0], lo = o[-1], hi = o[1];
+    const float zp = (cc & CS_HIGH) ? hi : m, zm = (cc & CS_HIGH) ? m : lo;
+    if ((cc & CC_OP) == CC_INTERIOR) return 4.f * ((a + b) + (d + f) + (zp + zm));
+    return (coarse_face(cc, 0) * a + coarse_face(cc, 1) * b) + (coarse_face(cc, 2) * d + coarse_face(cc, 3) * f) +
+           (coarse_face(cc, 4) * zp + coarse_face(cc, 5) * zm);
 }
-
-// fine x += P x_coarse on fluid fine cells (coarse fluid values only)
-__device__ void s_prolong(const SLev F, const SLev C) {
-    for (int i = threadIdx.x; i < F.n; i += blockDim.x) {
-        if (!is_fluid(F.code[i])) continue;
-        const int z = i % F.nz, y = (i / F.nz) % F.ny, x = i / (F.nz * F.ny);
-        const int p[3] = {(x & 1) ? x >> 1 : (x >> 1) - 1, (y & 1) ? y >> 1 : (y >> 1) - 1,
-                          (z & 1) ? z >> 1 : (z >> 1) - 1};
-        const float wl[3] = {(x & 1) ? 0.75f : 0.25f, (y & 1) ? 0.75f : 0.25f, (z & 1) ? 0.75f : 0.25f};
-        float sum = 0.f;
-        for (int o = 0; o < 8; o++) {
-            const int ox = o >> 2, oy = (o >> 1) & 1, oz = o & 1;
-            const int cx = p[0] + ox, cy = p[1] + oy, cz = p[2] + oz;
-            if (cx < 0 || cy < 0 || cz < 0 || cx >= C.nx || cy >= C.ny || cz >= C.nz) continue;
-            const int ci = sidx(C, cx, cy, cz);
-            if (!is_fluid(C.code[ci])) continue;
-            sum += (ox ? 1.f - wl[0] : wl[0]) * (oy ? 1.f - wl[1] : wl[1]) * (oz ? 1.f - wl[2] : wl[2]) * C.x[ci];
-        }
-        F.x[i] += sum * coarse_pscale(F.code[i]);
-    }
-    __syncthreads();
+__device__ __forceinline__ void slev_put(const SLev& L, int c, int p, float v) {
+    pool[L.xo + c * L.xc + p] = v;
+    if (L.lo && p < L.plane) L.lo[c * L.xc + p] = v;
+    if (L.hi && p >= L.n - L.plane) L.hi[c * L.xc + p - (L.n - L.plane)] = v;
 }
-
-// Levels ls..last in one CTA's shared memory, dense (z fastest), laid out from
-// `smem` level by level: x, f, r (n floats each), then the codes (n words).  load_f: level ls's rhs comes from global memory
-// (otherwise the caller's restriction writes it into this layout).
-__device__ void smem_levels_init(const MGChain& C, float* smem, SLev* S, bool load_f) {
-    if (threadIdx.x == 0) {
-        float* p = smem;
-        for (int l = C.ls; l <= C.last; l++) {
-            const MGLev& G = C.lev[l];
-            SLev& L = S[l];
-            L.nx = G.nx; L.ny = G.ny; L.nz = G.nz;
-            L.n = G.nx * G.ny * G.nz;
-            L.x = p; p += L.n;
-            L.f = p; p += L.n;
-            L.r = p; p += L.n;
-            L.code = reinterpret_cast<uint32_t*>(p);
-            p += L.n;
-        }
-    }
-    __syncthreads();
-    for (int l = C.ls; l <= C.last; l++) {
-        const MGLev& G = C.lev[l];
-        const SLev L = S[l];
-        for (int i = threadIdx.x; i < L.n; i += blockDim.x) {
-            const int z = i % L.nz, t = i / L.nz;
-            const long long gi = (long long)t * G.pz + z;
-            const int odd = (t / L.ny + t % L.ny + z) & 1;
-            L.code[i] = G.ccode[gi] | (odd ? CS_ODD : 0);
-            L.x[i] = 0.f;
-            if (l == C.ls && load_f) L.f[i] = G.f[gi];
-        }
-    }
-    __syncthreads();
-}
-
-// the V-cycle over those levels; store_x: level ls's correction goes back to
-// global memory (otherwise the caller's prolongation reads it in place)
-__device__ void smem_levels_run(const MGChain& C, const SLev* S, bool store_x) {
-    for (int l = C.ls; l < C.last; l++) {
-        for (int k = 0; k < C.nu; k++) {
-            s_smooth(S[l], 0);
-            s_smooth(S[l], 1);
-        }
-        s_residual(S[l]);
-        s_restrict(S[l], S[l + 1]);
-    }
-    for (int k = 0; k < MG_BOTTOM_SWEEPS; k++) {
-        s_smooth(S[C.last], 0);
-        s_smooth(S[C.last], 1);
-    }
-    for (int k = 0; k < MG_BOTTOM_SWEEPS; k++) {
-        s_smooth(S[C.last], 1);
-        s_smooth(S[C.last], 0);
-    }
-    for (int l = C.last - 1; l >= C.ls; l--) {
-        s_prolong(S[l], S[l + 1]);
-        for (int k = 0; k < C.nu; k++) {
-            s_smooth(S[l], 1);
-            s_smooth(S[l], 0);
-        }
-    }
-    if (store_x) {
-        const MGLev& G = C.lev[C.ls];
-        for (int i = threadIdx.x; i < S[C.ls].n; i += blockDim.x)
-            G.x[(long long)(i / S[C.ls].nz) * G.pz + (i % S[C.ls].nz)] = S[C.ls].x[i];
+// scaled residual of the red cells (the black ones, just updated, have none)
+__device__ __noinline__ void slev_resid(const SLev& SL) {
+    const SLev L = SL;
+#pragma unroll 1
+    for (int p = threadIdx.x; p < L.n; p += blockDim.x) {
+        const uint32_t cc = __float_as_uint(pool[slev_co(L) + p]);
+        if (!is_fluid(cc)) continue;
+        pool[slev_ro(L) + p] =
+            coarse_resid(cc, pool[L.fo + p], pool[L.xo + p], slev_sum4(L, 0, p, cc)) * coarse_pscale(cc);
     }
 }
 
@@ -1452,41 +1410,6 @@ __device__ __forceinline__ unsigned cluster_size() {
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
     return n;
 }
-
-
-// ---- cluster levels held in distributed shared memory ------------------------
-// With MGChain::slab set, every CTA of the cluster holds P consecutive x planes
-// of each level lc .. ls-1 in its own shared memory (x, f, r and the codes, at
-// the same offsets in every CTA) and reads its neighbours' boundary planes
-// through distributed shared memory; the cluster barrier separates the passes.
-// The restriction into level ls writes straight into rank 0's shared-memory
-// levels, and the prolongation from ls reads them there, so only level lc's
-// rhs comes from global memory and only its correction goes back.
-// (CS_XLO / CS_XHI in the slab copies' codes: x - 1 / x + 1 lies in the previous / next CTA)
-
-struct DLev {
-    float *x, *f, *r;
-    uint32_t* code;
-    int nx, ny, nz, P, np, x0, plane;
-};
-
-__device__ __forceinline__ DLev dlev(const MGChain& C, int l, float* pool, unsigned rank) {
-    const MGLev& G = C.lev[l];
-    DLev D;
-    D.nx = G.nx; D.ny = G.ny; D.nz = G.nz;
-    D.P = C.P[l];
-    D.plane = G.ny * G.nz;
-    D.x0 = (int)rank * D.P;
-    D.np = max(0, min(D.P, G.nx - D.x0));
-    const int m = D.P * D.plane;
-    float* p = pool + C.off[l];
-    D.x = p;
-    D.f = p + m;
-    D.r = p + 2 * m;
-    D.code = reinterpret_cast<uint32_t*>(p + 3 * m);
-    return D;
-}
-
 // the same shared-memory location in cluster CTA `rank` (generic address)
 template <typename T>
 __device__ __forceinline__ T* dsm(T* p, unsigned rank) {
@@ -1495,202 +1418,249 @@ __device__ __forceinline__ T* dsm(T* p, unsigned rank) {
     return reinterpret_cast<T*>(out);
 }
 
-__device__ __forceinline__ float slab_nbsum4(const DLev& D, int i, uint32_t cc, const float* xp, const float* xn) {
-    if ((cc & (CC_OP | CS_XLO | CS_XHI)) == CC_INTERIOR)
-        return 4.f * (D.x[i + D.plane] + D.x[i - D.plane] + D.x[i + D.nz] + D.x[i - D.nz] + D.x[i + 1] + D.x[i - 1]);
-    float s = 0.f;
-    if (cc & 7u) s += coarse_face(cc, 0) * ((cc & CS_XHI) ? xn[i - (D.np - 1) * D.plane] : D.x[i + D.plane]);
-    if (cc & (7u << 3)) s += coarse_face(cc, 1) * ((cc & CS_XLO) ? xp[i + (D.P - 1) * D.plane] : D.x[i - D.plane]);
-    if (cc & (7u << 6)) s += coarse_face(cc, 2) * D.x[i + D.nz];
-    if (cc & (7u << 9)) s += coarse_face(cc, 3) * D.x[i - D.nz];
-    if (cc & (7u << 12)) s += coarse_face(cc, 4) * D.x[i + 1];
-    if (cc & (7u << 15)) s += coarse_face(cc, 5) * D.x[i - 1];
-    return s;
+// who runs a level: one warp, one CTA or the cluster
+enum { SYNC_WARP, SYNC_CTA, SYNC_CLUSTER };
+__device__ __forceinline__ void level_sync(int sync) {
+    if (sync == SYNC_CLUSTER) cluster_barrier();
+    else if (sync == SYNC_CTA) __syncthreads();
+    else __syncwarp();
 }
 
-// red-black half sweep; first: the other colour is still zero
-__device__ void slab_smooth(const DLev& D, int color, bool first, const float* xp, const float* xn) {
-    const int n = D.np * D.plane;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const uint32_t cc = D.code[i];
-        if (!smem_color(cc, color)) continue;
-        D.x[i] = coarse_solve(cc, D.f[i], first ? 0.f : slab_nbsum4(D, i, cc, xp, xn));
+// A cell's update in registers.  The six face weights (0, 1/4 .. 1) are three pairs of
+// 16-bit floats, which hold them exactly and unpack with one instruction each: an
+// update is 7 loads and ~25 instructions, half of what decoding the code takes.
+struct SOp {
+    uint32_t x, y, z;  // z: the pair's other cell, then the next pair's
+    float di, f;       // sign of di: set if the next pair is the one above
+};
+__device__ __forceinline__ uint32_t face_pair(uint32_t cc, int k) {
+    return (__float_as_uint(0.25f * coarse_face(cc, k)) >> 16) | __float_as_uint(0.25f * coarse_face(cc, k + 1));
+}
+__device__ __forceinline__ SOp slev_op(const SLev& L, int c, int p) {
+    const float* fp = pool + L.fo + c * L.fc + p;
+    const uint32_t cc = __float_as_uint(fp[2 * L.fc]), z = face_pair(cc, 4);
+    const bool high = (cc & CS_HIGH) != 0;
+    SOp o;
+    o.x = face_pair(cc, 0);
+    o.y = face_pair(cc, 2);
+    o.z = high ? (z << 16) | (z >> 16) : z;
+    o.di = high ? -fp[4 * L.fc] : fp[4 * L.fc];
+    o.f = fp[0];
+    return o;
+}
+__device__ __forceinline__ float w_lo(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float w_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+__device__ __forceinline__ void slev_update(const SLev& L, int c, int p, const SOp& op) {
+    const float* o = pool + L.xo + (1 - c) * L.xc + p;
+    const float xp = o[L.plane], xm = o[-L.plane], yp = o[L.pr], ym = o[-L.pr], m = o[0];
+    const float zn = o[signbit(op.di) ? 1 : -1];
+    const float sum = (w_lo(op.x) * xp + w_hi(op.x) * xm) + (w_lo(op.y) * yp + w_hi(op.y) * ym) +
+                      (w_lo(op.z) * m + w_hi(op.z) * zn);
+    slev_put(L, c, p, fabsf(op.di) * (op.f + sum));
+}
+// `passes` half sweeps, alternating, colour c first, by nt threads
+constexpr int SLEV_PAIRS = 4;  // pairs a thread keeps the operator of
+__device__ __noinline__ void level_smooth(const SLev& SL, int passes, int c, int sync, int nt) {
+    const SLev L = SL;
+    const int t = threadIdx.x;
+    if (L.n <= SLEV_PAIRS * nt) {
+        SOp op[2][SLEV_PAIRS];
+#pragma unroll
+        for (int i = 0; i < SLEV_PAIRS; i++) {
+            if (t + i * nt >= L.n) break;
+            op[0][i] = slev_op(L, c, t + i * nt);
+            op[1][i] = slev_op(L, 1 - c, t + i * nt);
+        }
+#pragma unroll 1
+        for (int k = 0; k < passes; k += 2) {
+#pragma unroll
+            for (int i = 0; i < SLEV_PAIRS; i++) {
+                if (t + i * nt >= L.n) break;
+                slev_update(L, c, t + i * nt, op[0][i]);
+            }
+            level_sync(sync);
+            if (k + 1 == passes) break;
+#pragma unroll
+            for (int i = 0; i < SLEV_PAIRS; i++) {
+                if (t + i * nt >= L.n) break;
+                slev_update(L, 1 - c, t + i * nt, op[1][i]);
+            }
+            level_sync(sync);
+        }
+        return;
+    }
+#pragma unroll 1
+    for (int k = 0; k < passes; k++) {
+#pragma unroll 1
+        for (int p = t; p < L.n; p += nt) slev_update(L, c ^ (k & 1), p, slev_op(L, c ^ (k & 1), p));
+        level_sync(sync);
     }
 }
 
-__device__ void slab_residual(const DLev& D, const float* xp, const float* xn) {
-    const int n = D.np * D.plane;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const uint32_t cc = D.code[i];
-        float rv = 0.f;
-        if (is_fluid(cc)) rv = coarse_resid(cc, D.f[i], D.x[i], slab_nbsum4(D, i, cc, xp, xn)) * coarse_pscale(cc);
-        D.r[i] = rv;
-    }
-}
+__device__ __forceinline__ float fw_weight(int d) { return (d == 0 || d == 1) ? 0.75f : 0.25f; }
 
-// coarse f = 0.5 * sum_fine P r from level l's slabs (r is zero off the fluid)
-// into level l + 1: the CTA's own slab, or rank 0's first shared-memory level
-// (its cells spread over the whole cluster)
-__device__ void slab_restrict(const MGChain& C, int l, float* pool, unsigned rank, unsigned cs, float* spool) {
-    const DLev F = dlev(C, l, pool, rank);
-    const MGLev& Gc = C.lev[l + 1];
-    const bool to_slab = l + 1 < C.ls;
-    const DLev D = dlev(C, l + 1, pool, rank);  // used only when to_slab
-    const int nsm = Gc.nx * Gc.ny * Gc.nz;
-    const int n = to_slab ? D.np * D.plane : nsm;
-    const int i0 = to_slab ? (int)threadIdx.x : (int)(rank * blockDim.x + threadIdx.x);
-    const int step = to_slab ? (int)blockDim.x : (int)(cs * blockDim.x);
-    float* fout = to_slab ? D.f : dsm(spool + nsm, 0);
-    const uint32_t* cin = to_slab ? D.code : reinterpret_cast<const uint32_t*>(dsm(spool + 3 * nsm, 0));
-    for (int i = i0; i < n; i += step) {
-        int cx, cy, cz;
-        if (to_slab) {
-            const int xl = i / D.plane, t = i - xl * D.plane;
-            cx = D.x0 + xl;
-            cy = t / Gc.nz;
-            cz = t - cy * Gc.nz;
-        } else {
-            cz = i % Gc.nz;
-            const int t = i / Gc.nz;
-            cy = t % Gc.ny;
-            cx = t / Gc.ny;
-        }
-        if (!is_fluid(cin[i])) {
-            fout[i] = 0.f;
-            continue;
-        }
+// D.f = 0.5 * sum P r over the red fine cells of F.  Fine plane fx lies in cluster CTA
+// fx / F.P; D's pairs i0, i0 + step, ... are this thread's, in CTA `drank`.
+__device__ __noinline__ void slev_restrict(const SLev& SF, const SLev& SD, int dn, int i0, int step, unsigned drank) {
+    const SLev F = SF, D = SD;
+    float* f = dsm(pool + D.fo, drank);
+    const float* diag = dsm(pool + slev_do(D), drank);
+#pragma unroll 1
+    for (int i = i0; i < 2 * dn; i += step) {
+        const int c = i >= dn, p = i - c * dn;
+        if (diag[c * D.fc + p] == 0.f) continue;
+        int xl, cy, j, par;
+        slev_pair(D, p, xl, cy, j, par);
+        const int cx = D.x0 + xl, cz = 2 * j + (par ^ c);
         float sum = 0.f;
+#pragma unroll
         for (int dx = -1; dx <= 2; dx++) {
             const int fx = 2 * cx + dx;
             if (fx < 0 || fx >= F.nx) continue;
-            const unsigned ro = (unsigned)(fx / F.P);
-            const float* rp = (ro == rank ? F.r : dsm(F.r, ro)) + (fx - (int)ro * F.P) * F.plane;
+            const int ro = (int)((unsigned)fx / (unsigned)F.P);
+            const float* plane = dsm(pool + slev_ro(F) + (fx - ro * F.P) * F.plane, (unsigned)ro);
 #pragma unroll
             for (int dy = -1; dy <= 2; dy++) {
                 const int fy = 2 * cy + dy;
                 if (fy < 0 || fy >= F.ny) continue;
-                const float wxy = fw_weight(dx) * fw_weight(dy);
-                const float* row = rp + fy * F.nz;
-#pragma unroll
-                for (int dz = -1; dz <= 2; dz++) {
-                    const int fz = 2 * cz + dz;
-                    if (fz < 0 || fz >= F.nz) continue;
-                    sum += wxy * fw_weight(dz) * row[fz];
-                }
+                // red: dz has the parity of dx + dy; dz = -1, 1 lie in pairs cz - 1 and cz, dz = 0, 2
+                // in cz and cz + 1
+                const bool odd = ((dx + dy) & 1) != 0;
+                const int ja = odd ? cz - 1 : cz;
+                const float* r = plane + fy * F.pr + ja;
+                const float ra = ja >= 0 ? r[0] : 0.f, rb = ja + 1 < F.pr ? r[1] : 0.f;
+                sum += fw_weight(dx) * fw_weight(dy) * (odd ? 0.25f * ra + 0.75f * rb : 0.75f * ra + 0.25f * rb);
             }
         }
-        fout[i] = 0.5f * sum;
+        f[c * D.fc + p] = 0.5f * sum;
     }
 }
 
-// fine x += P x_coarse on level l's fluid cells (coarse fluid values only), the
-// coarse level being level l + 1's slabs or rank 0's first shared-memory level
-__device__ void slab_prolong(const MGChain& C, int l, float* pool, unsigned rank, float* spool) {
-    const DLev F = dlev(C, l, pool, rank);
-    const MGLev& Gc = C.lev[l + 1];
-    const bool from_slab = l + 1 < C.ls;
-    const DLev D = dlev(C, l + 1, pool, rank);  // used only when from_slab
-    const int nsm = Gc.nx * Gc.ny * Gc.nz;
-    const float* sx0 = from_slab ? nullptr : dsm(spool, 0);
-    const uint32_t* sc0 = from_slab ? nullptr : reinterpret_cast<const uint32_t*>(dsm(spool + 3 * nsm, 0));
-    const int n = F.np * F.plane;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        if (!is_fluid(F.code[i])) continue;
-        const int xl = i / F.plane, t = i - xl * F.plane;
-        const int x = F.x0 + xl, y = t / F.nz, z = t - y * F.nz;
-        const int p[3] = {(x & 1) ? x >> 1 : (x >> 1) - 1, (y & 1) ? y >> 1 : (y >> 1) - 1,
-                          (z & 1) ? z >> 1 : (z >> 1) - 1};
-        const float wl[3] = {(x & 1) ? 0.75f : 0.25f, (y & 1) ? 0.75f : 0.25f, (z & 1) ? 0.75f : 0.25f};
+// x += P x_coarse on L's red cells; coarse plane cx lies in cluster CTA cx / D.P
+__device__ __noinline__ void slev_prolong(const SLev& SL, const SLev& SD) {
+    const SLev L = SL, D = SD;
+#pragma unroll 1
+    for (int p = threadIdx.x; p < L.n; p += blockDim.x) {
+        const uint32_t cc = __float_as_uint(pool[slev_co(L) + p]);
+        if (!is_fluid(cc)) continue;
+        int xl, y, j, par;
+        slev_pair(L, p, xl, y, j, par);
+        const int x = L.x0 + xl;
+        // z = 2j + par: coarse j with weight 3/4 and j + 1 or j - 1 with 1/4
+        const int jn = par ? j + 1 : j - 1;
         float sum = 0.f;
 #pragma unroll
-        for (int o = 0; o < 8; o++) {
-            const int ox = o >> 2, oy = (o >> 1) & 1, oz = o & 1;
-            const int cx = p[0] + ox, cy = p[1] + oy, cz = p[2] + oz;
-            if (cx < 0 || cy < 0 || cz < 0 || cx >= Gc.nx || cy >= Gc.ny || cz >= Gc.nz) continue;
-            float v;
-            uint32_t c;
-            if (from_slab) {
-                const unsigned ro = (unsigned)(cx / D.P);
-                const int li = ((cx - (int)ro * D.P) * Gc.ny + cy) * Gc.nz + cz;
-                v = (ro == rank ? D.x : dsm(D.x, ro))[li];
-                c = (ro == rank ? D.code : dsm(D.code, ro))[li];
-            } else {
-                const int ci = (cx * Gc.ny + cy) * Gc.nz + cz;
-                v = sx0[ci];
-                c = sc0[ci];
+        for (int ox = 0; ox < 2; ox++) {
+            const int cx = (x >> 1) - 1 + (x & 1) + ox;
+            if (cx < 0 || cx >= D.nx) continue;
+            const int ro = (int)((unsigned)cx / (unsigned)D.P);
+            const float* plane = dsm(pool + D.xo + (cx - ro * D.P) * D.plane, (unsigned)ro);
+            const float wx = (x & 1) != ox ? 0.75f : 0.25f;
+#pragma unroll
+            for (int oy = 0; oy < 2; oy++) {
+                const int cy = (y >> 1) - 1 + (y & 1) + oy;
+                if (cy < 0 || cy >= D.ny) continue;
+                // colour of coarse cell (cx, cy, z): (cx + cy + z) & 1
+                const float* row = plane + cy * D.pr;
+                const float a = row[((cx + cy + j) & 1) * D.xc + (j >> 1)];
+                const float b = jn >= 0 && jn < D.nz ? row[((cx + cy + jn) & 1) * D.xc + (jn >> 1)] : 0.f;
+                sum += wx * ((y & 1) != oy ? 0.75f : 0.25f) * (0.75f * a + 0.25f * b);
             }
-            if (!is_fluid(c)) continue;
-            sum += (ox ? 1.f - wl[0] : wl[0]) * (oy ? 1.f - wl[1] : wl[1]) * (oz ? 1.f - wl[2] : wl[2]) * v;
         }
-        F.x[i] += sum * coarse_pscale(F.code[i]);
+        slev_put(L, 0, p, pool[L.xo + p] + coarse_pscale(cc) * sum);
     }
 }
 
-__global__ void __launch_bounds__(MG_CLUSTER_THREADS) k_mg_coarse(const PcgArgs A, const __grid_constant__ MGChain C) {
-    pdl_enter();
-    if (A.st->done) return;  // the same value in every CTA of the cluster
-    extern __shared__ float pool[];
+// levels ls..last in rank 0's shared memory
+__device__ __noinline__ void smem_levels_run(const MGChain& C, const SLev* S) {
+#pragma unroll 1
+    for (int l = C.ls; l < C.last; l++) {
+        level_smooth(S[l], 2 * C.nu, 0, SYNC_CTA, blockDim.x);
+        slev_resid(S[l]);
+        __syncthreads();
+        slev_restrict(S[l], S[l + 1], S[l + 1].n, threadIdx.x, blockDim.x, 0);
+        __syncthreads();
+    }
+    // bottom level (at most 64 cells): symmetric Gauss-Seidel in one warp (red, black, ..,
+    // black, red; repeating the middle half sweep would change nothing)
+    if (threadIdx.x < 32) level_smooth(S[C.last], 4 * MG_BOTTOM_SWEEPS - 1, 0, SYNC_WARP, 32);
+    __syncthreads();
+#pragma unroll 1
+    for (int l = C.last - 1; l >= C.ls; l--) {
+        slev_prolong(S[l], S[l + 1]);
+        __syncthreads();
+        level_smooth(S[l], 2 * C.nu, 1, SYNC_CTA, blockDim.x);
+    }
+}
+
+__global__ void __launch_bounds__(MG_CLUSTER_THREADS, 1) k_mg_coarse(const PcgArgs A,
+                                                                     const __grid_constant__ MGChain C) {
     __shared__ SLev S[MG_MAX_LEVELS];
     const unsigned rank = cluster_rank(), cs = cluster_size();
-    if (C.slab) {
-        float* spool = pool + C.soff;
-        for (int l = C.lc; l < C.ls; l++) {
-            const DLev D = dlev(C, l, pool, rank);
-            const MGLev& G = C.lev[l];
-            for (int i = threadIdx.x; i < D.np * D.plane; i += blockDim.x) {
-                const int xl = i / D.plane, t = i - xl * D.plane, y = t / D.nz, z = t - y * D.nz;
-                const long long gi = ((long long)(D.x0 + xl) * G.ny + y) * G.pz + z;
-                uint32_t cc = G.ccode[gi];
-                if ((D.x0 + xl + y + z) & 1) cc |= CS_ODD;
-                if (xl == 0) cc |= CS_XLO;
-                if (xl == D.np - 1) cc |= CS_XHI;
-                D.code[i] = cc;
-                D.x[i] = 0.f;
-                if (l == C.lc) D.f[i] = G.f[gi];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // this CTA's levels: slabs lc .. ls-1, then (held by rank 0, known to all) ls .. last
+    const int first = C.slab ? C.lc : C.ls;
+    if (threadIdx.x == 0) {
+        int off = C.soff;
+        for (int l = first; l <= C.last; l++) {
+            if (l >= C.ls) {
+                slev_make(S[l], C.lev[l], off, C.lev[l].nx, 0);
+                off += (int)slev_floats(C.lev[l].nx, C.lev[l].ny, C.lev[l].nz);
+                continue;
+            }
+            slev_make(S[l], C.lev[l], C.off[l], C.P[l], (int)rank * C.P[l]);
+            if (S[l].np > 0) {
+                // the previous CTA's slab is full: its upper guard plane follows P planes
+                if (rank > 0) S[l].lo = dsm(pool + S[l].xo + C.P[l] * S[l].plane, rank - 1);
+                if (rank + 1 < cs && S[l].x0 + S[l].np < S[l].nx) S[l].hi = dsm(pool + S[l].xo - S[l].plane, rank + 1);
             }
         }
-        if (rank == 0) smem_levels_init(C, spool, S, false);
-        cluster_barrier();
-        for (int l = C.lc; l < C.ls; l++) {
-            const DLev D = dlev(C, l, pool, rank);
-            const float* xp = rank > 0 ? dsm(D.x, rank - 1) : nullptr;
-            const float* xn = rank + 1 < cs ? dsm(D.x, rank + 1) : nullptr;
-            for (int k = 0; k < C.nu; k++) {
-                slab_smooth(D, 0, k == 0, xp, xn);
-                cluster_barrier();
-                slab_smooth(D, 1, false, xp, xn);
-                cluster_barrier();
-            }
-            slab_residual(D, xp, xn);
-            cluster_barrier();
-            slab_restrict(C, l, pool, rank, cs, spool);
-            cluster_barrier();
-        }
-        if (rank == 0) smem_levels_run(C, S, false);
-        cluster_barrier();
-        for (int l = C.ls - 1; l >= C.lc; l--) {
-            const DLev D = dlev(C, l, pool, rank);
-            const float* xp = rank > 0 ? dsm(D.x, rank - 1) : nullptr;
-            const float* xn = rank + 1 < cs ? dsm(D.x, rank + 1) : nullptr;
-            slab_prolong(C, l, pool, rank, spool);
-            cluster_barrier();
-            for (int k = 0; k < C.nu; k++) {
-                slab_smooth(D, 1, false, xp, xn);
-                cluster_barrier();
-                slab_smooth(D, 0, false, xp, xn);
-                cluster_barrier();
-            }
-        }
-        // level lc's correction back to global memory (its slab alone: no other
-        // CTA reads this CTA's shared memory after the last barrier)
-        const DLev D = dlev(C, C.lc, pool, rank);
-        const MGLev& G = C.lev[C.lc];
-        for (int i = threadIdx.x; i < D.np * D.plane; i += blockDim.x) {
-            const int xl = i / D.plane, t = i - xl * D.plane, y = t / D.nz, z = t - y * D.nz;
-            G.x[((long long)(D.x0 + xl) * G.ny + y) * G.pz + z] = D.x[i];
+    }
+    __syncthreads();
+    // the codes were written before the solve's first V-cycle: they are loaded while
+    // the predecessor drains
+    for (int l = first; l <= C.last; l++)
+        if (l < C.ls || rank == 0) slev_init(S[l], C.lev[l]);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (A.st->done) return;  // the same value in every CTA of the cluster
+    __syncthreads();
+    if (C.ls == C.lc) {
+        // rank 0 runs every level alone
+        if (rank == 0) {
+            slev_load_f(S[C.ls], C.lev[C.ls]);
+            __syncthreads();
+            smem_levels_run(C, S);
+            slev_store_x(S[C.ls], C.lev[C.ls]);
         }
         return;
     }
+    if (C.slab) {
+        slev_load_f(S[C.lc], C.lev[C.lc]);
+        cluster_barrier();  // every slab's guard planes are zero before a neighbour writes them
+#pragma unroll 1
+        for (int l = C.lc; l < C.ls; l++) {
+            level_smooth(S[l], 2 * C.nu, 0, SYNC_CLUSTER, blockDim.x);
+            slev_resid(S[l]);
+            cluster_barrier();
+            // into the CTA's own slab, or into rank 0's first level, spread over the cluster
+            if (l + 1 < C.ls) slev_restrict(S[l], S[l + 1], S[l + 1].n, threadIdx.x, blockDim.x, rank);
+            else slev_restrict(S[l], S[l + 1], S[l + 1].n, rank * blockDim.x + threadIdx.x, cs * blockDim.x, 0);
+            cluster_barrier();
+        }
+        if (rank == 0) smem_levels_run(C, S);
+        cluster_barrier();
+#pragma unroll 1
+        for (int l = C.ls - 1; l >= C.lc; l--) {
+            slev_prolong(S[l], S[l + 1]);
+            cluster_barrier();
+            level_smooth(S[l], 2 * C.nu, 1, SYNC_CLUSTER, blockDim.x);
+        }
+        // level lc's correction back to global memory (its slab alone: no other
+        // CTA reads this CTA's shared memory after the last barrier)
+        slev_store_x(S[C.lc], C.lev[C.lc]);
+        return;
+    }
+    // levels lc .. ls-1 in global memory
     const long long i0 = (long long)rank * blockDim.x + threadIdx.x;
     const long long step = (long long)cs * blockDim.x;
     for (int l = C.lc; l < C.ls; l++) {
@@ -1704,12 +1674,14 @@ __global__ void __launch_bounds__(MG_CLUSTER_THREADS) k_mg_coarse(const PcgArgs 
         mg_for_range(L, i0, step, [&](int x, int y, int z0, long long c0) { residual_quad<false>(L, L.f, x, y, z0, c0); });
         cluster_barrier();
         const MGLev& Cl = C.lev[l + 1];
-        mg_for_range(Cl, i0, step, [&](int x, int y, int z0, long long c0) { restrict_quad<false>(L, Cl, x, y, z0, c0); });
+        mg_for_range(Cl, i0, step, [&](int x, int y, int z0, long long c0) { restrict_quad(L, Cl, x, y, z0, c0); });
         cluster_barrier();
     }
     if (rank == 0) {
-        smem_levels_init(C, pool, S, true);
-        smem_levels_run(C, S, true);
+        slev_load_f(S[C.ls], C.lev[C.ls]);
+        __syncthreads();
+        smem_levels_run(C, S);
+        slev_store_x(S[C.ls], C.lev[C.ls]);
     }
     cluster_barrier();
     for (int l = C.ls - 1; l >= C.lc; l--) {
@@ -1799,31 +1771,46 @@ __global__ void k_mg_code(MGLev F, MGLev L, uint32_t* code) {
 }
 
 // interpolation scale of a level's fluid cells from the next level's kinds
-// (outside the level = solid)
+// (outside the level = solid).  One thread per coarse cell: its eight children's
+// neighbours all lie in the 27 cells around it, mostly none of them solid (one
+// thread per fine cell with eight kind reads: 110 us at 256^3).
 template <bool FINE>
 __global__ void k_mg_pscale(MGLev F, MGLev Cl, const uint8_t* ckind, uint16_t* code, uint32_t* ccode) {
-    const long long n = (long long)F.nx * F.ny * F.nz;
+    const long long n = (long long)Cl.nx * Cl.ny * Cl.nz;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const unsigned iu = (unsigned)i, t = iu / (unsigned)F.nz, u = t / (unsigned)F.ny;
-    const int z = (int)(iu - t * (unsigned)F.nz), y = (int)(t - u * (unsigned)F.ny), x = (int)u;
-    const long long fi = ((long long)x * F.ny + y) * F.pz + z;
-    if (FINE ? !is_fluid(code[fi]) : !is_fluid(ccode[fi])) return;
-    const int px = (x >> 1) - 1 + (x & 1), py = (y >> 1) - 1 + (y & 1), pz = (z >> 1) - 1 + (z & 1);
-    int k = 0;
+    const unsigned iu = (unsigned)i, t = iu / (unsigned)Cl.nz, u = t / (unsigned)Cl.ny;
+    const int cz = (int)(iu - t * (unsigned)Cl.nz), cy = (int)(t - u * (unsigned)Cl.ny), cx = (int)u;
+    const long long ci = ((long long)cx * Cl.ny + cy) * Cl.pz + cz;
+    if (ckind[ci] != 0) return;  // no fluid child
+    unsigned solid = 0;          // bit 9 (dx + 1) + 3 (dy + 1) + dz + 1
 #pragma unroll
-    for (int o = 0; o < 8; o++) {
-        const int ox = o >> 2, oy = (o >> 1) & 1, oz = o & 1;
-        const int cx = px + ox, cy = py + oy, cz = pz + oz;
-        if (cx < 0 || cy < 0 || cz < 0 || cx >= Cl.nx || cy >= Cl.ny || cz >= Cl.nz) continue;
-        if (ckind[((long long)cx * Cl.ny + cy) * Cl.pz + cz] == 2) continue;
-        // the lower neighbour weighs 3 (of 4) for odd cells, 1 for even ones
-        k += ((x & 1) != ox ? 3 : 1) * ((y & 1) != oy ? 3 : 1) * ((z & 1) != oz ? 3 : 1);
+    for (int k = 0; k < 27; k++) {
+        const int x = cx + k / 9 - 1, y = cy + (k / 3) % 3 - 1, z = cz + k % 3 - 1;
+        const bool in = x >= 0 && y >= 0 && z >= 0 && x < Cl.nx && y < Cl.ny && z < Cl.nz;
+        if (!in || ckind[((long long)x * Cl.ny + y) * Cl.pz + z] == 2) solid |= 1u << k;
     }
-    const unsigned s = (unsigned)(64 - k) & 63u;
-    if (!s) return;
-    if (FINE) code[fi] = (uint16_t)(code[fi] | ((s & 3u) << 6) | ((s & 0x3Cu) << 9));
-    else ccode[fi] |= s << CC_SCALE;
+    if (!solid) return;
+    for (int o = 0; o < 8; o++) {
+        const int sx = o >> 2, sy = (o >> 1) & 1, sz = o & 1;
+        const int fx = 2 * cx + sx, fy = 2 * cy + sy, fz = 2 * cz + sz;
+        if (fx >= F.nx || fy >= F.ny || fz >= F.nz) continue;
+        const long long fi = ((long long)fx * F.ny + fy) * F.pz + fz;
+        if (FINE ? !is_fluid(code[fi]) : !is_fluid(ccode[fi])) continue;
+        // the child's eight coarse neighbours: the parent (weight 3 of 4 per axis) and the
+        // cells next to it on the child's side (1 of 4)
+        int k = 0;
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            const int ax = q >> 2, ay = (q >> 1) & 1, az = q & 1;
+            const int dx = ax ? 2 * sx - 1 : 0, dy = ay ? 2 * sy - 1 : 0, dz = az ? 2 * sz - 1 : 0;
+            if (!((solid >> (9 * (dx + 1) + 3 * (dy + 1) + dz + 1)) & 1u)) k += (ax ? 1 : 3) * (ay ? 1 : 3) * (az ? 1 : 3);
+        }
+        const unsigned s = (unsigned)(64 - k) & 63u;
+        if (!s) continue;
+        if (FINE) code[fi] = (uint16_t)(code[fi] | ((s & 3u) << 6) | ((s & 0x3Cu) << 9));
+        else ccode[fi] |= s << CC_SCALE;
+    }
 }
 
 // phi += x; x = 0   (fold the FP32 accumulator into the FP64 solution)
@@ -1871,7 +1858,8 @@ int solver_alloc(fsim_ctx* ctx) {
     int bps = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_update<float, 1>, PCG_THREADS, 0);
     if (bps < 1) bps = 1;
-    S.grid_blocks = ctx->num_sms * bps;
+    // a pass takes four bricks per block: no more blocks than a grid has bricks for
+    S.grid_blocks = (int)std::min<long long>((long long)ctx->num_sms * bps, (S.nbricks + 3) / 4);
     FSIM_CUDA_TRY(ctx, cudaMalloc(&S.partials, (size_t)S.grid_blocks * 4 * sizeof(double)));
     FSIM_CUDA_TRY(ctx, cudaMalloc(&S.counter, sizeof(unsigned)));
     FSIM_CUDA_TRY(ctx, cudaMemset(S.counter, 0, sizeof(unsigned)));
@@ -1965,19 +1953,20 @@ static MGLev mg_lev(const SolverBufs& S, int l, const float* f0, const float* f1
 static void mg_setup(fsim_ctx* ctx) {
     SolverBufs& S = ctx->sv;
     cudaStream_t st = ctx->stream;
+    // the residual passes visit only quads with fluid on level 0, the restriction reads all
+    cudaMemsetAsync(S.mg[0].r, 0, (size_t)S.mg[0].ncell * sizeof(float), st);
     for (size_t l = 1; l < S.mg.size(); l++) {
         MGLev F = mg_lev(S, (int)l - 1, nullptr, nullptr, nullptr);
         MGLev Cl = mg_lev(S, (int)l, nullptr, nullptr, nullptr);
         const long long n = S.mg[l].ncell;
         k_mg_coarsen<<<ceil_div(n, 256), 256, 0, st>>>(F, l == 1 ? nullptr : S.mg[l - 1].kind, ctx->flags, Cl,
                                                        S.mg[l].kind);
-        const long long nf = S.mg[l - 1].ncell;
         if (l == 1) {
             k_mg_code<true><<<ceil_div(n, 256), 256, 0, st>>>(F, Cl, S.mg[l].ccode);
-            k_mg_pscale<true><<<ceil_div(nf, 256), 256, 0, st>>>(F, Cl, S.mg[l].kind, S.code, nullptr);
+            k_mg_pscale<true><<<ceil_div(n, 256), 256, 0, st>>>(F, Cl, S.mg[l].kind, S.code, nullptr);
         } else {
             k_mg_code<false><<<ceil_div(n, 256), 256, 0, st>>>(F, Cl, S.mg[l].ccode);
-            k_mg_pscale<false><<<ceil_div(nf, 256), 256, 0, st>>>(F, Cl, S.mg[l].kind, nullptr, S.mg[l - 1].ccode);
+            k_mg_pscale<false><<<ceil_div(n, 256), 256, 0, st>>>(F, Cl, S.mg[l].kind, nullptr, S.mg[l - 1].ccode);
         }
         ctx->launches += 3;
     }
@@ -1989,7 +1978,7 @@ static int mg_band_sweeps(const fsim_params& P, int l) {
 }
 
 // z = V-cycle(r); r is the current PCG residual (r0 or r1 by device state).
-// first_fused: the first level-0 sweep was done by k_update; dot_mode >= 0: the
+// first_fused: the first red half sweep on level 0 was done by k_update_q; dot_mode >= 0: the
 // last level-0 sweep also computes z.r and the CG scalars (k_red modes).
 static void mg_vcycle(fsim_ctx* ctx, const PcgArgs& A, int l, const float* r0, const float* r1, float* z,
                       bool first_fused, int dot_mode) {
@@ -2018,14 +2007,12 @@ static void mg_vcycle(fsim_ctx* ctx, const PcgArgs& A, int l, const float* r0, c
         size_t smem = 0;
         for (int k = C.last; k >= 0; k--) {
             const MGLevelBufs& b = S.mg[l + k];
-            const long long n = (long long)b.nx * b.ny * b.nz;
-            if (n > MG_SMEM_CELLS) break;
+            if ((long long)b.nx * b.ny * ((b.nz + 1) & ~1) > MG_SMEM_CELLS) break;
             C.ls = k;
         }
         for (int k = C.ls; k <= C.last; k++) {
             const MGLevelBufs& b = S.mg[l + k];
-            const long long n = (long long)b.nx * b.ny * b.nz;
-            smem += (size_t)(4 * n) * sizeof(float);
+            smem += (size_t)slev_floats(b.nx, b.ny, b.nz) * sizeof(float);
         }
         // levels lc .. ls-1 as x slabs in the cluster's distributed shared memory
         // when they fit beside rank 0's levels (else they run in global memory)
@@ -2033,14 +2020,13 @@ static void mg_vcycle(fsim_ctx* ctx, const PcgArgs& A, int l, const float* r0, c
         for (int k = 0; k < C.ls; k++) {
             const MGLevelBufs& b = S.mg[l + k];
             const int P = ceil_div(b.nx, S.mg_cluster);
-            const long long m = (long long)P * b.ny * b.nz;
             C.P[k] = P;
             C.off[k] = (int)slab_floats;
-            slab_floats += (size_t)((4 * m + 3) & ~3ll);
+            slab_floats += (size_t)((slev_floats(P, b.ny, b.nz) + 3) & ~3ll);
         }
-        C.soff = (int)slab_floats;
         const size_t slab_bytes = slab_floats * sizeof(float) + smem;
         C.slab = (C.ls > 0 && slab_bytes <= (size_t)MG_CLUSTER_SMEM) ? 1 : 0;
+        C.soff = C.slab ? (int)slab_floats : 0;
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(S.mg_cluster);
         cfg.blockDim = dim3(MG_CLUSTER_THREADS);
@@ -2064,11 +2050,14 @@ static void mg_vcycle(fsim_ctx* ctx, const PcgArgs& A, int l, const float* r0, c
         if (l == 0) launch_pdl(k_mg_smooth<true>, nb, PCG_THREADS, st, A, L, color, first);
         else launch_pdl(k_mg_smooth<false>, nb, PCG_THREADS, st, A, L, color, first);
     };
+    // the first red half sweep was done by k_update_q (level 0) or the restriction
     for (int k = 0; k < NU; k++) {
-        if (k == 0 && l == 0 && first_fused) continue;
-        smooth(0, k == 0);
+        if (k > 0 || !(l > 0 || first_fused)) {
+            smooth(0, k == 0);
+            ctx->launches += 1;
+        }
         smooth(1, 0);
-        ctx->launches += 2;
+        ctx->launches += 1;
     }
     const int NB = mg_band_sweeps(P, l);
     auto smooth_band = [&](int color) {
@@ -2082,9 +2071,8 @@ static void mg_vcycle(fsim_ctx* ctx, const PcgArgs& A, int l, const float* r0, c
     if (l == 0) launch_pdl(k_mg_residual<true>, nb, PCG_THREADS, st, A, L);
     else launch_pdl(k_mg_residual<false>, nb, PCG_THREADS, st, A, L);
     MGLev Cl = mg_lev(S, l + 1, nullptr, nullptr, nullptr);
-    const int nbc = std::min(G, ceil_div(S.mg[l + 1].ncell, 256));
-    if (l == 0) launch_pdl(k_mg_restrict<true>, nbc, PCG_THREADS, st, A.st, L, Cl);
-    else launch_pdl(k_mg_restrict<false>, nbc, PCG_THREADS, st, A.st, L, Cl);
+    launch_pdl(k_mg_restrict, std::min(ctx->num_sms * 8, ceil_div(S.mg[l + 1].ncell, 256)), PCG_THREADS, st, A.st, L, Cl,
+               S.mg[l + 1].ncell > 32768 ? 1 : 0);
     mg_vcycle(ctx, A, l + 1, nullptr, nullptr, nullptr, false, -1);
     if (l == 0) launch_pdl(k_mg_prolong<true>, nb, PCG_THREADS, st, A, L, Cl);
     else launch_pdl(k_mg_prolong<false>, nb, PCG_THREADS, st, A, L, Cl);
@@ -2137,7 +2125,7 @@ void solver_free(fsim_ctx* ctx) {
 // ||b - A phi|| (previous pressure) against ||b - A guess||, FP32 per cell and
 // FP64 per thread; the last block records which one seeds PCG.
 __global__ void __launch_bounds__(PCG_THREADS) k_guess_judge(const PcgArgs a, const float* guess) {
-    __shared__ double scratch[32 * 2];
+    __shared__ double scratch[PCG_THREADS * 2];
     double acc[2] = {0.0, 0.0};
     const int nact = *a.nactive;
     for (int bk = blockIdx.x; bk < nact; bk += gridDim.x) {
@@ -2221,7 +2209,7 @@ static int run_pcg(fsim_ctx* ctx, PcgArgs& A, Vecs<T> v, int precision, int prec
     // z = M^-1 r and sigma (mode 0 setup, 1 iteration, 2 after a fold)
     auto precondition = [&](int mode, bool black_done) {
         if (mg) {
-            // mode 1: k_update already did the first sweep; the V-cycle ends with z.r
+            // mode 1: k_update_q already did the first half sweep; the V-cycle ends with z.r
             mg_vcycle(ctx, A, 0, (const float*)(const void*)v.r[0], (const float*)(const void*)v.r[1],
                       (float*)(void*)v.z, mode == 1, mode);
         } else {
@@ -2427,7 +2415,7 @@ int solve_pressure(fsim_ctx* ctx, double dt, int precision, int tol_mode, double
     sa.phi = S.phi;
     sa.brick_flag = S.brick_flag;
     k_setup<<<ceil_div(g.ncell, 256), 256, 0, st>>>(sa);
-    k_compact_bricks<<<1, 1024, 0, st>>>(S.brick_flag, S.nbricks, S.nby, S.nbz, S.brick_xyz, S.d_nactive);
+    k_compact_bricks<<<1, COMPACT_THREADS, 0, st>>>(S.brick_flag, S.nbricks, S.nby, S.nbz, S.brick_xyz, S.d_nactive);
     ctx->launches += 2;
     fetch_small(&ctx->h_misc[1], S.d_nactive, (int)sizeof(int), st);
 
