@@ -26,7 +26,7 @@ struct ConvLaunch {
     int ys, yo;                // output channel stride / offset
     unsigned* err;
     const CUtensorMap* mx;     // input map (conv_act_map)
-    const CUtensorMap* mw;     // weight map (conv_wt_map)
+    const __nv_bfloat16* wgt;  // weights packed for the layer's tile (conv_pack_index)
 };
 
 struct WgradLaunch {
@@ -37,11 +37,21 @@ struct WgradLaunch {
     const CUtensorMap* mg;     // gradient map [vox][cout] (wgrad_g_map)
 };
 
-bool conv_act_map(CUtensorMap* m, const void* base, int n, int d, int h, int w, int c, int taps);
-bool conv_wt_map(CUtensorMap* m, const void* base, int taps, int rows, int kdim, int nt);
+// d-planes and output channels of a CTA's tile (a function of the layer and the device);
+// the input's map is encoded and the weights are packed for them
+struct ConvTile {
+    int planes, nt;
+};
+ConvTile conv_tile(int taps, int n, int d, int h, int w, int cin, int cout);
+bool conv_act_map(CUtensorMap* m, const void* base, int n, int d, int h, int w, int c, int taps, int planes);
 bool wgrad_x_map(CUtensorMap* m, const void* base, int n, int d, int h, int w, int c, int taps);
 bool wgrad_g_map(CUtensorMap* m, const void* base, int n, int d, int h, int w, int c, int taps);
-int conv_nt(int taps, int cout);
+// place of weight (position t of taps, output channel n of nout, input channel c): what a
+// CTA needs of 8 input channels for its nt output channels is one contiguous block, in
+// the order of the tensor core's core matrices ([tap][nt][8 channels])
+__host__ __device__ inline long long conv_pack_index(int taps, int nout, int nt, int t, int n, int c) {
+    return (((long long)(c >> 3) * (nout / nt) + n / nt) * taps + t) * nt * 8 + (n % nt) * 8 + (c & 7);
+}
 int launch_conv_mma(const ConvLaunch& L, cudaStream_t s);
 int launch_conv_wgrad(const WgradLaunch& L, cudaStream_t s);
 
@@ -54,9 +64,9 @@ enum { NET_LAYERS = 17, NET_MAX_BATCH = 64 };
 struct NetLayer {
     int taps, cin, cout;
     long long w_off, b_off;          // offsets (floats) of weight / bias in the flat parameters
-    __nv_bfloat16* wb = nullptr;     // [taps][cout][cin]
-    __nv_bfloat16* wt = nullptr;     // [taps][cin][cout]
-    CUtensorMap mw, mwt;             // forward / input-gradient weight maps
+    __nv_bfloat16* wb = nullptr;     // forward weights, packed for nt output channels per CTA
+    __nv_bfloat16* wt = nullptr;     // input-gradient weights, packed for ntt
+    int nt = 16, ntt = 16;           // (of the workspace's shape)
 };
 
 struct NetShape {

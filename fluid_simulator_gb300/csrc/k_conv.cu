@@ -2,29 +2,27 @@
 // 5th-generation tensor cores (tcgen05, TMEM accumulators, TMA operands).
 //
 // Tensors are BF16 in NDHWC order ([n][d][h][w][c], c fastest).  Weights are
-// BF16 [tap][cout][cin] (tap = (kd*3 + kh)*3 + kw for 3x3x3, a single tap for
-// the pointwise convolutions).  Accumulation is FP32.
+// BF16, packed per 8 input channels and N tile (conv_pack_index); accumulation is FP32.
 //
 // Forward / input-gradient kernels: implicit GEMM
 //   D[m, n] = sum_{tap, c} X[voxel(m) + off(tap), c] * W[tap, n, c]
-// over output tiles of 8 (w) x 16 (h) x 4 (d) voxels and NT output channels:
+// over output tiles of 8 (w) x 16 (h) x P (d) voxels and NT output channels:
 // k_conv_pers (3x3x3 layers) is persistent, one CTA per SM walking the tiles
 // with warp-specialized roles (described at the kernel); k_conv_mma (the
 // pointwise down-convolutions) gives each CTA one tile.  Per 16-channel chunk
-// of the input a CTA loads ONE halo box of the
-// input (10 x 18 x 6 voxels for 3x3x3, zero-filled outside the volume, which
-// is the padding) and the chunk's weights for all taps with TMA, in the
-// no-swizzle K-major core-matrix layout (8 rows x 16 bytes per core matrix,
-// the two 8-channel halves of the chunk in separate planes).  Every tap is then
-// one tcgen05.mma (M = 128 voxels of one d-plane, N = NT, K = 16) whose A
-// descriptor simply starts at the shifted halo row: row groups of 8 voxels are
-// 16-byte rows, so a shift by (kw, kh, kd) is a start offset of
-// ((kd*18 + kh)*10 + kw) * 16 bytes.  The four d-planes accumulate into four
-// TMEM column blocks.  Input-gradient (dgrad) is the same kernel on the output
-// gradient with the per-tap transposed weights [tap][cin][cout] read at tap
-// 26 - t.  The epilogue reads TMEM with tcgen05.ld, adds the bias, applies
-// ReLU or a ReLU-derivative mask, and stores BF16 at a channel stride/offset
-// (so encoder outputs land directly in their concatenation slice).
+// of the input a CTA loads ONE halo box of the input (10 x 18 x (P + 2) voxels for
+// 3x3x3, zero-filled outside the volume, which is the padding) and the chunk's
+// weights for all taps (packed in that order, one contiguous copy), in the no-swizzle K-major core-matrix layout (8
+// rows x 16 bytes per core matrix, the two 8-channel halves of the chunk in separate
+// planes).  A shift by (kh, kw) is a start offset of the A descriptor: row groups of
+// 8 voxels are 16-byte rows, ((plane*18 + kh)*10 + kw) * 16 bytes.  One tcgen05.mma
+// multiplies the 128 voxels of an input plane by the weights of all three kd side by
+// side (M = 128, N = 3 NT, K = 16): its N blocks are the products for the output
+// planes pl - 2, pl - 1, pl, whose TMEM column blocks are neighbours.  Input-gradient
+// (dgrad) is the same kernel on the output gradient with the per-tap transposed
+// weights, (kh, kw) read backwards.  The epilogue reads TMEM with tcgen05.ld, adds the
+// bias, applies ReLU or a ReLU-derivative mask, and stores BF16 at a channel
+// stride/offset (so encoder outputs land directly in their concatenation slice).
 //
 // Weight-gradient kernel (k_conv_wgrad): D[(tap, c), n] = sum_v X[v + off(tap), c]
 // * G[v, n] with K = voxels, operands in the MN-major layout (described there).
@@ -39,7 +37,7 @@
 
 namespace {
 
-constexpr int TW = 8, TH = 16, TD = 4;  // output tile (w, h, d); M = TW*TH = 128 per plane
+constexpr int TW = 8, TH = 16;  // output tile (w, h); M = TW*TH = 128 per plane
 constexpr int CONV_THREADS = 128;
 constexpr int SMEM_LIMIT = 227 * 1024 - 1024;  // opt-in maximum minus room for static shared memory
 constexpr long long SPIN_LIMIT = 1ll << 31;  // clock cycles, about one second
@@ -75,12 +73,11 @@ __device__ __forceinline__ void tma_5d(void* dst, const CUtensorMap* map, int c0
         "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(s32(bar))
         : "memory");
 }
-__device__ __forceinline__ void tma_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(s32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(s32(bar))
-        : "memory");
+// contiguous copy; both addresses and the size are multiples of 16 bytes
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(s32(dst)),
+                 "l"(src), "r"(bytes), "r"(s32(bar))
+                 : "memory");
 }
 
 // tcgen05 shared-memory matrix descriptor, K-major, no swizzle: core matrices
@@ -107,6 +104,30 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(bar))
                  : "memory");
+}
+// The issuing loops run on the whole warp and let one lane issue (predicated): control
+// flow stays uniform, so descriptors live in uniform registers.  With a single thread
+// branching off, every MMA first moved its operands there: 48 -> 16 channels at 128^3
+// 142 us, now 109; weight gradient of 16 -> 16 at 8 x 64^3 300 us, now 222.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ void mma_bf16_one(uint32_t lead, uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc,
+                                             uint32_t acc) {
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(lead)
+        : "memory");
+}
+__device__ __forceinline__ void mma_commit_one(uint32_t lead, uint64_t* bar) {
+    asm volatile(
+        "{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
+        " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(s32(bar)),
+        "r"(lead)
+        : "memory");
 }
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst, int ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(dst)), "r"(ncols)
@@ -137,10 +158,10 @@ __device__ __forceinline__ bool bf16_pos(unsigned short bits) { return !(bits & 
 // ---------------------------------------------------------------------------
 // forward / input-gradient
 // ---------------------------------------------------------------------------
-template <int TAPS>
+template <int TAPS, int PLANES>
 struct Halo {
     static constexpr int H = TAPS == 27 ? 1 : 0;
-    static constexpr int AW = TW + 2 * H, AH = TH + 2 * H, AD = TD + 2 * H;
+    static constexpr int AW = TW + 2 * H, AH = TH + 2 * H, AD = PLANES + 2 * H;
     static constexpr int ROWS = AW * AH * AD;
     static constexpr int KC = ROWS * 16;  // bytes of one 8-channel half
     static constexpr int A_BYTES = 2 * KC;
@@ -152,6 +173,7 @@ struct MmaArgs {
     int tiles_w, tiles_h, tiles_d, ntiles;
     int stages;
     int flip;            // weights read at tap 26 - t (input gradient)
+    const __nv_bfloat16* wgt;   // packed weights (conv_pack_index)
     const float* bias;   // [cout] or null
     int relu;
     const __nv_bfloat16* mask;  // ReLU-derivative mask (out *= mask > 0) or null
@@ -161,13 +183,14 @@ struct MmaArgs {
     unsigned* err;
 };
 
-template <int TAPS>
-__global__ void __launch_bounds__(CONV_THREADS) k_conv_mma(const MmaArgs a, const __grid_constant__ CUtensorMap tx,
-                                                           const __grid_constant__ CUtensorMap tw) {
-    using G = Halo<TAPS>;
+// pointwise (down-)convolutions: one tile of PLANES d-planes per CTA
+constexpr int POINT_MAX_STAGES = 8;
+template <int PLANES>
+__global__ void __launch_bounds__(CONV_THREADS) k_conv_mma(const MmaArgs a, const __grid_constant__ CUtensorMap tx) {
+    using G = Halo<1, PLANES>;
     extern __shared__ __align__(128) unsigned char smraw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>(((uintptr_t)smraw + 127) & ~(uintptr_t)127);
-    __shared__ __align__(8) uint64_t full[3], empty[3], done;
+    __shared__ __align__(8) uint64_t full[POINT_MAX_STAGES], empty[POINT_MAX_STAGES], done;
     __shared__ uint32_t tmem_base;
     __shared__ int s_fail;
 
@@ -180,10 +203,10 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv_mma(const MmaArgs a, cons
     t /= a.tiles_h;
     const int bd = (int)(t % a.tiles_d);
     const int nb = (int)(t / a.tiles_d);
-    const int w0 = bw * TW, h0 = bh * TH, d0 = bd * TD, n0 = nti * a.nt;
+    const int w0 = bw * TW, h0 = bh * TH, d0 = bd * PLANES, n0 = nti * a.nt;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int ncols = tmem_cols(TD * a.nt);
-    const int B_KC = TAPS * a.nt * 16;
+    const int ncols = tmem_cols(PLANES * a.nt);
+    const int B_KC = a.nt * 16;
     const int stage_bytes = G::A_BYTES + 2 * B_KC;
 
     if (threadIdx.x == 0) {
@@ -212,7 +235,8 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv_mma(const MmaArgs a, cons
 #pragma unroll
             for (int kc = 0; kc < 2; kc++) {
                 tma_5d(st + kc * G::KC, &tx, k * 16 + kc * 8, w0 - G::H, h0 - G::H, d0 - G::H, nb, &full[s]);
-                tma_3d(st + G::A_BYTES + kc * B_KC, &tw, k * 16 + kc * 8, n0, 0, &full[s]);
+                bulk_load(st + G::A_BYTES + kc * B_KC, a.wgt + ((long long)(k * 2 + kc) * a.cout + n0) * 8,
+                          (unsigned)B_KC, &full[s]);
             }
         };
         bool ok = true;
@@ -226,23 +250,19 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv_mma(const MmaArgs a, cons
             fence_after();
             const uint32_t abase = s32(sm + s * stage_bytes);
             const uint32_t bbase = abase + G::A_BYTES;
-#pragma unroll 1
-            for (int tap = 0; tap < TAPS; tap++) {
-                const int kd = tap / 9, kh = (tap / 3) % 3, kw = tap % 3;
-                const int wt = a.flip ? TAPS - 1 - tap : tap;
-                const uint64_t bdesc = sdesc(bbase + (uint32_t)(wt * a.nt * 16), (uint32_t)B_KC, 128);
+            const uint64_t bdesc = sdesc(bbase, (uint32_t)B_KC, 128);
 #pragma unroll
-                for (int zp = 0; zp < TD; zp++) {
-                    const int row = ((zp + kd) * G::AH + kh) * G::AW + kw;
-                    const uint64_t adesc =
-                        sdesc(abase + (uint32_t)(row * 16), (uint32_t)G::KC, (uint32_t)(G::AW * 16));
-                    mma_bf16(tmem + (uint32_t)(zp * a.nt), adesc, bdesc, idesc, (k > 0 || tap > 0) ? 1u : 0u);
-                }
+            for (int zp = 0; zp < PLANES; zp++) {
+                const uint64_t adesc =
+                    sdesc(abase + (uint32_t)(zp * G::AH * G::AW * 16), (uint32_t)G::KC, (uint32_t)(G::AW * 16));
+                mma_bf16(tmem + (uint32_t)(zp * a.nt), adesc, bdesc, idesc, k > 0 ? 1u : 0u);
             }
             mma_commit(&empty[s]);
-            if (k + a.stages < nchunk) {
-                if (!mbar_wait(&empty[s], (unsigned)((k / a.stages) & 1))) { ok = false; break; }
-                issue(k + a.stages);
+            // refill the stage of the chunk before this one: its MMAs have (nearly) finished
+            const int b = k - 1;
+            if (b >= 0 && b + a.stages < nchunk) {
+                if (!mbar_wait(&empty[b % a.stages], (unsigned)((b / a.stages) & 1))) { ok = false; break; }
+                issue(b + a.stages);
                 issued++;
             }
         }
@@ -263,7 +283,7 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv_mma(const MmaArgs a, cons
         const int m = warp * 32 + lane;
         const int vw = w0 + (m & 7), vh = h0 + (m >> 3);
 #pragma unroll 1
-        for (int zp = 0; zp < TD; zp++) {
+        for (int zp = 0; zp < PLANES; zp++) {
             const int vd = d0 + zp;
             const bool inside = vw < a.w && vh < a.h && vd < a.d;
             const long long vox = (((long long)nb * a.d + vd) * a.h + vh) * a.w + vw;
@@ -311,16 +331,23 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv_mma(const MmaArgs a, cons
 // ---------------------------------------------------------------------------
 // One CTA per SM walks the output tiles t = blockIdx.x, + gridDim.x, ...  Warp
 // 0 (one thread) streams (tile, 16-channel chunk) items into a ring of shared
-// memory stages with TMA, warp 1 (one thread) issues each item's 108 MMAs into
-// one of two TMEM accumulators, and warps 2-5 drain the other accumulator
+// memory stages with TMA, warp 1 issues each item's MMAs (nine per input plane) into
+// one of two TMEM accumulators, and warps 2-9 drain the other accumulator
 // (bias, ReLU or mask, BF16 stores) while the next tile accumulates, so loads,
 // MMAs and the epilogue of neighbouring tiles overlap instead of running one
 // after the other in every CTA.  When the layer has one N tile and its
 // weights fit beside two stages, all chunks' weights are loaded once and stay
 // resident; otherwise each stage carries its chunk's weights as above.
+// What bounds it: the MMAs' operand reads.  An MMA reads 4 KB of A whatever N is, so
+// wide N pays: with one MMA per tap and output plane (N = NT) a 16 -> 16 layer of 128^3
+// was 2916 MMAs of 61 cycles per CTA (98 us); with the three kd in one MMA, 1260 of 52
+// cycles, and loads (16-byte rows) and stores of the same length beside them: 50 us.
+// 48 -> 16: 260 us, now 110, 9% above its MMAs alone.  The sum of an output is taken in
+// the same order (chunk, kd, kh, kw).
 // Every wait is bounded; a timeout (or a role that gave up) makes all roles
 // stop, the copies in flight land, the issued MMAs finish, TMEM is freed.
-constexpr int PERS_THREADS = 192;
+constexpr int PERS_DRAIN = 8;  // draining warps
+constexpr int PERS_THREADS = 64 + 32 * PERS_DRAIN;
 constexpr int PERS_MAX_STAGES = 4;
 
 struct PersArgs {
@@ -335,6 +362,7 @@ struct TileAt {
     int w0, h0, d0, nb, n0;
 };
 
+template <int PLANES>
 __device__ __forceinline__ TileAt tile_at(const MmaArgs& a, int t) {
     TileAt c;
     const int nti = t % a.ntiles;
@@ -343,7 +371,7 @@ __device__ __forceinline__ TileAt tile_at(const MmaArgs& a, int t) {
     t /= a.tiles_w;
     c.h0 = (t % a.tiles_h) * TH;
     t /= a.tiles_h;
-    c.d0 = (t % a.tiles_d) * TD;
+    c.d0 = (t % a.tiles_d) * PLANES;
     c.nb = t / a.tiles_d;
     c.n0 = nti * a.nt;
     return c;
@@ -374,9 +402,10 @@ __device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t (&r)[16
         : "r"(taddr));
 }
 
-__global__ void __launch_bounds__(PERS_THREADS, 1) k_conv_pers(const PersArgs p, const __grid_constant__ CUtensorMap tx,
-                                                                const __grid_constant__ CUtensorMap tw) {
-    using G = Halo<27>;
+template <int PLANES>
+__global__ void __launch_bounds__(PERS_THREADS, 1) k_conv_pers(const PersArgs p,
+                                                                const __grid_constant__ CUtensorMap tx) {
+    using G = Halo<27, PLANES>;
     const MmaArgs& a = p.m;
     extern __shared__ __align__(128) unsigned char smraw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>(((uintptr_t)smraw + 127) & ~(uintptr_t)127);
@@ -385,7 +414,7 @@ __global__ void __launch_bounds__(PERS_THREADS, 1) k_conv_pers(const PersArgs p,
     __shared__ uint32_t tmem_base;
     __shared__ int s_stop, s_issued, s_consumed;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int S = a.stages;
     const int nchunk = a.cin >> 4;
     const int B_KC = 27 * a.nt * 16;
@@ -400,7 +429,7 @@ __global__ void __launch_bounds__(PERS_THREADS, 1) k_conv_pers(const PersArgs p,
         }
         for (int b = 0; b < 2; b++) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 4);
+            mbar_init(&acc_empty[b], PERS_DRAIN);
         }
         mbar_init(&wfull, 1);
         mbar_init(&done, 1);
@@ -413,74 +442,83 @@ __global__ void __launch_bounds__(PERS_THREADS, 1) k_conv_pers(const PersArgs p,
     fence_before();
     __syncthreads();
     fence_after();
-    const uint32_t tmem = tmem_base;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
     volatile int* stop = &s_stop;
 
     if (warp == 0) {
         if (lane == 0) {
             if (p.wres) {
                 mbar_expect_tx(&wfull, (unsigned)(nchunk * 2 * B_KC));
-                for (int k = 0; k < nchunk; k++)
-                    for (int kc = 0; kc < 2; kc++) tma_3d(wbase + (k * 2 + kc) * B_KC, &tw, k * 16 + kc * 8, 0, 0, &wfull);
+                for (int k = 0; k < 2 * nchunk; k++)
+                    bulk_load(wbase + k * B_KC, a.wgt + (long long)k * (B_KC / 2), (unsigned)B_KC, &wfull);
             }
             int issued = 0;
             for (int j = 0; j < items; j++) {
                 const int s = j % S;
                 if (j >= S && !mbar_wait_ab(&empty[s], (unsigned)(((j / S) - 1) & 1), stop, a.err)) break;
-                const TileAt c = tile_at(a, (int)blockIdx.x + (j / nchunk) * (int)gridDim.x);
+                const TileAt c = tile_at<PLANES>(a, (int)blockIdx.x + (j / nchunk) * (int)gridDim.x);
                 const int k = j % nchunk;
                 unsigned char* st = sm + s * p.stage_bytes;
                 mbar_expect_tx(&full[s], (unsigned)p.stage_bytes);
 #pragma unroll
                 for (int kc = 0; kc < 2; kc++) {
                     tma_5d(st + kc * G::KC, &tx, k * 16 + kc * 8, c.w0 - 1, c.h0 - 1, c.d0 - 1, c.nb, &full[s]);
-                    if (!p.wres) tma_3d(st + G::A_BYTES + kc * B_KC, &tw, k * 16 + kc * 8, c.n0, 0, &full[s]);
+                    if (!p.wres)
+                        bulk_load(st + G::A_BYTES + kc * B_KC, a.wgt + ((long long)(k * 2 + kc) * a.cout + c.n0) * 27 * 8,
+                                  (unsigned)B_KC, &full[s]);
                 }
                 issued = j + 1;
             }
             s_issued = issued;
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = idesc_bf16(a.nt);
-            bool ok = !p.wres || mbar_wait_ab(&wfull, 0, stop, a.err);
+        {
+            const uint32_t lead = elect_one() ? 1u : 0u;
+            const uint32_t idesc[3] = {idesc_bf16(a.nt), idesc_bf16(2 * a.nt), idesc_bf16(3 * a.nt)};
+            const bool ok = !p.wres || __all_sync(0xffffffffu, mbar_wait_ab(&wfull, 0, stop, a.err));
             int consumed = 0;
             for (int j = 0; ok && j < items; j++) {
                 const int s = j % S, ti = j / nchunk, k = j % nchunk, buf = ti & 1;
-                if (!mbar_wait_ab(&full[s], (unsigned)((j / S) & 1), stop, a.err)) break;
+                if (!__all_sync(0xffffffffu, mbar_wait_ab(&full[s], (unsigned)((j / S) & 1), stop, a.err))) break;
                 consumed = j + 1;
-                if (k == 0 && ti >= 2 && !mbar_wait_ab(&acc_empty[buf], (unsigned)(((ti >> 1) - 1) & 1), stop, a.err))
+                if (k == 0 && ti >= 2 &&
+                    !__all_sync(0xffffffffu, mbar_wait_ab(&acc_empty[buf], (unsigned)(((ti >> 1) - 1) & 1), stop, a.err)))
                     break;
                 fence_after();
                 const uint32_t abase = s32(sm + s * p.stage_bytes);
                 const uint32_t bbase = p.wres ? s32(wbase + k * 2 * B_KC) : abase + G::A_BYTES;
-                // The 108 MMAs are unrolled with their descriptors formed by
-                // adding to two base descriptors (the start-address field is
-                // the byte address / 16, so a shift by `row` halo rows adds
-                // `row` and the next tap's weights add nt): one thread issues
-                // every MMA of the CTA and must not spend more time per MMA
-                // than the tensor core does.
+                // Unrolled, with descriptors formed by adding to two base
+                // descriptors (the start-address field is the byte address / 16, so
+                // a shift by `row` halo rows adds `row` and a weight row adds 1): one
+                // thread issues every MMA of the CTA and must not spend more time
+                // per MMA than the tensor core does.
                 const uint64_t ad0 = sdesc(abase, (uint32_t)G::KC, (uint32_t)(G::AW * 16));
-                const int bstep = a.flip ? -a.nt : a.nt;
-                const uint64_t bd0 = sdesc(bbase, (uint32_t)B_KC, 128) + (uint64_t)(a.flip ? 26 * a.nt : 0);
+                const uint64_t bd0 = sdesc(bbase, (uint32_t)B_KC, 128);
                 const uint32_t acc0 = tmem + (uint32_t)(buf * p.ncols);
-                const uint32_t accz[TD] = {acc0, acc0 + (uint32_t)a.nt, acc0 + (uint32_t)(2 * a.nt),
-                                           acc0 + (uint32_t)(3 * a.nt)};
 #pragma unroll
-                for (int tap = 0; tap < 27; tap++) {
-                    const int kd = tap / 9, kh = (tap / 3) % 3, kw = tap % 3;
-                    const uint64_t bdesc = bd0 + (uint64_t)(long long)(tap * bstep);
+                for (int pl = 0; pl < G::AD; pl++) {
+                    // input plane pl feeds output planes pl - kd, kd = lo .. hi
+                    const int lo = pl >= PLANES ? pl - PLANES + 1 : 0, hi = pl < 2 ? pl : 2;
+                    const uint32_t d = acc0 + (uint32_t)((pl - hi) * a.nt);
 #pragma unroll
-                    for (int zp = 0; zp < TD; zp++) {
-                        const int row = ((zp + kd) * G::AH + kh) * G::AW + kw;
-                        mma_bf16(accz[zp], ad0 + (uint64_t)row, bdesc, idesc, (k > 0 || tap > 0) ? 1u : 0u);
+                    for (int g = 0; g < 9; g++) {
+                        const uint64_t ad = ad0 + (uint64_t)((pl * G::AH + g / 3) * G::AW + g % 3);
+                        const int gw = (a.flip ? 8 - g : g) * 3;
+                        const uint64_t bd = bd0 + (uint64_t)((gw + 2 - hi) * a.nt);
+                        if (g == 0 && lo == 0 && k == 0) {
+                            // output plane pl's first product overwrites, the others add
+                            if (hi > 0) mma_bf16_one(lead, d, ad, bd, idesc[hi > 0 ? hi - 1 : 0], 1u);
+                            mma_bf16_one(lead, acc0 + (uint32_t)(pl * a.nt), ad, bd0 + (uint64_t)((gw + 2) * a.nt), idesc[0], 0u);
+                        } else {
+                            mma_bf16_one(lead, d, ad, bd, idesc[hi - lo], 1u);
+                        }
                     }
                 }
-                mma_commit(&empty[s]);
-                if (k == nchunk - 1) mma_commit(&acc_full[buf]);
+                mma_commit_one(lead, &empty[s]);
+                if (k == nchunk - 1) mma_commit_one(lead, &acc_full[buf]);
             }
-            s_consumed = consumed;
-            mma_commit(&done);  // arrives once every MMA issued above has completed
+            if (lane == 0) s_consumed = consumed;
+            mma_commit_one(lead, &done);  // arrives once every MMA issued above has completed
         }
     } else {
         const int q = warp & 3;  // the TMEM lane quarter this warp may access
@@ -489,53 +527,62 @@ __global__ void __launch_bounds__(PERS_THREADS, 1) k_conv_pers(const PersArgs p,
             const int buf = ti & 1;
             if (!mbar_wait_ab(&acc_full[buf], (unsigned)((ti >> 1) & 1), stop, a.err)) break;
             fence_after();
-            const TileAt c = tile_at(a, (int)blockIdx.x + ti * (int)gridDim.x);
+            const TileAt c = tile_at<PLANES>(a, (int)blockIdx.x + ti * (int)gridDim.x);
             const int vw = c.w0 + (m & 7), vh = c.h0 + (m >> 3);
             const uint32_t lane_addr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * p.ncols);
 #pragma unroll 1
-            for (int zp = 0; zp < TD; zp++) {
-                const int vd = c.d0 + zp;
-                const bool inside = vw < a.w && vh < a.h && vd < a.d;
-                const long long vox = (((long long)c.nb * a.d + vd) * a.h + vh) * a.w + vw;
+            for (int c0 = 0; c0 < a.nt; c0 += 16) {
+                const int ch = c.n0 + c0;
+                float bias[16];
+#pragma unroll
+                for (int j = 0; j < 16; j++) bias[j] = a.bias ? a.bias[ch + j] : 0.f;
+                // the warps of a lane quarter take every other plane
 #pragma unroll 1
-                for (int c0 = 0; c0 < a.nt; c0 += 32) {
-                    // two 16-column loads in flight before one wait (nt is 16, 32 or 64)
-                    uint32_t r[2][16];
-                    const int nh = a.nt - c0 >= 32 ? 2 : 1;
-                    tmem_ld16_async(lane_addr + (uint32_t)(zp * a.nt + c0), r[0]);
-                    if (nh == 2) tmem_ld16_async(lane_addr + (uint32_t)(zp * a.nt + c0 + 16), r[1]);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (!inside) continue;
-#pragma unroll
-                    for (int hh = 0; hh < 2; hh++) {
-                        if (hh >= nh) break;
-                        const int ch = c.n0 + c0 + hh * 16;
-                        float v[16];
-#pragma unroll
-                        for (int j = 0; j < 16; j++) v[j] = __uint_as_float(r[hh][j]);
-                        if (a.bias) {
-#pragma unroll
-                            for (int j = 0; j < 16; j++) v[j] += a.bias[ch + j];
-                        }
-                        if (a.relu) {
-#pragma unroll
-                            for (int j = 0; j < 16; j++) v[j] = fmaxf(v[j], 0.f);
-                        }
-                        if (a.mask) {
-                            const uint4* mp = reinterpret_cast<const uint4*>(a.mask + vox * a.ms + a.mo + ch);
-                            uint4 mv[2] = {mp[0], mp[1]};
-                            const unsigned short* mb = reinterpret_cast<const unsigned short*>(mv);
-#pragma unroll
-                            for (int j = 0; j < 16; j++)
-                                if (!bf16_pos(mb[j])) v[j] = 0.f;
-                        }
-                        __align__(16) __nv_bfloat162 o[8];
-#pragma unroll
-                        for (int j = 0; j < 8; j++) o[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-                        uint4* dst = reinterpret_cast<uint4*>(a.y + vox * a.ys + a.yo + ch);
-                        dst[0] = reinterpret_cast<const uint4*>(o)[0];
-                        dst[1] = reinterpret_cast<const uint4*>(o)[1];
+                for (int zp = (warp - 2) >> 2; zp < PLANES; zp += PERS_DRAIN / 4) {
+                    const int vd = c.d0 + zp;
+                    const bool inside = vw < a.w && vh < a.h && vd < a.d;
+                    const long long vox = (((long long)c.nb * a.d + vd) * a.h + vh) * a.w + vw;
+                    uint4 mv[2] = {};
+                    if (a.mask && inside) {
+                        const uint4* mp = reinterpret_cast<const uint4*>(a.mask + vox * a.ms + a.mo + ch);
+                        mv[0] = mp[0];
+                        mv[1] = mp[1];
                     }
+                    uint32_t r[16];
+                    tmem_ld16(lane_addr + (uint32_t)(zp * a.nt + c0), r);
+                    float v[16];
+#pragma unroll
+                    for (int j = 0; j < 16; j++) v[j] = __uint_as_float(r[j]);
+                    if (a.bias) {
+#pragma unroll
+                        for (int j = 0; j < 16; j++) v[j] += bias[j];
+                    }
+                    if (a.relu) {
+#pragma unroll
+                        for (int j = 0; j < 16; j++) v[j] = fmaxf(v[j], 0.f);
+                    }
+                    if (a.mask) {
+                        const unsigned short* mb = reinterpret_cast<const unsigned short*>(mv);
+#pragma unroll
+                        for (int j = 0; j < 16; j++)
+                            if (!bf16_pos(mb[j])) v[j] = 0.f;
+                    }
+                    __align__(16) __nv_bfloat162 o[8];
+#pragma unroll
+                    for (int j = 0; j < 8; j++) o[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+                    // lane pairs (neighbours along w) store one voxel's 32 bytes at a time: whole sectors
+                    const uint4 lo = reinterpret_cast<const uint4*>(o)[0], hi = reinterpret_cast<const uint4*>(o)[1];
+                    const bool odd = (lane & 1) != 0;
+                    uint4 x = odd ? lo : hi;
+                    x.x = __shfl_xor_sync(0xffffffffu, x.x, 1);
+                    x.y = __shfl_xor_sync(0xffffffffu, x.y, 1);
+                    x.z = __shfl_xor_sync(0xffffffffu, x.z, 1);
+                    x.w = __shfl_xor_sync(0xffffffffu, x.w, 1);
+                    const long long v0 = vox - (odd ? 1 : 0);
+                    __nv_bfloat16* dst = a.y + v0 * a.ys + a.yo + ch + (odd ? 8 : 0);
+                    const bool row = vh < a.h && vd < a.d;
+                    if (row && (vw & ~1) < a.w) *reinterpret_cast<uint4*>(dst) = odd ? x : lo;
+                    if (row && (vw | 1) < a.w) *reinterpret_cast<uint4*>(dst + a.ys) = odd ? hi : x;
                 }
             }
             fence_before();
@@ -671,7 +718,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_conv_wgrad(const WgArgs a, co
     __shared__ uint32_t tmem_base;
     __shared__ int s_stop, s_issued, s_consumed;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int chunk = (int)blockIdx.x % a.nchunk;
     const int part = ((int)blockIdx.x / a.nchunk) % a.nparts;
     const int ks = (int)blockIdx.x / (a.nchunk * a.nparts);
@@ -697,7 +744,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_conv_wgrad(const WgArgs a, co
     fence_before();
     __syncthreads();
     fence_after();
-    const uint32_t tmem = tmem_base;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
     volatile int* stop = &s_stop;
 
     if (warp == 12) {
@@ -730,13 +777,14 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_conv_wgrad(const WgArgs a, co
             s_issued = issued;
         }
     } else if (warp == 13) {
-        if (lane == 0) {
+        {
+            const uint32_t lead = elect_one() ? 1u : 0u;
             constexpr uint32_t idesc = idesc_bf16_mn(NT);
             int consumed = 0;
             bool ok = true;
             for (int j = 0; ok && j < my_tiles; j++) {
                 const int q = j & 1;
-                if (!mbar_wait_ab(&full[q], (unsigned)((j >> 1) & 1), stop, a.err)) break;
+                if (!__all_sync(0xffffffffu, mbar_wait_ab(&full[q], (unsigned)((j >> 1) & 1), stop, a.err))) break;
                 consumed = j + 1;
                 fence_after();
                 const uint32_t xb = s32(sm + q * a.stage_bytes), gb = xb + W::X_BYTES;
@@ -754,7 +802,8 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_conv_wgrad(const WgArgs a, co
                         const int pp = TAPS == 1 ? p >> 1 : p, np = TAPS == 1 ? (planes + 1 - pt) / 2 : planes;
                         const int use = pp / a.interval, at = pp - use * a.interval;
                         if (at == 0 && use > 0 &&
-                            !mbar_wait_ab(&acc_empty[pt], (unsigned)((use - 1) & 1), stop, a.err)) {
+                            !__all_sync(0xffffffffu,
+                                        mbar_wait_ab(&acc_empty[pt], (unsigned)((use - 1) & 1), stop, a.err))) {
                             ok = false;
                             break;
                         }
@@ -765,15 +814,15 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_conv_wgrad(const WgArgs a, co
                         for (int hp = 0; hp < TH / 2; hp++)
 #pragma unroll
                             for (int k = 0; k < W::PACC; k++)  // kw = k
-                                mma_bf16(acc0 + (uint32_t)(k * NT), adp + (uint64_t)(2 * hp * W::XW + k),
+                                mma_bf16_one(lead, acc0 + (uint32_t)(k * NT), adp + (uint64_t)(2 * hp * W::XW + k),
                                          bdz + (uint64_t)(2 * hp * TW), idesc, (hp > 0 || at > 0) ? 1u : 0u);
-                        if (at == a.interval - 1 || pp == np - 1) mma_commit(&acc_full[pt]);
+                        if (at == a.interval - 1 || pp == np - 1) mma_commit_one(lead, &acc_full[pt]);
                     }
                 }
-                mma_commit(&empty[q]);
+                mma_commit_one(lead, &empty[q]);
             }
-            s_consumed = ok ? consumed : -1;
-            mma_commit(&done);  // arrives once every MMA issued above has completed
+            if (lane == 0) s_consumed = ok ? consumed : -1;
+            mma_commit_one(lead, &done);  // arrives once every MMA issued above has completed
         }
     } else if (warp < 4 * W::PARTS) {
         const int pt = warp >> 2;
@@ -816,30 +865,79 @@ int pick_nt(int cout, int ntmax) {
 
 }  // namespace
 
-// activations [n][d][h][w][c] bf16 read in halo boxes of 8 channels
-bool conv_act_map(CUtensorMap* m, const void* base, int n, int d, int h, int w, int c, int taps) {
+static int sm_count() {
+    static int sms[64] = {0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    if (!sms[dev] && cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    return sms[dev];
+}
+
+// stages of a 3x3x3 tile of `planes` planes and nt output channels that fit in
+// shared memory; wres: the weights of all chunks stay resident
+static int pers_stages(int planes, int nt, int cin, int cout, bool& wres, int& stage_bytes) {
+    const int A = 2 * (TW + 2) * (TH + 2) * (planes + 2) * 16, B = 2 * 27 * nt * 16, room = SMEM_LIMIT - 128;
+    const long long w_all = (long long)(cin / 16) * B;
+    wres = nt == cout && w_all + 2 * A <= room;
+    stage_bytes = wres ? A : A + B;
+    const int n = wres ? (int)((room - w_all) / A) : room / stage_bytes;
+    return n < PERS_MAX_STAGES ? n : PERS_MAX_STAGES;
+}
+
+// The tile with the least estimated time: waves of tiles over the SMs times the MMAs of
+// one.  Deep tiles read fewer input planes per output plane (8: 10, 2: 4), so they win
+// wherever they fill the chip; on the small coarse layers shallow tiles and fewer
+// channels per CTA give it more CTAs (64 -> 64 channels at 16^3: 8 CTAs of 4 planes x 64
+// channels 24 us, 64 of 2 x 16 10 us; at 32^3: 64 CTAs of 4 planes 24, 128 of 2 14).
+ConvTile conv_tile(int taps, int n, int d, int h, int w, int cin, int cout) {
+    const int sms = sm_count() > 0 ? sm_count() : 1;
+    if (taps != 27) {
+        // pointwise: a plane at a time and fewer channels per CTA until every SM has two
+        // tiles (512 -> 64 channels at 16^3: 8 CTAs 28 us, 128 22)
+        ConvTile t{4, pick_nt(cout, 128)};
+        auto ctas = [&] {
+            return (long long)ceil_div(w, TW) * ceil_div(h, TH) * ceil_div(d, t.planes) * n * (cout / t.nt);
+        };
+        if (ctas() < 2 * sms) t.planes = 1;
+        while (ctas() < sms && t.nt % 32 == 0) t.nt /= 2;
+        return t;
+    }
+    ConvTile best{0, 0};
+    double least = 0.0;
+    for (int planes : {8, 4, 2}) {
+        for (int nt = pick_nt(cout, 64); nt >= 16; nt -= 16) {
+            bool wres;
+            int bytes;
+            if (cout % nt || 2 * tmem_cols(planes * nt) > 512 || pers_stages(planes, nt, cin, cout, wres, bytes) < 2)
+                continue;
+            // cycles of an MMA of N columns (its operands at ~100 bytes a cycle), of the box's
+            // 16-byte rows
+            auto mma = [](int N) { return 39.0 + 0.31 * N; };
+            const double mmas = 9.0 * (2 * mma(nt) + 2 * mma(2 * nt) + (planes - 2) * mma(3 * nt));
+            const double rows = 1.2 * 2 * (TW + 2) * (TH + 2) * (planes + 2), item = mmas > rows ? mmas : rows;
+            const long long tiles =
+                (long long)ceil_div(w, TW) * ceil_div(h, TH) * ceil_div(d, planes) * n * (cout / nt);
+            const double cost = (double)((tiles + sms - 1) / sms) * (item * (cin / 16)) + 400.0 * planes;
+            if (!best.planes || cost < least) {
+                best = ConvTile{planes, nt};
+                least = cost;
+            }
+        }
+    }
+    return best;
+}
+
+// activations [n][d][h][w][c] bf16 read in halo boxes of 8 channels and `planes` output planes
+bool conv_act_map(CUtensorMap* m, const void* base, int n, int d, int h, int w, int c, int taps, int planes) {
     auto enc = encoder();
     if (!enc || (reinterpret_cast<uintptr_t>(base) & 15) || c % 16) return false;
     const int H = taps == 27 ? 1 : 0;
     cuuint64_t dims[5] = {(cuuint64_t)c, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)d, (cuuint64_t)n};
     cuuint64_t str[4] = {(cuuint64_t)c * 2, (cuuint64_t)c * 2 * w, (cuuint64_t)c * 2 * w * h,
                          (cuuint64_t)c * 2 * w * h * d};
-    cuuint32_t box[5] = {8, (cuuint32_t)(TW + 2 * H), (cuuint32_t)(TH + 2 * H), (cuuint32_t)(TD + 2 * H), 1};
+    cuuint32_t box[5] = {8, (cuuint32_t)(TW + 2 * H), (cuuint32_t)(TH + 2 * H), (cuuint32_t)(planes + 2 * H), 1};
     cuuint32_t es[5] = {1, 1, 1, 1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, str, box, es,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// weights [taps][rows][kdim] bf16 read as (8 of kdim) x nt rows x all taps
-bool conv_wt_map(CUtensorMap* m, const void* base, int taps, int rows, int kdim, int nt) {
-    auto enc = encoder();
-    if (!enc || (reinterpret_cast<uintptr_t>(base) & 15) || kdim % 16) return false;
-    cuuint64_t dims[3] = {(cuuint64_t)kdim, (cuuint64_t)rows, (cuuint64_t)taps};
-    cuuint64_t str[2] = {(cuuint64_t)kdim * 2, (cuuint64_t)kdim * 2 * rows};
-    cuuint32_t box[3] = {8, (cuuint32_t)nt, (cuuint32_t)taps};
-    cuuint32_t es[3] = {1, 1, 1};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, str, box, es,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -870,21 +968,48 @@ bool wgrad_g_map(CUtensorMap* m, const void* base, int n, int d, int h, int w, i
     return wgrad_map(m, base, (long long)n * d, h, w, c, wgrad_nt(taps, c) / 8, TW, TH);
 }
 
-int conv_nt(int taps, int cout) { return pick_nt(cout, taps == 27 ? 64 : 128); }
+template <int PLANES>
+static int launch_pointwise(MmaArgs& a, unsigned grid, const ConvLaunch& L, cudaStream_t s) {
+    const int nchunk = a.cin / 16, stage = Halo<1, PLANES>::A_BYTES + 2 * a.nt * 16;
+    if (stage + 128 > SMEM_LIMIT) return FSIM_E_INVALID;
+    // as many CTAs per SM as TMEM holds accumulators of, at most four, with two to eight
+    // pipeline stages each (the issuing loop refills a stage one chunk late): their loads, MMAs and epilogues overlap (one CTA per SM took 41 us
+    // for 128 -> 32 channels at 64^3, now 27)
+    const int fit = 512 / tmem_cols(PLANES * a.nt), ctas = fit < 4 ? fit : 4, room = SMEM_LIMIT / ctas - 1024;
+    a.stages = 1;
+    while (a.stages < POINT_MAX_STAGES && a.stages < nchunk && (a.stages + 1) * stage + 128 <= room) a.stages++;
+    if (a.stages < 2 && nchunk > 1) return FSIM_E_INVALID;
+    int smem = a.stages * stage + 128;
+    const int least = SMEM_LIMIT / (ctas + 1) + 1024;  // no more CTAs than that
+    if (smem < least) smem = least;
+    if (set_smem_limit((const void*)k_conv_mma<PLANES>, SMEM_LIMIT) != cudaSuccess) return FSIM_E_CUDA;
+    k_conv_mma<PLANES><<<grid, CONV_THREADS, smem, s>>>(a, *L.mx);
+    return cudaGetLastError() == cudaSuccess ? FSIM_OK : FSIM_E_CUDA;
+}
+
+template <int PLANES>
+static int launch_pers(const PersArgs& p, int ctas, int smem, const ConvLaunch& L, cudaStream_t s) {
+    if (set_smem_limit((const void*)k_conv_pers<PLANES>, SMEM_LIMIT) != cudaSuccess) return FSIM_E_CUDA;
+    k_conv_pers<PLANES><<<ctas, PERS_THREADS, smem, s>>>(p, *L.mx);
+    return cudaGetLastError() == cudaSuccess ? FSIM_OK : FSIM_E_CUDA;
+}
 
 int launch_conv_mma(const ConvLaunch& L, cudaStream_t s) {
     const int taps = L.taps;
     if ((taps != 27 && taps != 1) || L.cin % 16 || L.cout % 16 || L.cin <= 0 || L.cout <= 0) return FSIM_E_INVALID;
+    if (reinterpret_cast<uintptr_t>(L.wgt) & 15) return FSIM_E_INVALID;  // (bulk copies)
     if (L.ys % 8 || L.yo % 8 || (L.mask && (L.ms % 8 || L.mo % 8))) return FSIM_E_INVALID;
     MmaArgs a{};
     a.n = L.n; a.d = L.d; a.h = L.h; a.w = L.w;
     a.cin = L.cin; a.cout = L.cout;
-    a.nt = conv_nt(taps, L.cout);
+    const ConvTile tile = conv_tile(taps, L.n, L.d, L.h, L.w, L.cin, L.cout);
+    a.nt = tile.nt;
     a.tiles_w = ceil_div(L.w, TW);
     a.tiles_h = ceil_div(L.h, TH);
-    a.tiles_d = ceil_div(L.d, TD);
+    a.tiles_d = ceil_div(L.d, tile.planes);
     a.ntiles = L.cout / a.nt;
     a.flip = L.flip;
+    a.wgt = L.wgt;
     a.bias = L.bias;
     a.relu = L.relu;
     a.mask = L.mask; a.ms = L.ms; a.mo = L.mo;
@@ -896,49 +1021,22 @@ int launch_conv_mma(const ConvLaunch& L, cudaStream_t s) {
     if (taps == 27) {
         if (grid >= (1ll << 31)) return FSIM_E_INVALID;
         PersArgs p{};
-        const int A = Halo<27>::A_BYTES, B_KC = 27 * a.nt * 16, w_all = nchunk * 2 * B_KC;
+        bool wres;
         p.total_tiles = (int)grid;
-        p.ncols = tmem_cols(TD * a.nt);
-        if (2 * p.ncols > 512) return FSIM_E_INVALID;
-        const int room = SMEM_LIMIT - 128;
-        if (a.ntiles == 1 && w_all + 2 * A <= room) {
-            p.wres = 1;
-            p.stage_bytes = A;
-            a.stages = (room - w_all) / A;
-        } else {
-            p.wres = 0;
-            p.stage_bytes = A + 2 * B_KC;
-            a.stages = room / p.stage_bytes;
-        }
-        if (a.stages < 2) return FSIM_E_INVALID;
-        if (a.stages > PERS_MAX_STAGES) a.stages = PERS_MAX_STAGES;
+        p.ncols = tmem_cols(tile.planes * a.nt);
+        a.stages = pers_stages(tile.planes, a.nt, L.cin, L.cout, wres, p.stage_bytes);
+        p.wres = wres ? 1 : 0;
         p.m = a;
-        int smem = a.stages * p.stage_bytes + (p.wres ? w_all : 0) + 128;
+        int smem = a.stages * p.stage_bytes + (wres ? nchunk * 2 * 27 * a.nt * 16 : 0) + 128;
         if (smem < SMEM_LIMIT / 2 + 1024) smem = SMEM_LIMIT / 2 + 1024;  // one CTA per SM
-        static int sms[64] = {0};
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return FSIM_E_CUDA;
-        if (!sms[dev] && cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            return FSIM_E_CUDA;
-        const int ctas = grid < sms[dev] ? (int)grid : sms[dev];
-        if (set_smem_limit((const void*)k_conv_pers, SMEM_LIMIT) != cudaSuccess) return FSIM_E_CUDA;
-        k_conv_pers<<<ctas, PERS_THREADS, smem, s>>>(p, *L.mx, *L.mw);
-        return cudaGetLastError() == cudaSuccess ? FSIM_OK : FSIM_E_CUDA;
+        const int sms = sm_count();
+        if (!sms) return FSIM_E_CUDA;
+        const int ctas = grid < sms ? (int)grid : sms;
+        return tile.planes == 8   ? launch_pers<8>(p, ctas, smem, L, s)
+               : tile.planes == 4 ? launch_pers<4>(p, ctas, smem, L, s)
+                                  : launch_pers<2>(p, ctas, smem, L, s);
     }
-    const int a_bytes = Halo<1>::A_BYTES;
-    const int stage = a_bytes + 2 * a.nt * 16;
-    if (stage + 128 > SMEM_LIMIT) return FSIM_E_INVALID;
-    // as many pipeline stages (<= 3, <= chunks) as keep two CTAs on an SM: the
-    // second CTA's loads and epilogue overlap the first one's MMAs
-    int stages = 1;
-    while (stages < 3 && stages < nchunk && (stages + 1) * stage + 128 <= SMEM_LIMIT / 2) stages++;
-    a.stages = stages;
-    int smem = stages * stage + 128;
-    // the pointwise kernel's accumulator can take all of TMEM: one CTA per SM
-    if (smem < 160 * 1024) smem = 160 * 1024;
-    if (set_smem_limit((const void*)k_conv_mma<1>, SMEM_LIMIT) != cudaSuccess) return FSIM_E_CUDA;
-    k_conv_mma<1><<<(unsigned)grid, CONV_THREADS, smem, s>>>(a, *L.mx, *L.mw);
-    return cudaGetLastError() == cudaSuccess ? FSIM_OK : FSIM_E_CUDA;
+    return tile.planes == 4 ? launch_pointwise<4>(a, (unsigned)grid, L, s) : launch_pointwise<1>(a, (unsigned)grid, L, s);
 }
 
 template <int TAPS, int NT>

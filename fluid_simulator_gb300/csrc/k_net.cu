@@ -442,7 +442,9 @@ __global__ void k_adam(float* theta, float* grad, float* m, float* v, long long 
 }
 
 // wb[t][n][c] and wt[t][c][n] from the FP32 master [t][n][c]
-__global__ void k_pack_weights(const float* w, int taps, int cout, int cin, bf16* wb, bf16* wt) {
+// [taps][cout][cin] FP32 -> the packed BF16 operands.  3x3x3: the three kd of a (kh, kw)
+// side by side, in the order of the output planes that one input plane feeds (k_conv_pers)
+__global__ void k_pack_weights(const float* w, int taps, int cout, int cin, int nt, int ntt, bf16* wb, bf16* wt) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long total = (long long)taps * cout * cin;
     if (i >= total) return;
@@ -450,8 +452,9 @@ __global__ void k_pack_weights(const float* w, int taps, int cout, int cin, bf16
     const int nn = (int)((i / cin) % cout);
     const int t = (int)(i / ((long long)cin * cout));
     const bf16 b = __float2bfloat16_rn(w[i]);
-    wb[i] = b;
-    wt[((long long)t * cin + c) * cout + nn] = b;
+    const int tb = taps == 27 ? (t % 9) * 3 + 2 - t / 9 : t, tt = taps == 27 ? (t % 9) * 3 + t / 9 : t;
+    wb[conv_pack_index(taps, cout, nt, tb, nn, c)] = b;
+    wt[conv_pack_index(taps, cin, ntt, tt, c, nn)] = b;
 }
 
 // ---- solver hook ------------------------------------------------------------
@@ -578,8 +581,8 @@ int pack_all_weights(fsim_net* net) {
     for (int l = 0; l < NET_LAYERS; l++) {
         const NetLayer& L = net->L[l];
         const long long tot = (long long)L.taps * L.cout * L.cin;
-        k_pack_weights<<<nblk(tot), NT_THREADS, 0, net->stream>>>(net->theta + L.w_off, L.taps, L.cout, L.cin, L.wb,
-                                                                  L.wt);
+        k_pack_weights<<<nblk(tot), NT_THREADS, 0, net->stream>>>(net->theta + L.w_off, L.taps, L.cout, L.cin, L.nt,
+                                                                  L.ntt, L.wb, L.wt);
     }
     net->launches += NET_LAYERS;
     NET_TRY(cudaGetLastError());
@@ -629,7 +632,6 @@ int ensure_ws(fsim_net* net, int n, int d, int h, int w, bool train) {
     NET_TRY(cudaMalloc(&mem, bytes));
     net->ws = mem;
     net->ws_bytes = bytes;
-    net->shape = s;
     char* base = (char*)mem;
     net->act.resize(NACT);
     for (int i = 0; i < NACT; i++) net->act[i] = NetBuf{(bf16*)(base + aoff[i]), kActC[i], kActL[i]};
@@ -648,12 +650,17 @@ int ensure_ws(fsim_net* net, int n, int d, int h, int w, bool train) {
     for (int l = 0; l < NET_LAYERS; l++) {
         const NetBuf& in = net->act[kIn[l]];
         const int lv = in.lev;
-        if (!conv_act_map(&net->amap[l], in.p, n, d >> lv, h >> lv, w >> lv, in.c, net->L[l].taps))
+        NetLayer& L = net->L[l];
+        const ConvTile t = conv_tile(L.taps, n, d >> lv, h >> lv, w >> lv, L.cin, L.cout);
+        L.nt = t.nt;
+        if (!conv_act_map(&net->amap[l], in.p, n, d >> lv, h >> lv, w >> lv, in.c, L.taps, t.planes))
             return fail(net, "tensor map of a network activation failed", FSIM_E_CUDA);
         if (train && l > 0) {
             const NetBuf& gz = net->gbuf[kGz[l]];
-            if (!conv_act_map(&net->amap[NET_LAYERS + l], gz.p, n, d >> gz.lev, h >> gz.lev, w >> gz.lev, gz.c,
-                              net->L[l].taps))
+            const ConvTile tg = conv_tile(L.taps, n, d >> gz.lev, h >> gz.lev, w >> gz.lev, L.cout, L.cin);
+            L.ntt = tg.nt;
+            if (!conv_act_map(&net->amap[NET_LAYERS + l], gz.p, n, d >> gz.lev, h >> gz.lev, w >> gz.lev, gz.c, L.taps,
+                              tg.planes))
                 return fail(net, "tensor map of a network gradient failed", FSIM_E_CUDA);
         }
         if (train) {
@@ -664,6 +671,10 @@ int ensure_ws(fsim_net* net, int n, int d, int h, int w, bool train) {
                 return fail(net, "tensor map of a weight-gradient operand failed", FSIM_E_CUDA);
         }
     }
+    // the packing follows the shape; the next pass may come on another stream
+    if (int rc = pack_all_weights(net)) return rc;
+    NET_TRY(cudaStreamSynchronize(net->stream));
+    net->shape = s;
     return FSIM_OK;
 }
 
@@ -687,7 +698,7 @@ int conv_fwd(fsim_net* net, int l) {
     c.yo = kOutOff[l];
     c.err = net->d_err;
     c.mx = &net->amap[l];
-    c.mw = &L.mw;
+    c.wgt = L.wb;
     net->launches++;
     return launch_conv_mma(c, net->stream);
 }
@@ -791,7 +802,7 @@ int conv_bwd(fsim_net* net, int l) {
     c.yo = 0;
     c.err = net->d_err;
     c.mx = &net->amap[NET_LAYERS + l];
-    c.mw = &L.mwt;
+    c.wgt = L.wt;
     net->launches++;
     rc = launch_conv_mma(c, net->stream);
     if (rc) return fail(net, "input-gradient launch failed", rc);
@@ -972,9 +983,6 @@ int fsim_net_create(uint64_t seed, float out_scale, fsim_net** out) {
         wp += cnt;
         L.wt = wp;
         wp += cnt;
-        if (!conv_wt_map(&L.mw, L.wb, L.taps, L.cout, L.cin, conv_nt(L.taps, L.cout)) ||
-            !conv_wt_map(&L.mwt, L.wt, L.taps, L.cin, L.cout, conv_nt(L.taps, L.cin)))
-            return bad("weight tensor maps");
     }
     // He initialisation (fan-in of the real inputs), zero biases, zero head
     std::vector<float> h((size_t)off, 0.f);
@@ -1198,13 +1206,14 @@ int fsim_net_conv(int taps, int mode, int n, int d, int h, int w, int cin, int c
     if (rc == FSIM_OK) {
         if (x) k_to_bf16<<<nblk(vox * cin), NT_THREADS, 0, s>>>(fx, vox * cin, bx);
         if (g) k_to_bf16<<<nblk(vox * cout), NT_THREADS, 0, s>>>(fg, vox * cout, bg);
-        if (wgt) k_pack_weights<<<nblk(nw), NT_THREADS, 0, s>>>(fw, taps, cout, cin, bw, bwt);
         CUtensorMap mx, mw;
         if (mode == 0 || mode == 1) {
             const bool m0 = mode == 0;
             const int kin = m0 ? cin : cout, kout = m0 ? cout : cin;
-            if (!conv_act_map(&mx, m0 ? bx : bg, n, d, h, w, kin, taps) ||
-                !conv_wt_map(&mw, m0 ? bw : bwt, taps, kout, kin, conv_nt(taps, kout))) {
+            const ConvTile tile = conv_tile(taps, n, d, h, w, kin, kout);
+            k_pack_weights<<<nblk(nw), NT_THREADS, 0, s>>>(fw, taps, cout, cin, m0 ? tile.nt : 16, m0 ? 16 : tile.nt, bw,
+                                                           bwt);
+            if (!conv_act_map(&mx, m0 ? bx : bg, n, d, h, w, kin, taps, tile.planes)) {
                 rc = FSIM_E_CUDA;
                 g_conv_err = "tensor map encoding failed";
             } else {
@@ -1219,7 +1228,7 @@ int fsim_net_conv(int taps, int mode, int n, int d, int h, int w, int cin, int c
                 c.yo = 0;
                 c.err = err;
                 c.mx = &mx;
-                c.mw = &mw;
+                c.wgt = m0 ? bw : bwt;
                 rc = launch_conv_mma(c, s);
                 if (rc) g_conv_err = std::string("convolution launch: ") + cudaGetErrorString(cudaGetLastError());
                 if (rc == FSIM_OK) k_to_f32<<<nblk(nout), NT_THREADS, 0, s>>>(bo, nout, fo);
