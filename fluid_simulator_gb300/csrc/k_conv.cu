@@ -108,7 +108,7 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
 // The issuing loops run on the whole warp and let one lane issue (predicated): control
 // flow stays uniform, so descriptors live in uniform registers.  With a single thread
 // branching off, every MMA first moved its operands there: 48 -> 16 channels at 128^3
-// 142 us, now 109; weight gradient of 16 -> 16 at 8 x 64^3 300 us, now 222.
+// 142 us, now 109; weight gradient of 16 -> 16 at 8 x 64^3 300 us, then 222.
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
     asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}" : "=r"(p));
@@ -627,8 +627,10 @@ __global__ void __launch_bounds__(PERS_THREADS, 1) k_conv_pers(const PersArgs p,
 // own four warps while the other parts' MMAs run.  One CTA per SM: warps 0-11 drain
 // and finally add to the gradient, warp 12 streams tiles through two stages, warp
 // 13 issues the MMAs.  Every wait is bounded, as in k_conv_pers.
-// What bounds it: the MMAs' operand reads (A 4 KB, B 32 N bytes per MMA at 128 bytes
-// per cycle: 36 cycles at N = 16, 288 MMAs per tile).  Training pass of 8 x 64^3:
+// What bounds it: the MMAs' operand reads, 4 KB of A per MMA whatever N is (~50 cycles).
+// With 16 output channels N is two neighbouring planes of G: X planes z .. z + 3 fill
+// M = 128, and the block of X plane p and G plane z belongs to kd = p - z (16 -> 16 at
+// 8 x 64^3: 222 us with one plane, 112 with two).  Training pass of 8 x 64^3:
 // 15.8 ms of weight gradients with the kernel this one replaced (threads
 // transposing 27 shifted copies of X into shared memory, two bytes at a time).
 constexpr int WG_THREADS = 448;  // 12 draining warps, TMA, MMA
@@ -647,12 +649,16 @@ struct Wg {
     static constexpr int PACC = TAPS == 27 ? 3 : 1;     // accumulators of a part
 };
 
+// planes of G side by side in an MMA's N (see below)
+template <int TAPS, int NT>
+constexpr int wgrad_zp = TAPS == 27 && NT == 16 ? 2 : 1;
+
 struct WgArgs {
     int cin, cout;
     int n, d, h, w;
     int tiles_w, tiles_h, tiles_d, tiles;
     int nchunk, nparts, ksplit;
-    int interval;            // planes per drain of an accumulator
+    int interval;            // steps (planes or pairs of planes) per drain of an accumulator
     int stage_bytes, ncols;
     float* dw;               // [taps][cout][cin], accumulated
     unsigned* err;
@@ -669,7 +675,7 @@ template <int TAPS, int NT>
 __device__ __forceinline__ void wgrad_drain(const WgArgs& a, uint32_t tmem, int pt, int uses, int chunk, int cpart,
                                             uint64_t* acc_full, uint64_t* acc_empty, volatile int* stop) {
     using W = Wg<TAPS>;
-    constexpr int COLS = W::PACC * NT;
+    constexpr int ZP = wgrad_zp<TAPS, NT>, NC = ZP * NT, COLS = W::PACC * NC;
     const int lane = threadIdx.x & 31, q = (threadIdx.x >> 5) & 3;
     const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(pt * COLS);
     float r[COLS];
@@ -694,16 +700,22 @@ __device__ __forceinline__ void wgrad_drain(const WgArgs& a, uint32_t tmem, int 
         __syncwarp();
         if (lane == 0) mbar_arrive(acc_empty);
     }
-    // row m = (kd, octet, channel); rows past the used groups hold sums over other data
+    // row m = (X plane, octet, channel), column block z = G plane: kd = X plane - z; blocks with
+    // another kd hold sums nobody needs
     const int m = q * 32 + lane;
-    const int kd = (m >> 3) / W::OCT, c = chunk * W::OCT * 8 + ((m >> 3) % W::OCT) * 8 + (m & 7);
-    if (kd >= (TAPS == 27 ? 3 : 1) || c >= a.cin) return;
+    const int xp = (m >> 3) / W::OCT, c = chunk * W::OCT * 8 + ((m >> 3) % W::OCT) * 8 + (m & 7);
+    if (c >= a.cin) return;
 #pragma unroll
-    for (int k = 0; k < W::PACC; k++) {
-        const int tap = TAPS == 27 ? kd * 9 + pt * 3 + k : 0;
-        float* o = a.dw + ((long long)tap * a.cout + cpart * NT) * a.cin + c;
+    for (int z = 0; z < ZP; z++) {
+        const int kd = xp - z;
+        if (kd < 0 || kd >= (TAPS == 27 ? 3 : 1)) continue;
 #pragma unroll
-        for (int j = 0; j < NT; j++) atomicAdd(o + (long long)j * a.cin, r[k * NT + j]);
+        for (int k = 0; k < W::PACC; k++) {
+            const int tap = TAPS == 27 ? kd * 9 + pt * 3 + k : 0;
+            float* o = a.dw + ((long long)tap * a.cout + cpart * NT) * a.cin + c;
+#pragma unroll
+            for (int j = 0; j < NT; j++) atomicAdd(o + (long long)j * a.cin, r[k * NC + z * NT + j]);
+        }
     }
 }
 
@@ -712,6 +724,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_conv_wgrad(const WgArgs a, co
                                                               const __grid_constant__ CUtensorMap tg) {
     using W = Wg<TAPS>;
     constexpr int G_PLANE = (NT >> 3) * W::G_OCT;
+    constexpr int ZP = wgrad_zp<TAPS, NT>, NC = ZP * NT;
     extern __shared__ __align__(128) unsigned char smraw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>(((uintptr_t)smraw + 127) & ~(uintptr_t)127);
     __shared__ __align__(8) uint64_t full[2], empty[2], acc_full[3], acc_empty[3], done;
@@ -723,7 +736,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_conv_wgrad(const WgArgs a, co
     const int part = ((int)blockIdx.x / a.nchunk) % a.nparts;
     const int ks = (int)blockIdx.x / (a.nchunk * a.nparts);
     const int my_tiles = (a.tiles - 1 - ks) / a.ksplit + 1;  // ks < ksplit <= tiles
-    const int planes = my_tiles * W::PD;
+    const int steps = my_tiles * (W::PD / ZP);
 
     if (threadIdx.x == 0) {
         for (int q = 0; q < 2; q++) {
@@ -779,7 +792,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_conv_wgrad(const WgArgs a, co
     } else if (warp == 13) {
         {
             const uint32_t lead = elect_one() ? 1u : 0u;
-            constexpr uint32_t idesc = idesc_bf16_mn(NT);
+            constexpr uint32_t idesc = idesc_bf16_mn(NC);
             int consumed = 0;
             bool ok = true;
             for (int j = 0; ok && j < my_tiles; j++) {
@@ -791,15 +804,15 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_conv_wgrad(const WgArgs a, co
                 const uint64_t ad0 = sdesc_mn(xb, W::XW * 16, W::X_OCT);
                 const uint64_t bd0 = sdesc_mn(gb, TW * 16, W::G_OCT);
 #pragma unroll 1
-                for (int z = 0; ok && z < W::PD; z++) {
-                    const int p = j * W::PD + z;  // pointwise: plane p >> 1 of part p & 1
+                for (int z = 0; ok && z < W::PD; z += ZP) {
+                    const int p = (j * W::PD + z) / ZP;  // pointwise: plane p >> 1 of part p & 1
                     // start-address fields are in 16-byte units
                     const uint64_t adz = ad0 + (uint64_t)(z * W::X_PLANE / 16);
                     const uint64_t bdz = bd0 + (uint64_t)(z * G_PLANE / 16);
 #pragma unroll 1
                     for (int pt = 0; pt < W::PARTS; pt++) {
                         if (TAPS == 1 && (p & 1) != pt) continue;
-                        const int pp = TAPS == 1 ? p >> 1 : p, np = TAPS == 1 ? (planes + 1 - pt) / 2 : planes;
+                        const int pp = TAPS == 1 ? p >> 1 : p, np = TAPS == 1 ? (steps + 1 - pt) / 2 : steps;
                         const int use = pp / a.interval, at = pp - use * a.interval;
                         if (at == 0 && use > 0 &&
                             !__all_sync(0xffffffffu,
@@ -809,12 +822,12 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_conv_wgrad(const WgArgs a, co
                         }
                         fence_after();
                         const uint64_t adp = adz + (uint64_t)(TAPS == 27 ? pt * W::XW : 0);  // kh = pt
-                        const uint32_t acc0 = tmem + (uint32_t)(pt * W::PACC * NT);
+                        const uint32_t acc0 = tmem + (uint32_t)(pt * W::PACC * NC);
 #pragma unroll
                         for (int hp = 0; hp < TH / 2; hp++)
 #pragma unroll
                             for (int k = 0; k < W::PACC; k++)  // kw = k
-                                mma_bf16_one(lead, acc0 + (uint32_t)(k * NT), adp + (uint64_t)(2 * hp * W::XW + k),
+                                mma_bf16_one(lead, acc0 + (uint32_t)(k * NC), adp + (uint64_t)(2 * hp * W::XW + k),
                                          bdz + (uint64_t)(2 * hp * TW), idesc, (hp > 0 || at > 0) ? 1u : 0u);
                         if (at == a.interval - 1 || pp == np - 1) mma_commit_one(lead, &acc_full[pt]);
                     }
@@ -826,7 +839,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_conv_wgrad(const WgArgs a, co
         }
     } else if (warp < 4 * W::PARTS) {
         const int pt = warp >> 2;
-        const int np = TAPS == 27 ? planes : (planes + 1 - pt) / 2;
+        const int np = TAPS == 27 ? steps : (steps + 1 - pt) / 2;
         wgrad_drain<TAPS, NT>(a, tmem, pt, (np + a.interval - 1) / a.interval, chunk, part, &acc_full[pt],
                               &acc_empty[pt], stop);
     }
@@ -1061,15 +1074,16 @@ static int launch_wgrad(const WgradLaunch& L, cudaStream_t s) {
     const int groups = a.nchunk * a.nparts;
     a.ksplit = sms / groups > 0 ? sms / groups : 1;
     if (a.ksplit > a.tiles) a.ksplit = a.tiles;
-    // Drain depth (8 MMAs per plane): an eighth of the CTA's planes or less, 1 to 8.
-    // Draining after every plane costs the MMAs a third of their rate (8 x 64^3,
-    // 16 -> 16: 326 us against 230), and this stays below the depth at which the
-    // sums were as exact as before (all of a quarter as many voxels).
-    const int planes = ceil_div(a.tiles, a.ksplit) * W::PD / (TAPS == 1 ? 2 : 1);
+    // Drain depth (8 MMAs per step, a plane or a pair): an eighth of the CTA's steps or
+    // less, 1 to 8.  Draining after every plane cost the MMAs a third of their rate (8 x
+    // 64^3, 16 -> 16: 326 us against 230), and this stays below the depth at which the
+    // sums were as exact as with the kernel before (all of a quarter as many voxels).
+    constexpr int ZP = wgrad_zp<TAPS, NT>;
+    const int steps = ceil_div(a.tiles, a.ksplit) * (W::PD / ZP) / (TAPS == 1 ? 2 : 1);
     a.interval = 1;
-    while (a.interval < 8 && 2 * a.interval * 10 <= planes) a.interval *= 2;
+    while (a.interval < 8 && 2 * a.interval * 10 <= steps) a.interval *= 2;
     a.stage_bytes = W::X_BYTES + W::PD * (NT / 8) * W::G_OCT;
-    a.ncols = tmem_cols(TAPS == 27 ? W::ACC * NT : 2 * NT);
+    a.ncols = tmem_cols(TAPS == 27 ? W::ACC * ZP * NT : 2 * NT);
     a.dw = L.dw;
     a.err = L.err;
     // the unused M groups of the last planes read past the X box, into the stage's G box
