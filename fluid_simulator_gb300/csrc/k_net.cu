@@ -65,37 +65,37 @@ __global__ void k_to_f32(const bf16* in, long long n, float* out) {
 
 // ---- space-to-depth (2x2x2 stride-2 down-convolution = s2d + pointwise) -----
 // dst[coarse][(sd*4 + sh*2 + sw)*C + c] = src[2*coarse + (sd, sh, sw)][c]
+template <typename I>
 __global__ void k_s2d(const bf16* src, int ss, int so, int C, int n, int D, int H, int W, bf16* dst) {
     const int oct = C / 8;
-    const long long total = (long long)n * (D / 2) * (H / 2) * (W / 2) * 8 * oct;
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const I total = (I)n * (D / 2) * (H / 2) * (W / 2) * 8 * oct;
+    const I i = (I)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
-    const int o = (int)(i % oct);
-    long long t = i / oct;
-    const int sub = (int)(t % 8);
-    const long long cv = t / 8;  // coarse voxel
-    const int cw = (int)(cv % (W / 2)), chh = (int)((cv / (W / 2)) % (H / 2));
-    const long long cdn = cv / ((long long)(W / 2) * (H / 2));  // n * D/2 + cd
-    const int cd = (int)(cdn % (D / 2));
-    const int nb = (int)(cdn / (D / 2));
+    const int o = (int)(i % (I)oct);
+    const I t = i / (I)oct;
+    const int sub = (int)(t & 7);
+    const I cv = t >> 3;  // coarse voxel
+    const I row = cv / (I)(W / 2), pl = row / (I)(H / 2), smp = pl / (I)(D / 2);
+    const int cw = (int)(cv - row * (W / 2)), chh = (int)(row - pl * (H / 2)), cd = (int)(pl - smp * (D / 2));
+    const int nb = (int)smp;
     const int fd = 2 * cd + (sub >> 2), fh = 2 * chh + ((sub >> 1) & 1), fw = 2 * cw + (sub & 1);
     const long long fv = (((long long)nb * D + fd) * H + fh) * W + fw;
-    *reinterpret_cast<uint4*>(dst + cv * 8 * C + sub * C + o * 8) =
+    *reinterpret_cast<uint4*>(dst + (long long)cv * 8 * C + sub * C + o * 8) =
         *reinterpret_cast<const uint4*>(src + fv * ss + so + o * 8);
 }
 
 // out[fine][c] = (gs[coarse][sub*C + c] + gc[fine][gco + c]) * (m[fine][mo + c] > 0)
+template <typename I>
 __global__ void k_d2s_add_mask(const bf16* gs, const bf16* gc, int gcs, int gco, const bf16* m, int ms, int mo,
                                int C, int n, int D, int H, int W, bf16* out) {
     const int oct = C / 8;
-    const long long total = (long long)n * D * H * W * oct;
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const I total = (I)n * D * H * W * oct;
+    const I i = (I)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
-    const int o = (int)(i % oct);
-    const long long fv = i / oct;
-    const int fw = (int)(fv % W), fh = (int)((fv / W) % H);
-    const long long fdn = fv / ((long long)W * H);
-    const int fd = (int)(fdn % D), nb = (int)(fdn / D);
+    const I vi = i / (I)oct, row = vi / (I)W, pl = row / (I)H, smp = pl / (I)D;
+    const int o = (int)(i - vi * oct);
+    const int fw = (int)(vi - row * W), fh = (int)(row - pl * H), fd = (int)(pl - smp * D), nb = (int)smp;
+    const long long fv = (long long)vi;
     const long long cv = (((long long)nb * (D / 2) + fd / 2) * (H / 2) + fh / 2) * (W / 2) + fw / 2;
     const int sub = ((fd & 1) << 2) | ((fh & 1) << 1) | (fw & 1);
     float a[8], b[8], mk[8];
@@ -198,51 +198,56 @@ __global__ void __launch_bounds__(NT_THREADS, 3) k_upsample(const bf16* src, int
     }
 }
 
-// weights of coarse index k in the fine samples near it (adjoint of up_src)
-__device__ __forceinline__ int up_adj(int k, int nc, int (&f)[6], float (&w)[6]) {
-    int cnt = 0;
-    for (int ff = 2 * k - 2; ff <= 2 * k + 3; ff++) {
-        if (ff < 0 || ff >= 2 * nc) continue;
-        int i0, i1;
-        float l1;
-        up_src(ff, nc, i0, i1, l1);
-        float wt = 0.f;
-        if (i0 == k) wt += 1.f - l1;
-        if (i1 == k) wt += l1;
-        if (wt != 0.f) {
-            f[cnt] = ff;
-            w[cnt] = wt;
-            cnt++;
-        }
-    }
-    return cnt;
+// Adjoint of up_src: coarse k receives fine 2k - 1 .. 2k + 2 with weights 1/4, 3/4, 3/4,
+// 1/4; at a border the missing sample's weight goes to its neighbour (clamping).
+__device__ __forceinline__ void up_adj(int k, int nc, float (&w)[4]) {
+    w[0] = k > 0 ? 0.25f : 0.f;
+    w[1] = k > 0 ? 0.75f : 1.f;
+    w[2] = k < nc - 1 ? 0.75f : 1.f;
+    w[3] = k < nc - 1 ? 0.25f : 0.f;
 }
 
-// out[coarse][c] = (sum_fine w * g[fine][c]) * (m[coarse][c] > 0); g channel stride gs (offset 0)
+// out[coarse][c] = (sum_fine w * g[fine][c]) * (m[coarse][c] > 0); g channel stride gs (offset 0).
+// Bound by the 64 reads per output octet, which L1 serves: with run-time lists of samples
+// and 64-bit index arithmetic 178 us for 32 channels at 8 x 64^3, now 92.
+template <typename I>
 __global__ void k_upsample_bwd(const bf16* g, int gs, const bf16* m, int C, int n, int D, int H, int W, bf16* out) {
     const int oct = C / 8;
-    const long long total = (long long)n * D * H * W * oct;
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const I total = (I)n * D * H * W * oct;
+    const I i = (I)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
-    const int o = (int)(i % oct);
-    const long long cv = i / oct;
-    const int cw = (int)(cv % W), chh = (int)((cv / W) % H);
-    const long long cdn = cv / ((long long)W * H);
-    const int cd = (int)(cdn % D), nb = (int)(cdn / D);
-    int fd[6], fh[6], fw[6];
-    float wd[6], wh[6], ww[6];
-    const int nd = up_adj(cd, D, fd, wd), nh = up_adj(chh, H, fh, wh), nw = up_adj(cw, W, fw, ww);
+    const I vi = i / (I)oct, row = vi / (I)W, pl = row / (I)H, smp = pl / (I)D;
+    const int o = (int)(i - vi * oct);
+    const int cw = (int)(vi - row * W), chh = (int)(row - pl * H), cd = (int)(pl - smp * D), nb = (int)smp;
+    const long long cv = (long long)vi;
+    float wd[4], wh[4], ww[4];
+    up_adj(cd, D, wd);
+    up_adj(chh, H, wh);
+    up_adj(cw, W, ww);
     const int FD = 2 * D, FH = 2 * H, FW = 2 * W;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int a = 0; a < nd; a++)
-        for (int b = 0; b < nh; b++)
-            for (int c = 0; c < nw; c++) {
-                const float wt = wd[a] * wh[b] * ww[c];
-                float v[8];
-                ld8(g + ((((long long)nb * FD + fd[a]) * FH + fh[b]) * FW + fw[c]) * gs + o * 8, v);
 #pragma unroll
-                for (int j = 0; j < 8; j++) acc[j] += wt * v[j];
+    for (int a = 0; a < 4; a++) {
+        if (wd[a] == 0.f) continue;
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            if (wh[b] == 0.f) continue;
+            const bf16* p = g + ((((long long)nb * FD + 2 * cd - 1 + a) * FH + 2 * chh - 1 + b) * FW + 2 * cw - 1) * gs + o * 8;
+            const float wab = wd[a] * wh[b];
+            float v[4][8];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                if (ww[c] != 0.f) ld8(p + (long long)c * gs, v[c]);
             }
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                if (ww[c] == 0.f) continue;
+                const float wt = wab * ww[c];
+#pragma unroll
+                for (int j = 0; j < 8; j++) acc[j] += wt * v[c][j];
+            }
+        }
+    }
     float mk[8];
     ld8(m + cv * C + o * 8, mk);
 #pragma unroll
@@ -273,20 +278,50 @@ __global__ void k_head(const bf16* d0, long long vox, const float* wgt, const fl
 //   L_s = ||r|| / ||b|| + lam ||e|| / ||target||,   loss = mean_s L_s.
 // Pass 1 stores r and adds the per-sample sums of r^2, e^2, target^2, b^2;
 // k_loss_coef turns them into the loss and the per-sample gradient factors;
-// pass 2 writes dloss/dout = c_r A r + c_e e.  Warps never straddle two
-// samples (each sample's voxel count is a multiple of 512).
+// pass 2 writes dloss/dout = c_r A r + c_e e.  Blocks of 512 voxels never straddle
+// two samples (each sample's voxel count is a multiple of 512).
+//
+// Pass 1's sums are kept as FP32 pairs (value and rounding error, ~48 bits) until the
+// block adds them to the FP64 sums: FP64 arithmetic runs at 1/64 of the FP32 rate, and
+// summing doubles across every warp with four atomics each took 229 us at 8 x 64^3 (the
+// second pass, which moves as much, 29); now 43.
+struct FF {
+    float hi = 0.f, lo = 0.f;
+    __device__ __forceinline__ void add(float v, float e) {  // + v + e
+        const float s = hi + v, b = s - hi;
+        lo += ((hi - (s - b)) + (v - b)) + e;
+        hi = s;
+    }
+    // squares that FP32 cannot hold with their rounding error go to the FP64 sum at once
+    __device__ __forceinline__ void add_square(float v, double* sum) {
+        if (fabsf(v) <= 1e15f && fabsf(v) >= 1e-15f) {
+            const float p = v * v;
+            add(p, __fmaf_rn(v, v, -p));
+        } else if (v != 0.f) {
+            atomicAdd(sum, (double)v * v);
+        }
+    }
+};
+constexpr int LOSS_VPT = 512 / NT_THREADS;  // voxels per thread
 __device__ __forceinline__ bool vox_solid(const bf16* x0, long long v) { return __bfloat162float(x0[v * 16 + 2]) > 0.5f; }
 
-template <bool GRAD>
+template <bool GRAD, typename I>
 __global__ void k_loss(const float* out, const float* target, const uint8_t* mask, const bf16* x0, int n, int D,
                        int H, int W, float* r, float* gout, double* sums, const float* coef) {
     const long long per = (long long)D * H * W;
-    const long long vox = (long long)n * per;
-    const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    double q[4] = {0.0, 0.0, 0.0, 0.0};
-    const int smp = (int)(min(v, vox - 1) / per);
-    if (v < vox && mask[v]) {
-        const int w = (int)(v % W), h = (int)((v / W) % H), d = (int)((v / ((long long)W * H)) % D);
+    const int smp = (int)((I)blockIdx.x * 512 / (I)per);
+    FF q[4];
+#pragma unroll
+    for (int it = 0; it < LOSS_VPT; it++) {
+        const I vi = (I)blockIdx.x * 512 + it * NT_THREADS + threadIdx.x;
+        const long long v = (long long)vi;
+        if (!mask[v]) {
+            if (GRAD) gout[v] = 0.f;
+            else r[v] = 0.f;
+            continue;
+        }
+        const I row = vi / (I)W, pl = row / (I)H;
+        const int w = (int)(vi - row * W), h = (int)(row - pl * H), d = (int)(pl % (I)D);
         const long long off[6] = {1, -1, W, -(long long)W, (long long)W * H, -(long long)W * H};
         const bool in[6] = {w + 1 < W, w > 0, h + 1 < H, h > 0, d + 1 < D, d > 0};
         int ns = 0;
@@ -303,22 +338,29 @@ __global__ void k_loss(const float* out, const float* target, const uint8_t* mas
             gout[v] = coef[2 * smp] * ((float)ns * r[v] - nb) + coef[2 * smp + 1] * ev;
         } else {
             const float rv = (float)ns * ev - nb;
-            const float bv = __bfloat162float(x0[v * 16]);
             r[v] = rv;
-            q[0] = (double)rv * rv;
-            q[1] = (double)ev * ev;
-            q[2] = (double)target[v] * target[v];
-            q[3] = (double)bv * bv;
+            q[0].add_square(rv, sums + 4 * smp);
+            q[1].add_square(ev, sums + 4 * smp + 1);
+            q[2].add_square(target[v], sums + 4 * smp + 2);
+            q[3].add_square(__bfloat162float(x0[v * 16]), sums + 4 * smp + 3);
         }
-    } else if (v < vox) {
-        if (GRAD) gout[v] = 0.f;
-        else r[v] = 0.f;
     }
     if (!GRAD) {
+        __shared__ double part[4][NT_THREADS / 32];
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            for (int o = 16; o > 0; o >>= 1) q[k] += __shfl_xor_sync(0xffffffffu, q[k], o);
-            if ((threadIdx.x & 31) == 0 && q[k] != 0.0) atomicAdd(&sums[4 * smp + k], q[k]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const float hi = __shfl_xor_sync(0xffffffffu, q[k].hi, o), lo = __shfl_xor_sync(0xffffffffu, q[k].lo, o);
+                q[k].add(hi, lo);
+            }
+            if ((threadIdx.x & 31) == 0) part[k][threadIdx.x >> 5] = (double)q[k].hi + (double)q[k].lo;
+        }
+        __syncthreads();
+        if (threadIdx.x < 4) {
+            double t = 0.0;
+            for (int k = 0; k < NT_THREADS / 32; k++) t += part[threadIdx.x][k];
+            if (t != 0.0) atomicAdd(&sums[4 * smp + threadIdx.x], t);
         }
     }
 }
@@ -411,18 +453,33 @@ __global__ void k_head_bwd(const bf16* d0, const float* gout, long long vox, con
     }
 }
 
-// gb[c] += sum_v g[v][c]   (C in {16, 32, 64})
+// gb[c] += sum_v g[v][c]   (C in {16, 32, 64}); a thread sums eight neighbouring channels
+// (one 16-byte load a voxel: 25 us with 2-byte loads for 16 channels at 8 x 64^3, now 13)
 __global__ void k_bias_grad(const bf16* g, long long vox, int C, float* gb) {
-    __shared__ float red[NT_THREADS];
-    const int c = threadIdx.x % C, lane = threadIdx.x / C, lanes = NT_THREADS / C;
-    float s = 0.f;
-    for (long long v = (long long)blockIdx.x * lanes + lane; v < vox; v += (long long)gridDim.x * lanes)
-        s += __bfloat162float(g[v * C + c]);
-    red[threadIdx.x] = s;
+    __shared__ float red[8][NT_THREADS + 1];
+    const int oct = C >> 3, o = threadIdx.x % oct, lane = threadIdx.x / oct, lanes = NT_THREADS / oct;
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const long long step = (long long)gridDim.x * lanes;
+#pragma unroll 4
+    for (long long v = (long long)blockIdx.x * lanes + lane; v < vox; v += step) {
+        float a[8];
+        ld8(g + v * C + o * 8, a);
+#pragma unroll
+        for (int j = 0; j < 8; j++) s[j] += a[j];
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j++) red[j][threadIdx.x] = s[j];
     __syncthreads();
-    if (lane == 0) {
-        for (int k = 1; k < lanes; k++) s += red[k * C + c];
-        atomicAdd(gb + c, s);
+    // eight threads per channel, then one
+    const int c = threadIdx.x >> 3, part = threadIdx.x & 7;
+    for (int c0 = 0; c0 < C; c0 += NT_THREADS / 8) {
+        const int cc = c0 + c;
+        float t = 0.f;
+        if (cc < C)
+            for (int k = part; k < lanes; k += 8) t += red[cc & 7][k * oct + (cc >> 3)];
+#pragma unroll
+        for (int d = 4; d > 0; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
+        if (cc < C && part == 0) atomicAdd(gb + cc, t);
     }
 }
 
@@ -708,7 +765,8 @@ int s2d(fsim_net* net, int src, int so, int C, int dst) {
     const int lv = s.lev;
     const NetShape& sh = net->shape;
     const long long total = level_vox(sh, lv + 1) * 8 * (C / 8);
-    k_s2d<<<nblk(total), NT_THREADS, 0, net->stream>>>(s.p, s.c, so, C, sh.n, sh.d >> lv, sh.h >> lv, sh.w >> lv,
+    auto* k = total < (1ll << 31) ? k_s2d<uint32_t> : k_s2d<unsigned long long>;
+    k<<<nblk(total), NT_THREADS, 0, net->stream>>>(s.p, s.c, so, C, sh.n, sh.d >> lv, sh.h >> lv, sh.w >> lv,
                                                        net->act[dst].p);
     net->launches++;
     return FSIM_OK;
@@ -775,7 +833,7 @@ int conv_bwd(fsim_net* net, int l) {
     int rc = launch_conv_wgrad(wg, net->stream);
     if (rc) return fail(net, "weight-gradient launch failed", rc);
     const long long vox = level_vox(sh, lv);
-    int bl = (int)std::min<long long>((vox + 255) / 256, 1024);
+    const int bl = (int)std::min<long long>((vox * (L.cout / 8) + 2047) / 2048, 4 * 152);
     k_bias_grad<<<bl, NT_THREADS, 0, net->stream>>>(gz.p, vox, L.cout, net->grad + L.b_off);
     net->launches += 2;
     if (kGin[l] < 0) return FSIM_OK;
@@ -814,9 +872,9 @@ int up_bwd(fsim_net* net, int gcat, int mask, int out) {
     const int lv = m.lev;
     const NetShape& sh = net->shape;
     const long long total = level_vox(sh, lv) * (m.c / 8);
-    k_upsample_bwd<<<nblk(total), NT_THREADS, 0, net->stream>>>(net->gbuf[gcat].p, net->gbuf[gcat].c, m.p, m.c, sh.n,
-                                                                sh.d >> lv, sh.h >> lv, sh.w >> lv,
-                                                                net->gbuf[out].p);
+    auto* k = total < (1ll << 31) ? k_upsample_bwd<uint32_t> : k_upsample_bwd<unsigned long long>;
+    k<<<nblk(total), NT_THREADS, 0, net->stream>>>(net->gbuf[gcat].p, net->gbuf[gcat].c, m.p, m.c, sh.n, sh.d >> lv,
+                                                   sh.h >> lv, sh.w >> lv, net->gbuf[out].p);
     net->launches++;
     return FSIM_OK;
 }
@@ -826,9 +884,9 @@ int d2s(fsim_net* net, int gs2d, int gcat, int cat, int off, int C, int out) {
     const int lv = gc.lev;
     const NetShape& sh = net->shape;
     const long long total = level_vox(sh, lv) * (C / 8);
-    k_d2s_add_mask<<<nblk(total), NT_THREADS, 0, net->stream>>>(net->gbuf[gs2d].p, gc.p, gc.c, off, net->act[cat].p,
-                                                                net->act[cat].c, off, C, sh.n, sh.d >> lv,
-                                                                sh.h >> lv, sh.w >> lv, net->gbuf[out].p);
+    auto* k = total < (1ll << 31) ? k_d2s_add_mask<uint32_t> : k_d2s_add_mask<unsigned long long>;
+    k<<<nblk(total), NT_THREADS, 0, net->stream>>>(net->gbuf[gs2d].p, gc.p, gc.c, off, net->act[cat].p, net->act[cat].c, off,
+                                                   C, sh.n, sh.d >> lv, sh.h >> lv, sh.w >> lv, net->gbuf[out].p);
     net->launches++;
     return FSIM_OK;
 }
@@ -838,12 +896,15 @@ int net_backward(fsim_net* net, const float* target, const uint8_t* mask, float*
     const NetShape& sh = net->shape;
     if (sh.n > NET_MAX_BATCH) return fail(net, "training batch larger than 64 samples", FSIM_E_INVALID);
     NET_TRY(cudaMemsetAsync(net->d_sums, 0, sizeof(double) * 4 * sh.n, net->stream));
-    k_loss<false><<<nblk(vox), NT_THREADS, 0, net->stream>>>(net->out, target, mask, net->act[X0].p, sh.n, sh.d, sh.h,
-                                                             sh.w, net->res, nullptr, net->d_sums, nullptr);
+    auto* pass1 = vox < (1ll << 31) ? k_loss<false, uint32_t> : k_loss<false, unsigned long long>;
+    auto* pass2 = vox < (1ll << 31) ? k_loss<true, uint32_t> : k_loss<true, unsigned long long>;
+    const unsigned nb = (unsigned)(vox / 512);
+    pass1<<<nb, NT_THREADS, 0, net->stream>>>(net->out, target, mask, net->act[X0].p, sh.n, sh.d, sh.h, sh.w, net->res,
+                                              nullptr, net->d_sums, nullptr);
     k_loss_coef<<<1, 32, 0, net->stream>>>(net->d_sums, sh.n, net->loss_l2_weight, net->d_coef, net->d_loss,
                                            loss_out);
-    k_loss<true><<<nblk(vox), NT_THREADS, 0, net->stream>>>(net->out, target, mask, net->act[X0].p, sh.n, sh.d, sh.h,
-                                                            sh.w, net->res, net->gout, nullptr, net->d_coef);
+    pass2<<<nb, NT_THREADS, 0, net->stream>>>(net->out, target, mask, net->act[X0].p, sh.n, sh.d, sh.h, sh.w, net->res,
+                                              net->gout, nullptr, net->d_coef);
     k_head_bwd<<<nblk(vox), NT_THREADS, 0, net->stream>>>(net->act[D0].p, net->gout, vox, net->theta + net->head_w,
                                                           net->out_scale, net->gbuf[GD0].p, net->grad + net->head_w,
                                                           net->grad + net->head_b);
