@@ -42,6 +42,24 @@ __device__ __forceinline__ void st8(bf16* p, const float (&v)[8]) {
     *reinterpret_cast<uint4*>(p) = u;
 }
 
+// acc[0..7] += w * v[0..7] as four packed FMAs (the same roundings as eight single ones);
+// a BF16 pair unpacks with one instruction a value
+__device__ __forceinline__ void fma8(unsigned long long (&acc)[4], float w, const uint4& v) {
+    const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+    unsigned long long w2;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(w2) : "f"(w));
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        unsigned long long f;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(f) : "r"(u[j] << 16), "r"(u[j] & 0xffff0000u));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[j]) : "l"(w2), "l"(f));
+    }
+}
+__device__ __forceinline__ void unpack8(const unsigned long long (&acc)[4], float (&v)[8]) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) asm("mov.b64 {%0, %1}, %2;" : "=f"(v[2 * j]), "=f"(v[2 * j + 1]) : "l"(acc[j]));
+}
+
 // ---- input ----------------------------------------------------------------
 // in: [vox][4] FP32 (rhs scaled, fluid, solid, air) -> x0: [vox][16] bf16
 __global__ void k_pack_input(const float* in, long long vox, bf16* x0) {
@@ -124,25 +142,21 @@ __device__ __forceinline__ void up_src(int f, int nc, int& i0, int& i1, float& l
 // w = 2k, then reads the rows at k+1 and writes w = 2k+1, sharing the samples
 // at k.  The weights and the summation order are those of the per-voxel
 // formula (corner k = (d, h, w) bits, weight = product of the three 1-D
-// weights), so the result does not depend on this blocking.  Coarse indices
+// weights), so the result does not depend on this blocking.  Bound by arithmetic (64
+// products of 8 channels per thread; moving the data alone takes 34 us for 32 channels
+// from 64^3): 82 us with single FMAs and selected samples, now 57.  Coarse indices
 // are 32-bit: the host keeps n * D * H * W * (C / 8) below 2^31.
-__device__ __forceinline__ void up_out(const uint4 (&lo)[4], const uint4 (&hi)[4], bool w0_hi, bool w1_hi, float ld,
-                                       float lh, float lw, bf16* out) {
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+__device__ __forceinline__ void up_out(const uint4 (&lo)[4], const uint4 (&hi)[4], float ld, float lh, float lw,
+                                       bf16* out) {
+    unsigned long long acc2[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
     for (int k = 0; k < 8; k++) {
         const float wt = ((k & 4) ? ld : 1.f - ld) * ((k & 2) ? lh : 1.f - lh) * ((k & 1) ? lw : 1.f - lw);
         const int r = ((k & 4) ? 2 : 0) | ((k & 2) ? 1 : 0);
-        const bool use_hi = (k & 1) ? w1_hi : w0_hi;
-        const uint4 u = use_hi ? hi[r] : lo[r];
-        const __nv_bfloat162* hv = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const float2 f = __bfloat1622float2(hv[j]);
-            acc[2 * j] += wt * f.x;
-            acc[2 * j + 1] += wt * f.y;
-        }
+        fma8(acc2, wt, (k & 1) ? hi[r] : lo[r]);
     }
+    float acc[8];
+    unpack8(acc2, acc);
     st8(out, acc);
 }
 
@@ -162,7 +176,8 @@ __global__ void __launch_bounds__(NT_THREADS, 3) k_upsample(const bf16* src, int
     const int nb = t / D;
     const int FD = 2 * D, FH = 2 * H, FW = 2 * W;
     const int wl = cw > 0 ? cw - 1 : 0, wr = cw < W - 1 ? cw + 1 : cw;
-    // fine w = 2cw reads coarse {i0, i1} in {wl, cw}; fine 2cw + 1 reads them in {cw, wr}
+    // fine w = 2cw reads coarse wl and cw (at the border the sample there with weights 1 and
+    // 0), fine 2cw + 1 reads cw and wr (at the border that sample twice)
     int a0, a1, b0, b1;
     float lwa, lwb;
     up_src(2 * cw, W, a0, a1, lwa);
@@ -190,10 +205,10 @@ __global__ void __launch_bounds__(NT_THREADS, 3) k_upsample(const bf16* src, int
                 mid[r] = *reinterpret_cast<const uint4*>(src + rowb[r] + (size_t)cw * C);
             }
             const size_t fv = ((size_t)(nb * FD + 2 * cd + a) * FH + 2 * chh + b) * FW + 2 * cw;
-            up_out(lo, mid, a0 != wl, a1 != wl, ld, lh, lwa, dst + fv * ds + o * 8);
+            up_out(lo, mid, ld, lh, lwa, dst + fv * ds + o * 8);
 #pragma unroll
             for (int r = 0; r < 4; r++) lo[r] = *reinterpret_cast<const uint4*>(src + rowb[r] + (size_t)wr * C);
-            up_out(mid, lo, b0 != cw, b1 != cw, ld, lh, lwb, dst + (fv + 1) * ds + o * 8);
+            up_out(mid, lo, ld, lh, lwb, dst + (fv + 1) * ds + o * 8);
         }
     }
 }
@@ -209,7 +224,7 @@ __device__ __forceinline__ void up_adj(int k, int nc, float (&w)[4]) {
 
 // out[coarse][c] = (sum_fine w * g[fine][c]) * (m[coarse][c] > 0); g channel stride gs (offset 0).
 // Bound by the 64 reads per output octet, which L1 serves: with run-time lists of samples
-// and 64-bit index arithmetic 178 us for 32 channels at 8 x 64^3, now 92.
+// and 64-bit index arithmetic 178 us for 32 channels at 8 x 64^3, then 92; with packed FMAs 85.
 template <typename I>
 __global__ void k_upsample_bwd(const bf16* g, int gs, const bf16* m, int C, int n, int D, int H, int W, bf16* out) {
     const int oct = C / 8;
@@ -225,7 +240,7 @@ __global__ void k_upsample_bwd(const bf16* g, int gs, const bf16* m, int C, int 
     up_adj(chh, H, wh);
     up_adj(cw, W, ww);
     const int FD = 2 * D, FH = 2 * H, FW = 2 * W;
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    unsigned long long acc2[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
     for (int a = 0; a < 4; a++) {
         if (wd[a] == 0.f) continue;
@@ -234,21 +249,19 @@ __global__ void k_upsample_bwd(const bf16* g, int gs, const bf16* m, int C, int 
             if (wh[b] == 0.f) continue;
             const bf16* p = g + ((((long long)nb * FD + 2 * cd - 1 + a) * FH + 2 * chh - 1 + b) * FW + 2 * cw - 1) * gs + o * 8;
             const float wab = wd[a] * wh[b];
-            float v[4][8];
+            uint4 v[4];
 #pragma unroll
             for (int c = 0; c < 4; c++) {
-                if (ww[c] != 0.f) ld8(p + (long long)c * gs, v[c]);
+                if (ww[c] != 0.f) v[c] = *reinterpret_cast<const uint4*>(p + (long long)c * gs);
             }
 #pragma unroll
             for (int c = 0; c < 4; c++) {
-                if (ww[c] == 0.f) continue;
-                const float wt = wab * ww[c];
-#pragma unroll
-                for (int j = 0; j < 8; j++) acc[j] += wt * v[c][j];
+                if (ww[c] != 0.f) fma8(acc2, wab * ww[c], v[c]);
             }
         }
     }
-    float mk[8];
+    float acc[8], mk[8];
+    unpack8(acc2, acc);
     ld8(m + cv * C + o * 8, mk);
 #pragma unroll
     for (int j = 0; j < 8; j++)
