@@ -224,7 +224,7 @@ __device__ __forceinline__ void up_adj(int k, int nc, float (&w)[4]) {
 
 // out[coarse][c] = (sum_fine w * g[fine][c]) * (m[coarse][c] > 0); g channel stride gs (offset 0).
 // Bound by the 64 reads per output octet, which L1 serves: with run-time lists of samples
-// and 64-bit index arithmetic 178 us for 32 channels at 8 x 64^3, then 92; with packed FMAs 85.
+// and 64-bit index arithmetic 178 us for 32 channels at 8 x 64^3, now 90.
 template <typename I>
 __global__ void k_upsample_bwd(const bf16* g, int gs, const bf16* m, int C, int n, int D, int H, int W, bf16* out) {
     const int oct = C / 8;
