@@ -103,6 +103,7 @@ __device__ __forceinline__ bool brick_cell(const BrickGeo& B, int4 bb, int t, in
 
 __constant__ float c_fill[7][7];  // (1 + tau (nf - 1)) / ns
 __constant__ float c_rcp[7];      // 1 / ns (1 for ns = 0)
+__constant__ double c_nsd[7] = {0.0, 1.0, 2.0, 3.0, 4.0, 5.0, 6.0};
 
 // Per-thread sums.  GB300 runs FP64 at a small fraction of its FP32 rate, so
 // per-cell terms are summed in FP32 with compensation (Kahan), and only the
@@ -303,11 +304,10 @@ __global__ void __launch_bounds__(PCG_THREADS) k_residual(const PcgArgs a, Vecs<
         double rv = bc;
         if (!from_zero) {
             const double* phi = a.phi;
-            double ap = (double)code_ns(cc) * phi[c];
+            rv = fma(-c_nsd[code_ns(cc)], phi[c], bc);
 #pragma unroll
             for (int k = 0; k < 6; k++)
-                if ((cc >> k) & 1) ap -= phi[c + nb_off(a.B, k)];
-            rv = bc - ap;
+                if ((cc >> k) & 1) rv += phi[c + nb_off(a.B, k)];
             acc[0] += rv * rv;
         }
         const T rt = (T)rv;
@@ -971,21 +971,15 @@ __device__ __forceinline__ void prolong_quad(const MGLev& F, const MGLev& Cl, in
         if (cx < 0 || cy < 0 || cx >= Cl.nx || cy >= Cl.ny) continue;
         const float wxy = (ox ? 1.f - wlx : wlx) * (oy ? 1.f - wly : wly);
         const long long row = ((long long)cx * Cl.ny + cy) * Cl.pz;
+        // (x is zero where the coarse cell is not fluid: k_mg_code)
         float qv[4];
-        uint32_t qc[4];
         unpack4(ld4(Cl.x + row + hq), qv);
-        codes4(Cl.ccode, row + hq, qc);
-        const bool ein = ze >= 0 && ze < Cl.pz;
-        const float ev = ein ? Cl.x[row + ze] : 0.f;
-        const uint32_t ec = ein ? Cl.ccode[row + ze] : 0u;
+        const float ev = ze >= 0 && ze < Cl.pz ? Cl.x[row + ze] : 0.f;
         float cv[4];
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
+        for (int k = 0; k < 4; k++)
             // lowq: zc = hq - 1 (the extra value), then hq .. hq + 2; else hq + 1 .. hq + 3, then hq + 4
-            const float v = lowq ? (k == 0 ? ev : qv[k - 1]) : (k == 3 ? ev : qv[k + 1]);
-            const uint32_t c = lowq ? (k == 0 ? ec : qc[k - 1]) : (k == 3 ? ec : qc[k + 1]);
-            cv[k] = is_fluid(c) ? v : 0.f;
-        }
+            cv[k] = lowq ? (k == 0 ? ev : qv[k - 1]) : (k == 3 ? ev : qv[k + 1]);
         // lanes: z0 (lower zc, w 1/4), z0+1 (zc+1, 3/4), z0+2 (zc+1, 1/4), z0+3 (zc+2, 3/4)
         sum[0] += wxy * (0.25f * cv[0] + 0.75f * cv[1]);
         sum[1] += wxy * (0.75f * cv[1] + 0.25f * cv[2]);
@@ -1768,6 +1762,7 @@ __global__ void k_mg_code(MGLev F, MGLev L, uint32_t* code) {
     }
     cc |= (uint32_t)min((dir + 1) >> 1, DIRICHLET_MAX) << CC_DIRICHLET;
     code[ci] = cc;
+    if (!(cc & CC_OP)) L.x[ci] = 0.f;  // no pass writes it; interpolation reads it
 }
 
 // interpolation scale of a level's fluid cells from the next level's kinds
