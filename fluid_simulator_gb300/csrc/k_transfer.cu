@@ -110,68 +110,97 @@ __device__ __forceinline__ void p2g_face_axis(const float (&f)[3], const float (
         kb = h * cm[b];
         kc = h * cm[c] * (c == 2 ? zr : 1.f);
     }
+    const float kn = wn[1] * ka;
+    const float Kj[3] = {K - 0.5f * kb, K + 0.5f * kb, K + 1.5f * kb}, Kk[3] = {-0.5f * kc, 0.5f * kc, 1.5f * kc};
 #pragma unroll
     for (int j = 0; j < 3; j++)
 #pragma unroll
         for (int kk = 0; kk < 3; kk++) {
             const float wbc = wt[b][j] * wt[c][kk];
-            const float cbc = K + kb * ((float)j - 0.5f) + kc * ((float)kk - 0.5f);
-#pragma unroll
-            for (int ii = 0; ii < 2; ii++) {
-                const float w = wn[ii] * wbc;
-                const int e = (ii * 3 + j) * 3 + kk;
-                acc[OW + e] += w;
-                acc[OV + e] += w * (APIC ? cbc + ka * (float)ii : K);
-            }
+            const int e = j * 3 + kk;
+            acc[OW + e] += wn[0] * wbc;
+            acc[OW + 9 + e] += wn[1] * wbc;
+            const float t = wbc * (APIC ? Kj[j] + Kk[kk] : K);
+            acc[OV + e] += wn[0] * t;
+            acc[OV + 9 + e] += wn[1] * t;
+            if (APIC) acc[OV + 9 + e] += kn * wbc;
         }
 }
 
-template <int AX, int OW, int OV, int NA, class S>
-__device__ __forceinline__ void p2g_flush_axis(const float (&acc)[NA], int cx, int cy, int cz, int x0, int y0,
-                                               int z0, float* s_vw, float* s_w) {
-    constexpr int b = AX == 0 ? 1 : 0, c = AX == 2 ? 1 : 2;
-    constexpr int PX = S::PX, PY = S::PY, TZ = S::PZ;
-    constexpr int NCELL = PX * PY * TZ;
+// bit e of the result: entry e of the NX x NY x NZ stencil (offsets -1, 0, ..) of the cell at
+// (lx, ly, lz) lies in the tile
+template <int NX, int NY, int NZ, class S>
+__device__ __forceinline__ unsigned p2g_inside(int lx, int ly, int lz) {
+    unsigned m = ~0u;
 #pragma unroll
-    for (int e = 0; e < 18; e++) {
-        if (acc[OW + e] == 0.f) continue;
-        int o[3];
-        o[AX] = e / 9 - 1;
-        o[b] = (e / 3) % 3 - 1;
-        o[c] = e % 3 - 1;
-        const int lx = cx + o[0] - x0, ly = cy + o[1] - y0, lz = cz + o[2] - z0;
-        if (lx < 0 || ly < 0 || lz < 0 || lx >= PX || ly >= PY || lz >= TZ) continue;
-        const int li = (lx * PY + ly) * TZ + lz;
-        atomicAdd(&s_vw[AX * NCELL + li], acc[OV + e]);
-        atomicAdd(&s_w[AX * NCELL + li], acc[OW + e]);
+    for (int i = 0; i < NX; i++) {
+        constexpr unsigned plane = (1u << (NY * NZ)) - 1u;
+        if ((unsigned)(lx + i - 1) >= (unsigned)S::PX) m &= ~(plane << (i * NY * NZ));
     }
+#pragma unroll
+    for (int j = 0; j < NY; j++) {
+        unsigned rows = 0;
+#pragma unroll
+        for (int i = 0; i < NX; i++) rows |= ((1u << NZ) - 1u) << ((i * NY + j) * NZ);
+        if ((unsigned)(ly + j - 1) >= (unsigned)S::PY) m &= ~rows;
+    }
+#pragma unroll
+    for (int k = 0; k < NZ; k++) {
+        unsigned col = 0;
+#pragma unroll
+        for (int i = 0; i < NX * NY; i++) col |= 1u << (i * NZ + k);
+        if ((unsigned)(lz + k - 1) >= (unsigned)S::PZ) m &= ~col;
+    }
+    return m;
 }
 
-template <bool APIC, class S>
-__global__ void __launch_bounds__(S::NTHREADS, S::MIN_BLOCKS) k_p2g(const P2GArgs a) {
-    constexpr int PX = S::PX, PY = S::PY, PZ = S::PZ, QX = S::QX, QY = S::QY, QZ = S::QZ;
-    constexpr int PCELLS = S::PCELLS, P2G_THREADS = S::NTHREADS;
-    extern __shared__ float sm[];
-    float* s_vw = sm;                // [3][PCELLS]
-    float* s_w = sm + 3 * PCELLS;   // [3][PCELLS]
+// adds the stencil of the face role AX (entry (ii * 3 + j) * 3 + k: normal offset ii - 1,
+// transverse offsets j - 1, k - 1) to the tile
+template <int AX, class S>
+__device__ __forceinline__ void p2g_flush_axis(const float (&acc)[36], int lx, int ly, int lz, float* s_vw, float* s_w) {
+    constexpr int NX = AX == 0 ? 2 : 3, NY = AX == 1 ? 2 : 3, NZ = AX == 2 ? 2 : 3;
+    const unsigned in = p2g_inside<NX, NY, NZ, S>(lx, ly, lz);
+    const int li = (lx * S::PY + ly) * S::PZ + lz;
+    float* vw = s_vw + AX * S::PCELLS + li;
+    float* w = s_w + AX * S::PCELLS + li;
+#pragma unroll
+    for (int x = 0; x < NX; x++)
+#pragma unroll
+        for (int y = 0; y < NY; y++)
+#pragma unroll
+            for (int z = 0; z < NZ; z++) {
+                const int e = AX == 0 ? (x * 3 + y) * 3 + z : AX == 1 ? (y * 3 + x) * 3 + z : (z * 3 + x) * 3 + y;
+                const int off = ((x - 1) * S::PY + y - 1) * S::PZ + z - 1;
+                if (!((in >> ((x * NY + y) * NZ + z)) & 1u) || acc[e] == 0.f) continue;
+                atomicAdd(vw + off, acc[18 + e]);
+                atomicAdd(w + off, acc[e]);
+            }
+}
+
+// The walk of one role's warps (ROLE 0-2: the faces of that axis, 3: cell centres), each
+// compiled on its own: the halo plane below the tile along a face's own axis is left out
+// (it reaches none of the tile's faces), array bases are constants, the products with the
+// normal weights are shared by weight and velocity sums, and whether an entry lies in the
+// tile is one bit.  21 % fewer instructions than one body for all roles, 256^3 APIC: 6.60
+// -> 6.06 ms in a step, 2.44 -> 2.13 with the particles in order (dam break).
+template <bool APIC, class S, int ROLE>
+__device__ __forceinline__ void p2g_walk(const P2GArgs& a, int x0, int y0, int z0, float* sm) {
+    constexpr int PX = S::PX, PY = S::PY, PZ = S::PZ, PCELLS = S::PCELLS;
+    float* s_vw = sm;
+    float* s_w = sm + 3 * PCELLS;
     float* s_avg = sm + 6 * PCELLS;
-    for (int k = threadIdx.x; k < 7 * PCELLS; k += blockDim.x) sm[k] = 0.f;
-    const int bt = blockIdx.x;
-    const int tz = bt % a.ntz, ty = (bt / a.ntz) % a.nty, tx = bt / (a.ntz * a.nty);
-    const int x0 = tx * PX, y0 = ty * PY, z0 = tz * PZ;
-    __syncthreads();
     const float h = a.g.h, zr = a.g.two_d ? (float)(a.g.hzd * a.g.hinvd) : 1.f;
     const float hinv3[3] = {a.g.hinv, a.g.hinv, a.g.hzinv};
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int role = warp & 3;
-    const int quads = P2G_THREADS / 128;
-    constexpr int HC = QX * QY * QZ;
+    const int quads = S::NTHREADS / 128;
+    constexpr int OX = ROLE == 0, OY = ROLE == 1, OZ = ROLE == 2;
+    constexpr int QX = S::QX - OX, QY = S::QY - OY, QZ = S::QZ - OZ, HC = QX * QY * QZ;
 
     for (int blk = warp >> 2; blk * 32 < HC; blk += quads) {
         const int hc = blk * 32 + lane;
         if (hc >= HC) continue;
         const int hz = hc % QZ, hy = (hc / QZ) % QY, hx = hc / (QZ * QY);
-        const int cx = x0 - 1 + hx, cy = y0 - 1 + hy, cz = z0 - 1 + hz;
+        const int cx = x0 - 1 + OX + hx, cy = y0 - 1 + OY + hy, cz = z0 - 1 + OZ + hz;
         if (cx < 0 || cy < 0 || cz < 0 || cx >= a.g.nx || cy >= a.g.ny || cz >= a.g.nz) continue;
         const long long cell = gidx(a.g, cx, cy, cz);
         const int beg = a.cstart[cell], end = a.cstart[cell + 1];
@@ -198,7 +227,7 @@ __global__ void __launch_bounds__(S::NTHREADS, S::MIN_BLOCKS) k_p2g(const P2GArg
             float wt[3][3];
 #pragma unroll
             for (int d = 0; d < 3; d++) tent3(f[d], wt[d]);
-            if (role == 3) {
+            if (ROLE == 3) {
 #pragma unroll
                 for (int ox = 0; ox < 3; ox++)
 #pragma unroll
@@ -211,30 +240,45 @@ __global__ void __launch_bounds__(S::NTHREADS, S::MIN_BLOCKS) k_p2g(const P2GArg
                 float cm[3] = {0.f, 0.f, 0.f};
                 if (APIC) {
 #pragma unroll
-                    for (int q = 0; q < 3; q++) cm[q] = a.p.c[3 * role + q][i];
+                    for (int q = 0; q < 3; q++) cm[q] = a.p.c[ROLE < 3 ? 3 * ROLE + q : 0][i];
                 }
-                const float va = a.p.v[role][i];
-                if (role == 0) p2g_face_axis<APIC, 0, 0, 18>(f, wt, va, cm, h, zr, acc);
-                else if (role == 1) p2g_face_axis<APIC, 1, 0, 18>(f, wt, va, cm, h, zr, acc);
+                const float va = a.p.v[ROLE < 3 ? ROLE : 0][i];
+                if (ROLE == 0) p2g_face_axis<APIC, 0, 0, 18>(f, wt, va, cm, h, zr, acc);
+                else if (ROLE == 1) p2g_face_axis<APIC, 1, 0, 18>(f, wt, va, cm, h, zr, acc);
                 else p2g_face_axis<APIC, 2, 0, 18>(f, wt, va, cm, h, zr, acc);
             }
         }
-        if (role == 3) {
+        const int lx = cx - x0, ly = cy - y0, lz = cz - z0;
+        if (ROLE == 3) {
+            const unsigned in = p2g_inside<3, 3, 3, S>(lx, ly, lz);
+            float* avg = s_avg + (lx * PY + ly) * PZ + lz;
 #pragma unroll
-            for (int e = 0; e < 27; e++) {
-                if (acc[e] == 0.f) continue;
-                const int lx = cx + e / 9 - 1 - x0, ly = cy + (e / 3) % 3 - 1 - y0, lz = cz + e % 3 - 1 - z0;
-                if (lx < 0 || ly < 0 || lz < 0 || lx >= PX || ly >= PY || lz >= PZ) continue;
-                atomicAdd(&s_avg[(lx * PY + ly) * PZ + lz], acc[e]);
-            }
-        } else if (role == 0) {
-            p2g_flush_axis<0, 0, 18, 36, S>(acc, cx, cy, cz, x0, y0, z0, s_vw, s_w);
-        } else if (role == 1) {
-            p2g_flush_axis<1, 0, 18, 36, S>(acc, cx, cy, cz, x0, y0, z0, s_vw, s_w);
+            for (int e = 0; e < 27; e++)
+                if (((in >> e) & 1u) && acc[e] != 0.f)
+                    atomicAdd(avg + ((e / 9 - 1) * PY + (e / 3) % 3 - 1) * PZ + e % 3 - 1, acc[e]);
         } else {
-            p2g_flush_axis<2, 0, 18, 36, S>(acc, cx, cy, cz, x0, y0, z0, s_vw, s_w);
+            p2g_flush_axis<ROLE < 3 ? ROLE : 0, S>(acc, lx, ly, lz, s_vw, s_w);
         }
     }
+}
+
+template <bool APIC, class S>
+__global__ void __launch_bounds__(S::NTHREADS, S::MIN_BLOCKS) k_p2g(const P2GArgs a) {
+    constexpr int PX = S::PX, PY = S::PY, PZ = S::PZ, PCELLS = S::PCELLS;
+    extern __shared__ float sm[];
+    float* s_vw = sm;                // [3][PCELLS]
+    float* s_w = sm + 3 * PCELLS;   // [3][PCELLS]
+    float* s_avg = sm + 6 * PCELLS;
+    for (int k = threadIdx.x; k < 7 * PCELLS; k += blockDim.x) sm[k] = 0.f;
+    const int bt = blockIdx.x;
+    const int tz = bt % a.ntz, ty = (bt / a.ntz) % a.nty, tx = bt / (a.ntz * a.nty);
+    const int x0 = tx * PX, y0 = ty * PY, z0 = tz * PZ;
+    __syncthreads();
+    const int role = (threadIdx.x >> 5) & 3;
+    if (role == 0) p2g_walk<APIC, S, 0>(a, x0, y0, z0, sm);
+    else if (role == 1) p2g_walk<APIC, S, 1>(a, x0, y0, z0, sm);
+    else if (role == 2) p2g_walk<APIC, S, 2>(a, x0, y0, z0, sm);
+    else p2g_walk<APIC, S, 3>(a, x0, y0, z0, sm);
     __syncthreads();
     for (int lc = threadIdx.x; lc < PCELLS; lc += blockDim.x) {
         const int lz = lc % PZ, ly = (lc / PZ) % PY, lx = lc / (PZ * PY);
