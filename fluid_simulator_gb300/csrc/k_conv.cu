@@ -187,6 +187,7 @@ struct MmaArgs {
 constexpr int POINT_MAX_STAGES = 8;
 template <int PLANES>
 __global__ void __launch_bounds__(CONV_THREADS) k_conv_mma(const MmaArgs a, const __grid_constant__ CUtensorMap tx) {
+    pdl_enter();
     using G = Halo<1, PLANES>;
     extern __shared__ __align__(128) unsigned char smraw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>(((uintptr_t)smraw + 127) & ~(uintptr_t)127);
@@ -405,6 +406,7 @@ __device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t (&r)[16
 template <int PLANES>
 __global__ void __launch_bounds__(PERS_THREADS, 1) k_conv_pers(const PersArgs p,
                                                                 const __grid_constant__ CUtensorMap tx) {
+    pdl_enter();
     using G = Halo<27, PLANES>;
     const MmaArgs& a = p.m;
     extern __shared__ __align__(128) unsigned char smraw[];
@@ -722,6 +724,7 @@ __device__ __forceinline__ void wgrad_drain(const WgArgs& a, uint32_t tmem, int 
 template <int TAPS, int NT>
 __global__ void __launch_bounds__(WG_THREADS, 1) k_conv_wgrad(const WgArgs a, const __grid_constant__ CUtensorMap tx,
                                                               const __grid_constant__ CUtensorMap tg) {
+    pdl_enter();
     using W = Wg<TAPS>;
     constexpr int G_PLANE = (NT >> 3) * W::G_OCT;
     constexpr int ZP = wgrad_zp<TAPS, NT>, NC = ZP * NT;
@@ -996,14 +999,14 @@ static int launch_pointwise(MmaArgs& a, unsigned grid, const ConvLaunch& L, cuda
     const int least = SMEM_LIMIT / (ctas + 1) + 1024;  // no more CTAs than that
     if (smem < least) smem = least;
     if (set_smem_limit((const void*)k_conv_mma<PLANES>, SMEM_LIMIT) != cudaSuccess) return FSIM_E_CUDA;
-    k_conv_mma<PLANES><<<grid, CONV_THREADS, smem, s>>>(a, *L.mx);
+    launch_net(k_conv_mma<PLANES>, grid, CONV_THREADS, smem, s, a, *L.mx);
     return cudaGetLastError() == cudaSuccess ? FSIM_OK : FSIM_E_CUDA;
 }
 
 template <int PLANES>
 static int launch_pers(const PersArgs& p, int ctas, int smem, const ConvLaunch& L, cudaStream_t s) {
     if (set_smem_limit((const void*)k_conv_pers<PLANES>, SMEM_LIMIT) != cudaSuccess) return FSIM_E_CUDA;
-    k_conv_pers<PLANES><<<ctas, PERS_THREADS, smem, s>>>(p, *L.mx);
+    launch_net(k_conv_pers<PLANES>, ctas, PERS_THREADS, smem, s, p, *L.mx);
     return cudaGetLastError() == cudaSuccess ? FSIM_OK : FSIM_E_CUDA;
 }
 
@@ -1092,7 +1095,7 @@ static int launch_wgrad(const WgradLaunch& L, cudaStream_t s) {
     if (smem > SMEM_LIMIT) return FSIM_E_INVALID;
     if (smem < SMEM_LIMIT / 2 + 1024) smem = SMEM_LIMIT / 2 + 1024;  // one CTA per SM (TMEM)
     if (set_smem_limit((const void*)k_conv_wgrad<TAPS, NT>, SMEM_LIMIT) != cudaSuccess) return FSIM_E_CUDA;
-    k_conv_wgrad<TAPS, NT><<<(unsigned)(groups * a.ksplit), WG_THREADS, smem, s>>>(a, *L.mx, *L.mg);
+    launch_net(k_conv_wgrad<TAPS, NT>, (unsigned)(groups * a.ksplit), WG_THREADS, smem, s, a, *L.mx, *L.mg);
     return cudaGetLastError() == cudaSuccess ? FSIM_OK : FSIM_E_CUDA;
 }
 

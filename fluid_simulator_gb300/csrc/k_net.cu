@@ -63,6 +63,7 @@ __device__ __forceinline__ void unpack8(const unsigned long long (&acc)[4], floa
 // ---- input ----------------------------------------------------------------
 // in: [vox][4] FP32 (rhs scaled, fluid, solid, air) -> x0: [vox][16] bf16
 __global__ void k_pack_input(const float* in, long long vox, bf16* x0) {
+    pdl_enter();
     const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= vox) return;
     const float4 q = *reinterpret_cast<const float4*>(in + v * 4);
@@ -85,6 +86,7 @@ __global__ void k_to_f32(const bf16* in, long long n, float* out) {
 // dst[coarse][(sd*4 + sh*2 + sw)*C + c] = src[2*coarse + (sd, sh, sw)][c]
 template <typename I>
 __global__ void k_s2d(const bf16* src, int ss, int so, int C, int n, int D, int H, int W, bf16* dst) {
+    pdl_enter();
     const int oct = C / 8;
     const I total = (I)n * (D / 2) * (H / 2) * (W / 2) * 8 * oct;
     const I i = (I)blockIdx.x * blockDim.x + threadIdx.x;
@@ -106,6 +108,7 @@ __global__ void k_s2d(const bf16* src, int ss, int so, int C, int n, int D, int 
 template <typename I>
 __global__ void k_d2s_add_mask(const bf16* gs, const bf16* gc, int gcs, int gco, const bf16* m, int ms, int mo,
                                int C, int n, int D, int H, int W, bf16* out) {
+    pdl_enter();
     const int oct = C / 8;
     const I total = (I)n * D * H * W * oct;
     const I i = (I)blockIdx.x * blockDim.x + threadIdx.x;
@@ -162,6 +165,7 @@ __device__ __forceinline__ void up_out(const uint4 (&lo)[4], const uint4 (&hi)[4
 
 __global__ void __launch_bounds__(NT_THREADS, 3) k_upsample(const bf16* src, int C, int n, int D, int H, int W,
                                                             bf16* dst, int ds) {
+    pdl_enter();
     const int oct = C >> 3;
     const int total = n * D * H * W * oct;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -227,6 +231,7 @@ __device__ __forceinline__ void up_adj(int k, int nc, float (&w)[4]) {
 // and 64-bit index arithmetic 178 us for 32 channels at 8 x 64^3, now 90.
 template <typename I>
 __global__ void k_upsample_bwd(const bf16* g, int gs, const bf16* m, int C, int n, int D, int H, int W, bf16* out) {
+    pdl_enter();
     const int oct = C / 8;
     const I total = (I)n * D * H * W * oct;
     const I i = (I)blockIdx.x * blockDim.x + threadIdx.x;
@@ -271,6 +276,7 @@ __global__ void k_upsample_bwd(const bf16* g, int gs, const bf16* m, int C, int 
 
 // ---- head (1x1x1, 16 -> 1) and loss ---------------------------------------
 __global__ void k_head(const bf16* d0, long long vox, const float* wgt, const float* bias, float scale, float* out) {
+    pdl_enter();
     const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= vox) return;
     float a[8], b[8];
@@ -321,6 +327,7 @@ __device__ __forceinline__ bool vox_solid(const bf16* x0, long long v) { return 
 template <bool GRAD, typename I>
 __global__ void k_loss(const float* out, const float* target, const uint8_t* mask, const bf16* x0, int n, int D,
                        int H, int W, float* r, float* gout, double* sums, const float* coef) {
+    pdl_enter();
     const long long per = (long long)D * H * W;
     const int smp = (int)((I)blockIdx.x * 512 / (I)per);
     FF q[4];
@@ -381,6 +388,7 @@ __global__ void k_loss(const float* out, const float* target, const uint8_t* mas
 // Loss and gradient factors from the per-sample sums (one warp).  A sample
 // whose residual, error, target or rhs is zero contributes nothing to that term.
 __global__ void k_loss_coef(const double* sums, int n, float lam, float* coef, double* loss, float* loss_out) {
+    pdl_enter();
     double l = 0.0;
     for (int s = threadIdx.x; s < n; s += 32) {
         const double rr = sums[4 * s], ee = sums[4 * s + 1], tt = sums[4 * s + 2], bb = sums[4 * s + 3];
@@ -420,6 +428,7 @@ __global__ void k_gather_batch(const uint8_t* types, const float* rhs, const flo
 // head backward: gz = dloss/d(pre-activation of d0), head weight / bias gradients
 __global__ void k_head_bwd(const bf16* d0, const float* gout, long long vox, const float* wgt, float scale, bf16* gz,
                            float* gw, float* gb) {
+    pdl_enter();
     const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     __shared__ float sw[17][NT_THREADS / 32];
     float contrib[17];
@@ -469,6 +478,7 @@ __global__ void k_head_bwd(const bf16* d0, const float* gout, long long vox, con
 // gb[c] += sum_v g[v][c]   (C in {16, 32, 64}); a thread sums eight neighbouring channels
 // (one 16-byte load a voxel: 25 us with 2-byte loads for 16 channels at 8 x 64^3, now 13)
 __global__ void k_bias_grad(const bf16* g, long long vox, int C, float* gb) {
+    pdl_enter();
     __shared__ float red[8][NT_THREADS + 1];
     const int oct = C >> 3, o = threadIdx.x % oct, lane = threadIdx.x / oct, lanes = NT_THREADS / oct;
     float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -779,7 +789,7 @@ int s2d(fsim_net* net, int src, int so, int C, int dst) {
     const NetShape& sh = net->shape;
     const long long total = level_vox(sh, lv + 1) * 8 * (C / 8);
     auto* k = total < (1ll << 31) ? k_s2d<uint32_t> : k_s2d<unsigned long long>;
-    k<<<nblk(total), NT_THREADS, 0, net->stream>>>(s.p, s.c, so, C, sh.n, sh.d >> lv, sh.h >> lv, sh.w >> lv,
+    launch_net(k, nblk(total), NT_THREADS, 0, net->stream, s.p, s.c, so, C, sh.n, sh.d >> lv, sh.h >> lv, sh.w >> lv,
                                                        net->act[dst].p);
     net->launches++;
     return FSIM_OK;
@@ -791,7 +801,7 @@ int upsample(fsim_net* net, int src, int dst) {
     const NetShape& sh = net->shape;
     const long long total = level_vox(sh, lv) * (s.c / 8);
     if (total >= (1ll << 31)) return fail(net, "up-sampling volume too large", FSIM_E_CAPACITY);
-    k_upsample<<<nblk(total), NT_THREADS, 0, net->stream>>>(s.p, s.c, sh.n, sh.d >> lv, sh.h >> lv, sh.w >> lv,
+    launch_net(k_upsample, nblk(total), NT_THREADS, 0, net->stream, s.p, s.c, sh.n, sh.d >> lv, sh.h >> lv, sh.w >> lv,
                                                             net->act[dst].p, net->act[dst].c);
     net->launches++;
     return FSIM_OK;
@@ -816,7 +826,7 @@ int net_forward(fsim_net* net) {
     upsample(net, D1, CAT0);
     if (!conv(15) || !conv(16)) return rc;
     const long long vox = level_vox(net->shape, 0);
-    k_head<<<nblk(vox), NT_THREADS, 0, net->stream>>>(net->act[D0].p, vox, net->theta + net->head_w,
+    launch_net(k_head, nblk(vox), NT_THREADS, 0, net->stream, net->act[D0].p, vox, net->theta + net->head_w,
                                                       net->theta + net->head_b, net->out_scale, net->out);
     net->launches++;
     NET_TRY(cudaGetLastError());
@@ -847,7 +857,7 @@ int conv_bwd(fsim_net* net, int l) {
     if (rc) return fail(net, "weight-gradient launch failed", rc);
     const long long vox = level_vox(sh, lv);
     const int bl = (int)std::min<long long>((vox * (L.cout / 8) + 2047) / 2048, 4 * 152);
-    k_bias_grad<<<bl, NT_THREADS, 0, net->stream>>>(gz.p, vox, L.cout, net->grad + L.b_off);
+    launch_net(k_bias_grad, bl, NT_THREADS, 0, net->stream, gz.p, vox, L.cout, net->grad + L.b_off);
     net->launches += 2;
     if (kGin[l] < 0) return FSIM_OK;
     // input gradient
@@ -886,7 +896,7 @@ int up_bwd(fsim_net* net, int gcat, int mask, int out) {
     const NetShape& sh = net->shape;
     const long long total = level_vox(sh, lv) * (m.c / 8);
     auto* k = total < (1ll << 31) ? k_upsample_bwd<uint32_t> : k_upsample_bwd<unsigned long long>;
-    k<<<nblk(total), NT_THREADS, 0, net->stream>>>(net->gbuf[gcat].p, net->gbuf[gcat].c, m.p, m.c, sh.n, sh.d >> lv,
+    launch_net(k, nblk(total), NT_THREADS, 0, net->stream, net->gbuf[gcat].p, net->gbuf[gcat].c, m.p, m.c, sh.n, sh.d >> lv,
                                                    sh.h >> lv, sh.w >> lv, net->gbuf[out].p);
     net->launches++;
     return FSIM_OK;
@@ -898,7 +908,7 @@ int d2s(fsim_net* net, int gs2d, int gcat, int cat, int off, int C, int out) {
     const NetShape& sh = net->shape;
     const long long total = level_vox(sh, lv) * (C / 8);
     auto* k = total < (1ll << 31) ? k_d2s_add_mask<uint32_t> : k_d2s_add_mask<unsigned long long>;
-    k<<<nblk(total), NT_THREADS, 0, net->stream>>>(net->gbuf[gs2d].p, gc.p, gc.c, off, net->act[cat].p, net->act[cat].c, off,
+    launch_net(k, nblk(total), NT_THREADS, 0, net->stream, net->gbuf[gs2d].p, gc.p, gc.c, off, net->act[cat].p, net->act[cat].c, off,
                                                    C, sh.n, sh.d >> lv, sh.h >> lv, sh.w >> lv, net->gbuf[out].p);
     net->launches++;
     return FSIM_OK;
@@ -912,13 +922,13 @@ int net_backward(fsim_net* net, const float* target, const uint8_t* mask, float*
     auto* pass1 = vox < (1ll << 31) ? k_loss<false, uint32_t> : k_loss<false, unsigned long long>;
     auto* pass2 = vox < (1ll << 31) ? k_loss<true, uint32_t> : k_loss<true, unsigned long long>;
     const unsigned nb = (unsigned)(vox / 512);
-    pass1<<<nb, NT_THREADS, 0, net->stream>>>(net->out, target, mask, net->act[X0].p, sh.n, sh.d, sh.h, sh.w, net->res,
+    launch_net(pass1, nb, NT_THREADS, 0, net->stream, net->out, target, mask, net->act[X0].p, sh.n, sh.d, sh.h, sh.w, net->res,
                                               nullptr, net->d_sums, nullptr);
-    k_loss_coef<<<1, 32, 0, net->stream>>>(net->d_sums, sh.n, net->loss_l2_weight, net->d_coef, net->d_loss,
+    launch_net(k_loss_coef, 1, 32, 0, net->stream, net->d_sums, sh.n, net->loss_l2_weight, net->d_coef, net->d_loss,
                                            loss_out);
-    pass2<<<nb, NT_THREADS, 0, net->stream>>>(net->out, target, mask, net->act[X0].p, sh.n, sh.d, sh.h, sh.w, net->res,
+    launch_net(pass2, nb, NT_THREADS, 0, net->stream, net->out, target, mask, net->act[X0].p, sh.n, sh.d, sh.h, sh.w, net->res,
                                               net->gout, nullptr, net->d_coef);
-    k_head_bwd<<<nblk(vox), NT_THREADS, 0, net->stream>>>(net->act[D0].p, net->gout, vox, net->theta + net->head_w,
+    launch_net(k_head_bwd, nblk(vox), NT_THREADS, 0, net->stream, net->act[D0].p, net->gout, vox, net->theta + net->head_w,
                                                           net->out_scale, net->gbuf[GD0].p, net->grad + net->head_w,
                                                           net->grad + net->head_b);
     net->launches += 4;
@@ -1135,7 +1145,7 @@ int fsim_net_forward(fsim_net* net, int n, int d, int h, int w, const float* in,
     const long long vox = (long long)n * d * h * w;
     Staged sin;
     if ((rc = stage_in(net, in, (size_t)vox * 16, where, sin))) return rc;
-    k_pack_input<<<nblk(vox), NT_THREADS, 0, net->stream>>>((const float*)sin.p, vox, net->act[X0].p);
+    launch_net(k_pack_input, nblk(vox), NT_THREADS, 0, net->stream, (const float*)sin.p, vox, net->act[X0].p);
     net->launches++;
     rc = net_forward(net);
     unstage(net, sin);

@@ -626,10 +626,12 @@ long long p2g_tiles(const GridGeom& g) {
 // 4x4x8 / 4x8x8 / 8x8x16 / 8x16x16: 32^3 dam 64 / 69 / 83 / 140 / 210, 48^3 dam
 // 90 / 83 / 98 / 168 / 249, 64^3 dam 145 / 120 / 109 / 169 / 260, 90x61x75 half
 // filled 294 / 244 / 220 / 198 / 288, 96^3 dam 408 / 317 / 263 / 245 / 362, 128^3
-// dam 941 / 707 / 571 / 467 / 445.
+// dam 941 / 707 / 571 / 467 / 445 (before the walks were one per role).  Seven quads per
+// 4x8x8 tile instead of three: 64x64x40 dam 80 -> 73, half filled 112 -> 106; at 4x4x8 and
+// 4x4x4 it gains on one scene what it loses on the other.
 constexpr long long P2G_MIN_TILES = 480;
 using T1 = P2GShape<8, 8, 16, 384, 2>;
-using T2 = P2GShape<4, 8, 8, 384, 2>;
+using T2 = P2GShape<4, 8, 8, 896, 1>;  // seven quads: 19 cell blocks in three rounds
 using T3 = P2GShape<4, 4, 8, 384, 2>;
 using T4 = P2GShape<4, 4, 4, 384, 2>;
 cudaError_t p2g_fast(const P2GArgs& a, bool apic, cudaStream_t stream) {
