@@ -166,6 +166,31 @@ __device__ __forceinline__ bool last_block_reduce(double (&v)[K], unsigned is_ma
     return true;
 }
 
+// ---- programmatic dependent launch -------------------------------------------
+// Chains of short kernels are launched with programmatic stream serialisation, so each
+// grid is scheduled while its predecessor drains.  Every such kernel lets its successor
+// launch at once and then waits for its predecessor's completion (and memory) before it
+// touches any data: the order of the stream is unchanged.  Saves 1-2 us a launch.
+__device__ __forceinline__ void pdl_enter() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_dep(void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                       Args&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+
 // ---- SplitMix64 (Steele, Lea, Flood 2014) as a counter-based generator -----
 __host__ __device__ inline uint64_t splitmix64(uint64_t ctr) {
     uint64_t z = ctr * 0x9E3779B97F4A7C15ull;

@@ -7,33 +7,9 @@
 #include <cuda_runtime.h>
 
 #include <string>
-#include <utility>
 #include <vector>
 
 #include "fsim_common.cuh"
-
-// Programmatic dependent launch: the kernels of a pass are launched with programmatic
-// stream serialisation, so a grid is scheduled while its predecessor drains (a pass is 25
-// to 85 launches).  Each lets its successor launch at once and then waits for its
-// predecessor's completion before it touches any data: the order of the stream stands.
-__device__ __forceinline__ void pdl_enter() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-template <typename... KArgs, typename... Args>
-void launch_net(void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, Args&&... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
-}
 
 // One launch of the tensor-core convolution (forward, or input gradient when
 // flip is set and the weights are the per-tap transposed copy).

@@ -999,14 +999,14 @@ static int launch_pointwise(MmaArgs& a, unsigned grid, const ConvLaunch& L, cuda
     const int least = SMEM_LIMIT / (ctas + 1) + 1024;  // no more CTAs than that
     if (smem < least) smem = least;
     if (set_smem_limit((const void*)k_conv_mma<PLANES>, SMEM_LIMIT) != cudaSuccess) return FSIM_E_CUDA;
-    launch_net(k_conv_mma<PLANES>, grid, CONV_THREADS, smem, s, a, *L.mx);
+    launch_dep(k_conv_mma<PLANES>, grid, CONV_THREADS, smem, s, a, *L.mx);
     return cudaGetLastError() == cudaSuccess ? FSIM_OK : FSIM_E_CUDA;
 }
 
 template <int PLANES>
 static int launch_pers(const PersArgs& p, int ctas, int smem, const ConvLaunch& L, cudaStream_t s) {
     if (set_smem_limit((const void*)k_conv_pers<PLANES>, SMEM_LIMIT) != cudaSuccess) return FSIM_E_CUDA;
-    launch_net(k_conv_pers<PLANES>, ctas, PERS_THREADS, smem, s, p, *L.mx);
+    launch_dep(k_conv_pers<PLANES>, ctas, PERS_THREADS, smem, s, p, *L.mx);
     return cudaGetLastError() == cudaSuccess ? FSIM_OK : FSIM_E_CUDA;
 }
 
@@ -1095,7 +1095,7 @@ static int launch_wgrad(const WgradLaunch& L, cudaStream_t s) {
     if (smem > SMEM_LIMIT) return FSIM_E_INVALID;
     if (smem < SMEM_LIMIT / 2 + 1024) smem = SMEM_LIMIT / 2 + 1024;  // one CTA per SM (TMEM)
     if (set_smem_limit((const void*)k_conv_wgrad<TAPS, NT>, SMEM_LIMIT) != cudaSuccess) return FSIM_E_CUDA;
-    launch_net(k_conv_wgrad<TAPS, NT>, (unsigned)(groups * a.ksplit), WG_THREADS, smem, s, a, *L.mx, *L.mg);
+    launch_dep(k_conv_wgrad<TAPS, NT>, (unsigned)(groups * a.ksplit), WG_THREADS, smem, s, a, *L.mx, *L.mg);
     return cudaGetLastError() == cudaSuccess ? FSIM_OK : FSIM_E_CUDA;
 }
 

@@ -789,7 +789,7 @@ int s2d(fsim_net* net, int src, int so, int C, int dst) {
     const NetShape& sh = net->shape;
     const long long total = level_vox(sh, lv + 1) * 8 * (C / 8);
     auto* k = total < (1ll << 31) ? k_s2d<uint32_t> : k_s2d<unsigned long long>;
-    launch_net(k, nblk(total), NT_THREADS, 0, net->stream, s.p, s.c, so, C, sh.n, sh.d >> lv, sh.h >> lv, sh.w >> lv,
+    launch_dep(k, nblk(total), NT_THREADS, 0, net->stream, s.p, s.c, so, C, sh.n, sh.d >> lv, sh.h >> lv, sh.w >> lv,
                                                        net->act[dst].p);
     net->launches++;
     return FSIM_OK;
@@ -801,7 +801,7 @@ int upsample(fsim_net* net, int src, int dst) {
     const NetShape& sh = net->shape;
     const long long total = level_vox(sh, lv) * (s.c / 8);
     if (total >= (1ll << 31)) return fail(net, "up-sampling volume too large", FSIM_E_CAPACITY);
-    launch_net(k_upsample, nblk(total), NT_THREADS, 0, net->stream, s.p, s.c, sh.n, sh.d >> lv, sh.h >> lv, sh.w >> lv,
+    launch_dep(k_upsample, nblk(total), NT_THREADS, 0, net->stream, s.p, s.c, sh.n, sh.d >> lv, sh.h >> lv, sh.w >> lv,
                                                             net->act[dst].p, net->act[dst].c);
     net->launches++;
     return FSIM_OK;
@@ -826,7 +826,7 @@ int net_forward(fsim_net* net) {
     upsample(net, D1, CAT0);
     if (!conv(15) || !conv(16)) return rc;
     const long long vox = level_vox(net->shape, 0);
-    launch_net(k_head, nblk(vox), NT_THREADS, 0, net->stream, net->act[D0].p, vox, net->theta + net->head_w,
+    launch_dep(k_head, nblk(vox), NT_THREADS, 0, net->stream, net->act[D0].p, vox, net->theta + net->head_w,
                                                       net->theta + net->head_b, net->out_scale, net->out);
     net->launches++;
     NET_TRY(cudaGetLastError());
@@ -857,7 +857,7 @@ int conv_bwd(fsim_net* net, int l) {
     if (rc) return fail(net, "weight-gradient launch failed", rc);
     const long long vox = level_vox(sh, lv);
     const int bl = (int)std::min<long long>((vox * (L.cout / 8) + 2047) / 2048, 4 * 152);
-    launch_net(k_bias_grad, bl, NT_THREADS, 0, net->stream, gz.p, vox, L.cout, net->grad + L.b_off);
+    launch_dep(k_bias_grad, bl, NT_THREADS, 0, net->stream, gz.p, vox, L.cout, net->grad + L.b_off);
     net->launches += 2;
     if (kGin[l] < 0) return FSIM_OK;
     // input gradient
@@ -896,7 +896,7 @@ int up_bwd(fsim_net* net, int gcat, int mask, int out) {
     const NetShape& sh = net->shape;
     const long long total = level_vox(sh, lv) * (m.c / 8);
     auto* k = total < (1ll << 31) ? k_upsample_bwd<uint32_t> : k_upsample_bwd<unsigned long long>;
-    launch_net(k, nblk(total), NT_THREADS, 0, net->stream, net->gbuf[gcat].p, net->gbuf[gcat].c, m.p, m.c, sh.n, sh.d >> lv,
+    launch_dep(k, nblk(total), NT_THREADS, 0, net->stream, net->gbuf[gcat].p, net->gbuf[gcat].c, m.p, m.c, sh.n, sh.d >> lv,
                                                    sh.h >> lv, sh.w >> lv, net->gbuf[out].p);
     net->launches++;
     return FSIM_OK;
@@ -908,7 +908,7 @@ int d2s(fsim_net* net, int gs2d, int gcat, int cat, int off, int C, int out) {
     const NetShape& sh = net->shape;
     const long long total = level_vox(sh, lv) * (C / 8);
     auto* k = total < (1ll << 31) ? k_d2s_add_mask<uint32_t> : k_d2s_add_mask<unsigned long long>;
-    launch_net(k, nblk(total), NT_THREADS, 0, net->stream, net->gbuf[gs2d].p, gc.p, gc.c, off, net->act[cat].p, net->act[cat].c, off,
+    launch_dep(k, nblk(total), NT_THREADS, 0, net->stream, net->gbuf[gs2d].p, gc.p, gc.c, off, net->act[cat].p, net->act[cat].c, off,
                                                    C, sh.n, sh.d >> lv, sh.h >> lv, sh.w >> lv, net->gbuf[out].p);
     net->launches++;
     return FSIM_OK;
@@ -922,13 +922,13 @@ int net_backward(fsim_net* net, const float* target, const uint8_t* mask, float*
     auto* pass1 = vox < (1ll << 31) ? k_loss<false, uint32_t> : k_loss<false, unsigned long long>;
     auto* pass2 = vox < (1ll << 31) ? k_loss<true, uint32_t> : k_loss<true, unsigned long long>;
     const unsigned nb = (unsigned)(vox / 512);
-    launch_net(pass1, nb, NT_THREADS, 0, net->stream, net->out, target, mask, net->act[X0].p, sh.n, sh.d, sh.h, sh.w, net->res,
+    launch_dep(pass1, nb, NT_THREADS, 0, net->stream, net->out, target, mask, net->act[X0].p, sh.n, sh.d, sh.h, sh.w, net->res,
                                               nullptr, net->d_sums, nullptr);
-    launch_net(k_loss_coef, 1, 32, 0, net->stream, net->d_sums, sh.n, net->loss_l2_weight, net->d_coef, net->d_loss,
+    launch_dep(k_loss_coef, 1, 32, 0, net->stream, net->d_sums, sh.n, net->loss_l2_weight, net->d_coef, net->d_loss,
                                            loss_out);
-    launch_net(pass2, nb, NT_THREADS, 0, net->stream, net->out, target, mask, net->act[X0].p, sh.n, sh.d, sh.h, sh.w, net->res,
+    launch_dep(pass2, nb, NT_THREADS, 0, net->stream, net->out, target, mask, net->act[X0].p, sh.n, sh.d, sh.h, sh.w, net->res,
                                               net->gout, nullptr, net->d_coef);
-    launch_net(k_head_bwd, nblk(vox), NT_THREADS, 0, net->stream, net->act[D0].p, net->gout, vox, net->theta + net->head_w,
+    launch_dep(k_head_bwd, nblk(vox), NT_THREADS, 0, net->stream, net->act[D0].p, net->gout, vox, net->theta + net->head_w,
                                                           net->out_scale, net->gbuf[GD0].p, net->grad + net->head_w,
                                                           net->grad + net->head_b);
     net->launches += 4;
@@ -1145,7 +1145,7 @@ int fsim_net_forward(fsim_net* net, int n, int d, int h, int w, const float* in,
     const long long vox = (long long)n * d * h * w;
     Staged sin;
     if ((rc = stage_in(net, in, (size_t)vox * 16, where, sin))) return rc;
-    launch_net(k_pack_input, nblk(vox), NT_THREADS, 0, net->stream, (const float*)sin.p, vox, net->act[X0].p);
+    launch_dep(k_pack_input, nblk(vox), NT_THREADS, 0, net->stream, (const float*)sin.p, vox, net->act[X0].p);
     net->launches++;
     rc = net_forward(net);
     unstage(net, sin);

@@ -244,6 +244,7 @@ __device__ __forceinline__ bool in_obstacle(const AdvectArgs& a, float px, float
 // general path inline (40 registers), now 805 (44 bytes a
 // particle: 430 us).
 __global__ void __launch_bounds__(256, 8) k_advect(const __grid_constant__ AdvectArgs a) {
+    pdl_enter();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = i < a.n;
     uint32_t key = FSIM_DEAD_KEY;
@@ -337,6 +338,7 @@ __device__ __forceinline__ int block_excl_scan(int v, int* total) {
 }
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_tile_sums(const int* in, long long n, int* sums) {
+    pdl_enter();
     const long long base = (long long)blockIdx.x * SCAN_TILE;
     int s = 0;
 #pragma unroll
@@ -357,6 +359,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_tile_sums(const int* in, long 
 
 // single block: exclusive scan of the tile sums in place (any count)
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(int* sums, int nt) {
+    pdl_enter();
     int carry = 0;
     for (int base = 0; base < nt; base += SCAN_THREADS) {
         int j = base + threadIdx.x;
@@ -371,6 +374,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(int* sums, int nt) {
 // out[j] = exclusive prefix of in, out[n] = total
 __global__ void __launch_bounds__(SCAN_THREADS) k_tile_scan(const int* in, long long n, const int* sums,
                                                             int* out) {
+    pdl_enter();
     const long long base = (long long)blockIdx.x * SCAN_TILE + (long long)threadIdx.x * SCAN_ITEMS;
     int v[SCAN_ITEMS];
     int local = 0;
@@ -440,6 +444,7 @@ __global__ void k_push_apart(ParticleBuf p, const uint32_t* perm, const int* cst
 
 __global__ void k_scatter(const uint32_t* key, const uint32_t* rank, const int* cstart, uint32_t* perm,
                           long long n) {
+    pdl_enter();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t k = key[i];
@@ -462,6 +467,7 @@ __device__ __forceinline__ void cswap(uint32_t& a, uint32_t& b, bool up) {
 }
 
 __global__ void k_cell_order(uint32_t* perm, const int* cstart, long long ncell) {
+    pdl_enter();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= ncell) return;
     const int beg = cstart[c], end = cstart[c + 1];
@@ -642,14 +648,14 @@ __global__ void __launch_bounds__(GFX_THREADS) k_gfx(ParticleBuf p, long long n,
 
 void launch_advect(const AdvectArgs& a, cudaStream_t s) {
     if (a.n <= 0) return;
-    k_advect<<<ceil_div(a.n, 256), 256, 0, s>>>(a);
+    launch_dep(k_advect, ceil_div(a.n, 256), 256, 0, s, a);
 }
 
 void launch_scan(const int* in, int* out, long long n, int* block_sums, cudaStream_t s) {
     const int nt = ceil_div(n, SCAN_TILE);
-    k_tile_sums<<<nt, SCAN_THREADS, 0, s>>>(in, n, block_sums);
-    k_scan_sums<<<1, SCAN_THREADS, 0, s>>>(block_sums, nt);
-    k_tile_scan<<<nt, SCAN_THREADS, 0, s>>>(in, n, block_sums, out);
+    launch_dep(k_tile_sums, nt, SCAN_THREADS, 0, s, in, n, block_sums);
+    launch_dep(k_scan_sums, 1, SCAN_THREADS, 0, s, block_sums, nt);
+    launch_dep(k_tile_scan, nt, SCAN_THREADS, 0, s, in, n, block_sums, out);
 }
 
 void launch_push_apart(ParticleBuf p, const uint32_t* perm, const int* cstart, const GridGeom& g, long long n,
@@ -662,8 +668,8 @@ void launch_push_apart(ParticleBuf p, const uint32_t* perm, const int* cstart, c
 void launch_scatter(const uint32_t* key, const uint32_t* rank, const int* cstart, uint32_t* perm,
                     long long n, long long ncell, cudaStream_t s) {
     if (n <= 0) return;
-    k_scatter<<<ceil_div(n, 256), 256, 0, s>>>(key, rank, cstart, perm, n);
-    k_cell_order<<<ceil_div(ncell, 256), 256, 0, s>>>(perm, cstart, ncell);
+    launch_dep(k_scatter, ceil_div(n, 256), 256, 0, s, key, rank, cstart, perm, n);
+    launch_dep(k_cell_order, ceil_div(ncell, 256), 256, 0, s, perm, cstart, ncell);
 }
 
 void launch_gather(ParticleBuf src, ParticleBuf dst, const uint32_t* perm, const int* cstart,

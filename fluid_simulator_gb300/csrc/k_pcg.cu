@@ -43,29 +43,9 @@
 
 namespace {
 
-// Programmatic dependent launch: the kernels of one PCG iteration are launched
-// with programmatic stream serialisation, so each grid is scheduled while its
-// predecessor drains.  Every such kernel lets its successor launch at once and
-// then waits for its predecessor's completion (and memory) before touching any
-// data, so the ordering of the stream is unchanged.
-__device__ __forceinline__ void pdl_enter() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 template <typename... KArgs, typename... Args>
 void launch_pdl(void (*kern)(KArgs...), unsigned grid, unsigned block, cudaStream_t st, Args&&... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+    launch_dep(kern, grid, block, 0, st, std::forward<Args>(args)...);
 }
 
 constexpr int BRX = 2, BRY = 4, BRZ = 32;

@@ -165,6 +165,7 @@ __device__ __forceinline__ bool make_sprite(const Cam& cam, const float* pw, flo
 // for all sprites, which read it instead of unprojecting the pixel for every fragment
 // (28 operations and five divisions of ~200).
 __global__ void k_rays(Cam cam, int W, int H, float4* ray) {
+    pdl_enter();
     const int id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= W * H) return;
     const int i = id % W, j = id / W;
@@ -266,6 +267,7 @@ constexpr int SPLAT_GATHER = 2048;
 __global__ void __launch_bounds__(256, 8) k_splat_depth(const fsim_particle_gfx* parts, long long n, int which, float thr,
                                                      Cam cam, float r, int W, int H, const float4* ray, int plain_proj,
                                                      unsigned* depth_bits, const float* scene, float* thick) {
+    pdl_enter();
     if (which != 2) {
         const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
         if (k >= n) return;
@@ -286,14 +288,12 @@ __global__ void __launch_bounds__(256, 8) k_splat_depth(const fsim_particle_gfx*
         splat(parts[k0 + list[i]].pos, cam, r, W, H, ray, plain_proj, depth_bits, scene, thick);
 }
 
-__global__ void k_fill(float* p, long long n, float v) {
+__global__ void k_clear(float* depth, float* thick, long long n) {
+    pdl_enter();
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) p[k] = v;
-}
-
-__global__ void k_fill4(float4* p, long long n, float4 v) {
-    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) p[k] = v;
+    if (k >= n) return;
+    depth[k] = 1.f;
+    thick[k] = 0.f;
 }
 
 // ---- 2, 4: separable blurs -----------------------------------------------------
@@ -368,6 +368,7 @@ __device__ __forceinline__ void blur_pixel(int mode, int axis, const float* src,
 // exponentials and clamped indices for every tap 29 us a pass at 1000 x 1000, now 20.
 __global__ void k_blur(int mode, int axis, const float* src, const float* dsrc, float* dst, int W, int H, Cam cam,
                        float size, float blur_scale, float falloff) {
+    pdl_enter();
     __shared__ float wtab[(BLUR_MAX_R + 1) * (BLUR_MAX_R + 1)];
     if (mode == 1) {
         for (int p = threadIdx.x; p <= BLUR_BI_R; p += blockDim.x) {
@@ -398,6 +399,7 @@ __device__ __forceinline__ void eye_at(const Cam& cam, const float* depth, int W
 }
 
 __global__ void k_normals(const float* depth, float4* nd, int W, int H, Cam cam) {
+    pdl_enter();
     const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= (long long)W * H) return;
     const int x = (int)(id % W), y = (int)(id / W);
@@ -539,6 +541,7 @@ __device__ void shade_light(const float* wp, const float* nrm_in, const float* v
 // per pixel instead of 5 (91 us at 1000 x 1000, now 36).
 constexpr int SHADE_X = 32, SHADE_Y = 8;
 __global__ void __launch_bounds__(SHADE_X * SHADE_Y) k_shade(const ShadeArgs a) {
+    pdl_enter();
     constexpr int PX = SHADE_X + 2, PY = SHADE_Y + 2;
     __shared__ float pos[3][PY * PX];
     const int tiles_x = (a.W + SHADE_X - 1) / SHADE_X;
@@ -838,45 +841,44 @@ int fsim_render_frame(fsim_renderer* r, const fsim_particle_gfx* particles, int6
     // 1. surface sprites into the cleared depth buffer, with their thickness
     //    (the thickness of all particles accumulates over passes 1 and 3)
     float* thick = prm->transparency_enabled ? r->thick : nullptr;
-    k_fill<<<nblk(np), 256, 0, s>>>(r->raw, np, 1.f);
-    k_fill<<<nblk(np), 256, 0, s>>>(r->thick, np, 0.f);
-    L += 2;
     // the pixels' eye rays stand in the normal buffer until pass 5 writes it
     const float* pm = k.proj.m;
     const int plain = pm[2] == 0.f && pm[6] == 0.f && pm[3] == 0.f && pm[7] == 0.f && pm[15] == 0.f && pm[11] < 0.f &&
                       pm[14] < 0.f;
+    launch_dep(k_clear, nblk(np), 256, 0, s, r->raw, r->thick, np);
+    L++;
     if (n > 0) {
-        k_rays<<<nblk(np), 256, 0, s>>>(k, W, H, r->nd);
+        launch_dep(k_rays, nblk(np), 256, 0, s, k, W, H, r->nd);
         L++;
     }
     if (n > 0) {
-        k_splat_depth<<<nblk(n), 256, 0, s>>>(dp, n, prm->spray_enabled ? 1 : 0, prm->spray_density_threshold, k,
+        launch_dep(k_splat_depth, nblk(n), 256, 0, s, dp, n, prm->spray_enabled ? 1 : 0, prm->spray_density_threshold, k,
                                               rad, W, H, r->nd, plain, reinterpret_cast<unsigned*>(r->raw), scene_depth, thick);
         L++;
     }
     // 2. smoothing, x into tmp then y into depth
     const int mode = prm->bilateral_filter ? 1 : 0;
-    k_blur<<<nblk(np), 256, 0, s>>>(mode, 0, r->raw, r->raw, r->tmp, W, H, k, prm->smoothing_size, prm->blur_scale,
+    launch_dep(k_blur, nblk(np), 256, 0, s, mode, 0, r->raw, r->raw, r->tmp, W, H, k, prm->smoothing_size, prm->blur_scale,
                                    prm->blur_depth_falloff);
-    k_blur<<<nblk(np), 256, 0, s>>>(mode, 1, r->tmp, r->tmp, r->depth, W, H, k, prm->smoothing_size,
+    launch_dep(k_blur, nblk(np), 256, 0, s, mode, 1, r->tmp, r->tmp, r->depth, W, H, k, prm->smoothing_size,
                                    prm->blur_scale, prm->blur_depth_falloff);
     L += 2;
     // 3. spray on top of the smoothed surface
     if (prm->spray_enabled && n > 0) {
-        k_splat_depth<<<(unsigned)((n + SPLAT_GATHER - 1) / SPLAT_GATHER), 256, 0, s>>>(dp, n, 2, prm->spray_density_threshold, k, rad, W, H, r->nd, plain,
+        launch_dep(k_splat_depth, (unsigned)((n + SPLAT_GATHER - 1) / SPLAT_GATHER), 256, 0, s, dp, n, 2, prm->spray_density_threshold, k, rad, W, H, r->nd, plain,
                                               reinterpret_cast<unsigned*>(r->depth), scene_depth, thick);
         L++;
     }
     // 4. thickness blurred x then y
     if (prm->transparency_enabled) {
-        k_blur<<<nblk(np), 256, 0, s>>>(2, 0, r->thick, r->depth, r->ttmp, W, H, k, prm->transparency_blur_size,
+        launch_dep(k_blur, nblk(np), 256, 0, s, 2, 0, r->thick, r->depth, r->ttmp, W, H, k, prm->transparency_blur_size,
                                        0.f, 0.f);
-        k_blur<<<nblk(np), 256, 0, s>>>(2, 1, r->ttmp, r->depth, r->thick, W, H, k, prm->transparency_blur_size,
+        launch_dep(k_blur, nblk(np), 256, 0, s, 2, 1, r->ttmp, r->depth, r->thick, W, H, k, prm->transparency_blur_size,
                                        0.f, 0.f);
         L += 2;
     }
     // 5. normals
-    k_normals<<<nblk(np), 256, 0, s>>>(r->depth, r->nd, W, H, k);
+    launch_dep(k_normals, nblk(np), 256, 0, s, r->depth, r->nd, W, H, k);
     L++;
     // 6. shading and composite
     ShadeArgs a;
@@ -902,7 +904,7 @@ int fsim_render_frame(fsim_renderer* r, const fsim_particle_gfx* particles, int6
     a.nl = prm->num_lights;
     std::memcpy(a.lights, prm->lights, sizeof(a.lights));
     std::memcpy(a.bg, prm->background, sizeof(a.bg));
-    k_shade<<<(unsigned)(((W + SHADE_X - 1) / SHADE_X) * ((H + SHADE_Y - 1) / SHADE_Y)), SHADE_X * SHADE_Y, 0, s>>>(a);
+    launch_dep(k_shade, (unsigned)(((W + SHADE_X - 1) / SHADE_X) * ((H + SHADE_Y - 1) / SHADE_Y)), SHADE_X * SHADE_Y, 0, s, a);
     L++;
     cudaEventRecord(r->ev1, s);
     r->timed = true;

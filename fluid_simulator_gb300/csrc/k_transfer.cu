@@ -264,6 +264,7 @@ __device__ __forceinline__ void p2g_walk(const P2GArgs& a, int x0, int y0, int z
 
 template <bool APIC, class S>
 __global__ void __launch_bounds__(S::NTHREADS, S::MIN_BLOCKS) k_p2g(const P2GArgs a) {
+    pdl_enter();
     constexpr int PX = S::PX, PY = S::PY, PZ = S::PZ, PCELLS = S::PCELLS;
     extern __shared__ float sm[];
     float* s_vw = sm;                // [3][PCELLS]
@@ -606,9 +607,9 @@ cudaError_t launch_p2g_shape(P2GArgs a, bool apic, cudaStream_t stream) {
     cudaError_t e = set_smem_limit((const void*)(apic ? k_p2g<true, S> : k_p2g<false, S>), S::SMEM);
     if (e != cudaSuccess) return e;
     if (apic)
-        k_p2g<true, S><<<nb, S::NTHREADS, S::SMEM, stream>>>(a);
+        return launch_dep(k_p2g<true, S>, nb, S::NTHREADS, S::SMEM, stream, a);
     else
-        k_p2g<false, S><<<nb, S::NTHREADS, S::SMEM, stream>>>(a);
+        return launch_dep(k_p2g<false, S>, nb, S::NTHREADS, S::SMEM, stream, a);
     return cudaGetLastError();
 }
 
