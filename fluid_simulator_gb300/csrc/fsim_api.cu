@@ -21,6 +21,7 @@ namespace {
 // ---- AoS <-> SoA ------------------------------------------------------------
 __global__ void k_aos_to_soa(const float* pos, const float* vel, const float* c, long long n, ParticleBuf d,
                              long long first, uint32_t id0, int ids) {
+    pdl_enter();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const long long j = first + i;
@@ -41,6 +42,7 @@ __global__ void k_aos_to_soa(const float* pos, const float* vel, const float* c,
 constexpr int AOS_THREADS = 256;
 __global__ void __launch_bounds__(AOS_THREADS) k_soa_to_aos(ParticleBuf s, long long n, float* pos, float* vel,
                                                             float* c) {
+    pdl_enter();
     __shared__ float sp[AOS_THREADS * 3], sv[AOS_THREADS * 3], sc[AOS_THREADS * 9];
     const long long i0 = (long long)blockIdx.x * AOS_THREADS, i = i0 + threadIdx.x;
     const int t = threadIdx.x;
@@ -606,7 +608,7 @@ static int upload_particles(fsim_ctx* ctx, const float* pos, const float* vel, c
             dc = t + 6 * n;
         }
     }
-    k_aos_to_soa<<<ceil_div(n, 256), 256, 0, ctx->stream>>>(dp, dv, dc, n, ctx->buf[ctx->cur], first,
+    launch_dep(k_aos_to_soa, ceil_div(n, 256), 256, 0, ctx->stream, dp, dv, dc, n, ctx->buf[ctx->cur], first,
                                                             ctx->next_id, ctx->prm.track_ids ? 1 : 0);
     CHECK_LAUNCH(ctx);
     if (tmp) FSIM_CUDA_TRY(ctx, cudaFreeAsync(tmp, ctx->stream));
@@ -678,7 +680,7 @@ int fsim_get_particles(fsim_ctx* ctx, float* pos, float* vel, float* c, int64_t 
     if (dst_index)
         k_soa_to_aos_at<<<ceil_div(n, 256), 256, 0, s>>>(ctx->buf[ctx->cur], n, dst_index, dp, dv, dc);
     else
-        k_soa_to_aos<<<ceil_div(n, AOS_THREADS), AOS_THREADS, 0, s>>>(ctx->buf[ctx->cur], n, dp, dv, dc);
+        launch_dep(k_soa_to_aos, ceil_div(n, AOS_THREADS), AOS_THREADS, 0, s, ctx->buf[ctx->cur], n, dp, dv, dc);
     CHECK_LAUNCH(ctx);
     if (where == FSIM_HOST) {
         if (pos) FSIM_CUDA_TRY(ctx, cudaMemcpyAsync(pos, dp, (size_t)n * 12, cudaMemcpyDeviceToHost, s));

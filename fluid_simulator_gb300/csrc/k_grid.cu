@@ -45,6 +45,7 @@ __device__ __forceinline__ bool covered(const ObsGeom& o, int x, int y, int z) {
 // threads over the covered index box extended by one cell on the low side
 __global__ void k_obstacle_faces(GridGeom g, ObsGeom o, const uint8_t* flags, float* u0, float* u1,
                                  float* u2, int ex, int ey, int ez) {
+    pdl_enter();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ex * ey * ez) return;
     const int x = o.mn[0] - 1 + t / (ey * ez), y = o.mn[1] - 1 + (t / ez) % ey, z = o.mn[2] - 1 + t % ez;
@@ -64,6 +65,7 @@ __global__ void k_obstacle_faces(GridGeom g, ObsGeom o, const uint8_t* flags, fl
 }
 
 __global__ void k_obstacle_cells(GridGeom g, ObsGeom o, uint8_t* flags, int ex, int ey, int ez) {
+    pdl_enter();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ex * ey * ez) return;
     const int x = o.mn[0] + t / (ey * ez), y = o.mn[1] + (t / ez) % ey, z = o.mn[2] + t % ez;
@@ -83,6 +85,7 @@ __device__ __forceinline__ bool is_border(const GridGeom& g, int top_solid, int 
 // row counts as SOLID, as the reference's aliased index resolves to the floor).
 __global__ void k_prep(GridGeom g, int top_solid, int walls, int post, float ginc, uint8_t* flags,
                        float* u0, float* u1, float* u2, float* w0, float* w1, float* w2) {
+    pdl_enter();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.ncell) return;
     int x, y, z;
@@ -129,6 +132,7 @@ __global__ void k_prep(GridGeom g, int top_solid, int walls, int post, float gin
 // read as sources in that pass, so the passes are order independent.
 __global__ void k_extrapolate(GridGeom g, int it, const uint8_t* flags, uint8_t* valid, float* v0,
                               float* v1, float* v2) {
+    pdl_enter();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.ncell) return;
     int x, y, z;
@@ -209,6 +213,7 @@ __global__ void k_sor(GridGeom g, const uint8_t* flags, float* vx, float* vy, fl
 
 __global__ void k_apply_pressure(GridGeom g, const uint8_t* flags, const double* p, double scale,
                                  float* v0, float* v1, float* v2) {
+    pdl_enter();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.ncell) return;
     int x, y, z;
@@ -241,6 +246,7 @@ __global__ void k_apply_pressure(GridGeom g, const uint8_t* flags, const double*
 // grid stays below 2^31 cells.
 __global__ void __launch_bounds__(256) k_copy16(const uint4* src, uint4* dst, long long n16, const uint8_t* tsrc,
                                                 uint8_t* tdst, int tail) {
+    pdl_enter();
     const long long step = (long long)gridDim.x * blockDim.x, i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     for (long long i = i0; i < n16; i += step) dst[i] = src[i];
     if (i0 < tail) tdst[i0] = tsrc[i0];
@@ -249,13 +255,14 @@ bool copy_dense(const GridGeom& g, const void* src, void* dst, int elem, cudaStr
     if (g.pz != g.nz || ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15)) return false;
     const long long bytes = (long long)g.nx * g.ny * g.nz * elem, n16 = bytes / 16;
     const int nb = (int)std::min<long long>(std::max<long long>((n16 + 255) / 256, 1), 152 * 32);
-    k_copy16<<<nb, 256, 0, s>>>(static_cast<const uint4*>(src), static_cast<uint4*>(dst), n16,
+    launch_dep(k_copy16, nb, 256, 0, s, static_cast<const uint4*>(src), static_cast<uint4*>(dst), n16,
                                 static_cast<const uint8_t*>(src) + n16 * 16, static_cast<uint8_t*>(dst) + n16 * 16,
                                 (int)(bytes - n16 * 16));
     return true;
 }
 template <typename T>
 __global__ void k_pad_to_dense(GridGeom g, const T* src, T* dst) {
+    pdl_enter();
     const unsigned j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= (unsigned)g.nx * g.ny * g.nz) return;
     const unsigned row = j / (unsigned)g.nz;
@@ -318,15 +325,14 @@ int launch_obstacle(fsim_ctx* ctx, const fsim_obstacle& ob) {
         if (ext[a] <= 0) return 0;
     }
     const int ex = ext[0] + 1, ey = ext[1] + 1, ez = ext[2] + 1;
-    k_obstacle_faces<<<ceil_div((long long)ex * ey * ez, 256), 256, 0, ctx->stream>>>(
-        g, o, ctx->flags, ctx->u[0], ctx->u[1], ctx->u[2], ex, ey, ez);
-    k_obstacle_cells<<<ceil_div((long long)ext[0] * ext[1] * ext[2], 256), 256, 0, ctx->stream>>>(
-        g, o, ctx->flags, ext[0], ext[1], ext[2]);
+    launch_dep(k_obstacle_faces, ceil_div((long long)ex * ey * ez, 256), 256, 0, ctx->stream, g, o, ctx->flags, ctx->u[0], ctx->u[1], ctx->u[2], ex, ey, ez);
+    launch_dep(k_obstacle_cells, ceil_div((long long)ext[0] * ext[1] * ext[2], 256), 256, 0, ctx->stream, g, o, ctx->flags, ext[0], ext[1], ext[2]);
     return 2;
 }
 
 namespace {
 __global__ void k_fetch_small(unsigned* dst, const unsigned* src, int words) {
+    pdl_enter();
     for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
     __threadfence_system();
 }
@@ -334,13 +340,13 @@ __global__ void k_fetch_small(unsigned* dst, const unsigned* src, int words) {
 
 void fetch_small(void* host, const void* dev, int bytes, cudaStream_t s) {
     // every caller's buffers are 4-byte aligned and a whole number of words
-    k_fetch_small<<<1, 32, 0, s>>>(static_cast<unsigned*>(host), static_cast<const unsigned*>(dev), (bytes + 3) / 4);
+    launch_dep(k_fetch_small, 1, 32, 0, s, static_cast<unsigned*>(host), static_cast<const unsigned*>(dev), (bytes + 3) / 4);
 }
 
 void launch_prep(fsim_ctx* ctx, int walls, int post, float gravity_inc) {
     const GridGeom& g = ctx->g;
     ctx->launches += 1;
-    k_prep<<<ceil_div(g.ncell, 256), 256, 0, ctx->stream>>>(
+    launch_dep(k_prep, ceil_div(g.ncell, 256), 256, 0, ctx->stream,
         g, ctx->prm.top_solid, walls, post, gravity_inc, ctx->flags, ctx->u[0], ctx->u[1], ctx->u[2],
         ctx->v2[0], ctx->v2[1], ctx->v2[2]);
 }
@@ -349,7 +355,7 @@ void launch_extrapolate(fsim_ctx* ctx) {
     const GridGeom& g = ctx->g;
     ctx->launches += 2;
     for (int it = 0; it < 2; it++)
-        k_extrapolate<<<ceil_div(g.ncell, 256), 256, 0, ctx->stream>>>(g, it, ctx->flags, ctx->valid,
+        launch_dep(k_extrapolate, ceil_div(g.ncell, 256), 256, 0, ctx->stream, g, it, ctx->flags, ctx->valid,
                                                                        ctx->v2[0], ctx->v2[1], ctx->v2[2]);
 }
 
@@ -373,7 +379,7 @@ void launch_apply_pressure(fsim_ctx* ctx, double dt) {
     const GridGeom& g = ctx->g;
     ctx->launches += 1;
     const double scale = dt / (ctx->prm.fluid_density * g.hd);
-    k_apply_pressure<<<ceil_div(g.ncell, 256), 256, 0, ctx->stream>>>(g, ctx->flags, ctx->sv.phi, scale,
+    launch_dep(k_apply_pressure, ceil_div(g.ncell, 256), 256, 0, ctx->stream, g, ctx->flags, ctx->sv.phi, scale,
                                                                       ctx->v2[0], ctx->v2[1], ctx->v2[2]);
 }
 
@@ -381,9 +387,9 @@ void launch_pad_to_dense(const GridGeom& g, const void* src, void* dst, int elem
     const long long n = (long long)g.nx * g.ny * g.nz;
     if (copy_dense(g, src, dst, elem, s)) return;
     const int nb = ceil_div(n, 256);
-    if (elem == 1) k_pad_to_dense<uint8_t><<<nb, 256, 0, s>>>(g, (const uint8_t*)src, (uint8_t*)dst);
-    else if (elem == 4) k_pad_to_dense<float><<<nb, 256, 0, s>>>(g, (const float*)src, (float*)dst);
-    else k_pad_to_dense<double><<<nb, 256, 0, s>>>(g, (const double*)src, (double*)dst);
+    if (elem == 1) launch_dep(k_pad_to_dense<uint8_t>, nb, 256, 0, s, g, (const uint8_t*)src, (uint8_t*)dst);
+    else if (elem == 4) launch_dep(k_pad_to_dense<float>, nb, 256, 0, s, g, (const float*)src, (float*)dst);
+    else launch_dep(k_pad_to_dense<double>, nb, 256, 0, s, g, (const double*)src, (double*)dst);
 }
 
 void launch_dense_to_pad(const GridGeom& g, const void* src, void* dst, int elem, cudaStream_t s) {

@@ -589,6 +589,7 @@ constexpr int GFX_THREADS = 256;
 // as five 4-byte stores at a 20-byte stride per lane.
 __global__ void __launch_bounds__(GFX_THREADS) k_gfx(ParticleBuf p, long long n, const float* avg, GridGeom g,
                                                      fsim_particle_gfx* out, int vec) {
+    pdl_enter();
     __shared__ __align__(16) float stage[GFX_THREADS * 5];
     const long long i0 = (long long)blockIdx.x * GFX_THREADS;
     const long long i = i0 + threadIdx.x;
@@ -700,5 +701,5 @@ void launch_gfx(ParticleBuf p, long long n, const float* avg, const GridGeom& g,
                 fsim_particle_gfx* out, cudaStream_t s) {
     if (n <= 0) return;
     const int vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0 ? 1 : 0;
-    k_gfx<<<ceil_div(n, GFX_THREADS), GFX_THREADS, 0, s>>>(p, n, avg, g, out, vec);
+    launch_dep(k_gfx, ceil_div(n, GFX_THREADS), GFX_THREADS, 0, s, p, n, avg, g, out, vec);
 }

@@ -1592,7 +1592,8 @@ __global__ void __launch_bounds__(MG_CLUSTER_THREADS, 1) k_mg_coarse(const PcgAr
     }
     __syncthreads();
     // the codes were written before the solve's first V-cycle: they are loaded while
-    // the predecessor drains
+    // the predecessor drains (the residual in between is an ordinary launch: it starts
+    // when they are complete, and nothing after it starts before it is)
     for (int l = first; l <= C.last; l++)
         if (l < C.ls || rank == 0) slev_init(S[l], C.lev[l]);
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -347,6 +347,7 @@ __global__ void __launch_bounds__(G2P_THREADS) k_g2p(const G2PArgs a, const __gr
                                                      const __grid_constant__ CUtensorMap m3,
                                                      const __grid_constant__ CUtensorMap m4,
                                                      const __grid_constant__ CUtensorMap m5) {
+    pdl_enter();
     constexpr int TX = S::TX, TY = S::TY, TZ = S::TZ, BY = S::BY, BZ = S::BZ, BOXN = S::BOXN, ROWS = S::ROWS;
     static_assert(ROWS == 16 || ROWS == 32 || ROWS == 64, "a row per lane of one or two warps");
     extern __shared__ __align__(128) unsigned char smraw[];
@@ -725,7 +726,7 @@ void launch_g2p_shape(G2PArgs a, int mode, const CUtensorMap* m, cudaStream_t st
         set_smem_limit((const void*)kern, smem);
         // PIC and APIC read the first three boxes only
         const int o = mode == FSIM_FLIP ? 3 : 0;
-        kern<<<nb, G2P_THREADS, smem, stream>>>(a, m[0], m[1], m[2], m[o], m[o + 1], m[o + 2]);
+        launch_dep(kern, nb, G2P_THREADS, smem, stream, a, m[0], m[1], m[2], m[o], m[o + 1], m[o + 2]);
     };
     if (mode == FSIM_PIC) go(k_g2p<0, S>);
     else if (mode == FSIM_FLIP) go(k_g2p<1, S>);
