@@ -49,14 +49,15 @@ struct P2GArgs {
     int ntx, nty, ntz;
 };
 
-// P2G tile (owned cells) and its one-cell halo: 8x16x16 owned cells, seven
-// FP32 shared accumulators per cell (face v and weight per axis, density) =
-// 57 KB, two 384-thread CTAs per SM.  Tile shapes measured on the 256^3 APIC
-// workload (kernel ms): 8x16x16 4.56, 6x16x16 4.71, 12x12x12 4.73,
-// 12x16x16 4.75, 8x12x24 4.79, 8x8x32 4.83, 16x16x8 4.96, 8x16x24 5.03.  A
-// tile narrow in x (the slowest axis of the cell order) spans fewer runs of
-// sorted particles, and the smaller shared-memory share leaves L1 more room
-// for the particle re-reads of the four warp roles.
+// P2G tile (owned cells) and its one-cell halo; seven FP32 shared accumulators per
+// cell (face v and weight per axis, density).  One CTA of seven warp quads per SM:
+// the same warps as two CTAs of three quads, but the accumulators take half the
+// shared memory, and what they leave is L1 for the particles, whose sectors a lane
+// reads eight times and four roles share.  At 256^3 (half filled, in a step / dam
+// break, particles in order), ms: two CTAs of 8x16x16 6.08 / 2.13; one of 8x16x16
+// 5.32 / 2.07, 8x8x16 5.62 / 2.35, 12x16x16 5.21 / 1.99, 16x12x16 4.67 / 1.90, 16x16x16
+// 4.69 / 1.83, 16x20x16 4.94 / 1.81, 20x16x16 4.95 / 1.86, 16x16x24 6.35 / 1.95 (less L1
+// again).  Halo cells read and walked: 1.58 times the cells at 8x16x16, 1.42 at 16x16x16.
 template <int X, int Y, int Z, int THREADS, int MINB>
 struct P2GShape {
     static constexpr int PX = X, PY = Y, PZ = Z, QX = X + 2, QY = Y + 2, QZ = Z + 2;
@@ -64,14 +65,13 @@ struct P2GShape {
     static constexpr int SMEM = 7 * PCELLS * (int)sizeof(float);
     static constexpr int NTHREADS = THREADS, MIN_BLOCKS = MINB;
 };
-// the default on large grids: 8x16x16 tiles (57,344 B), three warp quads per CTA, two
-// CTAs per SM; smaller tiles on smaller grids (p2g_fast)
-using P2GFast = P2GShape<8, 16, 16, 384, 2>;
+// the default on large grids (114,688 B); smaller tiles on smaller grids (p2g_fast)
+using P2GFast = P2GShape<16, 16, 16, 896, 1>;
 // bit-reproducible (fsim_params.deterministic): one warp quad per CTA, so each
 // shared accumulator is added to by a single warp in program order (a warp's
 // lanes hold distinct cells: one flush instruction never adds twice to an
-// address); 8x8x16 tiles (28,672 B), six CTAs per SM.  5.9 against 4.6 ms at
-// 256^3 (8x16x16 tiles with one quad: 8.1 ms).
+// address); 8x8x16 tiles (28,672 B), six CTAs per SM (8x16x16 tiles with one quad took
+// 1.4 times as long).
 using P2GDet = P2GShape<8, 8, 16, 128, 6>;
 
 // 1D tent weights of the three cell-centred nodes at relative -0.5, 0.5, 1.5
@@ -619,28 +619,29 @@ long long p2g_tiles(const GridGeom& g) {
     return (long long)ceil_div(g.nx, S::PX) * ceil_div(g.ny, S::PY) * ceil_div(g.nz, S::PZ);
 }
 
-// The largest tile that still gives P2G_MIN_TILES CTAs (about three per SM; part of
-// them hold no fluid).  A warp quad walks its tile's cell blocks one after the
-// other, 35 blocks for 8x16x16 tiles, so a grid of few large tiles takes as long
-// as one tile does: 16 CTAs and 167 us at 32^3.  Smaller tiles read more halo
-// cells (1.6 times the cells at 8x16x16, 2.0 at 8x8x8, 3.4 at 4x4x4), which costs
-// more than it gives once every SM is busy.  Sort + P2G in us, by tile 4x4x4 /
-// 4x4x8 / 4x8x8 / 8x8x16 / 8x16x16: 32^3 dam 64 / 69 / 83 / 140 / 210, 48^3 dam
-// 90 / 83 / 98 / 168 / 249, 64^3 dam 145 / 120 / 109 / 169 / 260, 90x61x75 half
-// filled 294 / 244 / 220 / 198 / 288, 96^3 dam 408 / 317 / 263 / 245 / 362, 128^3
-// dam 941 / 707 / 571 / 467 / 445 (before the walks were one per role).  Seven quads per
-// 4x8x8 tile instead of three: 64x64x40 dam 80 -> 73, half filled 112 -> 106; at 4x4x8 and
-// 4x4x4 it gains on one scene what it loses on the other.
-constexpr long long P2G_MIN_TILES = 480;
-using T1 = P2GShape<8, 8, 16, 384, 2>;
-using T2 = P2GShape<4, 8, 8, 896, 1>;  // seven quads: 19 cell blocks in three rounds
-using T3 = P2GShape<4, 4, 8, 384, 2>;
+// A warp quad walks its tile's blocks of 32 halo cells one after the other (203 blocks
+// over seven quads for 16x12x16), so few large tiles take as long as one tile does
+// (8x16x16 on 32^3: 16 CTAs, 167 us); smaller ones read more halo cells (1.6 times the
+// cells at 8x16x16, 2.0 at 8x8x8, 3.4 at 4x4x4).  A shape is taken from the number of its
+// tiles on, part of which hold no fluid, at which it measured faster than the next
+// smaller one.  k_p2g in us, 16x16x16 / 16x12x16 / 8x16x16 / 8x8x16 / 4x8x8: 90x61x75 half
+// filled (180 tiles of 16x12x16, 480 of 8x8x16) 278 / 186 / 157 / 144 / 168; 107x90x66 (280 of
+// 16x12x16) 197 / 152 / 185 / 168 / 209; 128^3 dam (512 of 16x16x16) 375 / 352 / 397 / 365 / 565;
+// 256^3 above.  Sort + P2G, 8x8x16 / 4x8x8 / 4x4x8 / 4x4x4 (two CTAs of three quads), dam and
+// half filled: 32^3 (256 of 4x4x8) 71 80 / 42 42 / 37 38 / 35 40; 48x40x32 (240 of 4x8x8) 82 83 /
+// 43 47 / 38 53 / 37 55; 40x56x44 (420) 83 89 / 45 68 / 50 73 / 51 73; 64x64x40 (640, 160 of 8x8x16)
+// 89 94 / 57 91 / 68 103 / 68 108.
+using T0 = P2GShape<16, 12, 16, 896, 1>;
+using T1 = P2GShape<8, 8, 16, 896, 1>;
+using T2 = P2GShape<4, 8, 8, 896, 1>;
+using T3 = P2GShape<4, 4, 8, 896, 1>;
 using T4 = P2GShape<4, 4, 4, 384, 2>;
 cudaError_t p2g_fast(const P2GArgs& a, bool apic, cudaStream_t stream) {
-    if (p2g_tiles<P2GFast>(a.g) >= P2G_MIN_TILES) return launch_p2g_shape<P2GFast>(a, apic, stream);
-    if (p2g_tiles<T1>(a.g) >= P2G_MIN_TILES) return launch_p2g_shape<T1>(a, apic, stream);
-    if (p2g_tiles<T2>(a.g) >= P2G_MIN_TILES) return launch_p2g_shape<T2>(a, apic, stream);
-    if (p2g_tiles<T3>(a.g) >= P2G_MIN_TILES) return launch_p2g_shape<T3>(a, apic, stream);
+    if (p2g_tiles<P2GFast>(a.g) >= 2048) return launch_p2g_shape<P2GFast>(a, apic, stream);
+    if (p2g_tiles<T0>(a.g) >= 270) return launch_p2g_shape<T0>(a, apic, stream);
+    if (p2g_tiles<T1>(a.g) >= 400) return launch_p2g_shape<T1>(a, apic, stream);
+    if (p2g_tiles<T2>(a.g) >= 240) return launch_p2g_shape<T2>(a, apic, stream);
+    if (p2g_tiles<T3>(a.g) >= 300) return launch_p2g_shape<T3>(a, apic, stream);
     return launch_p2g_shape<T4>(a, apic, stream);
 }
 
@@ -655,6 +656,7 @@ cudaError_t p2g_load_shape() {
 // may not trigger a lazy module load later)
 cudaError_t p2g_load_all() {
     cudaError_t e = p2g_load_shape<P2GFast>();
+    if (e == cudaSuccess) e = p2g_load_shape<T0>();
     if (e == cudaSuccess) e = p2g_load_shape<T1>();
     if (e == cudaSuccess) e = p2g_load_shape<T2>();
     if (e == cudaSuccess) e = p2g_load_shape<T3>();

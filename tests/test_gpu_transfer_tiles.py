@@ -55,11 +55,10 @@ def p2g_ref(shape, pos, vel, c):
         wts.append(den)
 
 
-# CTAs of 8x16x16 tiles below and above the change: 23x29x30 and 37x21x44 run 4x4x4 tiles,
-# 48^3 4x4x8, 64^3 and 66x70x50 4x8x8, 90x61x75 8x8x16, 128x112x128 (448) 8x8x16,
-# 128x128x120 (512) 8x16x16
-SHAPES = [(7, 9, 5), (23, 29, 30), (37, 21, 44), (48, 48, 48), (66, 70, 50), (90, 61, 75), (128, 112, 128),
-          (128, 128, 120)]
+# P2G tiles: 7x9x5 and 23x29x30 run 4x4x4, 37x21x44 4x4x8, 48^3 and 66x70x50 4x8x8, 90x61x75
+# 8x8x16, 107x90x66 (280) and the 128^3 ones 16x12x16, 208x208x200 (2197) 16x16x16
+SHAPES = [(7, 9, 5), (23, 29, 30), (37, 21, 44), (48, 48, 48), (66, 70, 50), (90, 61, 75), (107, 90, 66),
+          (128, 112, 128), (128, 128, 120), (208, 208, 200)]
 
 
 @pytest.mark.parametrize("transfer", [N.FLIP, N.APIC])
