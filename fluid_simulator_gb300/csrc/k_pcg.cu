@@ -445,11 +445,9 @@ __global__ void __launch_bounds__(PCG_THREADS) k_spmv(const PcgArgs a, Vecs<T> v
     }
 }
 
-// x += alpha s; r_new = r - alpha q; r.r, max|r|; then on r_new:
-//   PMODE 1: the black half of the red-black IC solve (the red half is k_red)
-//   PMODE 2: the first red-black Gauss-Seidel sweep of the multigrid V-cycle from
-//            zero (red z = r/ns, black z = (r + sum_j r_j/ns_j)/ns)
-template <typename T, int PMODE>
+// x += alpha s; r_new = r - alpha q; r.r, max|r|; then on r_new the black half of the
+// red-black IC solve (the red half is k_red)
+template <typename T>
 __global__ void __launch_bounds__(PCG_THREADS) k_update(const PcgArgs a, Vecs<T> v) {
     __shared__ double scratch[PCG_THREADS * 2];
     if (a.st->done) return;
@@ -472,7 +470,7 @@ __global__ void __launch_bounds__(PCG_THREADS) k_update(const PcgArgs a, Vecs<T>
         rn[c] = rv;
         rr.add(rv * rv);
         rmax = fmax(rmax, fabs(rv));
-        if (PMODE != 0 && ((x + y + z) & 1)) {
+        if ((x + y + z) & 1) {
             T sum = rv;
 #pragma unroll
             for (int k = 0; k < 6; k++)
@@ -481,10 +479,7 @@ __global__ void __launch_bounds__(PCG_THREADS) k_update(const PcgArgs a, Vecs<T>
                     const uint16_t cj = a.code[j];
                     sum += (ro[j] - alpha * v.q[j]) * recip_ns<T>(code_ns(cj));
                 }
-            if (PMODE == 1) v.z[c] = sum * (T)black_pivot_inv(a.code, c, cc, a.B);
-            else v.z[c] = sum * recip_ns<T>(code_ns(cc));
-        } else if (PMODE == 2) {
-            v.z[c] = rv * recip_ns<T>(code_ns(cc));
+            v.z[c] = sum * (T)black_pivot_inv(a.code, c, cc, a.B);
         }
     }
     double acc[2] = {rr.value(), (double)rmax};
@@ -1837,7 +1832,7 @@ int solver_alloc(fsim_ctx* ctx) {
     S.q = S.r + 5 * nc;
     S.plo = S.r + 6 * nc;
     int bps = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_update<float, 1>, PCG_THREADS, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_update<float>, PCG_THREADS, 0);
     if (bps < 1) bps = 1;
     // a pass takes four bricks per block: no more blocks than a grid has bricks for
     S.grid_blocks = (int)std::min<long long>((long long)ctx->num_sms * bps, (S.nbricks + 3) / 4);
@@ -2235,7 +2230,7 @@ static int run_pcg(fsim_ctx* ctx, PcgArgs& A, Vecs<T> v, int precision, int prec
             launch_pdl(k_update_q, G, PCG_THREADS, st, A, vf, L0);
         } else {
             k_spmv<T><<<G, PCG_THREADS, 0, st>>>(A, v);
-            k_update<T, 1><<<G, PCG_THREADS, 0, st>>>(A, v);
+            k_update<T><<<G, PCG_THREADS, 0, st>>>(A, v);
         }
         ctx->launches += 2;
     };
