@@ -1852,14 +1852,16 @@ int solver_alloc(fsim_ctx* ctx) {
     float psc[64];
     for (int i = 0; i < 64; i++) psc[i] = 64.f / (64 - i);
     FSIM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_pscale, psc, sizeof(psc)));
-    // multigrid hierarchy: halve until every dimension is <= 4
+    // multigrid hierarchy: halve (at least once) until every dimension is <= 4
     MGLevelBufs l0;
     l0.nx = g.nx; l0.ny = g.ny; l0.nz = g.nz; l0.pz = g.pz; l0.ncell = g.ncell;
     l0.code = S.code;
     FSIM_CUDA_TRY(ctx, cudaMalloc(&l0.r, nc * sizeof(float)));
     FSIM_CUDA_TRY(ctx, cudaMemset(l0.r, 0, nc * sizeof(float)));
     S.mg.push_back(l0);
-    while (std::max(S.mg.back().nx, std::max(S.mg.back().ny, S.mg.back().nz)) > 4) {
+    // at least one coarse level, also below a grid of 3 or 4 cells per axis: the bottom
+    // kernel reads coarse codes, and the cycle's level 0 computes z.r
+    do {
         const MGLevelBufs& f = S.mg.back();
         MGLevelBufs c;
         c.nx = (f.nx + 1) / 2; c.ny = (f.ny + 1) / 2; c.nz = (f.nz + 1) / 2; c.pz = (c.nz + 3) & ~3;
@@ -1875,7 +1877,7 @@ int solver_alloc(fsim_ctx* ctx) {
         FSIM_CUDA_TRY(ctx, cudaMemset(c.ccode, 0, c.ncell * sizeof(uint32_t)));
         FSIM_CUDA_TRY(ctx, cudaMemset(c.kind, 2, c.ncell));
         S.mg.push_back(c);
-    }
+    } while (std::max(S.mg.back().nx, std::max(S.mg.back().ny, S.mg.back().nz)) > 4);
     if ((long long)S.mg.back().nx * S.mg.back().ny * S.mg.back().nz > MG_BOTTOM_MAX) {
         ctx->err = "multigrid coarsest level too large";
         return FSIM_E_INVALID;
