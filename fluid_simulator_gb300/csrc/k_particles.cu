@@ -600,8 +600,9 @@ __global__ void __launch_bounds__(GFX_THREADS) k_gfx(ParticleBuf p, long long n,
         const float gx = px * g.hinv - 0.5f, gy = py * g.hinv - 0.5f, gz = pz * g.hzinv - 0.5f;
         const int bx = (int)gx, by = (int)gy, bz = (int)gz;
         float dens = 0.f;
-        if (bx >= 0 && by >= 0 && bz >= 0 && bx + 1 < g.nx && by + 1 < g.ny && bz + 1 < g.nz) {
-            // all eight cells exist: one address, and the weights' factors once
+        if (bx >= 0 && by >= 0 && bz >= 0 && bx < g.nx - 1 && by < g.ny - 1 && bz < g.nz - 1) {
+            // all eight cells exist: one address, and the weights' factors once (a position far
+            // outside the grid saturates its index: nothing is added to it before the test)
             const float* q = avg + gidx(g, bx, by, bz);
             const long long sy = g.pz, sx = (long long)g.ny * g.pz;
             const float a[8] = {q[0], q[1], q[sy], q[sy + 1], q[sx], q[sx + 1], q[sx + sy], q[sx + sy + 1]};
@@ -613,8 +614,9 @@ __global__ void __launch_bounds__(GFX_THREADS) k_gfx(ParticleBuf p, long long n,
         } else
 #pragma unroll
         for (int k = 0; k < 8; k++) {
-            const int x = bx + (k >> 2), y = by + ((k >> 1) & 1), z = bz + (k & 1);
-            if (x < 0 || y < 0 || z < 0 || x >= g.nx || y >= g.ny || z >= g.nz) continue;
+            const int ox = k >> 2, oy = (k >> 1) & 1, oz = k & 1;
+            if (bx < -ox || by < -oy || bz < -oz || bx >= g.nx - ox || by >= g.ny - oy || bz >= g.nz - oz) continue;
+            const int x = bx + ox, y = by + oy, z = bz + oz;
             const float w = (1.f - fabsf(gx - x)) * (1.f - fabsf(gy - y)) * (1.f - fabsf(gz - z));
             dens += w * avg[gidx(g, x, y, z)];
         }
