@@ -1981,16 +1981,15 @@ static void mg_vcycle(fsim_ctx* ctx, const PcgArgs& A, int l, const float* r0, c
         C.last = last - l;
         C.nu = NUC;
         // the levels from ls on run in shared memory (x, f, r floats + codes per cell)
+        // (long thin levels: their guard planes count, and they halve along one axis only)
         C.ls = C.last;
         size_t smem = 0;
         for (int k = C.last; k >= 0; k--) {
             const MGLevelBufs& b = S.mg[l + k];
-            if ((long long)b.nx * b.ny * ((b.nz + 1) & ~1) > MG_SMEM_CELLS) break;
+            const size_t bytes = (size_t)slev_floats(b.nx, b.ny, b.nz) * sizeof(float);
+            if ((long long)b.nx * b.ny * ((b.nz + 1) & ~1) > MG_SMEM_CELLS || smem + bytes > (size_t)MG_CLUSTER_SMEM) break;
+            smem += bytes;
             C.ls = k;
-        }
-        for (int k = C.ls; k <= C.last; k++) {
-            const MGLevelBufs& b = S.mg[l + k];
-            smem += (size_t)slev_floats(b.nx, b.ny, b.nz) * sizeof(float);
         }
         // levels lc .. ls-1 as x slabs in the cluster's distributed shared memory
         // when they fit beside rank 0's levels (else they run in global memory)
