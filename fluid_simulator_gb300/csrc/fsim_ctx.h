@@ -5,6 +5,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <array>
 #include <string>
 #include <vector>
 
@@ -77,7 +78,7 @@ struct SolverBufs {
     // (precision, preconditioner, sweep counts); up to four are kept
     static constexpr int kIterGraphs = 4;
     cudaGraphExec_t iter_exec[kIterGraphs] = {};
-    int iter_key[kIterGraphs] = {-1, -1, -1, -1};
+    std::array<int, 6> iter_key[kIterGraphs] = {};  // element size, multigrid, its sweeps
     int iter_kernels[kIterGraphs] = {};
     long long iter_used[kIterGraphs] = {};  // last use (for replacement)
     long long iter_clock = 0;

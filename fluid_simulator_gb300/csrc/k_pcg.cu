@@ -1950,9 +1950,15 @@ static void mg_setup(fsim_ctx* ctx) {
     }
 }
 
-// free-surface band sweeps on level l (only the finest level has a band; none unless asked for)
-static int mg_band_sweeps(const fsim_params& P, int l) {
-    return l == 0 && P.mg_boundary_sweeps > 0 ? P.mg_boundary_sweeps : 0;
+// the V-cycle's sweeps: level 0, separately launched coarse levels, cluster levels, and on
+// the free-surface band of level 0 (none unless asked for)
+struct MGSweeps {
+    int fine, coarse, cluster, band;
+};
+static MGSweeps mg_sweeps(const fsim_params& P) {
+    return {P.mg_sweeps > 0 ? P.mg_sweeps : MG_NU_DEFAULT, P.mg_coarse_sweeps > 0 ? P.mg_coarse_sweeps : MG_NU_COARSE_DEFAULT,
+            P.mg_cluster_sweeps > 0 ? P.mg_cluster_sweeps : MG_NU_COARSE_DEFAULT,
+            P.mg_boundary_sweeps > 0 ? P.mg_boundary_sweeps : 0};
 }
 
 // z = V-cycle(r); r is the current PCG residual (r0 or r1 by device state).
@@ -1960,10 +1966,8 @@ static int mg_band_sweeps(const fsim_params& P, int l) {
 // last level-0 sweep also computes z.r and the CG scalars (k_red modes).
 static void mg_vcycle(fsim_ctx* ctx, const PcgArgs& A, int l, const float* r0, const float* r1, float* z,
                       bool first_fused, int dot_mode) {
-    const fsim_params& P = ctx->prm;
-    const int NU = l == 0 ? (P.mg_sweeps > 0 ? P.mg_sweeps : MG_NU_DEFAULT)
-                          : (P.mg_coarse_sweeps > 0 ? P.mg_coarse_sweeps : MG_NU_COARSE_DEFAULT);
-    const int NUC = P.mg_cluster_sweeps > 0 ? P.mg_cluster_sweeps : MG_NU_COARSE_DEFAULT;
+    const MGSweeps sw = mg_sweeps(ctx->prm);
+    const int NU = l == 0 ? sw.fine : sw.coarse, NUC = sw.cluster;
     SolverBufs& S = ctx->sv;
     cudaStream_t st = ctx->stream;
     const int G = S.grid_blocks;
@@ -2036,7 +2040,7 @@ static void mg_vcycle(fsim_ctx* ctx, const PcgArgs& A, int l, const float* r0, c
         smooth(1, 0);
         ctx->launches += 1;
     }
-    const int NB = mg_band_sweeps(P, l);
+    const int NB = l == 0 ? sw.band : 0;
     auto smooth_band = [&](int color) {
         launch_pdl(k_mg_smooth_bnd, G, PCG_THREADS, st, A, L, (const int4*)S.bnd_quads, (const int*)S.d_nbnd, color);
         ctx->launches += 1;
@@ -2199,7 +2203,8 @@ static int run_pcg(fsim_ctx* ctx, PcgArgs& A, Vecs<T> v, int precision, int prec
         }
     };
     if (mg) mg_setup(ctx);
-    if (mg && mg_band_sweeps(ctx->prm, 0) > 0) {
+    const MGSweeps sw = mg_sweeps(ctx->prm);
+    if (mg && sw.band > 0) {
         if (!S.bnd_quads) {
             FSIM_CUDA_TRY(ctx, cudaMalloc(&S.bnd_quads, (size_t)(ctx->g.ncell / 4 + 1) * sizeof(int4)));
             FSIM_CUDA_TRY(ctx, cudaMalloc(&S.d_nbnd, sizeof(int)));
@@ -2235,9 +2240,9 @@ static int run_pcg(fsim_ctx* ctx, PcgArgs& A, Vecs<T> v, int precision, int prec
         }
         ctx->launches += 2;
     };
-    const int key = (int)sizeof(T) * 10000000 + (mg ? 1000000 : 0) + ctx->prm.mg_sweeps * 10000 +
-                    ctx->prm.mg_coarse_sweeps * 100 + ctx->prm.mg_cluster_sweeps +
-                    (ctx->prm.mg_boundary_sweeps + 1) * 100000000;
+    // (all that the captured launches depend on)
+    const std::array<int, 6> key = mg ? std::array<int, 6>{(int)sizeof(T), 1, sw.fine, sw.coarse, sw.cluster, sw.band}
+                                      : std::array<int, 6>{(int)sizeof(T), 0, 0, 0, 0, 0};
     int gi = -1;
     for (int k = 0; k < SolverBufs::kIterGraphs; k++)
         if (S.iter_exec[k] && S.iter_key[k] == key) gi = k;
