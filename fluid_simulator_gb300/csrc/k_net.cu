@@ -300,27 +300,11 @@ __global__ void k_head(const bf16* d0, long long vox, const float* wgt, const fl
 // pass 2 writes dloss/dout = c_r A r + c_e e.  Blocks of 512 voxels never straddle
 // two samples (each sample's voxel count is a multiple of 512).
 //
-// Pass 1's sums are kept as FP32 pairs (value and rounding error, ~48 bits) until the
-// block adds them to the FP64 sums: FP64 arithmetic runs at 1/64 of the FP32 rate, and
-// summing doubles across every warp with four atomics each took 229 us at 8 x 64^3 (the
-// second pass, which moves as much, 29); now 43.
-struct FF {
-    float hi = 0.f, lo = 0.f;
-    __device__ __forceinline__ void add(float v, float e) {  // + v + e
-        const float s = hi + v, b = s - hi;
-        lo += ((hi - (s - b)) + (v - b)) + e;
-        hi = s;
-    }
-    // squares that FP32 cannot hold with their rounding error go to the FP64 sum at once
-    __device__ __forceinline__ void add_square(float v, double* sum) {
-        if (fabsf(v) <= 1e15f && fabsf(v) >= 1e-15f) {
-            const float p = v * v;
-            add(p, __fmaf_rn(v, v, -p));
-        } else if (v != 0.f) {
-            atomicAdd(sum, (double)v * v);
-        }
-    }
-};
+// Pass 1's sums are FP64 from the first square on.  FP64 arithmetic runs at 1/64 of the
+// FP32 rate, so a thread adds its voxels with one FMA a square, and the block sums through
+// shared memory (block_reduce).  Summing doubles across every warp with four atomics each
+// took 229 us at 8 x 64^3 (the second pass, which moves as much, 29); now 62 with half of
+// the voxels in the mask (FP32 pairs of 48 bits up to the block sum: 43).
 constexpr int LOSS_VPT = 512 / NT_THREADS;  // voxels per thread
 __device__ __forceinline__ bool vox_solid(const bf16* x0, long long v) { return __bfloat162float(x0[v * 16 + 2]) > 0.5f; }
 
@@ -330,7 +314,7 @@ __global__ void k_loss(const float* out, const float* target, const uint8_t* mas
     pdl_enter();
     const long long per = (long long)D * H * W;
     const int smp = (int)((I)blockIdx.x * 512 / (I)per);
-    FF q[4];
+    double q[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for (int it = 0; it < LOSS_VPT; it++) {
         const I vi = (I)blockIdx.x * 512 + it * NT_THREADS + threadIdx.x;
@@ -359,29 +343,18 @@ __global__ void k_loss(const float* out, const float* target, const uint8_t* mas
         } else {
             const float rv = (float)ns * ev - nb;
             r[v] = rv;
-            q[0].add_square(rv, sums + 4 * smp);
-            q[1].add_square(ev, sums + 4 * smp + 1);
-            q[2].add_square(target[v], sums + 4 * smp + 2);
-            q[3].add_square(__bfloat162float(x0[v * 16]), sums + 4 * smp + 3);
+            const double sq[4] = {rv, ev, target[v], __bfloat162float(x0[v * 16])};
+#pragma unroll
+            for (int k = 0; k < 4; k++) q[k] = fma(sq[k], sq[k], q[k]);
         }
     }
     if (!GRAD) {
-        __shared__ double part[4][NT_THREADS / 32];
+        __shared__ double scratch[NT_THREADS * 4];
+        block_reduce<4>(q, 0, scratch);
+        if (threadIdx.x == 0)
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float hi = __shfl_xor_sync(0xffffffffu, q[k].hi, o), lo = __shfl_xor_sync(0xffffffffu, q[k].lo, o);
-                q[k].add(hi, lo);
-            }
-            if ((threadIdx.x & 31) == 0) part[k][threadIdx.x >> 5] = (double)q[k].hi + (double)q[k].lo;
-        }
-        __syncthreads();
-        if (threadIdx.x < 4) {
-            double t = 0.0;
-            for (int k = 0; k < NT_THREADS / 32; k++) t += part[threadIdx.x][k];
-            if (t != 0.0) atomicAdd(&sums[4 * smp + threadIdx.x], t);
-        }
+            for (int k = 0; k < 4; k++)
+                if (q[k] != 0.0) atomicAdd(&sums[4 * smp + k], q[k]);
     }
 }
 
