@@ -1,0 +1,33 @@
+"""What a frame costs follows from what it shows: device times of frames that differ in one
+thing, the least of many, on an otherwise idle GPU.  The bounds leave room for noise; the
+faults they are set against cost factors of 1.2 and more."""
+import numpy as np
+import pytest
+
+from fluid_simulator_gb300 import native as N
+
+pytestmark = pytest.mark.gpu
+
+
+def frame_ms(r, pts, cam, prm, frames=30):
+    ms = []
+    for _ in range(frames):
+        r.frame(pts, cam, prm)
+        ms.append(r.stats()[0])
+    return min(ms)
+
+
+def camera(w, h, eye=(2.5, 1.7, 2.8)):
+    yaw, pitch = N.look_at_angles(eye, (0.5, 0.5, 0.5))
+    return N.camera(eye, yaw, pitch, fov=40.0, aspect=w / h, near=0.05, far=60.0)
+
+
+def test_background_costs_no_weights(gpu):
+    """An empty frame: the Gaussian filter, whose weights are 676 exponentials, costs what the
+    bilateral one with 36 does (1.3 with a table per block)."""
+    w, h = 3840, 2160
+    r = N.Renderer(w, h)
+    none = np.zeros((0, 5), np.float32)
+    g, b = (frame_ms(r, none, camera(w, h), N.default_render_params(bilateral_filter=f)) for f in (0, 1))
+    r.close()
+    assert g <= 1.1 * b
