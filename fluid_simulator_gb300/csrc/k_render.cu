@@ -30,6 +30,7 @@
 
 struct fsim_renderer {
     int W = 0, H = 0;
+    int sms = 1;
     cudaStream_t own = nullptr;
     float* raw = nullptr;     // sprite depth (before smoothing)
     float* depth = nullptr;   // smoothed depth + spray
@@ -261,13 +262,20 @@ __device__ __forceinline__ void splat(const float* pos, const Cam& cam, float r,
 }
 
 // which: 0 all particles, 1 surface (density >= threshold), 2 spray (below).  The spray is
-// a few particles of many: a block gathers the ones among SPLAT_GATHER before it splats
-// them (with one thread per particle 3.4 of 32 lanes worked).  1000 x 1000 pixels, 8M
+// a few particles of many: a block gathers the ones among `gather` before it splats them
+// (with one thread per particle 3.4 of 32 lanes worked).  1000 x 1000 pixels, 8M
 // particles: surface 629 us and spray 130 before, now 405 and 55.
 constexpr int SPLAT_GATHER = 2048;
+// A block's spray is splatted by its 256 threads in turn, so where a frame has little else
+// a wide gather leaves the chip idle (2048 sprites, all spray, 1000 x 1000: one block and
+// 3570 us a frame, eight of 256 618): eight blocks per SM come first, then wider ones.
+static int splat_gather(long long n, int sms) {
+    const long long per = (n + 8ll * sms - 1) / (8ll * sms), g = (per + 255) / 256 * 256;
+    return (int)(g < 256 ? 256 : g > SPLAT_GATHER ? SPLAT_GATHER : g);
+}
 __global__ void __launch_bounds__(256, 8) k_splat_depth(const fsim_particle_gfx* parts, long long n, int which, float thr,
                                                      Cam cam, float r, int W, int H, const float4* ray, int plain_proj,
-                                                     unsigned* depth_bits, const float* scene, float* thick) {
+                                                     unsigned* depth_bits, const float* scene, float* thick, int gather) {
     pdl_enter();
     if (which != 2) {
         const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -280,8 +288,8 @@ __global__ void __launch_bounds__(256, 8) k_splat_depth(const fsim_particle_gfx*
     __shared__ int list[SPLAT_GATHER], count;
     if (threadIdx.x == 0) count = 0;
     __syncthreads();
-    const long long k0 = (long long)blockIdx.x * SPLAT_GATHER;
-    const int m = (int)min((long long)SPLAT_GATHER, n - k0);
+    const long long k0 = (long long)blockIdx.x * gather;
+    const int m = (int)min((long long)gather, n - k0);
     for (int i = threadIdx.x; i < m; i += blockDim.x)
         if (parts[k0 + i].density < thr) list[atomicAdd(&count, 1)] = i;
     __syncthreads();
@@ -790,7 +798,10 @@ int fsim_render_create(int width, int height, fsim_renderer** out) {
     r->W = width;
     r->H = height;
     const size_t np = (size_t)width * height;
-    bool ok = cudaStreamCreateWithFlags(&r->own, cudaStreamNonBlocking) == cudaSuccess &&
+    int dev = 0;
+    bool ok = cudaGetDevice(&dev) == cudaSuccess &&
+              cudaDeviceGetAttribute(&r->sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+              cudaStreamCreateWithFlags(&r->own, cudaStreamNonBlocking) == cudaSuccess &&
               cudaMalloc(&r->raw, np * 4) == cudaSuccess && cudaMalloc(&r->depth, np * 4) == cudaSuccess &&
               cudaMalloc(&r->tmp, np * 4) == cudaSuccess && cudaMalloc(&r->thick, np * 4) == cudaSuccess &&
               cudaMalloc(&r->ttmp, np * 4) == cudaSuccess && cudaMalloc(&r->nd, np * 16) == cudaSuccess &&
@@ -859,7 +870,7 @@ int fsim_render_frame(fsim_renderer* r, const fsim_particle_gfx* particles, int6
     }
     if (n > 0) {
         launch_dep(k_splat_depth, nblk(n), 256, 0, s, dp, n, prm->spray_enabled ? 1 : 0, prm->spray_density_threshold, k,
-                                              rad, W, H, r->nd, plain, reinterpret_cast<unsigned*>(r->raw), scene_depth, thick);
+                                              rad, W, H, r->nd, plain, reinterpret_cast<unsigned*>(r->raw), scene_depth, thick, 0);
         L++;
     }
     // 2. smoothing, x into tmp then y into depth
@@ -871,8 +882,9 @@ int fsim_render_frame(fsim_renderer* r, const fsim_particle_gfx* particles, int6
     L += 2;
     // 3. spray on top of the smoothed surface
     if (prm->spray_enabled && n > 0) {
-        launch_dep(k_splat_depth, (unsigned)((n + SPLAT_GATHER - 1) / SPLAT_GATHER), 256, 0, s, dp, n, 2, prm->spray_density_threshold, k, rad, W, H, r->nd, plain,
-                                              reinterpret_cast<unsigned*>(r->depth), scene_depth, thick);
+        const int gather = splat_gather(n, r->sms);
+        launch_dep(k_splat_depth, nblk(n, gather), 256, 0, s, dp, n, 2, prm->spray_density_threshold, k, rad, W, H, r->nd, plain,
+                   reinterpret_cast<unsigned*>(r->depth), scene_depth, thick, gather);
         L++;
     }
     // 4. thickness blurred x then y

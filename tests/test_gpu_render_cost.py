@@ -31,3 +31,17 @@ def test_background_costs_no_weights(gpu):
     g, b = (frame_ms(r, none, camera(w, h), N.default_render_params(bilateral_filter=f)) for f in (0, 1))
     r.close()
     assert g <= 1.1 * b
+
+
+def test_spray_costs_what_surface_does(gpu):
+    """2048 sprites as spray and as surface (spray: 5 times as long from one block)."""
+    rng = np.random.default_rng(2)
+    r = N.Renderer(1000, 1000)
+    prm = N.default_render_params(particle_radius=0.02, smoothing_size=0.06, transparency_blur_size=0.06)
+    pts = rng.random((2048, 5)).astype(np.float32)
+    ms = []
+    for density in (0.0, 8.0):
+        pts[:, 4] = density
+        ms.append(frame_ms(r, pts, camera(1000, 1000), prm))
+    r.close()
+    assert ms[0] <= 1.5 * ms[1]
