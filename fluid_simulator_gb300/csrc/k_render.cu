@@ -39,7 +39,7 @@ struct fsim_renderer {
     float* ttmp = nullptr;    // thickness blur scratch
     float4* nd = nullptr;     // normal + depth
     float4* color = nullptr;  // composited frame
-    float* tab = nullptr;     // the blurs' weights
+    float* tab = nullptr;     // the blurs' weights, then the eye rays by axis
     fsim_particle_gfx* parts = nullptr;  // staging for host particles / fsim_render_ctx
     long long parts_cap = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -163,25 +163,31 @@ __device__ __forceinline__ bool make_sprite(const Cam& cam, const float* pw, flo
     return s.x0 <= s.x1 && s.y0 <= s.y1;
 }
 
-// Eye ray of every pixel (the eye-space point at its centre on the near plane): the same
-// for all sprites, which read it instead of unprojecting the pixel for every fragment
-// (28 operations and five divisions of ~200).
-__global__ void k_rays(Cam cam, int W, int H, float4* ray) {
-    pdl_enter();
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= W * H) return;
-    const int i = id % W, j = id / W;
+// Eye ray of pixel (i, j): the eye-space point at its centre on the near plane.
+__device__ __forceinline__ void eye_ray(const Cam& cam, int W, int H, int i, int j, float* d) {
     const float nd4[4] = {((float)i + 0.5f) / (float)W * 2.f - 1.f, ((float)j + 0.5f) / (float)H * 2.f - 1.f, -1.f,
                           1.f};
     float o[4];
     mul4(cam.proj_inv, nd4, o);
-    ray[id] = make_float4(o[0] / o[3], o[1] / o[3], o[2] / o[3], 0.f);
+    d[0] = o[0] / o[3];
+    d[1] = o[1] / o[3];
+    d[2] = o[2] / o[3];
+}
+// Under a projection whose inverse keeps x and y apart (any but a sheared or rotated one)
+// a ray's x depends on the column alone, its y on the row, and its z is the same for all:
+// W + H + 1 numbers, tabulated once a frame (k_tables), which stay in L1.  The zero products
+// left out change no sum.  Unprojecting the pixel for every fragment is 28 operations and
+// five divisions of ~200; a table of all rays was 16 bytes written per pixel and read per
+// fragment (2M sprites at 1000 x 1000: 436 us a frame with it, 366 now; 1000 small ones at
+// 3840 x 2160: 382 and 330).
+inline bool rays_by_axis(const Cam& cam) {
+    const float* m = cam.proj_inv.m;
+    return m[1] == 0.f && m[2] == 0.f && m[3] == 0.f && m[4] == 0.f && m[6] == 0.f && m[7] == 0.f;
 }
 
-// Sprite coordinate of the pixel with eye ray dr: false outside the quad.  On return P is
+// Sprite coordinate of the pixel with eye ray d: false outside the quad.  On return P is
 // the eye-space point of the billboard plane under the pixel centre.
-__device__ __forceinline__ bool sprite_hit(const float4 dr, const Sprite& s, float r, float& px, float& py, float* P) {
-    const float d[3] = {dr.x, dr.y, dr.z};
+__device__ __forceinline__ bool sprite_hit(const float* d, const Sprite& s, float& px, float& py, float* P) {
     const float den = dot3(d, s.za);
     if (!(den > 0.f)) return false;
     const float t = dot3(s.c, s.za) / den;
@@ -214,7 +220,8 @@ __device__ __forceinline__ float window_depth(const Cam& cam, const float* p, bo
 // particles deep in the fluid) only adds its thickness; and between the near and the far
 // plane every fragment passes the clip test and, without a scene, the depth test.  The
 // margins cover the rounding of the depths.
-__device__ __forceinline__ void splat(const float* pos, const Cam& cam, float r, int W, int H, const float4* ray,
+template <bool AXES>
+__device__ __forceinline__ void splat(const float* pos, const Cam& cam, float r, int W, int H, const float* ray,
                                       int plain_proj, unsigned* depth_bits, const float* scene, float* thick) {
     Sprite s;
     if (!make_sprite(cam, pos, r, W, H, s)) return;
@@ -227,11 +234,16 @@ __device__ __forceinline__ void splat(const float* pos, const Cam& cam, float r,
         if (zf == zf) front = zf - 4e-6f;
         deep = front > 1e-5f && zb < 1.f - 1e-5f;
     }
-    for (int j = s.y0; j <= s.y1; j++)
+    float d[3];  // eye ray
+    if (AXES) d[2] = ray[W + H];
+    for (int j = s.y0; j <= s.y1; j++) {
+        if (AXES) d[1] = ray[W + j];
         for (int i = s.x0; i <= s.x1; i++) {
             const int pix = j * W + i;
             float px, py, P[3];
-            if (!sprite_hit(ray[pix], s, r, px, py, P)) continue;
+            if (AXES) d[0] = ray[i];
+            else eye_ray(cam, W, H, i, j, d);
+            if (!sprite_hit(d, s, px, py, P)) continue;
             // particle_sprites_depth.fs
             const float nx = px * 2.f, ny = -py * 2.f;  // texCoord * 2 - 1
             const float r2 = nx * nx + ny * ny;
@@ -259,6 +271,7 @@ __device__ __forceinline__ void splat(const float* pos, const Cam& cam, float r,
             z = fminf(fmaxf(z, 0.f), 1.f);  // gl_FragDepth is clamped to the depth range
             atomicMin(&depth_bits[pix], __float_as_uint(z));  // z >= 0: bits order as floats
         }
+    }
 }
 
 // which: 0 all particles, 1 surface (density >= threshold), 2 spray (below).  The spray is
@@ -273,8 +286,9 @@ static int splat_gather(long long n, int sms) {
     const long long per = (n + 8ll * sms - 1) / (8ll * sms), g = (per + 255) / 256 * 256;
     return (int)(g < 256 ? 256 : g > SPLAT_GATHER ? SPLAT_GATHER : g);
 }
+template <bool AXES>
 __global__ void __launch_bounds__(256, 8) k_splat_depth(const fsim_particle_gfx* parts, long long n, int which, float thr,
-                                                     Cam cam, float r, int W, int H, const float4* ray, int plain_proj,
+                                                     Cam cam, float r, int W, int H, const float* ray, int plain_proj,
                                                      unsigned* depth_bits, const float* scene, float* thick, int gather) {
     pdl_enter();
     if (which != 2) {
@@ -282,7 +296,7 @@ __global__ void __launch_bounds__(256, 8) k_splat_depth(const fsim_particle_gfx*
         if (k >= n) return;
         const fsim_particle_gfx pg = parts[k];
         if (which == 1 && pg.density < thr) return;
-        splat(pg.pos, cam, r, W, H, ray, plain_proj, depth_bits, scene, thick);
+        splat<AXES>(pg.pos, cam, r, W, H, ray, plain_proj, depth_bits, scene, thick);
         return;
     }
     __shared__ int list[SPLAT_GATHER], count;
@@ -294,7 +308,7 @@ __global__ void __launch_bounds__(256, 8) k_splat_depth(const fsim_particle_gfx*
         if (parts[k0 + i].density < thr) list[atomicAdd(&count, 1)] = i;
     __syncthreads();
     for (int i = threadIdx.x; i < count; i += blockDim.x)
-        splat(parts[k0 + list[i]].pos, cam, r, W, H, ray, plain_proj, depth_bits, scene, thick);
+        splat<AXES>(parts[k0 + list[i]].pos, cam, r, W, H, ray, plain_proj, depth_bits, scene, thick);
 }
 
 // The blurs' weights depend on the tap and the pixel's radius alone (26 Gaussian radii, and
@@ -313,11 +327,19 @@ __device__ __forceinline__ float blur_weight(int q, float blur_scale) {
     return expf((float)(-p * p) / sd2 * 0.5f);
 }
 
-// the cleared images, and what depends on the frame's parameters alone
-__global__ void k_clear(float* depth, float* thick, long long n, float blur_scale, float* wtab) {
+// what depends on the frame's parameters alone: the blurs' weights and the rays by axis
+__global__ void k_tables(Cam cam, int W, int H, float blur_scale, float* tab) {
+    pdl_enter();
+    const int q = blockIdx.x * blockDim.x + threadIdx.x, e = q - BLUR_TAB;  // e: column, row, or the rays' z
+    if (e > W + H) return;
+    float d[3];
+    if (e >= 0) eye_ray(cam, W, H, e < W ? e : 0, e < W ? 0 : e - W, d);
+    tab[q] = e < 0 ? blur_weight(q, blur_scale) : e < W ? d[0] : e < W + H ? d[1] : d[2];
+}
+
+__global__ void k_clear(float* depth, float* thick, long long n) {
     pdl_enter();
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    for (long long q = k; q < BLUR_TAB; q += (long long)gridDim.x * blockDim.x) wtab[q] = blur_weight((int)q, blur_scale);
     if (k >= n) return;
     depth[k] = 1.f;
     thick[k] = 0.f;
@@ -805,7 +827,7 @@ int fsim_render_create(int width, int height, fsim_renderer** out) {
               cudaMalloc(&r->raw, np * 4) == cudaSuccess && cudaMalloc(&r->depth, np * 4) == cudaSuccess &&
               cudaMalloc(&r->tmp, np * 4) == cudaSuccess && cudaMalloc(&r->thick, np * 4) == cudaSuccess &&
               cudaMalloc(&r->ttmp, np * 4) == cudaSuccess && cudaMalloc(&r->nd, np * 16) == cudaSuccess &&
-              cudaMalloc(&r->color, np * 16) == cudaSuccess && cudaMalloc(&r->tab, BLUR_TAB * 4) == cudaSuccess && cudaEventCreate(&r->ev0) == cudaSuccess &&
+              cudaMalloc(&r->color, np * 16) == cudaSuccess && cudaMalloc(&r->tab, ((size_t)BLUR_TAB + width + height + 1) * 4) == cudaSuccess && cudaEventCreate(&r->ev0) == cudaSuccess &&
               cudaEventCreate(&r->ev1) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
@@ -858,19 +880,17 @@ int fsim_render_frame(fsim_renderer* r, const fsim_particle_gfx* particles, int6
     // 1. surface sprites into the cleared depth buffer, with their thickness
     //    (the thickness of all particles accumulates over passes 1 and 3)
     float* thick = prm->transparency_enabled ? r->thick : nullptr;
-    // the pixels' eye rays stand in the normal buffer until pass 5 writes it
+    const float* ray = r->tab + BLUR_TAB;
+    auto* splat_depth = rays_by_axis(k) ? k_splat_depth<true> : k_splat_depth<false>;
     const float* pm = k.proj.m;
     const int plain = pm[2] == 0.f && pm[6] == 0.f && pm[3] == 0.f && pm[7] == 0.f && pm[15] == 0.f && pm[11] < 0.f &&
                       pm[14] < 0.f;
-    launch_dep(k_clear, nblk(np), 256, 0, s, r->raw, r->thick, np, prm->blur_scale, r->tab);
-    L++;
+    launch_dep(k_tables, nblk(BLUR_TAB + W + H + 1), 256, 0, s, k, W, H, prm->blur_scale, r->tab);
+    launch_dep(k_clear, nblk(np), 256, 0, s, r->raw, r->thick, np);
+    L += 2;
     if (n > 0) {
-        launch_dep(k_rays, nblk(np), 256, 0, s, k, W, H, r->nd);
-        L++;
-    }
-    if (n > 0) {
-        launch_dep(k_splat_depth, nblk(n), 256, 0, s, dp, n, prm->spray_enabled ? 1 : 0, prm->spray_density_threshold, k,
-                                              rad, W, H, r->nd, plain, reinterpret_cast<unsigned*>(r->raw), scene_depth, thick, 0);
+        launch_dep(splat_depth, nblk(n), 256, 0, s, dp, n, prm->spray_enabled ? 1 : 0, prm->spray_density_threshold, k, rad, W, H,
+                   ray, plain, reinterpret_cast<unsigned*>(r->raw), scene_depth, thick, 0);
         L++;
     }
     // 2. smoothing, x into tmp then y into depth
@@ -883,7 +903,7 @@ int fsim_render_frame(fsim_renderer* r, const fsim_particle_gfx* particles, int6
     // 3. spray on top of the smoothed surface
     if (prm->spray_enabled && n > 0) {
         const int gather = splat_gather(n, r->sms);
-        launch_dep(k_splat_depth, nblk(n, gather), 256, 0, s, dp, n, 2, prm->spray_density_threshold, k, rad, W, H, r->nd, plain,
+        launch_dep(splat_depth, nblk(n, gather), 256, 0, s, dp, n, 2, prm->spray_density_threshold, k, rad, W, H, ray, plain,
                    reinterpret_cast<unsigned*>(r->depth), scene_depth, thick, gather);
         L++;
     }
