@@ -359,7 +359,7 @@ __device__ __forceinline__ float screen_extent(const Cam& cam, const float* eye,
 
 // mode 0: Gaussian depth, 1: bilateral depth, 2: Gaussian thickness (src = thickness, dsrc = depth)
 __device__ __forceinline__ void blur_pixel(int mode, int axis, const float* src, const float* dsrc, float* dst, int W,
-                                           int H, const Cam& cam, float size, float falloff, const float* wtab,
+                                           int H, const Cam& cam, float size, float falloff, const float* weights,
                                            int id, float cur) {
     const int x = id % W, y = id / W;
     const float u = ((float)x + 0.5f) / (float)W, v = ((float)y + 0.5f) / (float)H;
@@ -376,7 +376,7 @@ __device__ __forceinline__ void blur_pixel(int mode, int axis, const float* src,
         for (int p = -R; p <= R; p++) {
             const float s = tap(p);
             if (s < 1.f) {
-                const float w = wtab[p < 0 ? -p : p];
+                const float w = weights[p < 0 ? -p : p];
                 const float r2 = (s - cur) * falloff;
                 const float g = expf(-r2 * r2);
                 acc = acc + s * w * g;
@@ -389,7 +389,7 @@ __device__ __forceinline__ void blur_pixel(int mode, int axis, const float* src,
     int ks = (int)(ext * (float)tex) * 2 + 1;
     ks = ks > 51 ? 51 : (ks < 3 ? 3 : ks);
     const int R = ks / 2;
-    const float* wr = wtab + R * (BLUR_MAX_R + 1);
+    const float* wr = weights + R * (BLUR_MAX_R + 1);
     auto add = [&](float s, float w) {
         if (mode == 2 || s < 1.f) {
             wsum = wsum + w;
@@ -406,23 +406,25 @@ __device__ __forceinline__ void blur_pixel(int mode, int axis, const float* src,
     dst[id] = acc / wsum;
 }
 
-// Blocks without a surface pixel (the depth is cleared there, the value stays) leave before
-// anything else; the others take the weights to shared memory.  With the table computed by
-// every block of every pass (~350 exponentials and divisions), a frame of 3840 x 2160 that
-// is nearly all background took 578 us, now 382; 1000 x 1000 with 22 % covered 462, now 436
-// (exponentials and clamped indices for every tap: 682).
+// Background pixels leave before anything else (the depth is cleared there, the value
+// stays), and no block prepares anything: with the table computed by every block of every
+// pass (~350 exponentials and divisions), a frame of 3840 x 2160 that is nearly all
+// background took 578 us; copying it to shared memory is no faster than reading it from
+// L1.  DEP: launched as a dependent kernel.  A block's wait for the kernel before costs what
+// a background block does, so a frame of many waves of blocks takes ordinary launches
+// (3840 x 2160: 330 us with dependent ones, now 273).
+template <bool DEP>
 __global__ void k_blur(int mode, int axis, const float* src, const float* dsrc, float* dst, int W, int H, Cam cam,
                        float size, float falloff, const float* weights) {
-    pdl_enter();
-    __shared__ float wtab[BLUR_GAUSS];
+    if (DEP) pdl_enter();
     const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    const float cur = id < W * H ? dsrc[id] : 1.f;
-    if (id < W * H && cur == 1.f) dst[id] = mode == 2 ? 0.f : 1.f;
-    if (!__syncthreads_or(cur != 1.f)) return;
-    const int first = mode == 1 ? BLUR_GAUSS : 0, count = mode == 1 ? BLUR_BI_R + 1 : BLUR_GAUSS;
-    for (int q = threadIdx.x; q < count; q += blockDim.x) wtab[q] = weights[first + q];
-    __syncthreads();
-    if (cur != 1.f) blur_pixel(mode, axis, src, dsrc, dst, W, H, cam, size, falloff, wtab, id, cur);
+    if (id >= W * H) return;
+    const float cur = dsrc[id];
+    if (cur == 1.f) {
+        dst[id] = mode == 2 ? 0.f : 1.f;
+        return;
+    }
+    blur_pixel(mode, axis, src, dsrc, dst, W, H, cam, size, falloff, weights + (mode == 1 ? BLUR_GAUSS : 0), id, cur);
 }
 
 // ---- 5: normals (normal_depth.fs) ---------------------------------------------
@@ -895,11 +897,14 @@ int fsim_render_frame(fsim_renderer* r, const fsim_particle_gfx* particles, int6
     }
     // 2. smoothing, x into tmp then y into depth
     const int mode = prm->bilateral_filter ? 1 : 0;
-    launch_dep(k_blur, nblk(np), 256, 0, s, mode, 0, r->raw, r->raw, r->tmp, W, H, k, prm->smoothing_size,
-               prm->blur_depth_falloff, r->tab);
-    launch_dep(k_blur, nblk(np), 256, 0, s, mode, 1, r->tmp, r->tmp, r->depth, W, H, k, prm->smoothing_size,
-               prm->blur_depth_falloff, r->tab);
-    L += 2;
+    const bool many = np >= 8ll * 256 * 8 * r->sms;  // eight waves of eight blocks per SM
+    auto blur = [&](int m, int axis, const float* src, const float* dsrc, float* dst, float size, float falloff) {
+        if (many) k_blur<false><<<nblk(np), 256, 0, s>>>(m, axis, src, dsrc, dst, W, H, k, size, falloff, r->tab);
+        else launch_dep(k_blur<true>, nblk(np), 256, 0, s, m, axis, src, dsrc, dst, W, H, k, size, falloff, r->tab);
+        L++;
+    };
+    blur(mode, 0, r->raw, r->raw, r->tmp, prm->smoothing_size, prm->blur_depth_falloff);
+    blur(mode, 1, r->tmp, r->tmp, r->depth, prm->smoothing_size, prm->blur_depth_falloff);
     // 3. spray on top of the smoothed surface
     if (prm->spray_enabled && n > 0) {
         const int gather = splat_gather(n, r->sms);
@@ -909,11 +914,8 @@ int fsim_render_frame(fsim_renderer* r, const fsim_particle_gfx* particles, int6
     }
     // 4. thickness blurred x then y
     if (prm->transparency_enabled) {
-        launch_dep(k_blur, nblk(np), 256, 0, s, 2, 0, r->thick, r->depth, r->ttmp, W, H, k, prm->transparency_blur_size,
-                   0.f, r->tab);
-        launch_dep(k_blur, nblk(np), 256, 0, s, 2, 1, r->ttmp, r->depth, r->thick, W, H, k, prm->transparency_blur_size,
-                   0.f, r->tab);
-        L += 2;
+        blur(2, 0, r->thick, r->depth, r->ttmp, prm->transparency_blur_size, 0.f);
+        blur(2, 1, r->ttmp, r->depth, r->thick, prm->transparency_blur_size, 0.f);
     }
     // 5. normals
     launch_dep(k_normals, nblk(np), 256, 0, s, r->depth, r->nd, W, H, k);

@@ -47,14 +47,16 @@ def test_spray_costs_what_surface_does(gpu):
     assert ms[0] <= 1.5 * ms[1]
 
 
-def test_few_sprites_cost_little(gpu):
-    """A thousand sprites of a pixel or two add little to an empty frame (with an eye ray
-    tabulated for every pixel, a fifth of it)."""
-    w, h = 3840, 2160
-    r = N.Renderer(w, h)
+def test_few_sprites_cost_the_same_in_a_large_frame(gpu):
+    """What a thousand sprites of a pixel or two add to an empty frame does not grow with the
+    frame (16 times the pixels; with an eye ray tabulated for every pixel it did)."""
     prm = N.default_render_params(particle_radius=0.001, smoothing_size=0.06, transparency_blur_size=0.06)
     pts = np.random.default_rng(4).random((1000, 5)).astype(np.float32)
     pts[:, 4] = 8.0
-    some, none = (frame_ms(r, q, camera(w, h), prm) for q in (pts, pts[:0]))
-    r.close()
-    assert some <= 1.1 * none
+    add = []
+    for w, h in ((960, 540), (3840, 2160)):
+        r = N.Renderer(w, h)
+        some, none = (frame_ms(r, q, camera(w, h), prm) for q in (pts, pts[:0]))
+        add.append(some - none)
+        r.close()
+    assert add[1] <= 3 * add[0]

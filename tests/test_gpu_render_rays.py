@@ -41,3 +41,24 @@ def test_rays(gpu, port_lib, view, w, h, n):
     th = r.read(N.IMG_THICKNESS)
     assert (np.abs(th - ref["thickness"]) > 1e-5 * max(ref["thickness"].max(), 1e-30)).mean() <= 0.002
     r.close()
+
+
+@pytest.mark.parametrize("bilateral", [0, 1])
+def test_large_frame(gpu, port_lib, bilateral):
+    """More pixels than two waves of blocks (a blur thread takes several), no multiple of a
+    block's: mostly background, a few sprites."""
+    w, h = 2051, 1303
+    rng = np.random.default_rng(1)
+    pts = (rng.random((60, 5)) * [1, 1, 1, 0, 3]).astype(np.float32)
+    cam = scene_camera(w, h)
+    prm = N.default_render_params(particle_radius=1 / 80, smoothing_size=0.02, transparency_blur_size=0.02,
+                                  bilateral_filter=bilateral, noise_scale=9.0)
+    r = N.Renderer(w, h)
+    r.frame(pts, cam, prm)
+    ref = O.render_frame(pts, cam, prm, w, h)
+    assert np.array_equal(r.read(N.IMG_RAW_DEPTH), ref["raw_depth"])
+    d = r.read(N.IMG_DEPTH)
+    assert np.array_equal(d < 1, ref["depth"] < 1) and np.abs(d - ref["depth"]).max() <= 2e-6
+    th = r.read(N.IMG_THICKNESS)
+    assert (np.abs(th - ref["thickness"]) > 1e-5 * ref["thickness"].max()).mean() <= 0.001
+    r.close()
