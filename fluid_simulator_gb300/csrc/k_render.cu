@@ -286,8 +286,8 @@ static int splat_gather(long long n, int sms) {
     const long long per = (n + 8ll * sms - 1) / (8ll * sms), g = (per + 255) / 256 * 256;
     return (int)(g < 256 ? 256 : g > SPLAT_GATHER ? SPLAT_GATHER : g);
 }
-template <bool AXES>
-__global__ void __launch_bounds__(256, 8) k_splat_depth(const fsim_particle_gfx* parts, long long n, int which, float thr,
+template <bool AXES, int MINB>
+__global__ void __launch_bounds__(256, MINB) k_splat_depth(const fsim_particle_gfx* parts, long long n, int which, float thr,
                                                      Cam cam, float r, int W, int H, const float* ray, int plain_proj,
                                                      unsigned* depth_bits, const float* scene, float* thick, int gather) {
     pdl_enter();
@@ -883,7 +883,12 @@ int fsim_render_frame(fsim_renderer* r, const fsim_particle_gfx* particles, int6
     //    (the thickness of all particles accumulates over passes 1 and 3)
     float* thick = prm->transparency_enabled ? r->thick : nullptr;
     const float* ray = r->tab + BLUR_TAB;
-    auto* splat_depth = rays_by_axis(k) ? k_splat_depth<true> : k_splat_depth<false>;
+    // Many sprites hide their latency with resident blocks (32 registers and 200 bytes spilled:
+    // 8M at 1000 x 1000 606 us a frame, 658 with 48 registers); a frame of at most four blocks
+    // per SM has none to add and takes the registers (500 sprites of ~10,000 pixels 8850 -> 7980 us)
+    const bool few = nblk(n) <= 4u * (unsigned)r->sms;
+    auto* splat_depth = rays_by_axis(k) ? (few ? k_splat_depth<true, 4> : k_splat_depth<true, 8>)
+                                        : (few ? k_splat_depth<false, 4> : k_splat_depth<false, 8>);
     const float* pm = k.proj.m;
     const int plain = pm[2] == 0.f && pm[6] == 0.f && pm[3] == 0.f && pm[7] == 0.f && pm[15] == 0.f && pm[11] < 0.f &&
                       pm[14] < 0.f;
