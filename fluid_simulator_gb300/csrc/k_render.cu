@@ -219,7 +219,11 @@ __device__ __forceinline__ float window_depth(const Cam& cam, const float* p, bo
 // nearer than its front, and a fragment behind the depth already there (most, many
 // particles deep in the fluid) only adds its thickness; and between the near and the far
 // plane every fragment passes the clip test and, without a scene, the depth test.  The
-// margins cover the rounding of the depths.
+// margins cover the rounding of the depths, also where near and far are close and a depth
+// (a |z| - b) / |z| is the difference of large products: the numerator is rounded
+// monotonically in z, so two depths are out of order by 2^-22 at most, whatever a is; and a
+// point of the billboard plane is nearer to the sprite's centre along z than r by more than
+// its rounding unless it is seen at a right angle.
 template <bool AXES>
 __device__ __forceinline__ void splat(const float* pos, const Cam& cam, float r, int W, int H, const float* ray,
                                       int plain_proj, unsigned* depth_bits, const float* scene, float* thick) {
