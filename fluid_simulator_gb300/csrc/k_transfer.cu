@@ -611,7 +611,6 @@ cudaError_t launch_p2g_shape(P2GArgs a, bool apic, cudaStream_t stream) {
         return launch_dep(k_p2g<true, S>, nb, S::NTHREADS, S::SMEM, stream, a);
     else
         return launch_dep(k_p2g<false, S>, nb, S::NTHREADS, S::SMEM, stream, a);
-    return cudaGetLastError();
 }
 
 template <class S>
@@ -619,18 +618,24 @@ long long p2g_tiles(const GridGeom& g) {
     return (long long)ceil_div(g.nx, S::PX) * ceil_div(g.ny, S::PY) * ceil_div(g.nz, S::PZ);
 }
 
-// A warp quad walks its tile's blocks of 32 halo cells one after the other (203 blocks
-// over seven quads for 16x12x16), so few large tiles take as long as one tile does
-// (8x16x16 on 32^3: 16 CTAs, 167 us); smaller ones read more halo cells (1.6 times the
+// A warp quad walks its tile's blocks of 32 halo cells one after the other (142 blocks of
+// cell centres over seven quads for 16x12x16), so few large tiles take as long as one tile
+// does (8x16x16 on 32^3: 16 CTAs, 167 us); smaller ones read more halo cells (1.6 times the
 // cells at 8x16x16, 2.0 at 8x8x8, 3.4 at 4x4x4).  A shape is taken from the number of its
-// tiles on, part of which hold no fluid, at which it measured faster than the next
-// smaller one.  k_p2g in us, 16x16x16 / 16x12x16 / 8x16x16 / 8x8x16 / 4x8x8: 90x61x75 half
-// filled (180 tiles of 16x12x16, 480 of 8x8x16) 278 / 186 / 157 / 144 / 168; 107x90x66 (280 of
-// 16x12x16) 197 / 152 / 185 / 168 / 209; 128^3 dam (512 of 16x16x16) 375 / 352 / 397 / 365 / 565;
-// 256^3 above.  Sort + P2G, 8x8x16 / 4x8x8 / 4x4x8 / 4x4x4 (two CTAs of three quads), dam and
-// half filled: 32^3 (256 of 4x4x8) 71 80 / 42 42 / 37 38 / 35 40; 48x40x32 (240 of 4x8x8) 82 83 /
-// 43 47 / 38 53 / 37 55; 40x56x44 (420) 83 89 / 45 68 / 50 73 / 51 73; 64x64x40 (640, 160 of 8x8x16)
-// 89 94 / 57 91 / 68 103 / 68 108.
+// tiles on, part of which hold no fluid, at which it measured no slower than the next
+// smaller one.  Sort + P2G of APIC particles in us on the layouts below, half filled / dam:
+//              16x16x16    16x12x16   8x8x16     4x8x8      4x4x8     4x4x4
+//   24^3       170 / 170   165 / 129  91 / 90    58 / 59    50 / 49   49 / 45
+//   32^3       218 / 211   169 / 164  95 / 92    59 / 61    54 / 50   57 / 51
+//   40^3       249 / 230   186 / 196  106 / 104  64 / 60    70 / 63   72 / 65
+//   64x64x40   255 / 250   212 / 203  110 / 109  109 / 88   121 / 99  126 / 101
+//   64^3       268 / 258   220 / 210  122 / 113  150 / 114  177 / 141
+//   80x64x64   275 / 272   226 / 222  157 / 116  178 / 134  211 / 169
+//   84^3       307 / 292   255 / 237  253 / 194  300 / 237
+//   96^3       324 / 306   286 / 252  307 / 258  413 / 328
+//   128^3      626 / 565   647 / 475  673 / 517  942 / 745
+//   192x160^2  1308 / 1009 1350 / 1023 1529 / 1188
+// (tiles: 64x64x40 192 of 8x8x16, 64^3 256; 84^3 252 of 16x12x16, 96^3 288; 40^3 250 of 4x8x8).
 using T0 = P2GShape<16, 12, 16, 896, 1>;
 using T1 = P2GShape<8, 8, 16, 896, 1>;
 using T2 = P2GShape<4, 8, 8, 896, 1>;
@@ -639,7 +644,8 @@ using T4 = P2GShape<4, 4, 4, 384, 2>;
 cudaError_t p2g_fast(const P2GArgs& a, bool apic, cudaStream_t stream) {
     if (p2g_tiles<P2GFast>(a.g) >= 2048) return launch_p2g_shape<P2GFast>(a, apic, stream);
     if (p2g_tiles<T0>(a.g) >= 270) return launch_p2g_shape<T0>(a, apic, stream);
-    if (p2g_tiles<T1>(a.g) >= 400) return launch_p2g_shape<T1>(a, apic, stream);
+    // (cells, not tiles: on 60^3 the 256 tiles are partly empty, 117 / 111 us, 4x8x8 128 / 106)
+    if ((long long)a.g.nx * a.g.ny * a.g.nz >= 240ll * T1::PCELLS) return launch_p2g_shape<T1>(a, apic, stream);
     if (p2g_tiles<T2>(a.g) >= 240) return launch_p2g_shape<T2>(a, apic, stream);
     if (p2g_tiles<T3>(a.g) >= 300) return launch_p2g_shape<T3>(a, apic, stream);
     return launch_p2g_shape<T4>(a, apic, stream);
