@@ -243,9 +243,11 @@ __global__ void k_apply_pressure(GridGeom g, const uint8_t* flags, const double*
 // ---- layout conversions ------------------------------------------------------
 // Rows without padding (pz == nz) between 16-byte aligned arrays are one contiguous
 // copy (a 256^3 float field: 54 -> 22 us); the division of the others is 32-bit, a
-// grid stays below 2^31 cells.  Those kernels are ordinary launches: a block that copies
-// 256 values is shorter than the wait of a dependent launch (255 x 250 x 253 out, floats
-// and bytes: 81 us with it, 66 and 49 without).
+// grid stays below 2^31 cells.  A block that copies 256 values is shorter than the wait of
+// a dependent launch, so beyond PAD_DEP_BLOCKS (the wait costs 0.3 us a wave of blocks, the
+// launch saves 1) the copy out is an ordinary launch (255 x 250 x 253, floats and bytes: 81
+// us as a dependent one, 66 and 49 so).
+constexpr unsigned PAD_DEP_BLOCKS = 4096;
 __global__ void __launch_bounds__(256) k_copy16(const uint4* src, uint4* dst, long long n16, const uint8_t* tsrc,
                                                 uint8_t* tdst, int tail) {
     pdl_enter();
@@ -264,6 +266,7 @@ bool copy_dense(const GridGeom& g, const void* src, void* dst, int elem, cudaStr
 }
 template <typename T>
 __global__ void k_pad_to_dense(GridGeom g, const T* src, T* dst) {
+    if (gridDim.x <= PAD_DEP_BLOCKS) pdl_enter();
     const unsigned j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= (unsigned)g.nx * g.ny * g.nz) return;
     const unsigned row = j / (unsigned)g.nz;
@@ -388,9 +391,13 @@ void launch_pad_to_dense(const GridGeom& g, const void* src, void* dst, int elem
     const long long n = (long long)g.nx * g.ny * g.nz;
     if (copy_dense(g, src, dst, elem, s)) return;
     const int nb = ceil_div(n, 256);
-    if (elem == 1) k_pad_to_dense<uint8_t><<<nb, 256, 0, s>>>(g, (const uint8_t*)src, (uint8_t*)dst);
-    else if (elem == 4) k_pad_to_dense<float><<<nb, 256, 0, s>>>(g, (const float*)src, (float*)dst);
-    else k_pad_to_dense<double><<<nb, 256, 0, s>>>(g, (const double*)src, (double*)dst);
+    auto out = [&](auto* kern, auto* from, auto* to) {
+        if ((unsigned)nb <= PAD_DEP_BLOCKS) launch_dep(kern, nb, 256, 0, s, g, from, to);
+        else kern<<<nb, 256, 0, s>>>(g, from, to);
+    };
+    if (elem == 1) out(k_pad_to_dense<uint8_t>, (const uint8_t*)src, (uint8_t*)dst);
+    else if (elem == 4) out(k_pad_to_dense<float>, (const float*)src, (float*)dst);
+    else out(k_pad_to_dense<double>, (const double*)src, (double*)dst);
 }
 
 void launch_dense_to_pad(const GridGeom& g, const void* src, void* dst, int elem, cudaStream_t s) {
