@@ -303,8 +303,8 @@ __global__ void k_head(const bf16* d0, long long vox, const float* wgt, const fl
 // Pass 1's sums are FP64 from the first square on.  FP64 arithmetic runs at 1/64 of the
 // FP32 rate, so a thread adds its voxels with one FMA a square, and the block sums through
 // shared memory (block_reduce).  Summing doubles across every warp with four atomics each
-// took 229 us at 8 x 64^3 (the second pass, which moves as much, 29); now 62 with half of
-// the voxels in the mask (FP32 pairs of 48 bits up to the block sum: 43).
+// took 229 us at 8 x 64^3 (the second pass, which moves as much, 29); now 47, and 62 with
+// half of the voxels in the mask (FP32 pairs of 48 bits up to the block sum: 43).
 constexpr int LOSS_VPT = 512 / NT_THREADS;  // voxels per thread
 __device__ __forceinline__ bool vox_solid(const bf16* x0, long long v) { return __bfloat162float(x0[v * 16 + 2]) > 0.5f; }
 

@@ -22,7 +22,7 @@
 // FP32; dot products, alpha/beta and the convergence test in FP64; the
 // solution accumulates in FP32 and is folded into an FP64 solution with the
 // true residual b' - A' p recomputed in FP64 whenever the recursive residual
-// has dropped by 10x since the last fold ("reliable updates"), and always
+// has dropped by 1000x since the last fold ("reliable updates", refine_digits), and always
 // before convergence is declared.  FSIM_PREC_FP32 never folds until the end;
 // FSIM_PREC_FP64 runs every vector in FP64.
 //

@@ -281,7 +281,7 @@ __device__ __forceinline__ void splat(const float* pos, const Cam& cam, float r,
 // which: 0 all particles, 1 surface (density >= threshold), 2 spray (below).  The spray is
 // a few particles of many: a block gathers the ones among `gather` before it splats them
 // (with one thread per particle 3.4 of 32 lanes worked).  1000 x 1000 pixels, 8M
-// particles: surface 629 us and spray 130 before, now 405 and 55.
+// particles: surface 629 us and spray 130 before, now 405 and 53.
 constexpr int SPLAT_GATHER = 2048;
 // A block's spray is splatted by its 256 threads in turn, so where a frame has little else
 // a wide gather leaves the chip idle (2048 sprites, all spray, 1000 x 1000: one block and
